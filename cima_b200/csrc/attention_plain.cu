@@ -1,6 +1,6 @@
-// Plain causal grouped-query attention: one warp per (query row, head), keys visited one by one
-// with a running (max, sum, accumulator) in float32.  It is the attention of the true 32-bit path
-// and the fallback for head sizes the fast kernels do not take.  Two sources of keys and values:
+// Plain causal grouped-query attention, all sums in float32: the attention of the true 32-bit path (k_attention_f32, head sizes
+// up to 256), and the fallback for head sizes that no other kernel takes (k_attention_plain: one warp per (query row, head),
+// keys visited one by one with a running (max, sum, accumulator)).  Two sources of keys and values:
 //   step  - the step's own qkv buffer (a prompt that starts at position 0: key j of a sequence is
 //           its row j), used for prefill;
 //   cache - the layer's pages through the slot's block table, used for decoding.
@@ -92,6 +92,249 @@ k_attention_plain(const TA* __restrict__ qkv, int ld, const TA* __restrict__ cac
   }
 }
 
+// ---------------------------------------------------------------------------------------------------- float32, head sizes up to 256
+// The attention of the 32-bit path.  Keys are taken in pieces of 32 neighbouring positions (32 b .. 32 b + 31): a piece has a
+// maximum, a sum and a weighted sum of values of its own, added up in ascending position, and the pieces are merged in
+// ascending b.  A result therefore depends on its own sequence and position only, whoever computes it: the same bits whole,
+// token by token or in a batch, from the step's rows or from pages.  (A warp that walked one key after another took 294 us at
+// 200 positions, a chain of some 1.4 us a key; bound by latency.)
+//
+// A block owns up to QV query vectors of one sequence and key head: neighbouring rows times the heads that share the key head,
+// so that a piece's keys and values serve them all.  Its warps take the pieces in turn, each through its own shared memory
+// (cp.async), a lane a key for the scores and a lane NI dims for the weighted sums; what a round of pieces gives is merged by
+// the block in their order.  A decode step has a row a block and 8 warps, a prompt as many rows as QV allows and 4.
+// Measured at the 0.5B shape: 14.0 us for 2 rows at some 200 positions (294), 109 us for prompts of 201 and 123 rows (153).
+constexpr int AF_KEYS = 32;
+
+struct AfArgs {
+  const float *qkv, *cache, *head_sink, *slopes;
+  const int *row_pos, *row_seq, *seq_slot, *seq_first_row;
+  float* out;
+  CimaPaged pg;
+  int ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, rows, heads;      // a block's rows, and heads of a key head
+  float scale, sink;
+};
+
+template <int HDP> constexpr int AF_QV = HDP <= 64 ? 32 : HDP <= 128 ? 24 : 16;
+static size_t af_smem(int hdp, int warps, int qv) {
+  return sizeof(float) * ((size_t)warps * 2 * AF_KEYS * (hdp + 4) + (size_t)2 * qv * hdp + (size_t)warps * qv * (hdp + 4) + (size_t)warps * 8 * AF_KEYS);
+}
+
+template <int HDP, bool FROM_CACHE, bool VEC>
+__global__ void __launch_bounds__(HDP <= 64 ? 256 : 128)
+k_attention_f32(const __grid_constant__ AfArgs a) {
+  constexpr int NI = HDP / 32, PITCH = HDP + 4, QVM = AF_QV<HDP>;
+  extern __shared__ __align__(16) float af[];
+  __shared__ float s_m[8][QVM], s_l[8][QVM], s_c[8][QVM], s_k[8][QVM], run_m[QVM], run_l[QVM];
+  __shared__ int s_any[8][QVM];
+  cima_pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  const int group = a.nh / a.nkv, per_kv = (group + a.heads - 1) / a.heads;      // blocks of heads of one key head
+  const int kvh = blockIdx.y / per_kv, h0 = kvh * group + (blockIdx.y % per_kv) * a.heads;
+  const int heads = min(a.heads, (kvh + 1) * group - h0), vh = kvh / a.v_group;
+  const int qvs_max = a.rows * a.heads, hd = a.hd, hdr = (hd + 3) & ~3;
+  float* Kt = af + (size_t)warp * 2 * AF_KEYS * PITCH;
+  float* Vt = Kt + AF_KEYS * PITCH;
+  float* Q = af + (size_t)warps * 2 * AF_KEYS * PITCH;          // [qv][HDP]
+  float* O = Q + (size_t)qvs_max * HDP;                          // [qv][HDP], the running weighted sums
+  float* part = O + (size_t)qvs_max * HDP;                       // [warp][qv][PITCH], a round's pieces
+  float* P = part + (size_t)warps * qvs_max * PITCH + (size_t)warp * 8 * AF_KEYS;      // [8][32], the warp's weights
+  const int t0 = blockIdx.x * a.rows, t1 = min(a.T, t0 + a.rows);
+
+  for (int r0 = t0; r0 < t1;) {                          // rows of one sequence at a time
+    const int seq = a.row_seq[r0];
+    int r1 = r0 + 1;
+    while (r1 < t1 && a.row_seq[r1] == seq) r1++;
+    const int qvs = (r1 - r0) * heads;                   // vector i: row r0 + i / heads, head h0 + i % heads
+    const int slot = FROM_CACHE ? a.seq_slot[seq] : 0, first = FROM_CACHE ? 0 : a.seq_first_row[seq];
+    int pmin = a.row_pos[r0], pmax = pmin;
+    for (int r = r0 + 1; r < r1; r++) { const int p = a.row_pos[r]; pmin = min(pmin, p); pmax = max(pmax, p); }
+    const int lo = a.window > 0 && pmin + 1 > a.window ? pmin + 1 - a.window : 0, kept = min(a.keep_first, lo);
+    const int b0 = lo / AF_KEYS, kept_pieces = min((kept + AF_KEYS - 1) / AF_KEYS, b0), pieces = kept_pieces + pmax / AF_KEYS - b0 + 1;
+    __syncthreads();                                     // the sequence before is done with Q, O and the running sums
+    for (int i = tid; i < qvs * HDP; i += blockDim.x) {
+      const int v = i / HDP, d = i - v * HDP;
+      Q[i] = d < hd ? a.qkv[(size_t)(r0 + v / heads) * a.ld + (size_t)(h0 + v % heads) * hd + d] : 0.f;
+      O[i] = 0.f;
+    }
+    for (int i = tid; i < qvs; i += blockDim.x) { run_m[i] = -1e30f; run_l[i] = 0.f; }
+    __syncthreads();
+    for (int base = 0; base < pieces; base += warps) {
+      const int mine = base + warp;
+      if (mine < pieces) {
+        const int b = mine < kept_pieces ? mine : b0 + mine - kept_pieces;
+        const int j = b * AF_KEYS + lane;
+        // what no row sees is not read (pages may hold anything there)
+        const bool seen = j <= pmax && (j >= lo || j < kept);
+        const float *kp = nullptr, *vp = nullptr;
+        if (seen) {
+          if (FROM_CACHE) {
+            const size_t at = a.pg.offset(slot, j, 0, kvh);
+            kp = a.cache + at;
+            vp = vh == kvh ? kp + a.pg.value_offset() : a.cache + a.pg.offset(slot, j, 1, vh);
+          } else {
+            kp = a.qkv + (size_t)(first + j) * a.ld + (size_t)(a.nh + kvh) * hd;
+            vp = a.qkv + (size_t)(first + j) * a.ld + (size_t)(a.nh + a.nkv + vh) * hd;
+          }
+        }
+        const unsigned have = __ballot_sync(0xffffffffu, seen);
+        for (int key = 0; key < AF_KEYS; key++) {
+          const float* ks = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(kp), key));
+          const float* vs = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(vp), key));
+          const bool ok = have >> key & 1;
+          if constexpr (VEC) {
+            for (int d = 4 * lane; d < HDP; d += 128) {
+              if (ok && d < hd) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(Kt + key * PITCH + d)), "l"(ks + d));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(Vt + key * PITCH + d)), "l"(vs + d));
+              } else {
+                *reinterpret_cast<float4*>(Kt + key * PITCH + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(Vt + key * PITCH + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < NI; i++) {
+              const int d = lane + 32 * i;
+              Kt[key * PITCH + d] = ok && d < hd ? ks[d] : 0.f;
+              Vt[key * PITCH + d] = ok && d < hd ? vs[d] : 0.f;
+            }
+          }
+        }
+        if constexpr (VEC) asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+        __syncwarp();
+        float* mypart = part + (size_t)warp * qvs_max * PITCH;
+        for (int v0 = 0; v0 < qvs; v0 += 8) {            // eight query vectors at a time
+          float s[8];
+          const float* q[8];
+#pragma unroll
+          for (int x = 0; x < 8; x++) { s[x] = 0.f; q[x] = Q + (size_t)min(v0 + x, qvs - 1) * HDP; }
+#pragma unroll 2
+          for (int d = 0; d < hdr; d += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(Kt + lane * PITCH + d);
+#pragma unroll
+            for (int x = 0; x < 8; x++) {
+              const float4 q4 = *reinterpret_cast<const float4*>(q[x] + d);
+              s[x] = fmaf(q4.x, k4.x, s[x]); s[x] = fmaf(q4.y, k4.y, s[x]);
+              s[x] = fmaf(q4.z, k4.z, s[x]); s[x] = fmaf(q4.w, k4.w, s[x]);
+            }
+          }
+          unsigned vis[8], all = 0xffffffffu;
+#pragma unroll
+          for (int x = 0; x < 8; x++) {
+            const int v = min(v0 + x, qvs - 1), h = h0 + v % heads, pos = a.row_pos[r0 + v / heads];
+            const int from = a.window > 0 && pos + 1 > a.window ? pos + 1 - a.window : 0;
+            const bool see = j <= pos && (j >= from || j < a.keep_first);
+            s[x] = s[x] * a.scale - (a.slopes ? a.slopes[h] : 0.f) * (float)(pos - j);
+            vis[x] = __ballot_sync(0xffffffffu, see);
+            all &= vis[x];
+            float m = see ? fmaxf(s[x], -1e30f) : -1e30f;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            const float p = see ? expf(s[x] - m) : 0.f;
+            float l = p;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+            P[x * AF_KEYS + lane] = p;
+            if (lane == 0 && v0 + x < qvs) { s_m[warp][v] = m; s_l[warp][v] = l; s_any[warp][v] = vis[x] != 0u; }
+          }
+          __syncwarp();
+          float o[8][NI];
+#pragma unroll
+          for (int x = 0; x < 8; x++)
+#pragma unroll
+            for (int i = 0; i < NI; i++) o[x][i] = 0.f;
+#pragma unroll 2
+          for (int k = 0; k < AF_KEYS; k += 4) {
+            float vv[4][NI];
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+              for (int i = 0; i < NI; i++) vv[e][i] = Vt[(k + e) * PITCH + lane + 32 * i];
+#pragma unroll
+            for (int x = 0; x < 8; x++) {
+              const float4 p4 = *reinterpret_cast<const float4*>(P + x * AF_KEYS + k);
+              const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+              if (all == 0xffffffffu) {
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+#pragma unroll
+                  for (int i = 0; i < NI; i++) o[x][i] = fmaf(p[e], vv[e][i], o[x][i]);
+              } else {                                   // a value that the row does not see stays out, whatever it is
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                  if (vis[x] >> (k + e) & 1) {
+#pragma unroll
+                    for (int i = 0; i < NI; i++) o[x][i] = fmaf(p[e], vv[e][i], o[x][i]);
+                  }
+              }
+            }
+          }
+#pragma unroll
+          for (int x = 0; x < 8; x++)
+            if (v0 + x < qvs) {
+#pragma unroll
+              for (int i = 0; i < NI; i++) mypart[(size_t)(v0 + x) * PITCH + lane + 32 * i] = o[x][i];
+            }
+          __syncwarp();                                  // the weights have been read
+        }
+      }
+      __syncthreads();
+      const int there = min(warps, pieces - base);
+      for (int v = tid; v < qvs; v += blockDim.x) {      // the factors of the round's pieces, in their order
+        float m = run_m[v], l = run_l[v];
+        for (int w = 0; w < there; w++) {
+          float c = 1.f, k = 0.f;
+          if (s_any[w][v]) {
+            const float m2 = fmaxf(m, s_m[w][v]);
+            c = expf(m - m2); k = expf(s_m[w][v] - m2);
+            l = l * c + s_l[w][v] * k;
+            m = m2;
+          }
+          s_c[w][v] = c; s_k[w][v] = k;
+        }
+        run_m[v] = m; run_l[v] = l;
+      }
+      __syncthreads();
+      for (int i = tid; i < qvs * HDP; i += blockDim.x) {
+        const int v = i / HDP, d = i - v * HDP;
+        float acc = O[i];
+        for (int w = 0; w < there; w++)
+          if (s_any[w][v]) acc = fmaf(part[((size_t)w * qvs_max + v) * PITCH + d], s_k[w][v], acc * s_c[w][v]);
+        O[i] = acc;
+      }
+      __syncthreads();
+    }
+    for (int i = tid; i < qvs * HDP; i += blockDim.x) {
+      const int v = i / HDP, d = i - v * HDP;
+      if (d >= hd) continue;
+      const int row = r0 + v / heads, h = h0 + v % heads;
+      const float m = run_m[v], l = run_l[v] + (a.head_sink ? expf(a.head_sink[h] - m) : a.sink * expf(-m));
+      const float gate = a.gate_col > 0 ? cima_sigmoid(a.qkv[(size_t)row * a.ld + a.gate_col + (size_t)h * hd + d]) : 1.0f;
+      a.out[(size_t)row * a.ldo + (size_t)h * hd + d] = O[i] * (l > 0.f ? 1.0f / l : 0.f) * gate;
+    }
+    r0 = r1;
+  }
+}
+
+template <int HDP, bool FROM_CACHE>
+static int launch_attention_f32(AfArgs a, bool vec, cudaStream_t stream) {
+  const int group = a.nh / a.nkv;
+  a.heads = group < AF_QV<HDP> ? group : AF_QV<HDP>;
+  const int per_kv = (group + a.heads - 1) / a.heads;
+  // few rows: a row a block, so that rows do not wait for one another; many: as many rows as share a block's keys
+  const bool few = (long long)a.T * a.nkv * per_kv <= 592;
+  a.rows = few ? 1 : AF_QV<HDP> / a.heads;
+  int warps = HDP <= 64 ? (few ? 8 : 4) : HDP <= 128 ? 4 : 2;
+  if (af_smem(HDP, warps, a.rows * a.heads) > 220 * 1024) warps /= 2;
+  const size_t smem = af_smem(HDP, warps, a.rows * a.heads);
+  auto kern = vec ? k_attention_f32<HDP, FROM_CACHE, true> : k_attention_f32<HDP, FROM_CACHE, false>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return cima_fail((int)e, "attention_plain: %zu bytes of shared memory are not available: %s", smem, cudaGetErrorString(e));
+  const dim3 grid((unsigned)((a.T + a.rows - 1) / a.rows), (unsigned)(a.nkv * per_kv));
+  return cima_launch(kern, grid, dim3(32 * warps), smem, stream, 1, a);
+}
+
 // from_cache 0: keys/values of the step (seq_first_row needed); 1: of the cache (table, seq_slot needed).
 extern "C" int cima_attention_plain(const void* qkv, int dtype, int ld, const void* cache, const int* table,
                                     int table_width, int ring, int page_size, const int* row_pos,
@@ -108,14 +351,25 @@ extern "C" int cima_attention_plain(const void* qkv, int dtype, int ld, const vo
   if (from_cache && (!cache || !table)) return cima_fail(CIMA_E_ARG, "attention_plain: decoding needs the cache and its block table");
   if (gate_col < 0 || (gate_col > 0 && gate_col + nh * hd > ld)) return cima_fail(CIMA_E_ARG, "attention_plain: %d gate values from column %d on exceed the rows of %d", nh * hd, gate_col, ld);
   CimaPaged pg{table, table_width, ring, page_size, nkv, hd, planes};
+  if (dtype == CIMA_F32 && hd <= 256) {
+    AfArgs a{(const float*)qkv, (const float*)cache, head_sink, slopes, row_pos, row_seq, seq_slot, seq_first_row, (float*)out, pg,
+             ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, 1, 1, scale, sink};
+    const bool vec = hd % 4 == 0 && (from_cache || ld % 4 == 0) && ((from_cache ? (uintptr_t)cache : (uintptr_t)qkv) & 15) == 0;
+    int rc;
+    if (hd <= 64) rc = from_cache ? launch_attention_f32<64, true>(a, vec, stream) : launch_attention_f32<64, false>(a, vec, stream);
+    else if (hd <= 128) rc = from_cache ? launch_attention_f32<128, true>(a, vec, stream) : launch_attention_f32<128, false>(a, vec, stream);
+    else rc = from_cache ? launch_attention_f32<256, true>(a, vec, stream) : launch_attention_f32<256, false>(a, vec, stream);
+    return rc ? rc : cima_launch_result();
+  }
   dim3 grid((T + 3) / 4, nh);
-#define LAUNCH(TA, FC) { int rc_ = hd <= 256 ? LAUNCH_NI(TA, FC, 8) : LAUNCH_NI(TA, FC, 32); if (rc_) return rc_; }
 #define LAUNCH_NI(TA, FC, NI) cima_launch(k_attention_plain<TA, FC, NI>, dim3(grid), dim3(128), (size_t)(0), stream, 1, (const TA*)qkv, ld, (const TA*)cache, pg, \
     row_pos, row_seq, seq_slot, seq_first_row, (TA*)out, ldo, T, nh, nkv, hd, scale, window, sink, keep_first, v_group, head_sink, gate_col, slopes)
-  if (dtype == CIMA_F32) { if (from_cache) LAUNCH(float, true) else LAUNCH(float, false) }
-  else if (dtype == CIMA_BF16) { if (from_cache) LAUNCH(__nv_bfloat16, true) else LAUNCH(__nv_bfloat16, false) }
-  else return cima_fail(CIMA_E_DTYPE, "attention_plain: dtype code %d is neither float32 nor bfloat16", dtype);
-#undef LAUNCH
+  int rc;
+  if (dtype == CIMA_F32) rc = from_cache ? LAUNCH_NI(float, true, 32) : LAUNCH_NI(float, false, 32);
+  else if (dtype != CIMA_BF16) return cima_fail(CIMA_E_DTYPE, "attention_plain: dtype code %d is neither float32 nor bfloat16", dtype);
+  else if (hd <= 256) rc = from_cache ? LAUNCH_NI(__nv_bfloat16, true, 8) : LAUNCH_NI(__nv_bfloat16, false, 8);
+  else rc = from_cache ? LAUNCH_NI(__nv_bfloat16, true, 32) : LAUNCH_NI(__nv_bfloat16, false, 32);
+  if (rc) return rc;
 #undef LAUNCH_NI
   return cima_launch_result();
 }

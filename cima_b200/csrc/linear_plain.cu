@@ -1,8 +1,9 @@
 // Plain matrix product for the true 32-bit path and for weights that are stored in 32-bit:
 //   out[m,n] = sum_k A[m,k] * W[n,k] (+ bias[n])        weights are [out, in], as in the checkpoint
-// FFMA only, no tensor cores and no reduced-precision mode.  Each output element is accumulated
-// by one thread over k = 0..K-1 in ascending order, so its value depends on its own row of A and
-// row of W only: the same bits whether the row comes alone, in a prompt or in a batch.
+// FFMA only, no tensor cores and no reduced-precision mode.  The order in which an output's products are added follows
+// from K alone, so its value depends on its own row of A and row of W only: the same bits whether the row comes alone, in a
+// prompt or in a batch.  k_linear_plain (bfloat16 activations or weights): one accumulator over k = 0..K-1 in ascending
+// order.  All in float32: see k_linear_f32_few and k_linear_f32_tile.
 //
 // Counterpart in the reference: k_gemm_f16 (src/kernels.cu:1410-1431; 16x16 tiles, one output per
 // thread, f32 accumulate) with k_bias (:390-393) and k_add (:75-78) behind it.
@@ -73,106 +74,365 @@ k_linear_plain(const TA* __restrict__ A, const TW* __restrict__ W, const float* 
   }
 }
 
-// The same for at most 8 rows (a decode step): one thread per output feature walks its row of W once, 64 k at a
-// time (sixteen independent 16-byte loads in flight per thread, then the products in ascending k), with one
-// accumulator per row of A.  The sequence of fused multiply-adds of an output element is exactly that of the
-// tiled kernel above, so the two give the same bits; this one streams the weights (a thread per output feature
-// is all the parallelism the fixed order leaves: some 1 TB/s at 3,584 features, 3 TB/s at 37,888) where the tiled
-// kernel, with a sixty-fourth of its tile in use, reaches a few percent of the memory's bandwidth.
-// The block's rows of A go through shared memory, 64 k at a time (every thread reads the same values).
-constexpr int FEW_ROWS = 8;
-constexpr int FEW_THREADS = 64;
-constexpr int FEW_K = 64;
+// ---------------------------------------------------------------------------------------------------- all in float32
+// The 32-bit path's own product.  An output's sum over k is cut into F32_GROUPS ranges of k (f32_group_len, from K alone);
+// a range is added up in ascending k by one accumulator, and the ranges' sums are added in their order.  Both kernels below
+// follow that order, so a row's bits depend on its own row of A and the weights only: the same alone, in a prompt or in a
+// batch, whatever tile or split serves it.  (One accumulator over all of K left a decode step one thread per output feature:
+// 75 us a product at the 0.5B shape, 0.3 TB/s.  Eight ranges give eight times the threads, and a shorter chain of roundings.)
+constexpr int F32_GROUPS = 8;
+__host__ __device__ inline int f32_group_len(int K) { return ((K + F32_GROUPS - 1) / F32_GROUPS + 15) & ~15; }
 
-template <typename TA, typename TW, typename TO, int MODE, bool VEC>
-__global__ void __launch_bounds__(FEW_THREADS)
-k_linear_plain_few(const TA* __restrict__ A, const TW* __restrict__ W, const float* __restrict__ bias,
-                   TO* __restrict__ out, int M, int N, int K, int lda, int ldo) {
-  cima_pdl_wait();
-  __shared__ __align__(16) float As[FEW_ROWS][FEW_K];
-  const int n = blockIdx.x * FEW_THREADS + threadIdx.x;
-  const bool live = n < N;
-  const TW* wr = W + (size_t)(live ? n : 0) * K;
-  float acc[FEW_ROWS];
-#pragma unroll
-  for (int m = 0; m < FEW_ROWS; m++) acc[m] = 0.f;
-  for (int k0 = 0; k0 < K; k0 += FEW_K) {
-    const int kn = min(FEW_K, K - k0);
-    float w[FEW_K];
-    if (VEC && kn == FEW_K) {
-#pragma unroll
-      for (int q = 0; q < FEW_K / 4; q++) {
-        const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(wr) + k0 + 4 * q);
-        w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
-      }
+__device__ __forceinline__ void f32_copy16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void f32_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N> __device__ __forceinline__ void f32_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+__device__ __forceinline__ void f32_finish(float* o, float v, const float* bias, int n, int mode) {
+  if (bias) v += bias[n];
+  *o = mode == LIN_ACCUM ? *o + v : v;
+}
+
+// At most 8 rows (a decode step): bound by the weights' bytes.  A block takes 8 output features, a warp one range of k of
+// them: its pieces of the 8 weight rows travel through shared memory by cp.async, whole 512-byte runs of a row at a time, up
+// to FEW_STAGES pieces in flight, the first ones before the kernel ahead has finished (weights do not depend on it).  Lane =
+// (feature, row mod 4): a lane walks its feature's range in order for one or two rows of A.  8 features a block and not more:
+// a narrow product (896 features) still covers 112 SMs, and a wide one keeps several blocks on each.  Measured inside a decode
+// step of the 0.5B shape, 2 rows: 9.5 us a product on average, 2.2 TB/s (74.8 us and 0.27 TB/s with a thread an output feature).
+constexpr int FEW_ROWS = 8, FEW_F = 8, FEW_K = 128, FEW_PITCH = FEW_K + 4, FEW_STAGES = 4, FEW_WARPS = F32_GROUPS;
+
+template <int MR, bool VEC>        // MR: rows of A a lane takes (rows r, r + 4)
+__global__ void __launch_bounds__(32 * FEW_WARPS)
+k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out,
+                 int M, int N, int K, int lda, int ldo, int mode, int stages) {
+  extern __shared__ __align__(16) float few_smem[];
+  __shared__ float red[FEW_WARPS][FEW_ROWS][FEW_F];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * FEW_F;
+  const int len = f32_group_len(K), k0 = min(K, warp * len), kn = min(K, k0 + len) - k0, chunks = (kn + FEW_K - 1) / FEW_K;
+  const int unit = (FEW_F + M) * FEW_PITCH;             // a stage: 8 rows of W, then M rows of A
+  float* mine = few_smem + (size_t)warp * stages * unit;
+  // a piece of one row: `rows` floats of it (from k0 + c FEW_K on) into dst; what lies beyond the range is zero
+  auto piece = [&](float* dst, const float* src, int c) {
+    const int left = kn - c * FEW_K;
+    if constexpr (VEC) {
+      if (4 * lane < left) f32_copy16(dst + 4 * lane, src + k0 + c * FEW_K + 4 * lane);
+      else *reinterpret_cast<float4*>(dst + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
 #pragma unroll
-      for (int q = 0; q < FEW_K; q++) w[q] = q < kn ? cima_to_f32<TW>(wr[k0 + q]) : 0.f;
+      for (int e = 0; e < FEW_K / 32; e++) dst[lane + 32 * e] = lane + 32 * e < left ? src[k0 + c * FEW_K + lane + 32 * e] : 0.f;
     }
-    __syncthreads();                                    // the previous chunk of A has been used
-    for (int e = threadIdx.x; e < M * FEW_K; e += FEW_THREADS) {
-      const int m = e / FEW_K, q = e - m * FEW_K;
-      As[m][q] = q < kn ? cima_to_f32<TA>(A[(size_t)m * lda + k0 + q]) : 0.f;
-    }
-    __syncthreads();
+  };
+  auto weights = [&](int c) {
+    float* s = mine + (c % stages) * unit;
 #pragma unroll
-    for (int m = 0; m < FEW_ROWS; m++) {
-      if (m < M) {
-        if (kn == FEW_K) {
+    for (int f = 0; f < FEW_F; f++) piece(s + f * FEW_PITCH, W + (size_t)min(n0 + f, N - 1) * K, c);
+  };
+  auto rows = [&](int c) {
+    float* s = mine + (c % stages) * unit + FEW_F * FEW_PITCH;
+    for (int m = 0; m < M; m++) piece(s + m * FEW_PITCH, A + (size_t)m * lda, c);
+  };
+  for (int c = 0; c < min(stages, chunks); c++) weights(c);
+  cima_pdl_wait();
+  for (int c = 0; c < stages; c++) {
+    if (c < chunks) rows(c);
+    f32_commit();                                       // (the first of these groups holds all the weights requested above)
+  }
+  const int f = lane & 7, r = lane >> 3;
+  const bool live = r < M;
+  float acc[MR];
 #pragma unroll
-          for (int q = 0; q < FEW_K; q += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(&As[m][q]);
-            acc[m] = fmaf(a.x, w[q], acc[m]);
-            acc[m] = fmaf(a.y, w[q + 1], acc[m]);
-            acc[m] = fmaf(a.z, w[q + 2], acc[m]);
-            acc[m] = fmaf(a.w, w[q + 3], acc[m]);
-          }
-        } else {
-          for (int q = 0; q < kn; q++) acc[m] = fmaf(As[m][q], w[q], acc[m]);
+  for (int i = 0; i < MR; i++) acc[i] = 0.f;
+  for (int c = 0; c < chunks; c++) {
+    if (stages == FEW_STAGES) f32_wait<FEW_STAGES - 1>();
+    else if (stages == 2) f32_wait<1>();
+    else f32_wait<0>();
+    __syncwarp();
+    const float* s = mine + (c % stages) * unit;
+    if (live) {
+      const float *w = s + f * FEW_PITCH, *a = s + (FEW_F + r) * FEW_PITCH;
+      const bool two = MR > 1 && r + 4 < M;
+      const float* a2 = two ? a + 4 * FEW_PITCH : a;
+      const int kc = (min(FEW_K, kn - c * FEW_K) + 3) & ~3;
+#pragma unroll 8
+      for (int k = 0; k < kc; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(w + k), y = *reinterpret_cast<const float4*>(a + k);
+        acc[0] = fmaf(y.x, x.x, acc[0]); acc[0] = fmaf(y.y, x.y, acc[0]);
+        acc[0] = fmaf(y.z, x.z, acc[0]); acc[0] = fmaf(y.w, x.w, acc[0]);
+        if constexpr (MR > 1) {
+          const float4 z = *reinterpret_cast<const float4*>(a2 + k);
+          acc[1] = fmaf(z.x, x.x, acc[1]); acc[1] = fmaf(z.y, x.y, acc[1]);
+          acc[1] = fmaf(z.z, x.z, acc[1]); acc[1] = fmaf(z.w, x.w, acc[1]);
         }
       }
     }
+    __syncwarp();                                       // the stage has been read by every lane
+    if (c + stages < chunks) { weights(c + stages); rows(c + stages); }
+    f32_commit();
   }
-  if (!live) return;
+  f32_wait<0>();
+  cima_pdl_trigger();
+  if (live) {
+    red[warp][r][f] = acc[0];
+    if (MR > 1 && r + 4 < M) red[warp][r + 4][f] = acc[MR - 1];
+  }
+  __syncthreads();
+  const int m = threadIdx.x / FEW_F, n = n0 + threadIdx.x % FEW_F;
+  if (m < M && n < N) {
+    float v = red[0][m][threadIdx.x % FEW_F];
 #pragma unroll
-  for (int m = 0; m < FEW_ROWS; m++) {
-    if (m >= M) break;
-    float v = acc[m];
-    if (bias) v += bias[n];
-    TO* o = out + (size_t)m * ldo + n;
-    if (MODE == LIN_ACCUM) *o = cima_from_f32<TO>(cima_to_f32<TO>(*o) + v);
-    else *o = cima_from_f32<TO>(v);
+    for (int g = 1; g < FEW_WARPS; g++) v += red[g][m][threadIdx.x % FEW_F];
+    f32_finish(out + (size_t)m * ldo + n, v, bias, n, mode);
   }
 }
 
-template <typename TA, typename TW, typename TO, int MODE>
-static int launch_few(const void* A, const void* W, const float* bias, void* out, int M, int N, int K, int lda, int ldo,
+// More rows: bound by the FP32 pipe.  Tiles of BM x 128 outputs, 256 threads with BM / 16 x 8 outputs each; the products run
+// two at a time (fma.rn.f32x2, the same rounding), for which shared memory holds each value of A twice.  The next 16 k travel
+// through registers while the current ones are multiplied.  SPLIT: a cluster of 8 blocks shares a tile, a range of k each,
+// and adds the ranges' sums in order through distributed shared memory (see launch_f32 for when).  Measured inside a prompt step
+// of the 0.5B shape, 201 + 123 rows: 122 us a product on average, 24 TFLOP/s (322 us with tiles of 64 x 64 and 4 x 4 a thread).
+constexpr int F32_BN = 128, F32_BK = 16, F32_WROW = F32_BN + 4;
+
+__device__ __forceinline__ unsigned long long f32_pair(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 f32_unpair(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void f32_fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+
+template <int BM>
+constexpr int f32_tile_floats() { return 2 * F32_BK * (2 * BM + 4 + F32_WROW); }
+template <int BM, bool SPLIT>
+constexpr size_t f32_tile_smem() {
+  const size_t stage = f32_tile_floats<BM>() * sizeof(float), tile = SPLIT ? (size_t)BM * (F32_BN + 4) * sizeof(float) : 0;
+  return stage > tile ? stage : tile;
+}
+
+template <int BM, bool SPLIT, bool VEC>
+__global__ void __launch_bounds__(256)
+k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out,
+                  int M, int N, int K, int lda, int ldo, int mode) {
+  constexpr int TM = BM / 16, AROW = 2 * BM + 4;
+  constexpr int NA = (BM * F32_BK / 4 + 255) / 256, NW = F32_BN * F32_BK / 4 / 256;      // 16-byte pieces a thread moves
+  extern __shared__ __align__(16) float f32_smem[];
+  float* As = f32_smem;                                 // [2][F32_BK][AROW], every value twice
+  float* Ws = f32_smem + 2 * F32_BK * AROW;             // [2][F32_BK][F32_WROW]
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int rank = SPLIT ? blockIdx.x % F32_GROUPS : 0;
+  const int m0 = blockIdx.y * BM, n0 = (SPLIT ? blockIdx.x / F32_GROUPS : blockIdx.x) * F32_BN;
+  const int len = f32_group_len(K);
+  const int kbeg = SPLIT ? min(K, rank * len) : 0, kend = SPLIT ? min(K, kbeg + len) : K;
+  cima_pdl_wait();
+
+  float4 ra[NA], rw[NW];
+  auto load4 = [&](const float* p, int k) {              // four values of a row from k on; zero beyond the range
+    if constexpr (VEC) return k < kend ? *reinterpret_cast<const float4*>(p + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    else return make_float4(k < kend ? p[k] : 0.f, k + 1 < kend ? p[k + 1] : 0.f, k + 2 < kend ? p[k + 2] : 0.f, k + 3 < kend ? p[k + 3] : 0.f);
+  };
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int i = 0; i < NA; i++) {
+      const int idx = tid + 256 * i;
+      if (BM * F32_BK / 4 >= 256 * (i + 1) || idx < BM * F32_BK / 4) ra[i] = load4(A + (size_t)min(m0 + idx / 4, M - 1) * lda, k + 4 * (idx % 4));
+    }
+#pragma unroll
+    for (int i = 0; i < NW; i++) {
+      const int idx = tid + 256 * i;
+      rw[i] = load4(W + (size_t)min(n0 + idx / 4, N - 1) * K, k + 4 * (idx % 4));
+    }
+  };
+  auto place = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < NA; i++) {
+      const int idx = tid + 256 * i;
+      if (BM * F32_BK / 4 >= 256 * (i + 1) || idx < BM * F32_BK / 4) {
+        float* p = As + (buf * F32_BK + 4 * (idx % 4)) * AROW + 2 * (idx / 4);
+        *reinterpret_cast<float2*>(p) = make_float2(ra[i].x, ra[i].x);
+        *reinterpret_cast<float2*>(p + AROW) = make_float2(ra[i].y, ra[i].y);
+        *reinterpret_cast<float2*>(p + 2 * AROW) = make_float2(ra[i].z, ra[i].z);
+        *reinterpret_cast<float2*>(p + 3 * AROW) = make_float2(ra[i].w, ra[i].w);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NW; i++) {
+      const int idx = tid + 256 * i;
+      float* p = Ws + (buf * F32_BK + 4 * (idx % 4)) * F32_WROW + idx / 4;
+      p[0] = rw[i].x; p[F32_WROW] = rw[i].y; p[2 * F32_WROW] = rw[i].z; p[3 * F32_WROW] = rw[i].w;
+    }
+  };
+
+  unsigned long long acc[TM][4];
+  float total[SPLIT ? 1 : TM][SPLIT ? 1 : 8];
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      acc[i][j] = 0ull;
+      if constexpr (!SPLIT) total[i][2 * j] = total[i][2 * j + 1] = 0.f;
+    }
+  const int tiles = kend > kbeg ? (kend - kbeg + F32_BK - 1) / F32_BK : 0;
+  const int per = len / F32_BK;                         // tiles of a range (SPLIT: the only one)
+  if (tiles > 0) { fetch(kbeg); place(0); }
+  int until = per;
+  for (int t = 0; t < tiles; t++) {
+    const int buf = t & 1;
+    if (t + 1 < tiles) fetch(kbeg + (t + 1) * F32_BK);
+    __syncthreads();
+    const float *as = As + buf * F32_BK * AROW + 2 * TM * ty, *ws = Ws + buf * F32_BK * F32_WROW + 4 * tx;
+#pragma unroll
+    for (int k = 0; k < F32_BK; k++) {
+      unsigned long long a[TM], w[4];
+#pragma unroll
+      for (int i = 0; i < TM; i += 2) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(as + k * AROW + 2 * i);
+        a[i] = v.x; a[i + 1] = v.y;
+      }
+      const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(ws + k * F32_WROW), v = *reinterpret_cast<const ulonglong2*>(ws + k * F32_WROW + 64);
+      w[0] = u.x; w[1] = u.y; w[2] = v.x; w[3] = v.y;
+#pragma unroll
+      for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) f32_fma2(acc[i][j], a[i], w[j]);
+    }
+    if constexpr (!SPLIT) {
+      if (--until == 0 || t + 1 == tiles) {             // a range is complete
+        until = per;
+#pragma unroll
+        for (int i = 0; i < TM; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float2 v = f32_unpair(acc[i][j]);
+            total[i][2 * j] += v.x;
+            total[i][2 * j + 1] += v.y;
+            acc[i][j] = 0ull;
+          }
+      }
+    }
+    if (t + 1 < tiles) place(buf ^ 1);                  // (last read before the barrier above)
+  }
+  cima_pdl_trigger();
+  const bool wide = ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  auto store4 = [&](int m, int n, float4 v) {
+    if (m >= M || n >= N) return;
+    float* o = out + (size_t)m * ldo + n;
+    if (wide && n + 3 < N) {
+      if (bias) { v.x += bias[n]; v.y += bias[n + 1]; v.z += bias[n + 2]; v.w += bias[n + 3]; }
+      if (mode == LIN_ACCUM) {
+        const float4 c = *reinterpret_cast<const float4*>(o);
+        v.x = c.x + v.x; v.y = c.y + v.y; v.z = c.z + v.z; v.w = c.w + v.w;
+      }
+      *reinterpret_cast<float4*>(o) = v;
+    } else {
+      const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (n + j < N) f32_finish(o + j, e[j], bias, n + j, mode);
+    }
+  };
+  if constexpr (SPLIT) {
+    constexpr int ROW = F32_BN + 4;
+    __syncthreads();                                    // the stages are free: the tile takes their place
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const float2 x = f32_unpair(acc[i][2 * j]), y = f32_unpair(acc[i][2 * j + 1]);
+        *reinterpret_cast<float4*>(f32_smem + (ty * TM + i) * ROW + 64 * j + 4 * tx) = make_float4(x.x, x.y, y.x, y.y);
+      }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    const unsigned base = (unsigned)__cvta_generic_to_shared(f32_smem);
+    constexpr int MINE = BM / F32_GROUPS;               // rows of the tile that this block finishes
+    for (int idx = tid; idx < MINE * (F32_BN / 4); idx += 256) {
+      const int m = rank * MINE + idx / (F32_BN / 4), n = 4 * (idx % (F32_BN / 4));
+      float4 s[F32_GROUPS];
+#pragma unroll
+      for (int g = 0; g < F32_GROUPS; g++) {
+        unsigned at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(base + (unsigned)((m * ROW + n) * sizeof(float))), "r"(g));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s[g].x), "=f"(s[g].y), "=f"(s[g].z), "=f"(s[g].w) : "r"(at) : "memory");
+      }
+      float4 v = s[0];
+#pragma unroll
+      for (int g = 1; g < F32_GROUPS; g++) { v.x += s[g].x; v.y += s[g].y; v.z += s[g].z; v.w += s[g].w; }
+      store4(m0 + m, n0 + n, v);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");      // nobody leaves while its tile is read
+  } else {
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        store4(m0 + ty * TM + i, n0 + 64 * j + 4 * tx, make_float4(total[i][4 * j], total[i][4 * j + 1], total[i][4 * j + 2], total[i][4 * j + 3]));
+  }
+}
+
+template <typename Kern>
+static int f32_allow(Kern kern, size_t smem) {
+  if (smem <= 48 * 1024) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e == cudaSuccess ? 0 : cima_fail((int)e, "linear_plain: %zu bytes of shared memory are not available: %s", smem, cudaGetErrorString(e));
+}
+
+template <int BM, bool SPLIT, bool VEC>
+static int launch_f32_tile(const float* A, const float* W, const float* bias, float* out, int mode, int M, int N, int K, int lda, int ldo,
+                           cudaStream_t stream) {
+  constexpr size_t smem = f32_tile_smem<BM, SPLIT>();
+  auto kern = k_linear_f32_tile<BM, SPLIT, VEC>;
+  if (int rc = f32_allow(kern, smem)) return rc;
+  const dim3 grid((unsigned)((N + F32_BN - 1) / F32_BN) * (SPLIT ? F32_GROUPS : 1), (unsigned)((M + BM - 1) / BM));
+  return cima_launch(kern, grid, dim3(256), smem, stream, SPLIT ? F32_GROUPS : 1, A, W, bias, out, M, N, K, lda, ldo, mode);
+}
+
+template <bool VEC>
+static int launch_f32(const float* A, const float* W, const float* bias, float* out, int mode, int M, int N, int K, int lda, int ldo,
                       cudaStream_t stream) {
-  const dim3 g((N + FEW_THREADS - 1) / FEW_THREADS);
-  const bool vec = sizeof(TW) == 4 && K % 4 == 0 && ((uintptr_t)W & 15) == 0;
-  int rc;
-  if (vec) rc = cima_launch(k_linear_plain_few<TA, TW, TO, MODE, true>, g, dim3(FEW_THREADS), (size_t)0, stream, 1, (const TA*)A, (const TW*)W, bias, (TO*)out, M, N, K, lda, ldo);
-  else rc = cima_launch(k_linear_plain_few<TA, TW, TO, MODE, false>, g, dim3(FEW_THREADS), (size_t)0, stream, 1, (const TA*)A, (const TW*)W, bias, (TO*)out, M, N, K, lda, ldo);
-  if (rc) return rc;
-  return cima_launch_result();
+  if (M <= FEW_ROWS) {
+    const int chunks = (f32_group_len(K) + FEW_K - 1) / FEW_K, unit = (FEW_F + M) * FEW_PITCH * (int)sizeof(float) * FEW_WARPS;
+    const int blocks = (N + FEW_F - 1) / FEW_F;
+    // the most pieces in flight that leave room for two blocks on an SM (one, where there are not two for each)
+    const int room = blocks > 148 ? 110 * 1024 : 220 * 1024;
+    const int stages = chunks >= FEW_STAGES && FEW_STAGES * unit <= room ? FEW_STAGES : chunks >= 2 ? 2 : 1;
+    const size_t smem = (size_t)stages * unit;
+    auto kern = M <= 4 ? k_linear_f32_few<1, VEC> : k_linear_f32_few<2, VEC>;
+    if (int rc = f32_allow(kern, smem)) return rc;
+    return cima_launch(kern, dim3((unsigned)blocks), dim3(32 * FEW_WARPS), smem, stream, 1, A, W, bias, out, M, N, K, lda, ldo, mode, stages);
+  }
+  // Tiles of 128 rows, or of 64 or 32 where those leave less of them empty; fewer tiles than three quarters of the SMs are shared by
+  // clusters of 8 blocks.
+  const int nt = (N + F32_BN - 1) / F32_BN;
+  const int bm = M <= 32 ? 32 : (M + 63) / 64 % 2 && M < 512 ? 64 : 128;
+  const bool split = K >= 2 * F32_GROUPS * F32_BK && (long long)nt * ((M + bm - 1) / bm) <= 111;
+#define F32_RUN(BM) return split ? launch_f32_tile<BM, true, VEC>(A, W, bias, out, mode, M, N, K, lda, ldo, stream) \
+                                 : launch_f32_tile<BM, false, VEC>(A, W, bias, out, mode, M, N, K, lda, ldo, stream)
+  if (bm == 32) F32_RUN(32);
+  if (bm == 64) F32_RUN(64);
+  F32_RUN(128);
+#undef F32_RUN
 }
 
 template <typename TA, typename TW, typename TO>
 static int launch_plain(const void* A, const void* W, const float* bias, void* out, int mode, int M, int N, int K,
                         int lda, int ldo, cudaStream_t stream) {
-  // (only the all-float32 combination, the 32-bit path's: each instantiation of that kernel costs seconds to compile)
   if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4 && sizeof(TO) == 4) {
-    if (M <= FEW_ROWS) {
-      if (mode == LIN_STORE) return launch_few<TA, TW, TO, LIN_STORE>(A, W, bias, out, M, N, K, lda, ldo, stream);
-      return launch_few<TA, TW, TO, LIN_ACCUM>(A, W, bias, out, M, N, K, lda, ldo, stream);
-    }
-  }
+    const bool vec = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    const int rc = vec ? launch_f32<true>((const float*)A, (const float*)W, bias, (float*)out, mode, M, N, K, lda, ldo, stream)
+                       : launch_f32<false>((const float*)A, (const float*)W, bias, (float*)out, mode, M, N, K, lda, ldo, stream);
+    return rc ? rc : cima_launch_result();
+  } else {
   dim3 grid((N + 63) / 64, (M + 63) / 64);
   if (mode == LIN_STORE)
     { int rc_ = cima_launch(k_linear_plain<TA, TW, TO, LIN_STORE>, dim3(grid), dim3(256), (size_t)(0), stream, 1, (const TA*)A, (const TW*)W, bias, (TO*)out, M, N, K, lda, ldo); if (rc_) return rc_; }
   else
     { int rc_ = cima_launch(k_linear_plain<TA, TW, TO, LIN_ACCUM>, dim3(grid), dim3(256), (size_t)(0), stream, 1, (const TA*)A, (const TW*)W, bias, (TO*)out, M, N, K, lda, ldo); if (rc_) return rc_; }
   return cima_launch_result();
+  }
 }
 
 // mode 0: out = A W^T (+ bias), stored as out_dtype.  mode 1: out += A W^T (+ bias); out must be float32.

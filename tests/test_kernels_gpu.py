@@ -112,6 +112,29 @@ def test_linear_plain_rows_are_independent(K, rows, N, K_):
     assert torch.equal(acc_full[33:33 + rows], acc_few)
 
 
+@pytest.mark.parametrize("N,K_", [(129, 256), (127, 260), (896, 4864), (20000, 896), (260, 1000), (130, 255), (40, 4864)])
+def test_linear_float32_the_same_bits_from_every_kernel(K, N, K_):
+    """Rows 1 to 8 (a warp a range of k), 9 to 32, 33 to 64, 65 and more (tiles of 32, 64 and 128 rows; shared by a cluster where a
+    product has few tiles, alone where it has many): one order of the sums, so one result; sizes around the tiles' edges, ranges of k
+    that end early, rows whose bytes are no multiple of 16.  Tolerance: K products in at most K / 8 + 31 steps a range (the last of them
+    shorter) and eight ranges, each step half an ulp of a sum that stays below the largest partial sum."""
+    M = 200
+    a, w, b = g(M, K_, seed=4), g(N, K_, seed=5, scale=0.1), g(N, seed=6)
+    want = a.double() @ w.double().t() + b.double()
+    full = torch.empty(M, N, device="cuda")
+    K.linear_plain(a.cuda(), w.cuda(), b.cuda(), full)
+    room = (K_ / 8 + 40) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()).max().item()
+    assert err(full, want) <= room
+    for rows in (1, 2, 4, 5, 8, 9, 32, 33, 64, 65, 128):
+        part = torch.full((rows, N), -777.0, device="cuda")
+        K.linear_plain(a[50:50 + rows].contiguous().cuda(), w.cuda(), b.cuda(), part)
+        assert torch.equal(part, full[50:50 + rows]), rows
+        acc, acc_full = torch.ones(rows, N, device="cuda"), torch.ones(M, N, device="cuda")
+        K.linear_plain(a[50:50 + rows].contiguous().cuda(), w.cuda(), None, acc, accumulate=True)
+        K.linear_plain(a.cuda(), w.cuda(), None, acc_full, accumulate=True)
+        assert torch.equal(acc, acc_full[50:50 + rows]), rows
+
+
 @pytest.mark.parametrize("M", [1, 3, 7, 8])
 @pytest.mark.parametrize("N,K_", [(200, 328), (1000, 192), (4608, 3584), (17, 8)])
 def test_linear_skinny_modes(K, M, N, K_):
@@ -317,6 +340,34 @@ def test_attention_decode_with_many_live_splits(K, nh, nkv, hd):
         K.profile = None
     assert [l.name for l in seen.launches] == ["attention_decode[64 splits]"]
     assert err(out[:1], want[:1]) <= TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window,keep", [(14, 2, 64, 0, 0), (4, 4, 128, 40, 0), (6, 2, 48, 33, 5), (3, 1, 200, 64, 40), (40, 1, 64, 0, 0), (2, 1, 30, 96, 32)])
+def test_attention_float32_the_same_bits_however_cut(K, nh, nkv, hd, window, keep):
+    """A float32 row's attention from the step's own rows, from the cache with many rows at once and from the cache row by row: the
+    same bits, around the borders of the 32-position pieces; with a sink, distance slopes and an infinity among the values that no
+    earlier row may notice.  Against the float64 statement on the rows in front of that infinity."""
+    n, page = 131, 16
+    tables, n_pages, width = scattered_tables([n], [1], page, seed=hd)
+    cpu, gpu = make_kv(n_pages, nkv, page, hd, 4, width, 0, 0, torch.float32, tables)
+    qkv = g(n, (nh + 2 * nkv) * hd, seed=7)
+    qkv[n - 1, (nh + nkv) * hd] = float("inf")
+    fill_cache(cpu, gpu, 1, qkv[:, nh * hd:(nh + nkv) * hd].reshape(n, nkv, hd), qkv[:, (nh + nkv) * hd:].reshape(n, nkv, hd))
+    scale, slopes = 1.0 / math.sqrt(hd), torch.linspace(0.0, 0.5, nh)
+    more = dict(sink=1.0, keep_first=keep)
+    bg, bc = batch_of([(1, 0, n)], "cuda"), batch_of([(1, 0, n)], "cpu")
+    step, cached, alone = (torch.empty(n, nh * hd, device="cuda") for _ in range(3))
+    args = (bg.row_pos, bg.row_seq, bg.seq_slot, bg.seq_first_row)
+    K.attention_plain(qkv.cuda(), None, *args, step, nh, nkv, hd, scale, window, False, slopes=slopes.cuda(), **more)
+    K.attention_plain(qkv.cuda(), gpu, *args, cached, nh, nkv, hd, scale, window, True, slopes=slopes.cuda(), **more)
+    for i in range(n):
+        b1 = batch_of([(1, i, 1)], "cuda")
+        K.attention_plain(qkv[i:i + 1].cuda(), gpu, b1.row_pos, b1.row_seq, b1.seq_slot, b1.seq_first_row, alone[i:i + 1], nh, nkv, hd, scale,
+                          window, True, slopes=slopes.cuda(), **more)
+    assert torch.equal(step[:n - 1], cached[:n - 1]) and torch.equal(step[:n - 1], alone[:n - 1]) and bool(step[:n - 1].isfinite().all())
+    want = torch.zeros(n, nh * hd, dtype=torch.float64)
+    REF.attention_plain(qkv, None, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_first_row, want, nh, nkv, hd, scale, window, False, slopes=slopes, **more)
+    assert err(step[:n - 1], want[:n - 1]) <= TOL["float32"]
 
 
 @pytest.mark.parametrize("dtype,page", [("float32", 16), ("bfloat16", 16), ("bfloat16", 64)])
