@@ -60,14 +60,19 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int HD, bool FROM_CACHE>
+// SPLIT: a block's key tiles are shared by n_splits blocks (blockIdx.y), which leave sums without the division and their
+// (maximum, denominator) for k_attention_merge.  For sequences that go on by a few rows behind a long context: 61 rows at
+// 16,000 positions of a 12-head shape are 12 blocks that walk 251 pages one after another; with 37 splits the 28 layers' step takes
+// 5.4 ms in place of 13.2 (kernels.py, extend_splits, says when).
+template <int HD, bool FROM_CACHE, bool SPLIT>
 __global__ void __launch_bounds__(WARPS * 32, 3)      // 3 blocks per SM: at most 168 registers
 k_attention_prefill(const __nv_bfloat16* __restrict__ qkv, int ld, const int* __restrict__ tile_seq,
                     const int* __restrict__ tile_row0, const int* __restrict__ seq_first_row,
                     const __nv_bfloat16* __restrict__ cache, CimaPaged pg, const int* __restrict__ seq_slot,
                     const int* __restrict__ seq_len,
                     __nv_bfloat16* __restrict__ out, int ldo, int T, int nh, int nkv, float scale, int window, float sink, int keep_first, int v_group,
-                    const float* __restrict__ head_sink, int gate_col, const float* __restrict__ slopes) {
+                    const float* __restrict__ head_sink, int gate_col, const float* __restrict__ slopes,
+                    float* __restrict__ part_o, float2* __restrict__ part_ml) {
   cima_pdl_wait();
   constexpr int ROW = HD + 8;
   constexpr int TILE = BN * ROW;
@@ -120,7 +125,9 @@ k_attention_prefill(const __nv_bfloat16* __restrict__ qkv, int ld, const int* __
   const int lo_key = (window > 0 && start + q0 + 1 > window) ? start + q0 + 1 - window : 0;
   const int t0 = lo_key / BN, t1 = (start + last_q) / BN + 1;
   const int nkeep = min((keep_first + BN - 1) / BN, t0);       // tiles of kept first positions that lie below the window's
-  const int n_iter = nkeep + t1 - t0;
+  const int all_iter = nkeep + t1 - t0;
+  const int share = SPLIT ? (all_iter + gridDim.y - 1) / gridDim.y : all_iter;
+  const int it0 = SPLIT ? min(all_iter, share * (int)blockIdx.y) : 0, n_iter = min(all_iter, it0 + share);      // this block's part of them
   auto tile_of = [&](int it) { return it < nkeep ? it : t0 + (it - nkeep); };
 
   auto issue = [&](int kt, int stage) {
@@ -155,9 +162,9 @@ k_attention_prefill(const __nv_bfloat16* __restrict__ qkv, int ld, const int* __
     }
   };
 
-  issue(tile_of(0), 0);
+  if (!SPLIT || it0 < n_iter) issue(tile_of(it0), it0 & 1);
   cp_async_commit();
-  for (int it = 0; it < n_iter; it++) {
+  for (int it = it0; it < n_iter; it++) {
     const int kt = tile_of(it);
     const int stage = it & 1;
     if (it + 1 < n_iter) issue(tile_of(it + 1), stage ^ 1);
@@ -275,6 +282,19 @@ k_attention_prefill(const __nv_bfloat16* __restrict__ qkv, int ld, const int* __
   }
   cp_async_wait<0>();
 
+  if constexpr (SPLIT) {
+    const int rows[2] = {r0, r1};
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      if (rows[r] >= len) continue;
+      const size_t at = ((size_t)(first + rows[r]) * nh + h) * gridDim.y + blockIdx.y;
+      if (t == 0) part_ml[at] = make_float2(m_run[r], l_run[r]);
+#pragma unroll
+      for (int j = 0; j < NTILES; j++) *reinterpret_cast<float2*>(part_o + at * HD + j * 8 + 2 * t) = make_float2(o[j][2 * r], o[j][2 * r + 1]);
+    }
+    return;
+  }
+
   // `sink` entries of score 0 without a value join the denominator (0: an ordinary softmax); maxima are base-2 scores
   // (or, with `head_sink`, one entry whose score is the head's own number)
   if (head_sink) sink = expf(head_sink[h]);
@@ -305,13 +325,68 @@ k_attention_prefill(const __nv_bfloat16* __restrict__ qkv, int ld, const int* __
   }
 }
 
-template <int HD, bool FROM_CACHE>
+// The splits of a row and head put together: a warp each, 2^(m_s - M) o_s summed in the order of the splits.  MAX_EXTEND_SPLITS / 32
+// (m, l) a lane, all requested at once; then four neighbouring dims a lane.
+constexpr int MAX_EXTEND_SPLITS = 64;
+__global__ void __launch_bounds__(128)
+k_attention_merge(const float* __restrict__ part_o, const float2* __restrict__ part_ml, __nv_bfloat16* __restrict__ out, int ldo, int T, int nh,
+                  int hd, int n_splits, float sink, const float* __restrict__ head_sink, const __nv_bfloat16* __restrict__ qkv, int ld, int gate_col) {
+  cima_pdl_wait();
+  __shared__ float sw[4][MAX_EXTEND_SPLITS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long unit = (long long)blockIdx.x * 4 + warp;
+  if (unit >= (long long)T * nh) return;
+  const int row = (int)(unit / nh), h = (int)(unit - (long long)row * nh);
+  const size_t base = (size_t)unit * n_splits;
+  float m[MAX_EXTEND_SPLITS / 32], l[MAX_EXTEND_SPLITS / 32], M = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < MAX_EXTEND_SPLITS / 32; i++) {
+    const int s = lane + 32 * i;
+    const float2 ml = s < n_splits ? part_ml[base + s] : make_float2(-INFINITY, 0.f);
+    m[i] = ml.x; l[i] = ml.y;
+    M = fmaxf(M, m[i]);
+  }
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  const float Ms = M == -INFINITY ? 0.f : M;
+  float L = 0.f;
+#pragma unroll
+  for (int i = 0; i < MAX_EXTEND_SPLITS / 32; i++) {
+    const float w = ex2(m[i] - Ms);                      // 0 for a split without keys
+    sw[warp][lane + 32 * i] = w;
+    L += w * l[i];
+  }
+  for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+  if (head_sink) sink = expf(head_sink[h]);
+  if (sink != 0.f) L += sink * ex2(-Ms);
+  const float inv = L > 0.f ? 1.0f / L : 0.f;
+  __syncwarp();
+  const int d = 4 * lane;
+  if (d >= hd) return;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int s = 0; s < n_splits; s++) {
+    const float4 v = *reinterpret_cast<const float4*>(part_o + (base + s) * hd + d);
+    const float w = sw[warp][s];
+    acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
+  }
+  float g[4] = {1.f, 1.f, 1.f, 1.f};
+  if (gate_col > 0) {
+    const __nv_bfloat16* gp = qkv + (size_t)row * ld + gate_col + (size_t)h * hd + d;
+#pragma unroll
+    for (int e = 0; e < 4; e++) g[e] = cima_sigmoid_fast(__bfloat162float(gp[e]));
+  }
+  uint32_t* op = reinterpret_cast<uint32_t*>(out + (size_t)row * ldo + (size_t)h * hd + d);
+  op[0] = pack_bf16(acc.x * inv * g[0], acc.y * inv * g[1]);
+  op[1] = pack_bf16(acc.z * inv * g[2], acc.w * inv * g[3]);
+}
+
+template <int HD, bool FROM_CACHE, bool SPLIT>
 int launch_prefill(const void* qkv, int ld, const int* tile_seq, const int* tile_row0, const int* seq_first_row,
                    const void* cache, const CimaPaged& pg, const int* seq_slot, const int* seq_len,
                    void* out, int ldo, int T, int n_tiles, int nh, int nkv, float scale, int window, float sink, int keep_first, int v_group,
-                   const float* head_sink, int gate_col, const float* slopes, cudaStream_t stream) {
+                   const float* head_sink, int gate_col, const float* slopes, int n_splits, float* part_o, float* part_ml, cudaStream_t stream) {
   if ((long long)n_tiles * nh > 0x7fffffffll) return cima_fail(CIMA_E_SIZE, "attention_prefill: %d blocks of rows x %d heads exceed one launch", n_tiles, nh);
-  auto kern = k_attention_prefill<HD, FROM_CACHE>;
+  auto kern = k_attention_prefill<HD, FROM_CACHE, SPLIT>;
   const size_t smem = (size_t)2 * 2 * BN * (HD + 8) * sizeof(__nv_bfloat16);
   static bool raised = false;
   if (smem > 48 * 1024 && !raised) {
@@ -319,10 +394,16 @@ int launch_prefill(const void* qkv, int ld, const int* tile_seq, const int* tile
     if (e != cudaSuccess) return cima_fail((int)e, "attention_prefill: cannot raise shared memory to %zu bytes: %s", smem, cudaGetErrorString(e));
     raised = true;
   }
-  { int rc_ = cima_launch(kern, dim3((unsigned)n_tiles * (unsigned)nh), dim3(WARPS * 32), (size_t)(smem), stream, 1, (const __nv_bfloat16*)qkv, ld, tile_seq, tile_row0, seq_first_row,
+  { int rc_ = cima_launch(kern, dim3((unsigned)n_tiles * (unsigned)nh, SPLIT ? n_splits : 1), dim3(WARPS * 32), (size_t)(smem), stream, 1, (const __nv_bfloat16*)qkv, ld, tile_seq, tile_row0, seq_first_row,
                                                         (const __nv_bfloat16*)cache, pg, seq_slot, seq_len,
-                                                        (__nv_bfloat16*)out, ldo, T, nh, nkv, scale, window, sink, keep_first, v_group, head_sink, gate_col, slopes); if (rc_) return rc_; }
-  return cima_launch_result();
+                                                        (__nv_bfloat16*)out, ldo, T, nh, nkv, scale, window, sink, keep_first, v_group, head_sink, gate_col, slopes, part_o, (float2*)part_ml); if (rc_) return rc_; }
+  if (int rc = cima_launch_result()) return rc;
+  if constexpr (SPLIT) {
+    const long long units = (long long)T * nh;
+    return cima_launch(k_attention_merge, dim3((unsigned)((units + 3) / 4)), dim3(128), (size_t)0, stream, 1, (const float*)part_o, (const float2*)part_ml,
+                       (__nv_bfloat16*)out, ldo, T, nh, HD, n_splits, sink, head_sink, (const __nv_bfloat16*)qkv, ld, gate_col);
+  }
+  return 0;
 }
 
 }  // namespace
@@ -345,7 +426,7 @@ extern "C" int cima_attention_prefill(const void* qkv, int ld, const int* tile_s
   if (T <= 0 || n_tiles <= 0) return 0;
   if (int rc = prefill_checks("attention_prefill", qkv, ld, out, ldo, hd, nh, nkv, keep_first, v_group, gate_col)) return rc;
   const CimaPaged none{nullptr, 0, 0, BN, nkv, hd};
-#define CASE(H) case H: return launch_prefill<H, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, nullptr, none, nullptr, nullptr, out, ldo, T, n_tiles, nh, nkv, scale, window, sink, keep_first, v_group, head_sink, gate_col, slopes, stream)
+#define CASE(H) case H: return launch_prefill<H, false, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, nullptr, none, nullptr, nullptr, out, ldo, T, n_tiles, nh, nkv, scale, window, sink, keep_first, v_group, head_sink, gate_col, slopes, 1, nullptr, nullptr, stream)
   switch (hd) {
     CASE(16); CASE(32); CASE(48); CASE(64); CASE(80); CASE(96); CASE(112); CASE(128);
   }
@@ -354,23 +435,28 @@ extern "C" int cima_attention_prefill(const void* qkv, int ld, const int* tile_s
 }
 
 // The same for sequences that go on: the rows of sequence s are the positions seq_len[s] - rows .. seq_len[s] - 1,
-// and every key, the step's own included, is read from the layer's pages (64 positions each).
+// and every key, the step's own included, is read from the layer's pages (64 positions each).  n_splits > 1: the key tiles of a
+// block of rows are shared by so many blocks; part_o [T, nh, n_splits, hd] and part_ml [T, nh, n_splits, 2] float32 are their scratch.
 extern "C" int cima_attention_extend(const void* qkv, int ld, const int* tile_seq, const int* tile_row0,
                                      const int* seq_first_row, const void* cache, const int* table, int table_width,
                                      int ring, int page_size, const int* seq_slot, const int* seq_len, void* out, int ldo,
                                      int T, int n_tiles, int nh, int nkv, int hd, float scale, int window,
                                      int planes, float sink, int keep_first, int v_group, const float* head_sink, int gate_col,
-                                     const float* slopes, cudaStream_t stream) {
+                                     const float* slopes, int n_splits, float* part_o, float* part_ml, cudaStream_t stream) {
   if (T <= 0 || n_tiles <= 0) return 0;
+  if (n_splits < 1 || n_splits > MAX_EXTEND_SPLITS) return cima_fail(CIMA_E_SIZE, "attention_extend: %d splits; 1 to %d are possible", n_splits, MAX_EXTEND_SPLITS);
+  if (n_splits > 1 && (!part_o || !part_ml || ((uintptr_t)part_o & 15) || ((uintptr_t)part_ml & 7))) return cima_fail(CIMA_E_ARG, "attention_extend: more than one split needs the scratch buffers (16- and 8-byte aligned)");
   if (planes != 1 && planes != 2) return cima_fail(CIMA_E_ARG, "attention_extend: %d planes; pages hold keys | values (2) or one shared vector (1)", planes);
   if (int rc = prefill_checks("attention_extend", qkv, ld, out, ldo, hd, nh, nkv, keep_first, v_group, gate_col)) return rc;
   if (page_size != BN) return cima_fail(CIMA_E_SIZE, "attention_extend: page size %d; this kernel takes %d", page_size, BN);
   if (!cache || !table || !seq_slot || !seq_len || ((uintptr_t)cache & 15)) return cima_fail(CIMA_E_ARG, "attention_extend: the cache (16-byte aligned), its block table, slots and lengths are needed");
   const CimaPaged pg{table, table_width, ring, page_size, nkv, hd, planes};
-#define CASE(H) case H: return launch_prefill<H, true>(qkv, ld, tile_seq, tile_row0, seq_first_row, cache, pg, seq_slot, seq_len, out, ldo, T, n_tiles, nh, nkv, scale, window, sink, keep_first, v_group, head_sink, gate_col, slopes, stream)
+#define RUN(H, S) launch_prefill<H, true, S>(qkv, ld, tile_seq, tile_row0, seq_first_row, cache, pg, seq_slot, seq_len, out, ldo, T, n_tiles, nh, nkv, scale, window, sink, keep_first, v_group, head_sink, gate_col, slopes, n_splits, part_o, part_ml, stream)
+#define CASE(H) case H: return n_splits > 1 ? RUN(H, true) : RUN(H, false)
   switch (hd) {
     CASE(16); CASE(32); CASE(48); CASE(64); CASE(80); CASE(96); CASE(112); CASE(128);
   }
 #undef CASE
+#undef RUN
   return cima_fail(CIMA_E_SIZE, "attention_extend: head_dim %d is not instantiated", hd);
 }

@@ -15,7 +15,7 @@ import torch
 from .csrc.build import BuildError, library_path
 
 F32, BF16 = 0, 1
-ABI_VERSION = 32
+ABI_VERSION = 33
 SPLIT_BLOCKS = 296          # blocks of the decode attention that one wave holds (two per SM, 148 SMs)
 TC_ATTENTION_MIN_LEN = 256  # prompts from this length on take the tcgen05 attention (head_dim 64 or 128)
 SPLIT_FEW_BLOCKS = 148      # below this many blocks at 8 splits, more splits are taken
@@ -30,6 +30,18 @@ SHORT_CONTEXT_BYTES = 96 * 1024   # up to this many bytes of keys and values (on
 def short_context(head_dim: int) -> int:
     """Positions (whole pages of 64) up to which the decode attention of this head size runs without splits."""
     return SHORT_CONTEXT_BYTES // (4 * head_dim) // 64 * 64
+
+
+EXTEND_BLOCKS = 444         # blocks of the attention of going-on rows that one wave holds (three per SM, 148 SMs)
+
+
+def extend_splits(blocks: int, max_len: int, window: int, keep_first: int) -> int:
+    """How many blocks share the key tiles of a block of rows that goes on from the cache: as many as fill one wave, each with
+    at least four tiles of 64 keys (a split costs its sums' way through memory and the merge's launch), 64 at most.
+    ``max_len``: positions of the longest sequence after the step (0: not known, one block then)."""
+    seen = max_len if window <= 0 else min(max_len, window + 128 + -(-keep_first // 64) * 64)
+    tiles = -(-seen // 64)
+    return max(1, min(64, tiles // 4, EXTEND_BLOCKS // max(1, blocks)))
 
 
 # epilogues of the skinny product
@@ -76,7 +88,8 @@ _SIGNATURES = {
                              _f, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _vp],
     "cima_attention_decode": [_vp, _i, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _vp],
     "cima_attention_prefill": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _vp, _i, _vp, _vp],
-    "cima_attention_extend": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _f, _i, _i, _vp, _i, _vp, _vp],
+    "cima_attention_extend": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _f, _i, _i, _vp, _i, _vp,
+                              _i, _vp, _vp, _vp],
     "cima_attention_extend_tc": [_vp, _i, _vp, _vp, _vp, _vp, ctypes.c_longlong, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                                  _f, _i, _vp, _i, _f, _vp, _i, _vp, _vp],
     "cima_row_norm_append": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _f, _vp, _vp, _i, _i, _i, _vp],
@@ -598,10 +611,11 @@ class Kernels:
 
     def attention_extend(self, qkv: torch.Tensor, kv, batch, out: torch.Tensor, n_heads: int, n_kv_heads: int,
                          head_dim: int, scale: float, window: int, sink: float = 0.0, keep_first: int = 0,
-                         v_group: int = 1, head_sink=None, gate_col: int = 0, slopes=None) -> None:
+                         v_group: int = 1, head_sink=None, gate_col: int = 0, slopes=None, n_splits: Optional[int] = None) -> None:
         """Flash attention of sequences that bring several rows to a cache that already holds keys (bf16, pages of
         64, head_dim <= 128): the rows of sequence s stand at positions seq_len[s] - rows .. seq_len[s] - 1, and all
-        keys, the step's own included, are read from the layer's pages.  ``batch`` brings the blocks of 64 rows."""
+        keys, the step's own included, are read from the layer's pages.  ``batch`` brings the blocks of 64 rows;
+        ``n_splits`` blocks share the keys of each (``extend_splits`` where None)."""
         self._need(qkv, "qkv", torch.bfloat16, 2); self._need(out, "out", torch.bfloat16, 2)
         self._need(kv.storage, "cache", torch.bfloat16, 5); self._need(kv.block_table, "block_table", torch.int32, 2)
         T = qkv.shape[0]
@@ -609,12 +623,20 @@ class Kernels:
         if tuple(out.shape) != (T, n_heads * head_dim) or batch.q_tile_seq.numel() != batch.q_tile_row0.numel():
             raise KernelError(f"attention_extend: out {tuple(out.shape)} or the block list do not fit")
         if not self._admit("attention_extend", *self._attention_work(qkv, n_heads, n_kv_heads, head_dim, kv.planes)): return
+        if n_splits is None:
+            n_splits = extend_splits(batch.q_tile_seq.numel() * n_heads, int(getattr(batch, "max_len", 0) or 0), window, keep_first)
+        part_o = part_ml = None
+        if n_splits > 1:
+            part_o = torch.empty(T * n_heads * n_splits * head_dim, dtype=torch.float32, device=qkv.device)
+            part_ml = torch.empty(T * n_heads * n_splits * 2, dtype=torch.float32, device=qkv.device)
         self._check(self.lib.cima_attention_extend(
             qkv.data_ptr(), qkv.shape[1], batch.q_tile_seq.data_ptr(), batch.q_tile_row0.data_ptr(),
             batch.seq_first_row.data_ptr(), kv.storage.data_ptr(), kv.block_table.data_ptr(), kv.block_table.shape[1],
             kv.ring_pages, kv.page_size, batch.seq_slot.data_ptr(), batch.seq_len.data_ptr(), out.data_ptr(), out.shape[1],
             T, batch.q_tile_seq.numel(), n_heads, n_kv_heads, head_dim, scale, window, kv.planes, sink, keep_first, v_group,
-            _ptr(head_sink), gate_col, _ptr(slopes), self._stream()), "attention_extend")
+            _ptr(head_sink), gate_col, _ptr(slopes), n_splits, _ptr(part_o), _ptr(part_ml), self._stream()), "attention_extend")
+        if n_splits > 1:
+            self.launches += 1
 
     def attention_prefill_tc(self, qkv: torch.Tensor, batch, out: torch.Tensor, n_heads: int, n_kv_heads: int,
                              head_dim: int, scale: float, window: int, kv=None, sink: float = 0.0, head_sink=None,

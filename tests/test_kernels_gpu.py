@@ -570,6 +570,35 @@ def test_attention_of_sequences_that_go_on(K, nh, nkv, hd, window, ring):
     assert torch.equal(out, out2)
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(12, 2, 128), (6, 2, 48), (3, 1, 16)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (300, 0), (130, 70)])
+def test_attention_of_going_on_rows_with_shared_keys(K, nh, nkv, hd, window, keep):
+    """The key tiles of a block of rows shared by 2, 5 and 64 blocks (more than there are tiles: some have none), for a sequence
+    deep into its cache, one that starts and one whose rows cross a page's edge; with a sink, a stored number a head, distance slopes
+    and gates; against the float64 statement and the launch that is not split."""
+    seqs, page, width = [(2, 1900, 70), (0, 0, 5), (1, 126, 3)], 64, 31
+    order = torch.randperm(4 * width, generator=torch.Generator().manual_seed(7)).tolist()
+    tables = {slot: order[slot * width:(slot + 1) * width] for slot in range(4)}
+    cpu, gpu = make_kv(4 * width, nkv, page, hd, 4, width, 0, window, torch.bfloat16, tables)
+    cpu.storage.copy_(g(*cpu.storage.shape, dtype=torch.bfloat16, seed=hd + window))
+    gpu.storage.copy_(cpu.storage)
+    T, scale, cols = sum(s[2] for s in seqs), 1.0 / math.sqrt(hd), (nh + 2 * nkv) * hd
+    qkv = g(T, cols + nh * hd, dtype=torch.bfloat16, seed=nh + T)
+    bc, bg = batch_of(seqs, "cpu"), batch_of(seqs, "cuda")
+    slopes, head_sink = torch.linspace(0.0, 0.02, nh), torch.linspace(-1.0, 2.0, nh)
+    for kw in (dict(sink=1.0), dict(head_sink=head_sink, slopes=slopes), dict(gate_col=cols)):
+        want = torch.zeros(T, nh * hd, dtype=torch.float64)
+        REF.attention_plain(qkv, cpu, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_first_row, want, nh, nkv, hd, scale, window, True, keep_first=keep, **kw)
+        dev = {k: v.cuda() if torch.is_tensor(v) else v for k, v in kw.items()}
+        whole = torch.full((T, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        K.attention_extend(qkv.cuda(), gpu, bg, whole, nh, nkv, hd, scale, window, keep_first=keep, n_splits=1, **dev)
+        assert err(whole, want) <= TOL["bfloat16"]
+        for n_splits in (2, 5, 64):
+            out = torch.full((T, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+            K.attention_extend(qkv.cuda(), gpu, bg, out, nh, nkv, hd, scale, window, keep_first=keep, n_splits=n_splits, **dev)
+            assert err(out, want) <= TOL["bfloat16"], (n_splits, list(kw))
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 128), (6, 1, 64)])
 @pytest.mark.parametrize("window", [0, 90, 300])
 def test_attention_of_sequences_that_go_on_by_many_rows_tcgen05(K, nh, nkv, hd, window):
