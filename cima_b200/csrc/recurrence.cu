@@ -16,6 +16,16 @@
 // partial sums, then a fixed shuffle tree over the 8 lanes, whatever the step: a token's result has the same bits whether
 // its sequence came whole, in pieces or one token at a time, alone or in a batch.  Everything is float32 but the loads of
 // q, k, v.
+//
+// A token is a chain of some 600 cycles (measured: 315 ns a token of the gate rule at key and value size 128), of which its
+// instructions fill a sixth, so few sequences leave the SMs waiting.  Long steps of the decay and the gate rule, whose states
+// nothing reads back before they are written, are therefore cut into segments of `seg` tokens that run side by side:
+//   PHASE 1   every segment but a sequence's last, from S = 0, without read-out: what it adds, E (and the product of its
+//             gates, D; the decay rule's is a power of its constant)
+//   combine   the state in front of every segment: S_0 = the stored state, S_(i+1) = D_i S_i + E_i
+//   PHASE 2   every segment from the state in front of it, with read-out; a sequence's last one stores the state
+// One and a half times the work, in place of the chain; PHASE 0 is the one launch for everything else.  Only bfloat16 rows are
+// cut: the 32-bit path keeps a token's bits whatever the cutting.
 #include "common.cuh"
 
 namespace {
@@ -34,15 +44,22 @@ __device__ __forceinline__ float rec_sum_over_lanes(float v) {        // over th
 
 // CPT: columns a thread owns (its columns stand 32 apart).  With two, every read of k, q and g from shared memory serves
 // both, but a block covers 64 columns and a sequence gets half as many blocks: measured slower for one prompt (1.2 ms
-// against 0.97 ms a layer of 2,048 tokens at key and value size 128), so the launch takes one.
+// against 0.97 ms a layer of 2,048 tokens at key and value size 128), so the launch takes one where a step is not cut.
 // MODE: 0 the decay rule, 1 the delta rule, 2 the gate rule.
-template <typename TQ, typename TV, int DIMP, int MODE, int CPT>
+struct RecSegments {
+  float* buf;                  // [sequence x max_segs, heads, dim, vdim]: what a segment adds, then the state in front of it
+  float* prod;                 // the gate rule: [sequence x max_segs, heads, dim], a segment's product of gates
+  int seg, max_segs;
+};
+
+template <typename TQ, typename TV, int DIMP, int MODE, int CPT, int PHASE>
 __global__ void __launch_bounds__(REC_THREADS)
 k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ldk, const TV* __restrict__ v, int ldv,
              const float* __restrict__ g, const float* __restrict__ beta, const float* __restrict__ decay,
              float* __restrict__ state, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row,
-             float* __restrict__ out, int heads, int kv_heads, int dim, int vdim) {
+             float* __restrict__ out, int heads, int kv_heads, int dim, int vdim, const RecSegments sg_) {
   constexpr bool DELTA = MODE == 1, GATE = MODE == 2, CHANNEL = MODE != 0;      // CHANNEL: a decay a key channel and token
+  constexpr bool READ = PHASE != 1;
   cima_pdl_wait();
   constexpr int RP = DIMP / REC_SPLIT;                  // rows of a column that one lane keeps
   constexpr int CH = DIMP > 128 ? 8 : 16;               // tokens staged at a time
@@ -53,19 +70,25 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
   __shared__ float sv[CH][COLS];
   __shared__ float so[CH][COLS];
   __shared__ float sb[CH];
-  const int seq = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
+  const int seq = PHASE == 0 ? blockIdx.z : blockIdx.z / sg_.max_segs, h = blockIdx.y, col0 = blockIdx.x * COLS;
+  const int skip = PHASE == 0 ? 0 : (blockIdx.z - seq * sg_.max_segs) * sg_.seg;      // the sequence's tokens in front of the segment
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rg = lane >> 2, lc = warp * 4 + (lane & 3);  // row group; the thread's columns are col0 + lc + 32 x
   const int kvh = h / (heads / kv_heads);
-  const int first = seq_first_row[seq], n = seq_first_row[seq + 1] - first;
-  float* st = state + (((size_t)seq_slot[seq] * heads + h) * dim) * (size_t)vdim + col0 + lc;
+  const int first = seq_first_row[seq] + skip, left = seq_first_row[seq + 1] - first;
+  if (PHASE != 0 && left <= 0) return;
+  const bool last = PHASE == 0 || left <= sg_.seg;
+  if (PHASE == 1 && last) return;
+  const int n = last ? left : sg_.seg;
+  const size_t in_unit = ((size_t)h * dim) * (size_t)vdim + col0 + lc, unit = (size_t)heads * dim * vdim;
+  float* st = PHASE == 0 ? state + seq_slot[seq] * unit + in_unit : sg_.buf + blockIdx.z * unit + in_unit;
   float S[CPT][RP];
 #pragma unroll
   for (int x = 0; x < CPT; x++)
 #pragma unroll
     for (int j = 0; j < RP; j++) {
       const int row = (j >> 2) * 32 + rg * 4 + (j & 3);
-      S[x][j] = (col0 + lc + 32 * x < vdim && row < dim) ? st[(size_t)row * vdim + 32 * x] : 0.f;
+      S[x][j] = (READ && col0 + lc + 32 * x < vdim && row < dim) ? st[(size_t)row * vdim + 32 * x] : 0.f;
     }
   const float dh = CHANNEL ? 1.f : decay[h];
   const int ldo = heads * vdim;
@@ -100,7 +123,7 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
       const size_t row = (size_t)(first + t0 + tt);
       const bool ok = tt < nt && i < dim;
       rk[r] = ok ? k[row * ldk + (size_t)kvh * dim + i] : zero_q;
-      rq[r] = ok ? q[row * ldq + (size_t)kvh * dim + i] : zero_q;
+      if (READ) rq[r] = ok ? q[row * ldq + (size_t)kvh * dim + i] : zero_q;
       if (DELTA) rgt[r] = ok ? g[(row * heads + h) * dim + i] : 1.f;
     }
 #pragma unroll
@@ -112,6 +135,7 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
     if (DELTA) rb = (int)threadIdx.x < nt ? beta[(size_t)(first + t0 + threadIdx.x) * heads + h] : 0.f;
   };
   if (n > 0) fetch(0);
+  float prod = 1.f;                                     // PHASE 1 of the gate rule: channel threadIdx.x's product of gates
 
   for (int t0 = 0; t0 < n; t0 += CH) {
     const int nt = min(CH, n - t0);
@@ -120,9 +144,12 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
     for (int r = 0; r < NLD; r++) {
       const int idx = threadIdx.x + r * REC_THREADS;
       const int tt = idx / DIMP, i = idx - tt * DIMP;
-      const float fk = cima_to_f32<TQ>(rk[r]), fq = cima_to_f32<TQ>(rq[r]);
+      const float fk = cima_to_f32<TQ>(rk[r]);
       if (!GATE) sk[tt][i] = DELTA ? fk : rec_silu(fk);
-      sq[tt][i] = DELTA ? fq : rec_silu(fq);
+      if (READ) {
+        const float fq = cima_to_f32<TQ>(rq[r]);
+        sq[tt][i] = DELTA ? fq : rec_silu(fq);
+      }
       if (DELTA) sg[tt][i] = rgt[r];
       if (GATE) sg[tt][i] = glow[r] + (1.0f - glow[r]) / (1.0f + expf(-(fk + gbias[r])));
     }
@@ -134,43 +161,63 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
     if (DELTA && threadIdx.x < CH) sb[threadIdx.x] = rb;
     __syncthreads();
     if (t0 + CH < n) fetch(t0 + CH);
+    if constexpr (GATE && PHASE == 1) {
+      if (blockIdx.x == 0 && (int)threadIdx.x < DIMP)
+        for (int tt = 0; tt < nt; tt++) prod *= sg[tt][threadIdx.x];
+    }
     if constexpr (GATE) {
       // Nothing of a token's read-out feeds the next token's update, so four tokens are taken together: their updates
       // follow one another row by row (S <- u + f (S - u), which is f S + (1 - f) u), their sums over the lanes run side
       // by side.  A token's own arithmetic is the same wherever it stands among the four.
-      static_assert(CPT == 1 || !GATE, "the gate rule runs one column a thread");
       constexpr int TB = 4;
       for (int tt = 0; tt < nt; tt += TB) {
-        float o0[TB], o1[TB];
+        float o0[TB][CPT], o1[TB][CPT];
 #pragma unroll
         for (int x = 0; x < TB; x++) {
-          o0[x] = o1[x] = 0.f;
+#pragma unroll
+          for (int c = 0; c < CPT; c++) o0[x][c] = o1[x][c] = 0.f;
           if (tt + x < nt) {
-            const float u = sv[tt + x][lc];
+            float u[CPT];
+#pragma unroll
+            for (int c = 0; c < CPT; c++) u[c] = sv[tt + x][lc + 32 * c];
 #pragma unroll
             for (int j = 0; j < RP; j += 4) {
               const int i = (j >> 2) * 32 + rg * 4;
               const float4 g4 = *reinterpret_cast<const float4*>(&sg[tt + x][i]);
-              const float4 q4 = *reinterpret_cast<const float4*>(&sq[tt + x][i]);
-              S[0][j] = fmaf(g4.x, S[0][j] - u, u); S[0][j + 1] = fmaf(g4.y, S[0][j + 1] - u, u);
-              S[0][j + 2] = fmaf(g4.z, S[0][j + 2] - u, u); S[0][j + 3] = fmaf(g4.w, S[0][j + 3] - u, u);
-              o0[x] = fmaf(S[0][j], q4.x, o0[x]); o1[x] = fmaf(S[0][j + 1], q4.y, o1[x]);
-              o0[x] = fmaf(S[0][j + 2], q4.z, o0[x]); o1[x] = fmaf(S[0][j + 3], q4.w, o1[x]);
+#pragma unroll
+              for (int c = 0; c < CPT; c++) {
+                S[c][j] = fmaf(g4.x, S[c][j] - u[c], u[c]); S[c][j + 1] = fmaf(g4.y, S[c][j + 1] - u[c], u[c]);
+                S[c][j + 2] = fmaf(g4.z, S[c][j + 2] - u[c], u[c]); S[c][j + 3] = fmaf(g4.w, S[c][j + 3] - u[c], u[c]);
+              }
+              if constexpr (READ) {
+                const float4 q4 = *reinterpret_cast<const float4*>(&sq[tt + x][i]);
+#pragma unroll
+                for (int c = 0; c < CPT; c++) {
+                  o0[x][c] = fmaf(S[c][j], q4.x, o0[x][c]); o1[x][c] = fmaf(S[c][j + 1], q4.y, o1[x][c]);
+                  o0[x][c] = fmaf(S[c][j + 2], q4.z, o0[x][c]); o1[x][c] = fmaf(S[c][j + 3], q4.w, o1[x][c]);
+                }
+              }
             }
           }
         }
-#pragma unroll
-        for (int x = 0; x < TB; x++) o0[x] += o1[x];
-#pragma unroll
-        for (int x = 0; x < TB; x++) o0[x] += __shfl_xor_sync(0xffffffffu, o0[x], 4);
-#pragma unroll
-        for (int x = 0; x < TB; x++) o0[x] += __shfl_xor_sync(0xffffffffu, o0[x], 8);
-#pragma unroll
-        for (int x = 0; x < TB; x++) o0[x] += __shfl_xor_sync(0xffffffffu, o0[x], 16);
-        if (rg == 0) {
+        if constexpr (READ) {
 #pragma unroll
           for (int x = 0; x < TB; x++)
-            if (tt + x < nt) so[tt + x][lc] = o0[x];
+#pragma unroll
+            for (int c = 0; c < CPT; c++) o0[x][c] += o1[x][c];
+#pragma unroll
+          for (int d = 4; d <= 16; d <<= 1)
+#pragma unroll
+            for (int x = 0; x < TB; x++)
+#pragma unroll
+              for (int c = 0; c < CPT; c++) o0[x][c] += __shfl_xor_sync(0xffffffffu, o0[x][c], d);
+          if (rg == 0) {
+#pragma unroll
+            for (int x = 0; x < TB; x++)
+#pragma unroll
+              for (int c = 0; c < CPT; c++)
+                if (tt + x < nt) so[tt + x][lc + 32 * c] = o0[x][c];
+          }
         }
       }
     } else {
@@ -211,22 +258,26 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
       for (int j = 0; j < RP; j += 4) {
         const int i = (j >> 2) * 32 + rg * 4;
         const float4 k4 = *reinterpret_cast<const float4*>(&sk[tt][i]);
-        const float4 q4 = *reinterpret_cast<const float4*>(&sq[tt][i]);
+        float4 q4;
+        if constexpr (READ) q4 = *reinterpret_cast<const float4*>(&sq[tt][i]);
 #pragma unroll
         for (int x = 0; x < CPT; x++) {
           S[x][j] = fmaf(k4.x, u[x], S[x][j]); S[x][j + 1] = fmaf(k4.y, u[x], S[x][j + 1]);
           S[x][j + 2] = fmaf(k4.z, u[x], S[x][j + 2]); S[x][j + 3] = fmaf(k4.w, u[x], S[x][j + 3]);
+          if constexpr (!READ) continue;
           o0[x] = fmaf(S[x][j], q4.x, o0[x]); o1[x] = fmaf(S[x][j + 1], q4.y, o1[x]);
           o0[x] = fmaf(S[x][j + 2], q4.z, o0[x]); o1[x] = fmaf(S[x][j + 3], q4.w, o1[x]);
         }
       }
 #pragma unroll
       for (int x = 0; x < CPT; x++) {
+        if constexpr (!READ) continue;
         const float o = rec_sum_over_lanes(o0[x] + o1[x]);
         if (rg == 0) so[tt][lc + 32 * x] = o;
       }
     }
     }
+    if constexpr (!READ) continue;
     __syncthreads();
     for (int idx = threadIdx.x; idx < nt * COLS; idx += REC_THREADS) {
       const int tt = idx / COLS, cc = idx - tt * COLS;
@@ -234,6 +285,11 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
     }
   }
   cima_pdl_trigger();        // the tokens are done: the next kernel may be set up while the state is stored
+  if (PHASE == 2) {
+    if (!last) return;
+    st = state + seq_slot[seq] * unit + in_unit;
+  }
+  if (GATE && PHASE == 1 && blockIdx.x == 0 && (int)threadIdx.x < dim) sg_.prod[((size_t)blockIdx.z * heads + h) * dim + threadIdx.x] = prod;
 #pragma unroll
   for (int x = 0; x < CPT; x++)
 #pragma unroll
@@ -243,21 +299,68 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
     }
 }
 
-template <typename TQ, typename TV, int MODE>
-int launch_recurrence(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const float* g, const float* beta,
-                      const float* decay, float* state, const int* seq_slot, const int* seq_first_row, float* out,
-                      int n_seqs, int heads, int kv_heads, int dim, int vdim, cudaStream_t stream) {
-  const int cpt = 1;      // two columns a thread (CPT 2) measured slower: half as many blocks, and the chain of a token is no shorter
-  const dim3 grid((vdim + REC_COLS * cpt - 1) / (REC_COLS * cpt), heads, n_seqs);
-#define RUN_C(D, C) return cima_launch(k_recurrence<TQ, TV, D, MODE, C>, grid, dim3(REC_THREADS), (size_t)0, stream, 1, (const TQ*)q, ldq, (const TQ*)k, ldk, \
-                                       (const TV*)v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, heads, kv_heads, dim, vdim)
-#define RUN(D) { RUN_C(D, 1); }
+// The segments' buffer turns from what every segment adds into the state in front of it.  A thread an element of a head's state.
+template <bool GATE>
+__global__ void __launch_bounds__(256)
+k_recurrence_combine(const float* __restrict__ state, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row,
+                     const float* __restrict__ decay, int heads, int dim, int vdim, const RecSegments sg_) {
+  cima_pdl_wait();
+  const int size = dim * vdim, e = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, seq = blockIdx.z;
+  if (e >= size) return;
+  const int segs = (seq_first_row[seq + 1] - seq_first_row[seq] + sg_.seg - 1) / sg_.seg;
+  const float power = GATE ? 0.f : powf(decay[h], (float)sg_.seg);
+  float S = state[((size_t)seq_slot[seq] * heads + h) * size + e];
+  for (int s0 = 0; s0 < segs; s0 += 8) {                 // eight segments' values requested before the first is used
+    float E[8], D[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const bool ok = s0 + i < segs - 1;                  // what the last segment adds was not made
+      const size_t at = ((size_t)seq * sg_.max_segs + (ok ? s0 + i : 0)) * heads + h;
+      E[i] = ok ? sg_.buf[at * size + e] : 0.f;
+      D[i] = !ok ? 0.f : GATE ? sg_.prod[at * dim + e / vdim] : power;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      if (s0 + i < segs) sg_.buf[(((size_t)seq * sg_.max_segs + s0 + i) * heads + h) * size + e] = S;
+      S = fmaf(D[i], S, E[i]);
+    }
+  }
+}
+
+template <typename TQ, typename TV, int MODE, int PHASE>
+int launch_phase(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const float* g, const float* beta,
+                 const float* decay, float* state, const int* seq_slot, const int* seq_first_row, float* out,
+                 int n_units, int heads, int kv_heads, int dim, int vdim, const RecSegments& sg, cudaStream_t stream) {
+  // Uncut, two columns a thread measured slower: half as many blocks, and the chain of a token is no shorter.  Segments fill the SMs
+  // with instructions instead, so there a read of k, q and g from shared memory serves two columns.
+  constexpr int cpt = PHASE == 0 ? 1 : 2;
+  const dim3 grid((vdim + REC_COLS * cpt - 1) / (REC_COLS * cpt), heads, n_units);
+#define RUN_C(D, C) return cima_launch(k_recurrence<TQ, TV, D, MODE, C, PHASE>, grid, dim3(REC_THREADS), (size_t)0, stream, 1, (const TQ*)q, ldq, (const TQ*)k, ldk, \
+                                       (const TV*)v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, heads, kv_heads, dim, vdim, sg)
+#define RUN(D) { RUN_C(D, cpt); }
   if (dim <= 32) RUN(32);
   if (dim <= 64) RUN(64);
   if (dim <= 128) RUN(128);
   RUN(256);
 #undef RUN
 #undef RUN_C
+}
+
+template <typename TQ, typename TV, int MODE>
+int launch_recurrence(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const float* g, const float* beta,
+                      const float* decay, float* state, const int* seq_slot, const int* seq_first_row, float* out,
+                      int n_seqs, int heads, int kv_heads, int dim, int vdim, const RecSegments& sg, cudaStream_t stream) {
+#define PHASE_ARGS q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out
+  if constexpr (MODE != 1) {
+    if (sg.max_segs > 1) {
+      if (int rc = launch_phase<TQ, TV, MODE, 1>(PHASE_ARGS, n_seqs * sg.max_segs, heads, kv_heads, dim, vdim, sg, stream)) return rc;
+      if (int rc = cima_launch(k_recurrence_combine<MODE == 2>, dim3((unsigned)((dim * vdim + 255) / 256), (unsigned)heads, (unsigned)n_seqs), dim3(256), (size_t)0,
+                               stream, 1, (const float*)state, seq_slot, seq_first_row, decay, heads, dim, vdim, sg)) return rc;
+      return launch_phase<TQ, TV, MODE, 2>(PHASE_ARGS, n_seqs * sg.max_segs, heads, kv_heads, dim, vdim, sg, stream);
+    }
+  }
+  return launch_phase<TQ, TV, MODE, 0>(PHASE_ARGS, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+#undef PHASE_ARGS
 }
 
 // Everything of the delta rule that is computed per token before the recurrence, in float32:
@@ -320,12 +423,17 @@ k_delta_prepare(const TA* __restrict__ qk, int ldqk, const TA* __restrict__ a, i
 // delta != 0: q, k float32 [T, kv_heads * dim] (prepared), v (vdtype) [T, ldv], g [T, heads * dim], beta [T, heads].
 // delta == 0: q, k, v of one dtype (vdtype), SiLU applied here; decay [heads].  out [T, heads * vdim] float32.
 // delta == 2 (the gate rule): q and k of v's dtype, k holding the gate's projection; g its bias and decay its lower bound,
-// both [heads * dim] and shared by all tokens.
+// both [heads * dim] and shared by all tokens.  max_segs > 1 (not the delta rule): the sequences are cut into at most so many
+// segments of `seg` tokens; buf [n_seqs * max_segs, heads, dim, vdim] and, for the gate rule, prod [n_seqs * max_segs, heads, dim]
+// float32 are their scratch.
 extern "C" int cima_recurrence(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, int vdtype,
                                const float* g, const float* beta, const float* decay, float* state, const int* seq_slot,
                                const int* seq_first_row, float* out, int T, int n_seqs, int heads, int kv_heads, int dim,
-                               int vdim, int delta, cudaStream_t stream) {
+                               int vdim, int delta, int seg, int max_segs, float* buf, float* prod, cudaStream_t stream) {
   if (T <= 0 || n_seqs <= 0) return 0;
+  if (max_segs > 1 && (delta == 1 || seg < 1 || !buf || (delta == 2 && !prod) || (long long)n_seqs * max_segs > 65535))
+    return cima_fail(CIMA_E_ARG, "recurrence: %d segments of %d tokens in %d sequences need their scratch, a rule without a delta and at most 65535 units", max_segs, seg, n_seqs);
+  const RecSegments sg{buf, prod, seg, max_segs};
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || heads > 65535 || n_seqs > 65535)
     return cima_fail(CIMA_E_SIZE, "recurrence: %d heads on %d key heads in %d sequences are not accepted", heads, kv_heads, n_seqs);
   if (dim <= 0 || dim > 256 || vdim <= 0) return cima_fail(CIMA_E_SIZE, "recurrence: key size %d must lie in 1..256 and value size %d be positive", dim, vdim);
@@ -333,8 +441,8 @@ extern "C" int cima_recurrence(const void* q, int ldq, const void* k, int ldk, c
   if (delta == 2) {
     if (!g || !decay) return cima_fail(CIMA_E_ARG, "recurrence: the gate rule needs the gate's bias and lower bound");
     int rc2;
-    if (vdtype == CIMA_F32) rc2 = launch_recurrence<float, float, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, stream);
-    else if (vdtype == CIMA_BF16) rc2 = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, stream);
+    if (vdtype == CIMA_F32) rc2 = launch_recurrence<float, float, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    else if (vdtype == CIMA_BF16) rc2 = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
     else return cima_fail(CIMA_E_DTYPE, "recurrence: dtype code %d is neither float32 nor bfloat16", vdtype);
     return rc2 ? rc2 : cima_launch_result();
   }
@@ -342,12 +450,12 @@ extern "C" int cima_recurrence(const void* q, int ldq, const void* k, int ldk, c
   if (!delta && !decay) return cima_fail(CIMA_E_ARG, "recurrence: the decay rule needs the heads' decays");
   int rc;
   if (delta) {
-    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, stream);
-    else if (vdtype == CIMA_BF16) rc = launch_recurrence<float, __nv_bfloat16, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, stream);
+    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    else if (vdtype == CIMA_BF16) rc = launch_recurrence<float, __nv_bfloat16, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
     else return cima_fail(CIMA_E_DTYPE, "recurrence: dtype code %d is neither float32 nor bfloat16", vdtype);
   } else {
-    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, stream);
-    else if (vdtype == CIMA_BF16) rc = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, stream);
+    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    else if (vdtype == CIMA_BF16) rc = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
     else return cima_fail(CIMA_E_DTYPE, "recurrence: dtype code %d is neither float32 nor bfloat16", vdtype);
   }
   return rc ? rc : cima_launch_result();

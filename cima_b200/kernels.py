@@ -101,7 +101,7 @@ _SIGNATURES = {
     "cima_dyt_add": [_vp, _vp, _vp, _vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "cima_embed_bigram": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _f, _i, ctypes.c_longlong, ctypes.c_longlong, _vp, _vp, _vp, _vp, _vp,
                           _i, _vp],
-    "cima_recurrence": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
+    "cima_recurrence": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
     "cima_delta_prepare": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "cima_delta_rule": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "cima_group_rmsnorm_gate": [_vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _f, _vp],
@@ -1031,6 +1031,20 @@ class Kernels:
             self.launches += 1
 
     # ------------------------------------------------------------------ recurrent mixers
+    RECURRENCE_SEGMENT = 128    # tokens of a segment of a long step's decay or gate rule
+
+    def recurrence_segments(self, batch, columns: int, dtype: torch.dtype) -> int:
+        """Into how many segments at most the step's sequences are cut by the decay and the gate rule (1: not at all); ``columns``:
+        blocks of 32 value channels, all heads.  Uncut, a sequence takes 600 cycles a token; cut, a block's token costs the SM some
+        110 cycles of instructions, half as many again for the first phase, and three launches and the states' way through memory
+        come to some 30,000 cycles: cut where that is less than the longest sequence's chain.  bfloat16 rows only (a 32-bit row has
+        the same bits however its sequence is cut)."""
+        rows = int(getattr(batch, "max_rows", 0) or 0)
+        segs = -(-rows // self.RECURRENCE_SEGMENT)
+        if dtype is not torch.bfloat16 or rows < 2 * self.RECURRENCE_SEGMENT or 1.2 * batch.n_rows * columns + 30000 > 600 * rows or batch.n_seqs * segs > 65535:
+            return 1
+        return segs
+
     def recurrence(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, batch, out: torch.Tensor,
                    heads: int, kv_heads: int, dim: int, vdim: int, g: Optional[torch.Tensor] = None,
                    beta: Optional[torch.Tensor] = None, decay: Optional[torch.Tensor] = None, gate=None) -> None:
@@ -1065,10 +1079,15 @@ class Kernels:
                            batch.n_seqs * heads * dim * vdim * 8 + T * (2 * kv_heads * dim * q.element_size() + heads * vdim * (4 + v.element_size())
                                                                         + (heads * dim * 4 if delta else 0)),
                            (8.0 if delta else 5.0) * T * heads * dim * vdim): return
+        segs = 1 if delta else self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype)
+        buf = torch.empty(batch.n_seqs * segs * heads * dim * vdim, dtype=torch.float32, device=q.device) if segs > 1 else None
         self._check(self.lib.cima_recurrence(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
                                              dtype_code(v.dtype), _ptr(g), _ptr(beta), _ptr(decay), state.data_ptr(),
                                              batch.seq_slot.data_ptr(), batch.seq_first_row.data_ptr(), out.data_ptr(), T,
-                                             batch.n_seqs, heads, kv_heads, dim, vdim, int(delta), self._stream()), "recurrence")
+                                             batch.n_seqs, heads, kv_heads, dim, vdim, int(delta), self.RECURRENCE_SEGMENT, segs, _ptr(buf), None,
+                                             self._stream()), "recurrence")
+        if segs > 1:
+            self.launches += 2
 
     def _recurrence_gate(self, q, k, v, state, batch, out, heads, kv_heads, dim, vdim, bias, lower) -> None:
         self._need(state, "state", torch.float32, 4); self._need(out, "out", torch.float32, 2)
@@ -1084,10 +1103,18 @@ class Kernels:
                               f"out {tuple(out.shape)} and the gate's vectors do not agree with {heads} heads of {dim} x {vdim}")
         if not self._admit("recurrence[gate]", batch.n_seqs * heads * dim * vdim * 8 + T * heads * ((2 * dim + vdim) * v.element_size() + vdim * 4),
                            5.0 * T * heads * dim * vdim): return
+        segs = self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype)
+        buf = prod = None
+        if segs > 1:
+            buf = torch.empty(batch.n_seqs * segs * heads * dim * vdim, dtype=torch.float32, device=q.device)
+            prod = torch.empty(batch.n_seqs * segs * heads * dim, dtype=torch.float32, device=q.device)
         self._check(self.lib.cima_recurrence(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
                                              dtype_code(v.dtype), bias.data_ptr(), None, lower.data_ptr(), state.data_ptr(),
                                              batch.seq_slot.data_ptr(), batch.seq_first_row.data_ptr(), out.data_ptr(), T,
-                                             batch.n_seqs, heads, kv_heads, dim, vdim, 2, self._stream()), "recurrence")
+                                             batch.n_seqs, heads, kv_heads, dim, vdim, 2, self.RECURRENCE_SEGMENT, segs, _ptr(buf), _ptr(prod),
+                                             self._stream()), "recurrence")
+        if segs > 1:
+            self.launches += 2
 
     def delta_prepare(self, qk: torch.Tensor, a: torch.Tensor, b: torch.Tensor, A_log: torch.Tensor, dt_bias: torch.Tensor,
                       qn: torch.Tensor, kn: torch.Tensor, g: torch.Tensor, beta: torch.Tensor, heads: int, kv_heads: int,

@@ -8,6 +8,7 @@ import sys
 
 import numpy as np
 import pytest
+from types import SimpleNamespace
 import torch
 
 import cima_b200
@@ -191,6 +192,15 @@ def test_recurrence_whole_in_pieces_and_token_by_token(heads, kv_heads, dim, vdi
         kv_heads = heads
     steps = [[20, 3, 9], [2, 2, 2], [1, 1, 1], [1, 0, 1], [17, 0, 1]]
     _recurrence_case(delta, heads, kv_heads, dim, vdim, dtype, steps, seed=dim + vdim)
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 40, 72), (1, 128, 33), (3, 16, 8), (1, 200, 64)])
+def test_decay_rule_of_long_sequences_in_segments(heads, dim, vdim):
+    """Sequences of two to six segments beside short ones, ends on and off a segment's border, and what goes on from them."""
+    seg = K().RECURRENCE_SEGMENT
+    steps = [[5 * seg + 60, 5, 2 * seg], [2 * seg + 1, 0, 1], [1, 1, seg + 2]]
+    assert K().recurrence_segments(SimpleNamespace(max_rows=steps[0][0], n_rows=sum(steps[0]), n_seqs=3), heads * -(-vdim // 32), torch.bfloat16) == 6
+    _recurrence_case(False, heads, heads, dim, vdim, "bfloat16", steps, seed=dim)
 
 
 def test_recurrence_long_decoding_holds_its_state():
