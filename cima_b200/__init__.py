@@ -47,6 +47,7 @@ class LM:
                  use_graphs: bool = True):
         from .engine import GenerationLoop, ModelStepper
         self.model = model
+        model.record_steps = use_graphs
         self.stepper = ModelStepper(model, max_batch=max_batch, use_graphs=use_graphs, pipeline=pipeline, retain=retain)
         self.loop = GenerationLoop(self.stepper, eos_ids)
 
@@ -125,8 +126,8 @@ def load(folder: Optional[str] = None, dtype: str = "bfloat16", max_tokens: int 
     (the tokens are fed forward on the device).  ``retain``: how many finished sequences stay in the cache for
     later prompts that begin with the same tokens (the next turn of a conversation runs only what is new; the
     reference keeps its one sequence so, src/models/mod.rs:1022-1058); they give way when a batch needs the room.
-    ``use_graphs``: record decode steps as CUDA graphs (a model with a part that is unfit for it decodes step by
-    step whatever is asked)."""
+    ``use_graphs``: record decode steps, and one-token steps of ``LM.step``, as CUDA graphs (a model with a part that is unfit
+    for it decodes step by step whatever is asked)."""
     from .engine import load_model
     model = load_model(folder, dtype=dtype, max_tokens=max_tokens, max_seqs=max_seqs, device=device, verbose=verbose,
                        config=config, seed=seed, draw=draw)

@@ -17,6 +17,28 @@ import torch
 from .batch import StepBatch, StepEntry, build_batch
 
 
+def one_token_batch(meta: torch.Tensor, n_seqs: int, max_len: int) -> StepBatch:
+    """A step of one token a sequence, all logits wanted, whose arrays are views of ``meta`` (int32 [6 n + 1], see
+    ``fill_meta``).  What a recorded step may know on the host is what every replay shares: the number of sequences and
+    their rows (one each).  Slots, positions and lengths change from replay to replay and exist on the device only
+    (``host_seq_slot`` / ``host_seq_len`` stay None; ``max_len`` bounds the sequences' positions after the step, 0 = unknown)."""
+    B, m = n_seqs, meta
+    return StepBatch(prefill=False, n_rows=B, n_seqs=B, n_want=B, max_len=max_len, want_all_in_order=True,
+                     tokens=m[0:B], row_pos=m[B:2 * B], row_seq=m[2 * B:3 * B], seq_slot=m[3 * B:4 * B], seq_first_row=m[4 * B:5 * B + 1],
+                     seq_len=m[5 * B + 1:6 * B + 1], want_rows=m[2 * B:3 * B], max_rows=1, host_seq_first_row=np.arange(B + 1, dtype=np.int32))
+
+
+def fill_meta(h: np.ndarray, slots: Sequence[int], tokens: Sequence[int], lengths: Sequence[int]) -> None:
+    """Sequence i sits in slots[i], holds lengths[i] positions and brings tokens[i]."""
+    B = len(slots)
+    h[0:B] = tokens
+    h[B:2 * B] = lengths                           # the new token's position
+    h[2 * B:3 * B] = np.arange(B)
+    h[3 * B:4 * B] = slots
+    h[4 * B:5 * B + 1] = np.arange(B + 1)
+    h[5 * B + 1:6 * B + 1] = np.asarray(lengths) + 1
+
+
 class DecodeGraph:
     """One batch size's captured step.  ``load`` sets its inputs for a set of sequences; ``run``
     does one step (the first run after construction executes eagerly and captures)."""
@@ -33,31 +55,17 @@ class DecodeGraph:
         dev = model.rt.device
         self.meta = torch.zeros(6 * B + 1, dtype=torch.int32, device=dev)
         self.meta_host = torch.zeros(6 * B + 1, dtype=torch.int32).pin_memory()
-        m = self.meta
-        self.tokens, self.row_pos, self.row_seq = m[0:B], m[B:2 * B], m[2 * B:3 * B]
-        self.seq_slot, self.seq_first_row, self.seq_len = m[3 * B:4 * B], m[4 * B:5 * B + 1], m[5 * B + 1:6 * B + 1]
+        self.batch = b = one_token_batch(self.meta, B, max_len)
+        self.tokens, self.row_pos, self.row_seq = b.tokens, b.row_pos, b.row_seq
+        self.seq_slot, self.seq_first_row, self.seq_len = b.seq_slot, b.seq_first_row, b.seq_len
         self.params = torch.zeros(B, 4, dtype=torch.float32, device=dev)
         self.chosen = torch.zeros(B, dtype=torch.int32, device=dev)
-        # What a recorded step may know on the host is what every replay shares: the number of sequences and their
-        # rows (one each).  Slots, positions and lengths change from replay to replay and exist on the device only
-        # (``host_seq_slot`` / ``host_seq_len`` stay None; ``max_len`` is the graph's bound, 0 = unknown).
-        self.batch = StepBatch(prefill=False, n_rows=B, n_seqs=B, n_want=B, max_len=max_len, want_all_in_order=True,
-                               tokens=self.tokens, row_pos=self.row_pos, row_seq=self.row_seq,
-                               seq_slot=self.seq_slot, seq_first_row=self.seq_first_row, seq_len=self.seq_len,
-                               want_rows=self.row_seq, max_rows=1, host_seq_first_row=np.arange(B + 1, dtype=np.int32))
         self.graph = None
         self.slots: List[int] = []
 
     def load(self, slots: Sequence[int], tokens: Sequence[int], lengths: Sequence[int], params: np.ndarray) -> None:
         """Inputs of the next step: sequence i sits in slots[i], holds lengths[i] positions and brings tokens[i]."""
-        B = self.B
-        h = self.meta_host.numpy()
-        h[0:B] = tokens
-        h[B:2 * B] = lengths                       # the new token's position
-        h[2 * B:3 * B] = np.arange(B)
-        h[3 * B:4 * B] = slots
-        h[4 * B:5 * B + 1] = np.arange(B + 1)
-        h[5 * B + 1:6 * B + 1] = np.asarray(lengths) + 1
+        fill_meta(self.meta_host.numpy(), slots, tokens, lengths)
         self.meta.copy_(self.meta_host, non_blocking=True)
         self.params.copy_(torch.from_numpy(params), non_blocking=False)
         self.slots = list(slots)
@@ -167,3 +175,44 @@ class PromptGraph:
             return out
         self.graph.replay()
         return self.logits
+
+
+MAX_STEP_GRAPHS = 16      # recorded one-token steps kept (by sequences, context class and stream); the one used longest ago gives way
+STEP_GRAPH_ROWS = 64      # most sequences of a recorded one-token step
+
+
+class StepGraph:
+    """``Model.step`` for sequences that bring one token each, all logits wanted, recorded: what a caller that feeds tokens
+    itself runs again and again.  Issued launch by launch, such a step waits for the host (about 100 us a layer: 2.75 ms at the
+    24 layers of the 0.5B shape, where the device works 0.5; 3.4 against 1.2 at 1.5B).  A shape's first step is issued as it is,
+    its second is recorded as well, from the third on the recording is replayed; every call gets logits of its own."""
+
+    def __init__(self, model, n_seqs: int, max_len: int):
+        self.model, self.n_seqs = model, n_seqs
+        self.meta = torch.zeros(6 * n_seqs + 1, dtype=torch.int32, device=model.rt.device)
+        self.batch = one_token_batch(self.meta, n_seqs, max_len)
+        self.graph = None
+        self.logits = None
+        self.uses = 0
+
+    def run(self, slots: Sequence[int], tokens: Sequence[int], lengths: Sequence[int]) -> torch.Tensor:
+        """Float32 logits [sequences, vocab].  The caller has reserved the new position of every slot and commits it."""
+        host = torch.empty(6 * self.n_seqs + 1, dtype=torch.int32, pin_memory=True)      # its own each time: the copy may still be under way
+        fill_meta(host.numpy(), slots, tokens, lengths)
+        self.meta.copy_(host, non_blocking=True)
+        if self.graph is not None:
+            self.graph.replay()
+            return self.logits.clone()
+        self.uses += 1
+        out = self.model.forward(self.batch)
+        if self.uses >= 2:
+            g, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                g.capture_begin(capture_error_mode="thread_local")
+                try:
+                    self.logits = self.model.forward(self.batch)      # recorded, not run
+                finally:
+                    g.capture_end()
+            self.graph = g
+        return out

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import dataclasses
 import sys
+from collections import OrderedDict
 from typing import Dict, List, Optional, Sequence
 
 import torch
@@ -72,6 +73,8 @@ class Model:
                 raise ValueError(f"layer {i}: a token input goes with a block of kind 'prenorm' and the model's own side table")
         self.config = None                                  # set by load_model
         self.step_rows = STEP_ROWS                          # a step of more rows runs in parts
+        self.record_steps = False                           # record one-token steps (``StepGraph``); an ``LM`` with graphs says so
+        self._step_graphs = OrderedDict()                   # (sequences, context bound, stream) -> StepGraph, the newest last
         self.embedding: Optional[torch.Tensor] = None
         self.bigram: Optional[torch.Tensor] = None          # the hashed bigram table, where the spec has one
         self.positions: Optional[torch.Tensor] = None       # the vectors added at each position, where the spec has a table
@@ -109,6 +112,7 @@ class Model:
         """``tensors``: name -> tensor, a dict or a ``TensorSource`` that fetches each tensor when it is asked for
         (every name of the plan is asked for once)."""
         s = self.spec
+        self._step_graphs.clear()
         table = tensors[s.embed_name]
         self.embedding = self.rt.matrix(table)
         if s.tie_head:
@@ -185,6 +189,7 @@ class Model:
         sched = self.spec.schedule
         shares = {site: self.spec.layers[layer].mixer.cache_from for site, layer in enumerate(sched)
                   if self.spec.layers[layer].mixer.cache_from is not None}
+        self._step_graphs.clear()                           # recorded with the cache before
         self.cache = KVCache(self._cache_requests(),
                              max_tokens, self.spec.max_position,
                              self.rt.dtype, self.rt.device, page_size=page_size, max_seqs=max_seqs,
@@ -238,6 +243,8 @@ class Model:
         limit = cache.most_tokens_going_on()
         if limit is not None and any(starts) and max(len(e.tokens) for e in entries) > limit:
             return self._step_in_rounds(entries, limit)
+        if self._recordable(entries):
+            return self._step_recorded(entries, starts)
         batch = build_batch(entries, starts, self.spec.vocab, self.rt.device)
         for e, s in zip(entries, starts):
             cache.reserve(e.slot, s + len(e.tokens))
@@ -245,6 +252,35 @@ class Model:
         logits = self.forward(batch)
         for e, s in zip(entries, starts):
             cache.commit(e.slot, s + len(e.tokens))
+        return logits
+
+    def _recordable(self, entries: Sequence[StepEntry]) -> bool:
+        """Whether the step runs through a ``StepGraph``: one token a sequence, every sequence's logits wanted, parts that may
+        be recorded, and nobody else recording or profiling."""
+        from .graph import STEP_GRAPH_ROWS
+        return (self.record_steps and len(entries) <= STEP_GRAPH_ROWS and all(len(e.tokens) == 1 and list(e.want) == [0] for e in entries)
+                and self.graph_safe and torch.device(self.rt.device).type == "cuda" and getattr(self.rt.kernels, "profile", None) is None
+                and not torch.cuda.is_current_stream_capturing())
+
+    def _step_recorded(self, entries: Sequence[StepEntry], starts: Sequence[int]) -> torch.Tensor:
+        from .graph import MAX_STEP_GRAPHS, StepGraph
+        check_entries(entries, self.spec.vocab)
+        cache, short = self.cache, self.short_context
+        for e, s in zip(entries, starts):
+            cache.reserve(e.slot, s + 1)
+        cache.flush()
+        # a stream's steps follow one another; another stream's have buffers of their own
+        key = (len(entries), short if max(starts) + 1 <= short else 0, torch.cuda.current_stream().cuda_stream)
+        g = self._step_graphs.get(key)
+        if g is None:
+            g = self._step_graphs[key] = StepGraph(self, key[0], key[1])
+            while len(self._step_graphs) > MAX_STEP_GRAPHS:
+                torch.cuda.synchronize()                    # the one that goes may still be running
+                self._step_graphs.popitem(last=False)
+        self._step_graphs.move_to_end(key)
+        logits = g.run([e.slot for e in entries], [int(e.tokens[0]) for e in entries], starts)
+        for e, s in zip(entries, starts):
+            cache.commit(e.slot, s + 1)
         return logits
 
     def _step_in_parts(self, entries: Sequence[StepEntry]) -> torch.Tensor:

@@ -573,3 +573,50 @@ def test_cima_bench_reports_a_decode_rate():
     line = json.loads(p.stdout.strip().split("\n")[-1])
     assert line["batch"] == 2 and line["gen_tokens"] == 12 and line["prompt_tokens"] == 9
     assert line["decode_tok_per_s_p50"] >= line["decode_tok_per_s_min"] > 0 and line["ttft_ms"] > 0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("name", ["tiny-b", "gisirax-tiny", "vunovik-tiny", "netezen-tiny"])
+def test_one_token_steps_recorded_give_what_issued_ones_give(name, dtype):
+    """``LM.step`` with a token a sequence: issued, recorded and replayed, over changing sets of sequences, a batch of another size in
+    between and a second stream, against a model that records nothing; logits handed out stay what they were, a refused token
+    leaves the sequences as they are, and a step that wants no logits is issued as before."""
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    kw = dict(config=SHAPES[name], seed=3, dtype=dtype, max_tokens=2048, max_seqs=8, verbose=False)
+    rec, ref = cima_b200.load(**kw), cima_b200.load(use_graphs=False, **kw)
+    assert rec.model.record_steps and not ref.model.record_steps
+    vocab = rec.spec.vocab
+    g = torch.Generator().manual_seed(5)
+    draw = lambda n: torch.randint(0, vocab, (n,), generator=g).tolist()
+    prompts = [draw(n) for n in (5, 70, 1)]
+    slots = [lm.model.cache.open(3) for lm in (rec, ref)]
+    for lm, s in zip((rec, ref), slots):
+        lm.step([StepEntry(a, p, [len(p) - 1]) for a, p in zip(s, prompts)])
+    kept = []
+
+    def both(ids, stream=None):
+        toks = draw(len(ids))
+        want = ref.step([StepEntry(slots[1][i], [t], [0]) for i, t in zip(ids, toks)])
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream or torch.cuda.current_stream()):
+            got = rec.step([StepEntry(slots[0][i], [t], [0]) for i, t in zip(ids, toks)])
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) if dtype == "float32" else (got - want).abs().max() <= 2e-2 * want.std()
+        kept.append((got, got.clone()))
+
+    side = torch.cuda.Stream()
+    for ids in ([0, 1, 2], [2, 0, 1], [1], [1, 2, 0], [0, 2], [1], [2], [0, 1, 2]):
+        both(ids)
+    for _ in range(3):
+        both([0, 1, 2], side)
+    both([2, 1, 0])
+    assert any(x.graph is not None for x in rec.model._step_graphs.values()) == rec.model.graph_safe and not ref.model._step_graphs
+    assert all(torch.equal(a, b) for a, b in kept)
+    before = [rec.model.cache.length(s) for s in slots[0]]
+    with pytest.raises(ValueError, match="token ids"):
+        rec.step([StepEntry(s, [vocab], [0]) for s in slots[0]])
+    assert [rec.model.cache.length(s) for s in slots[0]] == before
+    assert rec.step([StepEntry(slots[0][0], [1], [])]).shape[0] == 0
+    ref.step([StepEntry(slots[1][0], [1], [])])
+    both([0, 1, 2])
