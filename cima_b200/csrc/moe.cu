@@ -20,8 +20,8 @@
 //   many pairs, bfloat16   moe_sort_tiles lays every expert's pairs out from a multiple of 256 rows on and names each row
 //                          tile's expert; moe_gather_rows copies the rows of h to their places; the two products run on
 //                          the tcgen05 kernel (gemm_tcgen05_pair_grouped); moe_combine reads y through the pairs' places
-//   few pairs, bfloat16    moe_few: a warp computes one output feature for up to 8 pairs of an expert, streaming the
-//                          feature's weights with 16-byte loads (a decode step reads every touched expert once)
+//   few pairs, bfloat16    moe_few: a block computes 16 output features for up to 8 pairs of an expert at a time, its warps
+//                          streaming a range of k each with 16-byte loads (a decode step reads every touched expert once)
 #include "common.cuh"
 
 namespace {
@@ -507,112 +507,121 @@ k_moe_gather_rows(const uint4* __restrict__ src, const int* __restrict__ pos, ui
   for (int v = threadIdx.x; v < vecs; v += blockDim.x) d[v] = s[v];
 }
 
-// Few pairs (a decode step).  Block (x = tile of 32 pairs of one expert as moe_sort laid them out, y = 8 or 16 output
-// features): warp w owns feature n0 + w (and n0 + w + 8); its lanes stride the features' weights by 16 bytes and hold the sums
-// of up to 8 pairs at a time; a fixed shuffle tree adds the lanes.  MODE as in k_moe_gemm.
-constexpr int FEW_PAIRS = 8;
-constexpr int FEW_ROWS = 2;          // rows of weights a warp streams at once (4 measured the same: 0.663 against 0.659 ms a step)
+// Few pairs (a decode step): bound by the touched experts' weights.  Block (x = tile of 32 pairs of one expert as moe_sort laid
+// them out, y = 16 output features): the weights are the 16-row operand of mma.m16n8k16, up to 8 pairs its columns.  The sum
+// over k is shared by the block's 8 warps, a range each, whose sums are added in their order, so that a down product (few
+// features, a long sum) has work for every SM in more than one wave.  The order of k inside a product is free as long as both
+// operands follow it: lane (g, t) loads 16 neighbouring bytes of weight rows g and g + 8 and of pair g, 8 t values into each 32,
+// and uses them as its parts of two k-steps.  FEW_AHEAD such pieces are requested before the first is used.  MODE as in k_moe_gemm.
+// (A warp a feature with multiply-adds stood at 4.2 TB/s in the down product of 16 experts of 1,536 x 4,480 and 8 rows, 52.8 us: its
+// 1,536 blocks are 1.3 waves, and each began with a chain of dependent look-ups of its expert.)
+constexpr int FEW_PAIRS = 8, FEW_FEATURES = 16, FEW_WARPS = 8;
+__device__ __forceinline__ void few_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// 16 bytes, or zeros; volatile, so that a piece's requests stay in front of the products they are requested for
+__device__ __forceinline__ uint4 few_load(const void* p, bool ok) {
+  uint4 v;
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %5, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\nmov.b32 %2, 0;\nmov.b32 %3, 0;\n@p ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n}\n"
+               : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)ok));
+  return v;
+}
 template <int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * FEW_WARPS)
 k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
           const int* __restrict__ offsets, const int* __restrict__ tiles, const int* __restrict__ perm, int E, int top, int N,
           int K, int act, float limit, const float* __restrict__ weigh) {
+  constexpr int MT = MODE == 0 ? 2 : 1;                 // operand tiles of a block: gate and up
+  constexpr int AHEAD = MODE == 0 ? 2 : 4;
   cima_pdl_wait();
-  __shared__ int s_row[BM];
-  __shared__ int s_e, s_i0, s_n;
-  if (threadIdx.x == 0) {
-    const int tile = blockIdx.x;
-    int e = -1;
-    if (tile < tiles[E]) {
-      int lo = 0, hi = E - 1;
-      while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (tiles[mid] <= tile) lo = mid; else hi = mid - 1; }
-      e = lo;
-      while (tiles[e + 1] <= tile) e++;
-      s_i0 = offsets[e] + (tile - tiles[e]) * BM;
-      s_n = min(BM, offsets[e + 1] - s_i0);
+  __shared__ int s_row[BM], s_pair[BM], s_e, s_i0, s_n;
+  __shared__ float s_w[BM];
+  __shared__ float red[FEW_WARPS][MT * FEW_FEATURES][FEW_PAIRS + 1];
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
+  if (tid == 0) s_e = -1;
+  __syncthreads();
+  for (int e = tid; e < E; e += 32 * FEW_WARPS) {       // the expert whose row tiles hold this one
+    const int t0 = tiles[e], t1 = tiles[e + 1], o0 = offsets[e], o1 = offsets[e + 1];
+    if (t0 <= tile && tile < t1) {
+      s_e = e;
+      s_i0 = o0 + (tile - t0) * BM;
+      s_n = min(BM, o1 - s_i0);
     }
-    s_e = e;
   }
   __syncthreads();
   const int e = s_e;
   if (e < 0) return;
-  const int i0 = s_i0, nrows = s_n;
-  const int tid = (int)threadIdx.x;
-  __shared__ float s_w[BM];
-  if (tid < BM) {
-    s_row[tid] = tid < nrows ? (MODE != 1 ? perm[i0 + tid] / top : i0 + tid) : -1;
-    s_w[tid] = MODE != 1 && weigh && tid < nrows ? weigh[perm[i0 + tid]] : 1.0f;
+  const int i0 = s_i0, nrows = s_n, n0 = blockIdx.y * FEW_FEATURES;
+  if (tid < nrows) {
+    const int pair = perm[i0 + tid];
+    s_pair[tid] = pair;
+    s_row[tid] = MODE != 1 ? pair / top : i0 + tid;
+    s_w[tid] = MODE != 1 && weigh ? weigh[pair] : 1.0f;
   }
+  const int g = lane >> 2, t = lane & 3;
+  const __nv_bfloat16* w[MT][2];
+#pragma unroll
+  for (int m = 0; m < MT; m++)
+#pragma unroll
+    for (int x = 0; x < 2; x++) w[m][x] = W + ((size_t)e * (MT * N) + (size_t)m * N + min(n0 + g + 8 * x, N - 1)) * K + 8 * t;
+  const int pieces = (K + 31) / 32, share = (pieces + FEW_WARPS - 1) / FEW_WARPS;
+  const int beg = min(pieces, warp * share), end = min(pieces, beg + share);
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // A warp streams FEW_ROWS rows of weights at once, so that enough loads are in flight: a feature's gate and up rows
-  // (MODE 0) or the rows of features n and n + 8 (MODE 1); with four, two and four features.  With one row a warp the down
-  // product stood at 0.4 of the bandwidth (a decode step of the 1.5B shape at batch 8 took 0.72 ms, with two 0.66 ms).
-  constexpr int FEATS = MODE == 0 ? FEW_ROWS / 2 : FEW_ROWS;          // features a warp computes
-  const int n = blockIdx.y * (8 * FEATS) + warp;
-  if (n >= N) return;
-  const __nv_bfloat16* wrow[FEW_ROWS];
-  bool valid[FEATS];
-#pragma unroll
-  for (int f = 0; f < FEATS; f++) {
-    valid[f] = n + 8 * f < N;
-    const int nf = valid[f] ? n + 8 * f : n;
-    if (MODE == 0) {
-      wrow[2 * f] = W + ((size_t)e * 2 * N + nf) * K;
-      wrow[2 * f + 1] = wrow[2 * f] + (size_t)N * K;
-    } else {
-      wrow[f] = W + ((size_t)e * N + nf) * K;
-    }
-  }
   for (int r0 = 0; r0 < nrows; r0 += FEW_PAIRS) {
-    float acc[FEW_ROWS][FEW_PAIRS];
+    const __nv_bfloat16* a = A + (size_t)s_row[min(r0 + g, nrows - 1)] * lda + 8 * t;      // (a column without a pair is not read below)
+    float acc[MT][4];
 #pragma unroll
-    for (int j = 0; j < FEW_ROWS; j++)
+    for (int m = 0; m < MT; m++)
 #pragma unroll
-      for (int r = 0; r < FEW_PAIRS; r++) acc[j][r] = 0.f;
-    for (int k = lane * 8; k < K; k += 256) {
-      uint4 w4[FEW_ROWS];
+      for (int x = 0; x < 4; x++) acc[m][x] = 0.f;
+#pragma unroll 1
+    for (int p0 = beg; p0 < end; p0 += AHEAD) {
+      uint4 wv[AHEAD][MT][2], av[AHEAD];
 #pragma unroll
-      for (int j = 0; j < FEW_ROWS; j++) w4[j] = *reinterpret_cast<const uint4*>(wrow[j] + k);
+      for (int u = 0; u < AHEAD; u++) {
+        const int k = 32 * (p0 + u);
+        const bool ok = p0 + u < end && k + 8 * t < K;
 #pragma unroll
-      for (int r = 0; r < FEW_PAIRS; r++) {
-        if (r0 + r >= nrows) break;
-        const uint4 a4 = *reinterpret_cast<const uint4*>(A + (size_t)s_row[r0 + r] * lda + k);
-        const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&a4);
+        for (int m = 0; m < MT; m++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const float2 av = __bfloat1622float2(ap[q]);
-#pragma unroll
-          for (int j = 0; j < FEW_ROWS; j++) {
-            const float2 wv = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&w4[j])[q]);
-            acc[j][r] = fmaf(av.x, wv.x, acc[j][r]);
-            acc[j][r] = fmaf(av.y, wv.y, acc[j][r]);
-          }
-        }
+          for (int x = 0; x < 2; x++) wv[u][m][x] = few_load(w[m][x] + k, ok);
+        av[u] = few_load(a + k, ok);
       }
+#pragma unroll
+      for (int u = 0; u < AHEAD; u++)
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+          few_mma(acc[m], wv[u][m][0].x, wv[u][m][1].x, wv[u][m][0].y, wv[u][m][1].y, av[u].x, av[u].y);
+          few_mma(acc[m], wv[u][m][0].z, wv[u][m][1].z, wv[u][m][0].w, wv[u][m][1].w, av[u].z, av[u].w);
+        }
     }
 #pragma unroll
-    for (int r = 0; r < FEW_PAIRS; r++) {
+    for (int m = 0; m < MT; m++)
 #pragma unroll
-      for (int j = 0; j < FEW_ROWS; j++)
-        for (int o = 16; o > 0; o >>= 1) acc[j][r] += __shfl_xor_sync(0xffffffffu, acc[j][r], o);
-      if (lane == 0 && r0 + r < nrows) {
+      for (int x = 0; x < 4; x++) red[warp][m * FEW_FEATURES + g + 8 * (x >> 1)][2 * t + (x & 1)] = acc[m][x];
+    __syncthreads();
+    const int f = tid / FEW_PAIRS, r = tid % FEW_PAIRS, n = n0 + f;
+    if (f < FEW_FEATURES && n < N && r0 + r < nrows) {
+      float v[MT];
 #pragma unroll
-        for (int f = 0; f < FEATS; f++) {
-          if (!valid[f]) continue;
-          if (MODE == 2) {
-            const float z = __bfloat162float(__float2bfloat16_rn(acc[f][r] * s_w[r0 + r]));
-            reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(i0 + r0 + r) * N + n + 8 * f] = __float2bfloat16_rn(cima_ungated_act(z, act));
-          } else if (MODE == 0) {
-            // gate and up are rounded to bfloat16 before the activation, as stored projections would be
-            const float gt = __bfloat162float(__float2bfloat16_rn(acc[2 * f][r] * s_w[r0 + r])), uv = __bfloat162float(__float2bfloat16_rn(acc[2 * f + 1][r] * s_w[r0 + r]));
-            reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(i0 + r0 + r) * N + n + 8 * f] = __float2bfloat16_rn(cima_gated(gt, uv, act, limit));
-          } else {
-            reinterpret_cast<float*>(out)[(size_t)perm[i0 + r0 + r] * N + n + 8 * f] = acc[f][r];
-          }
-        }
+      for (int m = 0; m < MT; m++) {
+        v[m] = red[0][m * FEW_FEATURES + f][r];
+#pragma unroll
+        for (int x = 1; x < FEW_WARPS; x++) v[m] += red[x][m * FEW_FEATURES + f][r];
+      }
+      if (MODE == 2) {
+        const float z = __bfloat162float(__float2bfloat16_rn(v[0] * s_w[r0 + r]));
+        reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(i0 + r0 + r) * N + n] = __float2bfloat16_rn(cima_ungated_act(z, act));
+      } else if (MODE == 0) {
+        // gate and up are rounded to bfloat16 before the activation, as stored projections would be
+        const float gt = __bfloat162float(__float2bfloat16_rn(v[0] * s_w[r0 + r])), uv = __bfloat162float(__float2bfloat16_rn(v[MT - 1] * s_w[r0 + r]));
+        reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(i0 + r0 + r) * N + n] = __float2bfloat16_rn(cima_gated(gt, uv, act, limit));
+      } else {
+        reinterpret_cast<float*>(out)[(size_t)s_pair[r0 + r] * N + n] = v[0];
       }
     }
+    __syncthreads();
   }
 }
 }  // namespace
@@ -718,8 +727,7 @@ extern "C" int cima_moe_few(const void* a, int lda, const void* w, void* out, co
     return cima_fail(CIMA_E_SIZE, "moe_few: K %d and the row stride %d must be multiples of 8 and the operands 16-byte aligned", K, lda);
   if (mode < 0 || mode > 2) return cima_fail(CIMA_E_ARG, "moe_few: mode %d is none of 0 (gate | up), 1 (down), 2 (up without gates)", mode);
   if (mode == 2 ? !cima_ungated_known(act) : (act < 0 || act >= CIMA_GATED_COUNT)) return cima_fail(CIMA_E_ARG, "moe_few: activation code %d is unknown", act);
-  const int per_block = 8 * (mode == 0 ? FEW_ROWS / 2 : FEW_ROWS);          // features of a block: its 8 warps' 
-  const dim3 grid((unsigned)((P + BM - 1) / BM + E), (unsigned)((N + per_block - 1) / per_block));
+  const dim3 grid((unsigned)((P + BM - 1) / BM + E), (unsigned)((N + FEW_FEATURES - 1) / FEW_FEATURES));
   if (grid.y > 65535) return cima_fail(CIMA_E_SIZE, "moe_few: %d outputs exceed one launch", N);
   int rc;
   if (mode == 0) rc = cima_launch(k_moe_few<0>, grid, dim3(256), (size_t)0, stream, 1, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, out, offsets, tiles, perm, E, top, N, K, act, limit, weigh);
