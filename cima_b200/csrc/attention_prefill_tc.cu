@@ -26,6 +26,10 @@
 // Every wait on an mbarrier is bounded (2 s); a wait that runs out sets *error_flag, and all roles leave their
 // loops, free the tensor memory and return.
 //
+// With a window, `keep_first` positions stay visible below it: the tiles that hold them and lie below the window's are visited
+// first, under the mask.  `v_group` neighbouring key heads share one value head.  (A layer of differential attention of the
+// 3B Lipizen shape, 2,048 tokens: 46 us; 109 on the mma.sync kernel, which took these two before.)
+//
 // The reference's prefill attention is k_attn_prefill_tiled (src/kernels.cu:659-753): one warp per query row,
 // online softmax on CUDA cores; it has no tensor-core attention.
 #include "tcgen05.cuh"
@@ -65,6 +69,8 @@ struct AttnArgs {
   const __nv_bfloat16* gate;    // or null: the rows' own gates, gate[row * ld_gate + h * HD + d]; the result leaves times their sigmoid
   int ld_gate;
   const float* slopes;          // or null: [nh], slopes[h] * (distance from the query back to the key) is taken off the scaled score
+  int keep_first;               // with a window: so many of a sequence's first positions stay visible below it
+  int v_group;                  // so many neighbouring key heads share one value head
 };
 
 // Keys of a query block whose rows stand at positions p0 .. (at most p0 + 127, below len): tiles [first, last] of 64.
@@ -110,7 +116,9 @@ k_attention_prefill_tc(const __grid_constant__ CUtensorMap map_qkv, const __grid
   const int slot = FROM_CACHE ? a.seq_slot[seq] : 0;
   int first, last;
   key_tiles(q0, len, a.window, first, last);
-  const int n = last - first + 1;
+  const int nkeep = min((a.keep_first + BN - 1) / BN, first);      // tiles of kept first positions that lie below the window's
+  const int n = nkeep + last - first + 1, vh = kvh / a.v_group;
+  auto tile_of = [&](int j) { return j < nkeep ? j : first + j - nkeep; };
 
   if (threadIdx.x == 0 && (smem_u32(smem) & 1023u)) atomicExch(a.error_flag, 2);   // never seen; the tiles would be misread
   if (threadIdx.x == 0) {
@@ -148,22 +156,22 @@ k_attention_prefill_tc(const __grid_constant__ CUtensorMap map_qkv, const __grid
 #pragma unroll
       for (int kb = 0; kb < NH; kb++) tma_load_2d(sq + (size_t)kb * HALF_BYTES, &map_qkv, h * HD + 64 * kb, row_base + r0, q_full);
       for (int j = 0; j < n; j++) {
-        const int s = j & 1, k0 = (first + j) * BN;
+        const int s = j & 1, kt = tile_of(j), k0 = kt * BN;
         if (j >= 2 && !mbar_wait(&k_empty[s], ((j >> 1) - 1) & 1, a.error_flag, abort_flag)) break;
         mbar_expect_tx(&k_full[s], NH * KHALF_BYTES);
         // from the cache, map_k covers the layer's pages as rows of head_dim values: page, k or v, kv head, position
-        const int x = FROM_CACHE ? 0 : (a.nh + kvh) * HD, y = FROM_CACHE ? (page_of(first + j) * a.planes * a.nkv + kvh) * BN : row_base + k0;
+        const int x = FROM_CACHE ? 0 : (a.nh + kvh) * HD, y = FROM_CACHE ? (page_of(kt) * a.planes * a.nkv + kvh) * BN : row_base + k0;
 #pragma unroll
         for (int kb = 0; kb < NH; kb++)
           tma_load_2d(sk + (size_t)(NH * s + kb) * KHALF_BYTES, &map_k, x + 64 * kb, y, &k_full[s]);
       }
     } else if (lane == 1) {
       for (int j = 0; j < n; j++) {
-        const int s = j & 1, k0 = (first + j) * BN;
+        const int s = j & 1, kt = tile_of(j), k0 = kt * BN;
         if (j >= 2 && !mbar_wait(&v_empty[s], ((j >> 1) - 1) & 1, a.error_flag, abort_flag)) break;
         mbar_expect_tx(&v_full[s], V_BYTES);
-        const int x = FROM_CACHE ? 0 : (a.nh + a.nkv + kvh) * HD;
-        const int y = FROM_CACHE ? ((page_of(first + j) * a.planes + (a.planes - 1)) * a.nkv + kvh) * BN : row_base + k0;
+        const int x = FROM_CACHE ? 0 : (a.nh + a.nkv + vh) * HD;
+        const int y = FROM_CACHE ? ((page_of(kt) * a.planes + (a.planes - 1)) * a.nkv + vh) * BN : row_base + k0;
 #pragma unroll
         for (int kb = 0; kb < NH; kb++)
           tma_load_2d(sv + (size_t)s * V_BYTES + (size_t)kb * KHALF_BYTES, &map_k, x + 64 * kb, y, &v_full[s]);
@@ -227,7 +235,7 @@ k_attention_prefill_tc(const __grid_constant__ CUtensorMap map_qkv, const __grid
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < n && ok; j++) {
-      const int s = j & 1, k0 = (first + j) * BN;
+      const int s = j & 1, k0 = tile_of(j) * BN;
       ok = mbar_wait(&s_full[s], (j >> 1) & 1, a.error_flag, abort_flag);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -257,7 +265,7 @@ k_attention_prefill_tc(const __grid_constant__ CUtensorMap map_qkv, const __grid
 #pragma unroll
           for (int e = 0; e < 32; e++) {
             const int key = k0 + c * 32 + e;
-            if (key > key_hi || key < key_lo) raw[c][e] = 0xff800000u;            // -inf
+            if (key > key_hi || (key < key_lo && key >= a.keep_first)) raw[c][e] = 0xff800000u;            // -inf
             mx4[e & 3] = fmaxf(mx4[e & 3], __uint_as_float(raw[c][e]));
           }
       } else {
@@ -382,14 +390,16 @@ struct CacheSource {              // keys and values from a layer's pages; cache
 template <int HD, bool FROM_CACHE>
 int launch_attention_tc(const void* qkv, int ld, const int* tile_seq, const int* tile_row0, const int* seq_first_row,
                         const CacheSource& c, void* out, int ldo, int T, int n_tiles, int nh, int nkv, float scale,
-                        int window, int* error_flag, float sink, const float* head_sink, int gate_col, const float* slopes, cudaStream_t stream) {
+                        int window, int* error_flag, float sink, const float* head_sink, int gate_col, const float* slopes, int keep_first, int v_group,
+                        cudaStream_t stream) {
   if ((long long)n_tiles * nh > 0x7fffffffll) return cima_fail(CIMA_E_SIZE, "attention_prefill_tc: %d blocks of rows x %d heads exceed one launch", n_tiles, nh);
   CUtensorMap mq, mk;                                  // boxes of 128 rows (Q) and of 64 rows (K and V) by 64 columns
   // (with the keys in the cache only the queries' columns of a row are read, and the row may end there)
-  int rc = make_map(&mq, qkv, T, FROM_CACHE ? (long long)nh * HD : (long long)(nh + 2 * nkv) * HD, ld);
+  const long long cols = FROM_CACHE ? (long long)nh * HD : (long long)(nh + nkv + nkv / v_group) * HD;
+  int rc = make_map(&mq, qkv, T, cols, ld);
   if (rc) return rc;
   if (FROM_CACHE) rc = make_map(&mk, c.cache, c.n_pages * c.planes * nkv * BN, HD, HD, BN);
-  else rc = make_map(&mk, qkv, T, (long long)(nh + 2 * nkv) * HD, ld, BN);
+  else rc = make_map(&mk, qkv, T, cols, ld, BN);
   if (rc) return rc;
   constexpr int NH = HD / 64;
   const size_t smem = NH * (size_t)HALF_BYTES + 2 * NH * (size_t)KHALF_BYTES + 2 * (size_t)HD * 128 + 14 * 8 + 16;
@@ -401,7 +411,7 @@ int launch_attention_tc(const void* qkv, int ld, const int* tile_seq, const int*
     raised = true;
   }
   AttnArgs a{tile_seq, tile_row0, seq_first_row, c.seq_len, c.seq_slot, c.table, c.table_width, c.ring,
-             (__nv_bfloat16*)out, ldo, nh, nkv, window, scale, error_flag, c.planes, sink, head_sink, gate_col > 0 ? (const __nv_bfloat16*)qkv + gate_col : nullptr, ld, slopes};
+             (__nv_bfloat16*)out, ldo, nh, nkv, window, scale, error_flag, c.planes, sink, head_sink, gate_col > 0 ? (const __nv_bfloat16*)qkv + gate_col : nullptr, ld, slopes, keep_first, v_group};
   { int rc_ = cima_launch(k_attention_prefill_tc<HD, FROM_CACHE>, dim3((unsigned)n_tiles * (unsigned)nh), dim3(THREADS), smem, stream, 1, mq, mk, a); if (rc_) return rc_; }
   return cima_launch_result();
 }
@@ -409,12 +419,13 @@ int launch_attention_tc(const void* qkv, int ld, const int* tile_seq, const int*
 }  // namespace
 
 static int tc_checks(const char* who, const void* qkv, int ld, const void* out, int ldo, int nh, int nkv, int hd, const int* error_flag,
-                     int gate_col, bool queries_only = false) {
+                     int gate_col, int keep_first, int v_group, bool queries_only = false) {
+  if (keep_first < 0 || v_group < 1 || nkv <= 0 || nkv % v_group) return cima_fail(CIMA_E_ARG, "%s: keep_first %d must not be negative and %d kv heads be a multiple of v_group %d", who, keep_first, nkv, v_group);
   if (hd != 64 && hd != 128) return cima_fail(CIMA_E_SIZE, "%s: head_dim %d; this kernel takes 64 or 128", who, hd);
   if (nh <= 0 || nkv <= 0 || nh % nkv) return cima_fail(CIMA_E_SIZE, "%s: %d heads are not a multiple of %d kv heads", who, nh, nkv);
   if (gate_col < 0 || gate_col % 8 || (gate_col > 0 && gate_col + nh * hd > ld)) return cima_fail(CIMA_E_ARG, "%s: %d gate values from column %d (a multiple of 8) on exceed the rows of %d", who, nh * hd, gate_col, ld);
   if (ld % 8 || ldo % 8) return cima_fail(CIMA_E_SIZE, "%s: row strides (%d, %d) must be multiples of 8", who, ld, ldo);
-  if (ld < (queries_only ? nh : nh + 2 * nkv) * hd) return cima_fail(CIMA_E_SIZE, "%s: row stride %d is smaller than the heads of a row", who, ld);
+  if (ld < (queries_only ? nh : nh + nkv + nkv / v_group) * hd) return cima_fail(CIMA_E_SIZE, "%s: row stride %d is smaller than the heads of a row", who, ld);
   if ((((uintptr_t)qkv | (uintptr_t)out) & 15)) return cima_fail(CIMA_E_ARG, "%s: qkv and out must be 16-byte aligned", who);
   if (!error_flag) return cima_fail(CIMA_E_ARG, "%s: an error flag on the device is needed", who);
   if (nh > 65535 || nkv > 65535) return cima_fail(CIMA_E_SIZE, "%s: %d heads exceed one launch", who, nh);
@@ -427,13 +438,13 @@ static int tc_checks(const char* who, const void* qkv, int ld, const void* out, 
 extern "C" int cima_attention_prefill_tc(const void* qkv, int ld, const int* tile_seq, const int* tile_row0,
                                          const int* seq_first_row, void* out, int ldo, int T, int n_tiles, int nh,
                                          int nkv, int hd, float scale, int window, int* error_flag, float sink, const float* head_sink,
-                                         int gate_col, const float* slopes, cudaStream_t stream) {
+                                         int gate_col, const float* slopes, int keep_first, int v_group, cudaStream_t stream) {
   if (T <= 0 || n_tiles <= 0) return 0;
-  if (int rc = tc_checks("attention_prefill_tc", qkv, ld, out, ldo, nh, nkv, hd, error_flag, gate_col)) return rc;
+  if (int rc = tc_checks("attention_prefill_tc", qkv, ld, out, ldo, nh, nkv, hd, error_flag, gate_col, keep_first, v_group)) return rc;
   const CacheSource none{nullptr, 0, nullptr, nullptr, nullptr, 0, 0};
   if (hd == 64)
-    return launch_attention_tc<64, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, none, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, stream);
-  return launch_attention_tc<128, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, none, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, stream);
+    return launch_attention_tc<64, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, none, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
+  return launch_attention_tc<128, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, none, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
 }
 
 // The same for sequences that go on: the rows of sequence s are the positions seq_len[s] - rows .. seq_len[s] - 1, and
@@ -443,16 +454,16 @@ extern "C" int cima_attention_extend_tc(const void* qkv, int ld, const int* tile
                                         int table_width, int ring, int page_size, const int* seq_slot, const int* seq_len,
                                         void* out, int ldo, int T, int n_tiles, int nh, int nkv, int hd, float scale,
                                         int window, int* error_flag, int planes, float sink, const float* head_sink,
-                                        int gate_col, const float* slopes, cudaStream_t stream) {
+                                        int gate_col, const float* slopes, int keep_first, int v_group, cudaStream_t stream) {
   if (T <= 0 || n_tiles <= 0) return 0;
   if (planes != 1 && planes != 2) return cima_fail(CIMA_E_ARG, "attention_extend_tc: %d planes; pages hold keys | values (2) or one shared vector (1)", planes);
-  if (int rc = tc_checks("attention_extend_tc", qkv, ld, out, ldo, nh, nkv, hd, error_flag, gate_col, true)) return rc;
+  if (int rc = tc_checks("attention_extend_tc", qkv, ld, out, ldo, nh, nkv, hd, error_flag, gate_col, keep_first, v_group, true)) return rc;
   if (page_size != BN) return cima_fail(CIMA_E_SIZE, "attention_extend_tc: page size %d; this kernel takes %d", page_size, BN);
   if (!cache || !table || !seq_slot || !seq_len || ((uintptr_t)cache & 15) || n_pages <= 0)
     return cima_fail(CIMA_E_ARG, "attention_extend_tc: the cache (16-byte aligned), its block table, slots and lengths are needed");
   if (n_pages * planes * nkv * BN >= (1ll << 31)) return cima_fail(CIMA_E_SIZE, "attention_extend_tc: %lld pages exceed a tensor map's 32-bit row coordinate", n_pages);
   const CacheSource c{cache, n_pages, table, seq_slot, seq_len, table_width, ring, planes};
   if (hd == 64)
-    return launch_attention_tc<64, true>(qkv, ld, tile_seq, tile_row0, seq_first_row, c, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, stream);
-  return launch_attention_tc<128, true>(qkv, ld, tile_seq, tile_row0, seq_first_row, c, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, stream);
+    return launch_attention_tc<64, true>(qkv, ld, tile_seq, tile_row0, seq_first_row, c, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
+  return launch_attention_tc<128, true>(qkv, ld, tile_seq, tile_row0, seq_first_row, c, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
 }

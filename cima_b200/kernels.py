@@ -91,7 +91,7 @@ _SIGNATURES = {
     "cima_attention_extend": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _f, _i, _i, _vp, _i, _vp,
                               _i, _vp, _vp, _vp],
     "cima_attention_extend_tc": [_vp, _i, _vp, _vp, _vp, _vp, ctypes.c_longlong, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
-                                 _f, _i, _vp, _i, _f, _vp, _i, _vp, _vp],
+                                 _f, _i, _vp, _i, _f, _vp, _i, _vp, _i, _i, _vp],
     "cima_row_norm_append": [_vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _f, _vp, _vp, _i, _i, _i, _vp],
     "cima_token_side_few": [_vp, _vp, _i, _vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp],
     "cima_token_side_apply": [_vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _vp],
@@ -125,7 +125,7 @@ _SIGNATURES = {
 
     "cima_head_linear_append": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _i, _vp, _f, _vp, _vp, _i, _i, _i, _vp, _vp, _vp,
                                 _i, _vp],
-    "cima_attention_prefill_tc": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _f, _vp, _i, _vp, _vp],
+    "cima_attention_prefill_tc": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _f, _vp, _i, _vp, _i, _i, _vp],
     "cima_gemm_tcgen05_pair": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _vp],
     "cima_diff_combine": [_vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _f, _f, _f, _vp],
     "cima_scale_add_group_rmsnorm": [_vp, _vp, _f, _vp, _vp, _i, _i, _i, _i, _f, _vp],
@@ -564,24 +564,23 @@ class Kernels:
         also holds exp(head_sink[h]), an entry that is not scaled and carries no value.  ``gate_col`` > 0: a row of ``qkv`` holds
         one gate value for each value of its result from that column on, and the result leaves times their sigmoid.  ``slopes`` (float32 [n_heads]): slopes[h] * (i - j) is taken
         off the scaled score of the query at position i with the key at j."""
-        general = keep_first > 0 or v_group > 1        # the tcgen05 kernels take neither
         if (from_cache and qkv.dtype is torch.bfloat16 and kv.page_size == 64 and head_dim % 16 == 0
                 and head_dim <= 128 and batch.n_rows == batch.n_seqs):
             return self.attention_decode(qkv, kv, batch.seq_slot, batch.seq_len, out, n_heads, n_kv_heads, head_dim,
                                          scale, window, batch.max_len, early=after_append, sink=sink,
                                          keep_first=keep_first, v_group=v_group, head_sink=head_sink, gate_col=gate_col, slopes=slopes)
-        many = (not general and qkv.dtype is torch.bfloat16 and head_dim in (64, 128) and qkv.shape[1] % 8 == 0
+        many = (qkv.dtype is torch.bfloat16 and head_dim in (64, 128) and qkv.shape[1] % 8 == 0
                 and getattr(batch, "n_q_tiles_tc", 0) > 0 and getattr(batch, "max_rows", 0) >= TC_ATTENTION_MIN_LEN)
         if from_cache and many and kv.page_size == 64 and kv.storage.numel() // head_dim < 2 ** 31:
             return self.attention_prefill_tc(qkv, batch, out, n_heads, n_kv_heads, head_dim, scale, window, kv=kv, sink=sink,
-                                             head_sink=head_sink, gate_col=gate_col, slopes=slopes)
+                                             head_sink=head_sink, gate_col=gate_col, slopes=slopes, keep_first=keep_first, v_group=v_group)
         if (from_cache and qkv.dtype is torch.bfloat16 and kv.page_size == 64 and head_dim % 16 == 0
                 and head_dim <= 128 and qkv.shape[1] % 8 == 0 and getattr(batch, "n_q_tiles", 0) > 0):
             return self.attention_extend(qkv, kv, batch, out, n_heads, n_kv_heads, head_dim, scale, window, sink=sink,
                                          keep_first=keep_first, v_group=v_group, head_sink=head_sink, gate_col=gate_col, slopes=slopes)
         if not from_cache and many:
             return self.attention_prefill_tc(qkv, batch, out, n_heads, n_kv_heads, head_dim, scale, window, sink=sink,
-                                             head_sink=head_sink, gate_col=gate_col, slopes=slopes)
+                                             head_sink=head_sink, gate_col=gate_col, slopes=slopes, keep_first=keep_first, v_group=v_group)
         if (not from_cache and qkv.dtype is torch.bfloat16 and head_dim % 16 == 0 and head_dim <= 128
                 and qkv.shape[1] % 8 == 0 and getattr(batch, "n_q_tiles", 0) > 0):
             return self.attention_prefill(qkv, batch.q_tile_seq, batch.q_tile_row0, batch.seq_first_row, out,
@@ -640,7 +639,7 @@ class Kernels:
 
     def attention_prefill_tc(self, qkv: torch.Tensor, batch, out: torch.Tensor, n_heads: int, n_kv_heads: int,
                              head_dim: int, scale: float, window: int, kv=None, sink: float = 0.0, head_sink=None,
-                             gate_col: int = 0, slopes=None) -> None:
+                             gate_col: int = 0, slopes=None, keep_first: int = 0, v_group: int = 1) -> None:
         """Flash attention of ragged prompts on the tcgen05 tensor cores (bf16, head_dim 64 or 128): blocks of 128
         query rows, both products with their results in tensor memory.  ``batch`` brings the blocks
         (``q_tile_tc_*``).  Without ``kv`` the sequences start at position 0 and the keys are the step's own rows;
@@ -661,13 +660,13 @@ class Kernels:
                 batch.seq_first_row.data_ptr(), kv.storage.data_ptr(), kv.storage.shape[0], kv.block_table.data_ptr(),
                 kv.block_table.shape[1], kv.ring_pages, kv.page_size, batch.seq_slot.data_ptr(), batch.seq_len.data_ptr(),
                 out.data_ptr(), out.shape[1], T, batch.n_q_tiles_tc, n_heads, n_kv_heads, head_dim, scale, window,
-                self._error_flag.data_ptr(), kv.planes, sink, _ptr(head_sink), gate_col, _ptr(slopes), self._stream()), "attention_extend_tc")
+                self._error_flag.data_ptr(), kv.planes, sink, _ptr(head_sink), gate_col, _ptr(slopes), keep_first, v_group, self._stream()), "attention_extend_tc")
             return
         self._check(self.lib.cima_attention_prefill_tc(
             qkv.data_ptr(), qkv.shape[1], batch.q_tile_tc_seq.data_ptr(), batch.q_tile_tc_row0.data_ptr(),
             batch.seq_first_row.data_ptr(), out.data_ptr(),
             out.shape[1], T, batch.n_q_tiles_tc, n_heads, n_kv_heads, head_dim, scale, window,
-            self._error_flag.data_ptr(), sink, _ptr(head_sink), gate_col, _ptr(slopes), self._stream()), "attention_prefill_tc")
+            self._error_flag.data_ptr(), sink, _ptr(head_sink), gate_col, _ptr(slopes), keep_first, v_group, self._stream()), "attention_prefill_tc")
 
     def attention_decode(self, qkv: torch.Tensor, kv, seq_slot, seq_len, out: torch.Tensor, n_heads: int,
                          n_kv_heads: int, head_dim: int, scale: float, window: int, max_len: int = 0,

@@ -599,6 +599,34 @@ def test_attention_of_going_on_rows_with_shared_keys(K, nh, nkv, hd, window, kee
             assert err(out, want) <= TOL["bfloat16"], (n_splits, list(kw))
 
 
+@pytest.mark.parametrize("nh,nkv,hd,v_group", [(8, 4, 64, 2), (4, 2, 128, 1), (4, 4, 128, 4)])
+@pytest.mark.parametrize("window,keep", [(90, 70), (300, 5), (64, 200), (130, 64), (0, 0)])
+def test_attention_tcgen05_with_kept_positions_and_shared_values(K, nh, nkv, hd, v_group, window, keep):
+    """The tcgen05 attention where a window keeps first positions (none of them below it, some, whole tiles, more than the window's
+    first rows have) and key heads share value heads: prompts on their own rows, and sequences that go on from the cache; the
+    dispatcher takes it for both."""
+    nv, page, width, scale = nkv // v_group, 64, 9, 1.0 / math.sqrt(hd)
+    for seqs, cached in ([(0, 0, 420), (1, 0, 37)], False), ([(2, 100, 260), (0, 0, 5), (1, 380, 130)], True):
+        T, cols = sum(s[2] for s in seqs), (nh + nkv + nv) * hd
+        qkv = g(T, cols, dtype=torch.bfloat16, seed=nh + T)
+        bc, bg = batch_of(seqs, "cpu"), batch_of(seqs, "cuda")
+        cpu = gpu = None
+        if cached:
+            order = torch.randperm(4 * width, generator=torch.Generator().manual_seed(6)).tolist()
+            cpu, gpu = make_kv(4 * width, nkv, page, hd, 4, width, 0, window, torch.bfloat16, {s: order[s * width:(s + 1) * width] for s in range(4)})
+            cpu.storage.copy_(g(*cpu.storage.shape, dtype=torch.bfloat16, seed=hd + window + 1))
+            gpu.storage.copy_(cpu.storage)
+        want = torch.zeros(T, nh * hd, dtype=torch.float64)
+        REF.attention_plain(qkv, cpu, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_first_row, want, nh, nkv, hd, scale, window, cached, keep_first=keep, v_group=v_group)
+        out = torch.full((T, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        K.attention_prefill_tc(qkv.cuda(), bg, out, nh, nkv, hd, scale, window, kv=gpu, keep_first=keep, v_group=v_group)
+        assert K.device_errors() == 0
+        assert err(out, want) <= TOL["bfloat16"], cached
+        out2 = torch.full((T, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        K.attention(qkv.cuda(), gpu, bg, out2, nh, nkv, hd, scale, window, cached, keep_first=keep, v_group=v_group)
+        assert torch.equal(out, out2), cached
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 128), (6, 1, 64)])
 @pytest.mark.parametrize("window", [0, 90, 300])
 def test_attention_of_sequences_that_go_on_by_many_rows_tcgen05(K, nh, nkv, hd, window):
