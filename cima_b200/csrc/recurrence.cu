@@ -165,10 +165,11 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
       if (blockIdx.x == 0 && (int)threadIdx.x < DIMP)
         for (int tt = 0; tt < nt; tt++) prod *= sg[tt][threadIdx.x];
     }
-    if constexpr (GATE) {
+    if constexpr (!DELTA) {
       // Nothing of a token's read-out feeds the next token's update, so four tokens are taken together: their updates
-      // follow one another row by row (S <- u + f (S - u), which is f S + (1 - f) u), their sums over the lanes run side
-      // by side.  A token's own arithmetic is the same wherever it stands among the four.
+      // follow one another row by row (the gate rule's S <- u + f (S - u), which is f S + (1 - f) u), their sums over the
+      // lanes run side by side.  A token's own arithmetic is the same wherever it stands among the four.  (Decay rule, 16 heads of
+      // 128 x 128, a sequence of 2,048: 640 us token after token, 504 so, 217 so in segments; four of 531 to 1,080, 12 heads: 357, 283.)
       constexpr int TB = 4;
       for (int tt = 0; tt < nt; tt += TB) {
         float o0[TB][CPT], o1[TB][CPT];
@@ -183,11 +184,20 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
 #pragma unroll
             for (int j = 0; j < RP; j += 4) {
               const int i = (j >> 2) * 32 + rg * 4;
-              const float4 g4 = *reinterpret_cast<const float4*>(&sg[tt + x][i]);
+              if constexpr (GATE) {
+                const float4 g4 = *reinterpret_cast<const float4*>(&sg[tt + x][i]);
 #pragma unroll
-              for (int c = 0; c < CPT; c++) {
-                S[c][j] = fmaf(g4.x, S[c][j] - u[c], u[c]); S[c][j + 1] = fmaf(g4.y, S[c][j + 1] - u[c], u[c]);
-                S[c][j + 2] = fmaf(g4.z, S[c][j + 2] - u[c], u[c]); S[c][j + 3] = fmaf(g4.w, S[c][j + 3] - u[c], u[c]);
+                for (int c = 0; c < CPT; c++) {
+                  S[c][j] = fmaf(g4.x, S[c][j] - u[c], u[c]); S[c][j + 1] = fmaf(g4.y, S[c][j + 1] - u[c], u[c]);
+                  S[c][j + 2] = fmaf(g4.z, S[c][j + 2] - u[c], u[c]); S[c][j + 3] = fmaf(g4.w, S[c][j + 3] - u[c], u[c]);
+                }
+              } else {
+                const float4 k4 = *reinterpret_cast<const float4*>(&sk[tt + x][i]);
+#pragma unroll
+                for (int c = 0; c < CPT; c++) {
+                  S[c][j] = fmaf(k4.x, u[c], S[c][j] * dh); S[c][j + 1] = fmaf(k4.y, u[c], S[c][j + 1] * dh);
+                  S[c][j + 2] = fmaf(k4.z, u[c], S[c][j + 2] * dh); S[c][j + 3] = fmaf(k4.w, u[c], S[c][j + 3] * dh);
+                }
               }
               if constexpr (READ) {
                 const float4 q4 = *reinterpret_cast<const float4*>(&sq[tt + x][i]);
@@ -226,31 +236,24 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
       float u[CPT];
 #pragma unroll
       for (int x = 0; x < CPT; x++) u[x] = sv[tt][lc + 32 * x];
-      if (DELTA) {
-        float p0[CPT], p1[CPT];
+      float p0[CPT], p1[CPT];
 #pragma unroll
-        for (int x = 0; x < CPT; x++) p0[x] = p1[x] = 0.f;
+      for (int x = 0; x < CPT; x++) p0[x] = p1[x] = 0.f;
 #pragma unroll
-        for (int j = 0; j < RP; j += 4) {
-          const int i = (j >> 2) * 32 + rg * 4;
-          const float4 g4 = *reinterpret_cast<const float4*>(&sg[tt][i]);
-          const float4 k4 = *reinterpret_cast<const float4*>(&sk[tt][i]);
+      for (int j = 0; j < RP; j += 4) {
+        const int i = (j >> 2) * 32 + rg * 4;
+        const float4 g4 = *reinterpret_cast<const float4*>(&sg[tt][i]);
+        const float4 k4 = *reinterpret_cast<const float4*>(&sk[tt][i]);
 #pragma unroll
-          for (int x = 0; x < CPT; x++) {
-            S[x][j] *= g4.x; S[x][j + 1] *= g4.y; S[x][j + 2] *= g4.z; S[x][j + 3] *= g4.w;
-            p0[x] = fmaf(S[x][j], k4.x, p0[x]); p1[x] = fmaf(S[x][j + 1], k4.y, p1[x]);
-            p0[x] = fmaf(S[x][j + 2], k4.z, p0[x]); p1[x] = fmaf(S[x][j + 3], k4.w, p1[x]);
-          }
+        for (int x = 0; x < CPT; x++) {
+          S[x][j] *= g4.x; S[x][j + 1] *= g4.y; S[x][j + 2] *= g4.z; S[x][j + 3] *= g4.w;
+          p0[x] = fmaf(S[x][j], k4.x, p0[x]); p1[x] = fmaf(S[x][j + 1], k4.y, p1[x]);
+          p0[x] = fmaf(S[x][j + 2], k4.z, p0[x]); p1[x] = fmaf(S[x][j + 3], k4.w, p1[x]);
         }
-        const float b = sb[tt];
-#pragma unroll
-        for (int x = 0; x < CPT; x++) u[x] = b * (u[x] - rec_sum_over_lanes(p0[x] + p1[x]));
-      } else {
-#pragma unroll
-        for (int x = 0; x < CPT; x++)
-#pragma unroll
-          for (int j = 0; j < RP; j++) S[x][j] *= dh;
       }
+      const float b = sb[tt];
+#pragma unroll
+      for (int x = 0; x < CPT; x++) u[x] = b * (u[x] - rec_sum_over_lanes(p0[x] + p1[x]));
       float o0[CPT], o1[CPT];
 #pragma unroll
       for (int x = 0; x < CPT; x++) o0[x] = o1[x] = 0.f;
@@ -258,20 +261,17 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
       for (int j = 0; j < RP; j += 4) {
         const int i = (j >> 2) * 32 + rg * 4;
         const float4 k4 = *reinterpret_cast<const float4*>(&sk[tt][i]);
-        float4 q4;
-        if constexpr (READ) q4 = *reinterpret_cast<const float4*>(&sq[tt][i]);
+        const float4 q4 = *reinterpret_cast<const float4*>(&sq[tt][i]);
 #pragma unroll
         for (int x = 0; x < CPT; x++) {
           S[x][j] = fmaf(k4.x, u[x], S[x][j]); S[x][j + 1] = fmaf(k4.y, u[x], S[x][j + 1]);
           S[x][j + 2] = fmaf(k4.z, u[x], S[x][j + 2]); S[x][j + 3] = fmaf(k4.w, u[x], S[x][j + 3]);
-          if constexpr (!READ) continue;
           o0[x] = fmaf(S[x][j], q4.x, o0[x]); o1[x] = fmaf(S[x][j + 1], q4.y, o1[x]);
           o0[x] = fmaf(S[x][j + 2], q4.z, o0[x]); o1[x] = fmaf(S[x][j + 3], q4.w, o1[x]);
         }
       }
 #pragma unroll
       for (int x = 0; x < CPT; x++) {
-        if constexpr (!READ) continue;
         const float o = rec_sum_over_lanes(o0[x] + o1[x]);
         if (rg == 0) so[tt][lc + 32 * x] = o;
       }
