@@ -32,7 +32,7 @@
 //   rows, warp 5 makes T and M of chunk j + 1 and leaves them split into their terms, while chunk j is worked on.  (One warp that
 //   did all three took 5,900 cycles a chunk, twice what the columns' warps take.)
 #include "common.cuh"
-#include "delta_chunk.cuh"
+#include <cstddef>
 
 namespace {
 constexpr int DR_WARPS = 4, DR_THREADS = 32 * DR_WARPS, DR_COLS = 8 * DR_WARPS;
@@ -248,8 +248,35 @@ k_delta_rule(const TA* __restrict__ qkv, int ld, const TA* __restrict__ a, int l
 
 
 // ---------------------------------------------------------------------------------------------------- 16 tokens at a time
-constexpr int DC_WARPS = 4, DC_COLS = 16 * DC_WARPS, DC_THREADS = 32 * (DC_WARPS + 3), DC_STAGES = 5;
+constexpr int DC_T = 16, DC_WARPS = 4, DC_COLS = 16 * DC_WARPS, DC_THREADS = 32 * (DC_WARPS + 3), DC_STAGES = 5;
 constexpr int DC_TROW = 24, DC_VROW = DC_COLS + 8;      // padded rows of the 16 x 16 matrices' terms and of v
+
+typedef __nv_bfloat16 bf16;
+__device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void dc_ldmatrix(uint32_t (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void dc_ldmatrix_trans(uint32_t (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void dc_copy16(unsigned dst, const bf16* src) {             // 16 bytes, dst an address in shared memory
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+}
+// x, y as a sum of three bfloat16 terms each, packed in pairs (x in the low half)
+__device__ __forceinline__ void dc_split(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const float2 hf = __bfloat1622float2(h);
+  x -= hf.x; y -= hf.y;
+  const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
+  const float2 mf = __bfloat1622float2(m);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(x - mf.x, y - mf.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h); mid = *reinterpret_cast<const uint32_t*>(&m); lo = *reinterpret_cast<const uint32_t*>(&l);
+}
 
 template <int DIMP>
 struct __align__(16) DcShared {

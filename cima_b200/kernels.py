@@ -102,7 +102,6 @@ _SIGNATURES = {
     "cima_embed_bigram": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _f, _i, ctypes.c_longlong, ctypes.c_longlong, _vp, _vp, _vp, _vp, _vp,
                           _i, _vp],
     "cima_recurrence": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
-    "cima_channel_delta": [_vp, _i, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
     "cima_delta_prepare": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "cima_delta_rule": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "cima_group_rmsnorm_gate": [_vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _f, _vp],
@@ -1031,9 +1030,6 @@ class Kernels:
             self.launches += 1
 
     # ------------------------------------------------------------------ recurrent mixers
-    # rows of a step's longest sequence from which bfloat16 delta rules take 16 tokens at a time (12 heads of 128 x 128, 8 sequences
-    # of 40 rows: 45.5 us, the walk 46; longer ones gain, shorter ones are mostly a chunk's start)
-    CHANNEL_DELTA_ROWS = 32
     RECURRENCE_SEGMENT = 128    # tokens of a segment of a long step's decay or gate rule
 
     def recurrence_segments(self, batch, columns: int, dtype: torch.dtype) -> int:
@@ -1082,13 +1078,6 @@ class Kernels:
                            batch.n_seqs * heads * dim * vdim * 8 + T * (2 * kv_heads * dim * q.element_size() + heads * vdim * (4 + v.element_size())
                                                                         + (heads * dim * 4 if delta else 0)),
                            (8.0 if delta else 5.0) * T * heads * dim * vdim): return
-        if (delta and v.dtype is torch.bfloat16 and int(getattr(batch, "max_rows", 0) or 0) >= self.CHANNEL_DELTA_ROWS and dim <= 128 and dim % 4 == 0
-                and vdim % 8 == 0 and q.stride(0) % 4 == 0 and k.stride(0) % 4 == 0 and v.stride(0) % 8 == 0
-                and not any(t.data_ptr() & 15 for t in (q, k, v, g))):
-            self._check(self.lib.cima_channel_delta(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), g.data_ptr(),
-                                                    beta.data_ptr(), state.data_ptr(), batch.seq_slot.data_ptr(), batch.seq_first_row.data_ptr(),
-                                                    out.data_ptr(), T, batch.n_seqs, heads, kv_heads, dim, vdim, self._stream()), "channel_delta")
-            return
         segs = 1 if delta else self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype)
         buf = torch.empty(batch.n_seqs * segs * heads * dim * vdim, dtype=torch.float32, device=q.device) if segs > 1 else None
         self._check(self.lib.cima_recurrence(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),

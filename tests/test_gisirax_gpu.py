@@ -194,31 +194,6 @@ def test_recurrence_whole_in_pieces_and_token_by_token(heads, kv_heads, dim, vdi
     _recurrence_case(delta, heads, kv_heads, dim, vdim, dtype, steps, seed=dim + vdim)
 
 
-@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(2, 1, 16, 24), (3, 3, 40, 8), (2, 2, 128, 64), (1, 1, 8, 104), (2, 1, 100, 16), (1, 1, 64, 200)])
-def test_delta_rule_sixteen_tokens_at_a_time(heads, kv_heads, dim, vdim):
-    """Long bfloat16 steps, ends on and off a chunk's border, beside short sequences and what goes on from them token by token."""
-    n = K().CHANNEL_DELTA_ROWS
-    _recurrence_case(True, heads, kv_heads, dim, vdim, "bfloat16", [[5 * n + 7, 3, 16], [n, 1, 17], [1, 1, 1], [0, n + 1, 1]], seed=dim + vdim)
-
-
-def test_delta_rule_sixteen_tokens_at_a_time_with_extreme_decays():
-    """Decays of 0, of the smallest floats and of 1, steps of size 0 and 1, in any mixture of channels and tokens: what the walk gives."""
-    g = torch.Generator().manual_seed(3)
-    T, heads, dim, vdim = 70, 2, 128, 64
-    q, k = (torch.nn.functional.normalize(torch.randn(T, heads, dim, generator=g), dim=-1).view(T, -1).to(DEV) for _ in range(2))
-    v = torch.randn(T, heads * vdim, generator=g).to(torch.bfloat16).to(DEV)
-    pick = lambda values, *shape: torch.tensor(values)[torch.randint(0, len(values), shape, generator=g)].to(DEV)
-    gg, beta = pick([0.0, 1e-38, 1e-20, 0.3, 0.999, 1.0], T, heads * dim), pick([0.0, 0.5, 1.0], T, heads)
-    b = entries_batch([T], [0], [0])
-    outs, states = [], []
-    for rows in (T, 1):                        # the second batch says that its longest sequence has one row: the walk
-        b.max_rows = rows
-        state, o = torch.randn(1, heads, dim, vdim, generator=torch.Generator().manual_seed(9)).to(DEV), torch.empty(T, heads * vdim, device=DEV)
-        K().recurrence(q, k, v, state, b, o, heads, heads, dim, vdim, g=gg, beta=beta)
-        outs.append(o); states.append(state)
-    assert bool(outs[0].isfinite().all()) and close(outs[0], outs[1].cpu(), 2e-5) and close(states[0], states[1].cpu(), 2e-5)
-
-
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 40, 72), (1, 128, 33), (3, 16, 8), (1, 200, 64)])
 def test_decay_rule_of_long_sequences_in_segments(heads, dim, vdim):
     """Sequences of two to six segments beside short ones, ends on and off a segment's border, and what goes on from them."""
