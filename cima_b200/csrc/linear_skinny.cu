@@ -97,8 +97,9 @@ struct SkinnyRope {
 
 // NT: 8-row tiles of X (M <= 8 * NT).  MT: m-tiles per block (1, or 2 for the gated epilogue).
 // U: 32-wide k steps kept in flight per warp iteration.  NORM: X is bf16(x * w), see above.
-template <int NT, int MT, int U, int MODE, bool NORM>
-__global__ void __launch_bounds__(SK_WARPS * 32)
+// MINB: blocks that an SM has to hold (0: as many as the registers come to), see launch_skinny_gated.
+template <int NT, int MT, int U, int MODE, bool NORM, int MINB = 0>
+__global__ void __launch_bounds__(SK_WARPS * 32, MINB)
 k_linear_skinny(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ W,
                 const float* __restrict__ bias, void* __restrict__ out,
                 int M, int N, int K, int ldx, int ldo, int up_offset, SkinnyNorm nm, SkinnyRope rp) {
@@ -321,24 +322,27 @@ k_linear_skinny(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __rest
 // costs more than its parallelism brings, and clusters of odd size were slower than their neighbours.
 // Depends on the matrix and the device only, never on the rows of X, so that a row's sum has the same order
 // whatever the batch.
-static int cluster_size(int tiles, int K) {
-  static int resident = 0;
-  if (!resident) {
-    int dev = 0, sms = 0;
+static int sm_count() {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0, n = 0;
     cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    resident = sms * 4;
+    sms = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
   }
+  return sms;
+}
+static int cluster_size(int tiles, int K) {
+  const int resident = sm_count() * 4;
   int s = 1;
   while (s < 8 && tiles * (2 * s) <= resident && (2 * s) * SK_WARPS * 128 <= K) s *= 2;
   return s;
 }
 
-template <int NT, int MT, int U, int MODE, bool NORM>
+template <int NT, int MT, int U, int MODE, bool NORM, int MINB = 0>
 static int launch_skinny(const void* X, const void* W, const float* bias, void* out, int M, int N, int K, int ldx,
                          int ldo, int up_offset, const SkinnyNorm& nm, cudaStream_t stream,
                          const SkinnyRope& rp = SkinnyRope{}) {
-  auto kern = k_linear_skinny<NT, MT, U, MODE, NORM>;
+  auto kern = k_linear_skinny<NT, MT, U, MODE, NORM, MINB>;
   const size_t smem = ((size_t)SK_WARPS * MT * NT * 8 * SK_PAD + (size_t)MT * NT * 8 * SK_ROWS) * sizeof(float);
   if (smem > 48 * 1024) {
     static bool raised = false;     // one attribute per instantiation
@@ -356,6 +360,19 @@ static int launch_skinny(const void* X, const void* W, const float* bias, void* 
   return cima_launch_result();
 }
 
+// The gated product takes 70 to 80 registers, three blocks an SM.  Held to 64 it fits four, with a few bytes spilled: the better one
+// where all its blocks are then resident at once and would otherwise leave a second wave of a few (560 tiles, gate and up of
+// 1,536 x 8,960: 13.0 -> 10.1 us for one row, 13.8 -> 10.8 for eight, 4.1 -> 5.4 and 4.0 -> 5.1 TB/s), the worse one elsewhere
+// (304 tiles 4.4 and 5.5 us, 688 tiles 16.6 and 19.2, 1,184 tiles 43.3 and 46.3).  The order of the sums is the same.
+template <int NT, bool NORM>
+static int launch_skinny_gated(const void* X, const void* W, const float* bias, void* out, int M, int N, int K, int ldx, int ldo,
+                               const SkinnyNorm& nm, cudaStream_t stream) {
+  const int tiles = (N + SK_ROWS - 1) / SK_ROWS, blocks = tiles * cluster_size(tiles, K);
+  if (blocks > 3 * sm_count() && blocks <= 4 * sm_count())
+    return launch_skinny<NT, 2, 2, SK_SWIGLU, NORM, 4>(X, W, bias, out, M, N, K, ldx, ldo, N, nm, stream);
+  return launch_skinny<NT, 2, 2, SK_SWIGLU, NORM>(X, W, bias, out, M, N, K, ldx, ldo, N, nm, stream);
+}
+
 template <int NT, bool NORM>
 static int dispatch_mode(int mode, const void* X, const void* W, const float* bias, void* out, int M, int N, int K,
                          int ldx, int ldo, const SkinnyNorm& nm, cudaStream_t stream) {
@@ -364,7 +381,7 @@ static int dispatch_mode(int mode, const void* X, const void* W, const float* bi
     case SK_STORE: return launch_skinny<NT, 1, U, SK_STORE, NORM>(X, W, bias, out, M, N, K, ldx, ldo, 0, nm, stream);
     case SK_ACCUM: return launch_skinny<NT, 1, U, SK_ACCUM, NORM>(X, W, bias, out, M, N, K, ldx, ldo, 0, nm, stream);
     case SK_STORE_F32: return launch_skinny<NT, 1, U, SK_STORE_F32, NORM>(X, W, bias, out, M, N, K, ldx, ldo, 0, nm, stream);
-    case SK_SWIGLU: return launch_skinny<NT, 2, 2, SK_SWIGLU, NORM>(X, W, bias, out, M, N, K, ldx, ldo, N, nm, stream);
+    case SK_SWIGLU: return launch_skinny_gated<NT, NORM>(X, W, bias, out, M, N, K, ldx, ldo, nm, stream);
     default: return cima_fail(CIMA_E_ARG, "linear_skinny: mode %d is not one of 0..3", mode);
   }
 }

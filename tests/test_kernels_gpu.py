@@ -175,6 +175,25 @@ def test_linear_skinny_row_does_not_depend_on_batch(K):
         assert torch.equal(part, full[:m])
 
 
+@pytest.mark.parametrize("I,K_", [(7104, 72), (7105, 200), (8960, 264), (9472, 136), (9473, 72)])
+def test_linear_skinny_gated_around_one_wave_of_blocks(K, I, K_):
+    """444, 445, 560, 592 and 593 tiles of 16 features: three and four blocks on each of 148 SMs, and one more, with the folded norm
+    and without.  Tolerance: the result's rounding to bfloat16, 2^-8 of it, and float32 sums of up to 264 products before."""
+    from cima_b200.kernels import SK_SWIGLU
+    a, w = g(8, K_, dtype=torch.bfloat16, seed=I), g(2 * I, K_, dtype=torch.bfloat16, seed=1, scale=1.0 / math.sqrt(K_))
+    ssq = torch.rand(8, 5, generator=torch.Generator().manual_seed(2))
+    inv = 1.0 / torch.sqrt(ssq.double().sum(1, keepdim=True) / K_ + 1e-6)
+    plain, folded, one = (torch.empty(m, I, dtype=torch.bfloat16, device="cuda") for m in (8, 8, 1))
+    K.linear_skinny(a.cuda(), w.cuda(), None, plain, SK_SWIGLU)
+    K.linear_skinny(a[6:7].contiguous().cuda(), w.cuda(), None, one, SK_SWIGLU)
+    K.linear_skinny_norm(a.cuda(), ssq.cuda(), 1e-6, w.cuda(), None, folded, SK_SWIGLU)
+    for got, f in ((plain, 1.0), (folded, inv)):
+        z = f * (a.double() @ w.double().t())
+        want = REF.gate_act(z[:, :I], 0) * z[:, I:]
+        assert err(got, want) <= 2.0 ** -8 * (1 + 2.0 ** -6) * want.abs().max().item()
+    assert torch.equal(one, plain[6:7])
+
+
 def test_linear_skinny_refuses(K):
     from cima_b200.kernels import KernelError, SK_STORE
     a, w = g(9, 64, dtype=torch.bfloat16).cuda(), g(32, 64, dtype=torch.bfloat16).cuda()
