@@ -20,8 +20,8 @@
 //   many pairs, bfloat16   moe_sort_tiles lays every expert's pairs out from a multiple of 256 rows on and names each row
 //                          tile's expert; moe_gather_rows copies the rows of h to their places; the two products run on
 //                          the tcgen05 kernel (gemm_tcgen05_pair_grouped); moe_combine reads y through the pairs' places
-//   few pairs, bfloat16    moe_few: a block computes 16 output features for up to 8 pairs of an expert at a time, its warps
-//                          streaming a range of k each with 16-byte loads (a decode step reads every touched expert once)
+//   fewer, bfloat16        moe_few: a block computes 16 output features for up to 8 (32 where there are more) pairs of an expert
+//                          at a time, its warps streaming a range of k each with 16-byte loads (every touched expert is read once)
 #include "common.cuh"
 
 namespace {
@@ -527,17 +527,20 @@ __device__ __forceinline__ uint4 few_load(const void* p, bool ok) {
                : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)ok));
   return v;
 }
-template <int MODE>
+// NB: pairs of eight that a piece of weights serves at once (1 in a decode step of few sequences; 4, a whole tile of 32 pairs, where
+// an expert has more than eight on average: 192 pairs of 16 gated experts of 1,536 x 2,240 in 109 us, 1,024 in 248).  A row's sums
+// are the same either way.
+template <int MODE, int NB>
 __global__ void __launch_bounds__(32 * FEW_WARPS)
 k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
           const int* __restrict__ offsets, const int* __restrict__ tiles, const int* __restrict__ perm, int E, int top, int N,
           int K, int act, float limit, const float* __restrict__ weigh) {
   constexpr int MT = MODE == 0 ? 2 : 1;                 // operand tiles of a block: gate and up
-  constexpr int AHEAD = MODE == 0 ? 2 : 4;
+  constexpr int AHEAD = MODE == 0 || NB > 1 ? 2 : 4, COLS = NB * FEW_PAIRS;
   cima_pdl_wait();
   __shared__ int s_row[BM], s_pair[BM], s_e, s_i0, s_n;
   __shared__ float s_w[BM];
-  __shared__ float red[FEW_WARPS][MT * FEW_FEATURES][FEW_PAIRS + 1];
+  __shared__ float red[FEW_WARPS][MT * FEW_FEATURES][COLS + 1];
   const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
   if (tid == 0) s_e = -1;
   __syncthreads();
@@ -568,16 +571,20 @@ k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __r
   const int pieces = (K + 31) / 32, share = (pieces + FEW_WARPS - 1) / FEW_WARPS;
   const int beg = min(pieces, warp * share), end = min(pieces, beg + share);
   __syncthreads();
-  for (int r0 = 0; r0 < nrows; r0 += FEW_PAIRS) {
-    const __nv_bfloat16* a = A + (size_t)s_row[min(r0 + g, nrows - 1)] * lda + 8 * t;      // (a column without a pair is not read below)
-    float acc[MT][4];
+  for (int r0 = 0; r0 < nrows; r0 += COLS) {
+    const __nv_bfloat16* a[NB];                           // (a column without a pair is not read below)
+#pragma unroll
+    for (int y = 0; y < NB; y++) a[y] = A + (size_t)s_row[min(r0 + FEW_PAIRS * y + g, nrows - 1)] * lda + 8 * t;
+    float acc[MT][NB][4];
 #pragma unroll
     for (int m = 0; m < MT; m++)
 #pragma unroll
-      for (int x = 0; x < 4; x++) acc[m][x] = 0.f;
+      for (int y = 0; y < NB; y++)
+#pragma unroll
+        for (int x = 0; x < 4; x++) acc[m][y][x] = 0.f;
 #pragma unroll 1
     for (int p0 = beg; p0 < end; p0 += AHEAD) {
-      uint4 wv[AHEAD][MT][2], av[AHEAD];
+      uint4 wv[AHEAD][MT][2], av[AHEAD][NB];
 #pragma unroll
       for (int u = 0; u < AHEAD; u++) {
         const int k = 32 * (p0 + u);
@@ -586,23 +593,29 @@ k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __r
         for (int m = 0; m < MT; m++)
 #pragma unroll
           for (int x = 0; x < 2; x++) wv[u][m][x] = few_load(w[m][x] + k, ok);
-        av[u] = few_load(a + k, ok);
+#pragma unroll
+        for (int y = 0; y < NB; y++) av[u][y] = few_load(a[y] + k, ok);
       }
 #pragma unroll
       for (int u = 0; u < AHEAD; u++)
 #pragma unroll
         for (int m = 0; m < MT; m++) {
-          few_mma(acc[m], wv[u][m][0].x, wv[u][m][1].x, wv[u][m][0].y, wv[u][m][1].y, av[u].x, av[u].y);
-          few_mma(acc[m], wv[u][m][0].z, wv[u][m][1].z, wv[u][m][0].w, wv[u][m][1].w, av[u].z, av[u].w);
+#pragma unroll
+          for (int y = 0; y < NB; y++) few_mma(acc[m][y], wv[u][m][0].x, wv[u][m][1].x, wv[u][m][0].y, wv[u][m][1].y, av[u][y].x, av[u][y].y);
+#pragma unroll
+          for (int y = 0; y < NB; y++) few_mma(acc[m][y], wv[u][m][0].z, wv[u][m][1].z, wv[u][m][0].w, wv[u][m][1].w, av[u][y].z, av[u][y].w);
         }
     }
 #pragma unroll
     for (int m = 0; m < MT; m++)
 #pragma unroll
-      for (int x = 0; x < 4; x++) red[warp][m * FEW_FEATURES + g + 8 * (x >> 1)][2 * t + (x & 1)] = acc[m][x];
+      for (int y = 0; y < NB; y++)
+#pragma unroll
+        for (int x = 0; x < 4; x++) red[warp][m * FEW_FEATURES + g + 8 * (x >> 1)][FEW_PAIRS * y + 2 * t + (x & 1)] = acc[m][y][x];
     __syncthreads();
-    const int f = tid / FEW_PAIRS, r = tid % FEW_PAIRS, n = n0 + f;
-    if (f < FEW_FEATURES && n < N && r0 + r < nrows) {
+    for (int o = tid; o < FEW_FEATURES * COLS; o += 32 * FEW_WARPS) {
+      const int f = o / COLS, r = o % COLS, n = n0 + f;
+      if (n >= N || r0 + r >= nrows) continue;
       float v[MT];
 #pragma unroll
       for (int m = 0; m < MT; m++) {
@@ -730,8 +743,12 @@ extern "C" int cima_moe_few(const void* a, int lda, const void* w, void* out, co
   const dim3 grid((unsigned)((P + BM - 1) / BM + E), (unsigned)((N + FEW_FEATURES - 1) / FEW_FEATURES));
   if (grid.y > 65535) return cima_fail(CIMA_E_SIZE, "moe_few: %d outputs exceed one launch", N);
   int rc;
-  if (mode == 0) rc = cima_launch(k_moe_few<0>, grid, dim3(256), (size_t)0, stream, 1, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, out, offsets, tiles, perm, E, top, N, K, act, limit, weigh);
-  else if (mode == 2) rc = cima_launch(k_moe_few<2>, grid, dim3(256), (size_t)0, stream, 1, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, out, offsets, tiles, perm, E, top, N, K, act, limit, weigh);
-  else rc = cima_launch(k_moe_few<1>, grid, dim3(256), (size_t)0, stream, 1, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, out, offsets, tiles, perm, E, top, N, K, act, limit, weigh);
+#define RUN(M, NB) rc = cima_launch(k_moe_few<M, NB>, grid, dim3(256), (size_t)0, stream, 1, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, out, offsets, tiles, perm, E, top, N, K, act, limit, weigh)
+#define WIDTH(M) { if (P > FEW_PAIRS * E) RUN(M, 4); else RUN(M, 1); }
+  if (mode == 0) WIDTH(0)
+  else if (mode == 2) WIDTH(2)
+  else WIDTH(1)
+#undef WIDTH
+#undef RUN
   return rc ? rc : cima_launch_result();
 }

@@ -1467,8 +1467,8 @@ class Kernels:
         """x[t] += (with ``assign``: =) sum_j wgt[t, j] * W_down[e] (act(W_gate[e] h[t]) * (W_up[e] h[t])), e = idx[t, j], ascending j.
         gate_up [E, 2 ff, H] (an expert's gate rows, then its up rows), down [E, H, ff]; x float32 [T, H].  Four launches:
         the pairs sorted by expert, the two grouped products over tiles of one expert's pairs, the weighted sum.  The
-        products take one of three roads by the step's size and dtype alone (``MOE_TC_PAIRS``, ``MOE_FEW_PAIRS``): tcgen05
-        tiles of 256 pairs, a warp a feature for the few pairs of a decode step, or the plain tiles (any dtype and size).
+        products take one of three roads by the step's size, layout and dtype alone (``MOE_TC_PAIRS``): tcgen05 tiles of 256 pairs,
+        ``mma.sync`` tiles of 16 features and up to 32 pairs (bfloat16), or the plain tiles (any dtype, size and address).
         ``limit`` goes with the clamped form of the middle.  ``shared = (rows, gate, col)``: float32 rows [T, H] (a shared
         expert's output) that join the weighted sum in its launch, each row times sigmoid(gate[t, col]) (gate float32
         [T, n]; None: unweighted).  ``identity``: indices from E on are identity experts: their pairs are in no product and
@@ -1508,7 +1508,7 @@ class Kernels:
         bf16 = h.dtype is torch.bfloat16 and gate_up.dtype is torch.bfloat16 and H % 8 == 0 and ff % 8 == 0 and h.stride(0) % 8 == 0
         if bf16 and P >= self.MOE_TC_PAIRS:
             return self._moe_experts_tc(h, gate_up, down, idx, wgt, x, act, assign, limit, tail + own, gated, weigh_input)
-        few = bf16 and P <= self.MOE_FEW_PAIRS
+        few = bf16 and (P <= self.MOE_FEW_PAIRS or not any(t.data_ptr() & 15 for t in (h, gate_up, down)))
         meta = ordered if ordered is not None else torch.empty(2 * (E + 1) + P, dtype=torch.int32, device=dev)
         offsets, tiles, perm = meta[:E + 1], meta[E + 1:2 * (E + 1)], meta[2 * (E + 1):]
         z = torch.empty((P, ff), dtype=h.dtype, device=dev)
@@ -1539,8 +1539,13 @@ class Kernels:
             self._check(self.lib.cima_moe_combine(y.data_ptr(), given, None, x.data_ptr(), T, top, H, int(assign), *tail, *own,
                                                   self._stream()), "moe_combine")
 
-    MOE_TC_PAIRS = 1024      # from this many (row, choice) pairs on, bfloat16 experts run on the tcgen05 tiles of 256 pairs
-    MOE_FEW_PAIRS = 128      # up to this many, a warp computes a feature for the pairs of an expert (a decode step)
+    # From MOE_TC_PAIRS (row, choice) pairs on bfloat16 experts run on the tcgen05 tiles of 256 pairs, below on the mma.sync kernel: such
+    # steps are the experts' weights read once, which both do, the mma.sync one with less beside it, until its pairs take several
+    # passes over a tile of weights.  Sort, products and sum of 16 gated experts of 1,536 x 2,240, mma.sync, tcgen05 and plain tiles, us:
+    # 64 pairs 73 / 113 / 1,223, 192: 109 / 114 / 1,413, 512: 160 / 114 / 1,671, 1,024: 248 / 114 / 2,373; ungated ones of 1,536 x 4,480: 96: 104 / 208 /
+    # 1,740, 288: 157 / 265 / 1,800, 768: 289 / 292 / 2,943; 64 gated ones of 2,048 x 512, 256: 92 / 186, 1,024: 160 / 193, 2,048: 235 / 195.
+    # MOE_FEW_PAIRS: up to there the mma.sync kernel refuses operands off 16 bytes; beyond, those go to the plain tiles.
+    MOE_TC_PAIRS, MOE_FEW_PAIRS = 1024, 128
 
     def _moe_experts_tc(self, h, gate_up, down, idx, wgt, x, act, assign=False, limit: float = 0.0, tail=(None, None, 0, None, 0, None, F32),
                         gated: bool = True, weigh_input: bool = False) -> None:

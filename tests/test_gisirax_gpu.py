@@ -265,6 +265,25 @@ def test_router_choice_and_weights(E, top, groups, keep):
     assert torch.equal(x1, x2)
 
 
+@pytest.mark.parametrize("T,H,ff,E,top", [(1, 8, 8, 2, 1), (8, 264, 136, 3, 2), (40, 96, 272, 2, 1), (42, 1544, 24, 3, 3), (100, 72, 40, 1, 1), (9, 40, 16, 16, 4),
+                                          (190, 72, 136, 16, 4), (300, 264, 40, 40, 3), (1023, 64, 64, 2, 1), (129, 128, 72, 130, 1)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_experts_of_few_pairs(T, H, ff, E, top, gated):
+    """Sums over k that end inside a warp's pieces and leave warps without any, features that end inside a block's sixteen, an
+    expert with one pair, with 8, 9, 32 and 33 and more, gated and not; up to the last size below the tcgen05 tiles."""
+    assert T * top < K().MOE_TC_PAIRS
+    g = torch.Generator().manual_seed(T * H + E)
+    h = torch.randn(T, H, generator=g).bfloat16()
+    gu, dn = (torch.randn(E, (2 if gated else 1) * ff, H, generator=g) * H ** -0.5).bfloat16(), (torch.randn(E, H, ff, generator=g) * ff ** -0.5).bfloat16()
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32)
+    wgt, x = torch.rand(T, top, generator=g), torch.randn(T, H, generator=g)
+    xd, xr = x.to(DEV).clone(), x.clone()
+    kw = {} if gated else dict(gated=False, weigh_input=True)
+    K().moe_experts(h.to(DEV), gu.to(DEV), dn.to(DEV), idx.to(DEV), wgt.to(DEV), xd, 0, **kw)
+    REF.moe_experts(h, gu, dn, idx, wgt, xr, 0, **kw)
+    assert close(xd - x.to(DEV), xr - x, 1.2e-2)          # the middle's rounding to bfloat16 (2^-8) at its largest, and the weighted rows'
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("T,H,ff,E,top", [(1, 40, 24, 3, 3), (5, 96, 40, 8, 2), (200, 64, 56, 6, 1), (70, 100, 33, 10, 4),
                                           (1100, 64, 56, 6, 1), (600, 128, 200, 5, 2), (30, 256, 64, 4, 4)])
