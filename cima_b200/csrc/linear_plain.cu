@@ -75,13 +75,13 @@ k_linear_plain(const TA* __restrict__ A, const TW* __restrict__ W, const float* 
 }
 
 // ---------------------------------------------------------------------------------------------------- all in float32
-// The 32-bit path's own product.  An output's sum over k is cut into F32_GROUPS ranges of k (f32_group_len, from K alone);
-// a range is added up in ascending k by one accumulator, and the ranges' sums are added in their order.  Both kernels below
-// follow that order, so a row's bits depend on its own row of A and the weights only: the same alone, in a prompt or in a
-// batch, whatever tile or split serves it.  (One accumulator over all of K left a decode step one thread per output feature:
+// The 32-bit path's own product.  An output's sum over k is cut into F32_GROUPS ranges of k (f32_group_len, from K alone; sums of
+// at most F32_ONE_RANGE stay one range, as there is little to share); a range is added up in ascending k by one accumulator, and
+// the ranges' sums are added in their order.  Both kernels below follow that order, so a row's bits depend on its own row of A and
+// the weights only: the same alone, in a prompt or in a batch, whatever tile or split serves it.  (One accumulator over all of K left a decode step one thread per output feature:
 // 75 us a product at the 0.5B shape, 0.3 TB/s.  Eight ranges give eight times the threads, and a shorter chain of roundings.)
-constexpr int F32_GROUPS = 8;
-__host__ __device__ inline int f32_group_len(int K) { return ((K + F32_GROUPS - 1) / F32_GROUPS + 15) & ~15; }
+constexpr int F32_GROUPS = 8, F32_ONE_RANGE = 512;
+__host__ __device__ inline int f32_group_len(int K) { return ((K <= F32_ONE_RANGE ? K : (K + F32_GROUPS - 1) / F32_GROUPS) + 15) & ~15; }
 
 __device__ __forceinline__ void f32_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
@@ -95,12 +95,12 @@ __device__ __forceinline__ void f32_finish(float* o, float v, const float* bias,
 }
 
 // At most 8 rows (a decode step): bound by the weights' bytes.  A block takes 8 output features, a warp one range of k of
-// them: its pieces of the 8 weight rows travel through shared memory by cp.async, whole 512-byte runs of a row at a time, up
+// them: its pieces of the 8 weight rows travel through shared memory by cp.async, 256-byte runs of a row at a time, up
 // to FEW_STAGES pieces in flight, the first ones before the kernel ahead has finished (weights do not depend on it).  Lane =
 // (feature, row mod 4): a lane walks its feature's range in order for one or two rows of A.  8 features a block and not more:
 // a narrow product (896 features) still covers 112 SMs, and a wide one keeps several blocks on each.  Measured inside a decode
 // step of the 0.5B shape, 2 rows: 9.5 us a product on average, 2.2 TB/s (74.8 us and 0.27 TB/s with a thread an output feature).
-constexpr int FEW_ROWS = 8, FEW_F = 8, FEW_K = 128, FEW_PITCH = FEW_K + 4, FEW_STAGES = 4, FEW_WARPS = F32_GROUPS;
+constexpr int FEW_ROWS = 8, FEW_F = 8, FEW_K = 64, FEW_PITCH = FEW_K + 4, FEW_STAGES = 4, FEW_WARPS = F32_GROUPS;
 
 template <int MR, bool VEC>        // MR: rows of A a lane takes (rows r, r + 4)
 __global__ void __launch_bounds__(32 * FEW_WARPS)
@@ -112,25 +112,27 @@ k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const
   const int len = f32_group_len(K), k0 = min(K, warp * len), kn = min(K, k0 + len) - k0, chunks = (kn + FEW_K - 1) / FEW_K;
   const int unit = (FEW_F + M) * FEW_PITCH;             // a stage: 8 rows of W, then M rows of A
   float* mine = few_smem + (size_t)warp * stages * unit;
-  // a piece of one row: `rows` floats of it (from k0 + c FEW_K on) into dst; what lies beyond the range is zero
+  // half a warp brings a piece of one row (from k0 + c FEW_K on) to dst; what lies beyond the range is zero
+  const int half = lane >> 4, at = 4 * (lane & 15);
   auto piece = [&](float* dst, const float* src, int c) {
-    const int left = kn - c * FEW_K;
+    const int left = kn - c * FEW_K - at;
+    src += k0 + c * FEW_K + at;
     if constexpr (VEC) {
-      if (4 * lane < left) f32_copy16(dst + 4 * lane, src + k0 + c * FEW_K + 4 * lane);
-      else *reinterpret_cast<float4*>(dst + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (left > 0) f32_copy16(dst + at, src);
+      else *reinterpret_cast<float4*>(dst + at) = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
 #pragma unroll
-      for (int e = 0; e < FEW_K / 32; e++) dst[lane + 32 * e] = lane + 32 * e < left ? src[k0 + c * FEW_K + lane + 32 * e] : 0.f;
+      for (int e = 0; e < 4; e++) dst[at + e] = e < left ? src[e] : 0.f;
     }
   };
   auto weights = [&](int c) {
     float* s = mine + (c % stages) * unit;
 #pragma unroll
-    for (int f = 0; f < FEW_F; f++) piece(s + f * FEW_PITCH, W + (size_t)min(n0 + f, N - 1) * K, c);
+    for (int f = half; f < FEW_F; f += 2) piece(s + f * FEW_PITCH, W + (size_t)min(n0 + f, N - 1) * K, c);
   };
   auto rows = [&](int c) {
     float* s = mine + (c % stages) * unit + FEW_F * FEW_PITCH;
-    for (int m = 0; m < M; m++) piece(s + m * FEW_PITCH, A + (size_t)m * lda, c);
+    for (int m = half; m < M; m += 2) piece(s + m * FEW_PITCH, A + (size_t)m * lda, c);
   };
   for (int c = 0; c < min(stages, chunks); c++) weights(c);
   cima_pdl_wait();
@@ -186,29 +188,16 @@ k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const
   }
 }
 
-// More rows: bound by the FP32 pipe.  Tiles of BM x 128 outputs, 256 threads with BM / 16 x 8 outputs each; the products run
-// two at a time (fma.rn.f32x2, the same rounding), for which shared memory holds each value of A twice.  The next 16 k travel
-// through registers while the current ones are multiplied.  SPLIT: a cluster of 8 blocks shares a tile, a range of k each,
-// and adds the ranges' sums in order through distributed shared memory (see launch_f32 for when).  Measured inside a prompt step
-// of the 0.5B shape, 201 + 123 rows: 122 us a product on average, 24 TFLOP/s (322 us with tiles of 64 x 64 and 4 x 4 a thread).
+// More rows: bound by the FP32 pipe.  Tiles of BM x 128 outputs, 256 threads with BM / 16 x 8 outputs each.  The next 16 k travel
+// through registers while the current ones are multiplied.  (Products two at a time, fma.rn.f32x2, want every value of A twice in
+// shared memory and were no faster.)  SPLIT: a cluster of 8 blocks shares a tile, a range of k each, and adds the ranges' sums in
+// order through distributed shared memory (see launch_f32 for when).  Measured, the 0.5B shape's products of 324 rows: 93 us on
+// average, 26 TFLOP/s (322 us with tiles of 64 x 64 and 4 x 4 a thread); alone and shared: 1,152 x 896 95 and 30 us, 9,728 x 896 187 and
+// 186, 896 x 4,864 491 and 124; tiles of 64 rows for 37 rows of 1,152 x 896: 11.5, of 128: 17.
 constexpr int F32_BN = 128, F32_BK = 16, F32_WROW = F32_BN + 4;
 
-__device__ __forceinline__ unsigned long long f32_pair(float x, float y) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float2 f32_unpair(unsigned long long v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void f32_fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-
 template <int BM>
-constexpr int f32_tile_floats() { return 2 * F32_BK * (2 * BM + 4 + F32_WROW); }
+constexpr int f32_tile_floats() { return 2 * F32_BK * (BM + 4 + F32_WROW); }
 template <int BM, bool SPLIT>
 constexpr size_t f32_tile_smem() {
   const size_t stage = f32_tile_floats<BM>() * sizeof(float), tile = SPLIT ? (size_t)BM * (F32_BN + 4) * sizeof(float) : 0;
@@ -216,13 +205,13 @@ constexpr size_t f32_tile_smem() {
 }
 
 template <int BM, bool SPLIT, bool VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, SPLIT ? 2 : 1)
 k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out,
                   int M, int N, int K, int lda, int ldo, int mode) {
-  constexpr int TM = BM / 16, AROW = 2 * BM + 4;
+  constexpr int TM = BM / 16, AROW = BM + 4;
   constexpr int NA = (BM * F32_BK / 4 + 255) / 256, NW = F32_BN * F32_BK / 4 / 256;      // 16-byte pieces a thread moves
   extern __shared__ __align__(16) float f32_smem[];
-  float* As = f32_smem;                                 // [2][F32_BK][AROW], every value twice
+  float* As = f32_smem;                                 // [2][F32_BK][AROW]
   float* Ws = f32_smem + 2 * F32_BK * AROW;             // [2][F32_BK][F32_WROW]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int rank = SPLIT ? blockIdx.x % F32_GROUPS : 0;
@@ -253,11 +242,8 @@ k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, cons
     for (int i = 0; i < NA; i++) {
       const int idx = tid + 256 * i;
       if (BM * F32_BK / 4 >= 256 * (i + 1) || idx < BM * F32_BK / 4) {
-        float* p = As + (buf * F32_BK + 4 * (idx % 4)) * AROW + 2 * (idx / 4);
-        *reinterpret_cast<float2*>(p) = make_float2(ra[i].x, ra[i].x);
-        *reinterpret_cast<float2*>(p + AROW) = make_float2(ra[i].y, ra[i].y);
-        *reinterpret_cast<float2*>(p + 2 * AROW) = make_float2(ra[i].z, ra[i].z);
-        *reinterpret_cast<float2*>(p + 3 * AROW) = make_float2(ra[i].w, ra[i].w);
+        float* p = As + (buf * F32_BK + 4 * (idx % 4)) * AROW + idx / 4;
+        p[0] = ra[i].x; p[AROW] = ra[i].y; p[2 * AROW] = ra[i].z; p[3 * AROW] = ra[i].w;
       }
     }
 #pragma unroll
@@ -268,14 +254,13 @@ k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, cons
     }
   };
 
-  unsigned long long acc[TM][4];
-  float total[SPLIT ? 1 : TM][SPLIT ? 1 : 8];
+  float acc[TM][8], total[SPLIT ? 1 : TM][SPLIT ? 1 : 8];
 #pragma unroll
   for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      acc[i][j] = 0ull;
-      if constexpr (!SPLIT) total[i][2 * j] = total[i][2 * j + 1] = 0.f;
+    for (int j = 0; j < 8; j++) {
+      acc[i][j] = 0.f;
+      if constexpr (!SPLIT) total[i][j] = 0.f;
     }
   const int tiles = kend > kbeg ? (kend - kbeg + F32_BK - 1) / F32_BK : 0;
   const int per = len / F32_BK;                         // tiles of a range (SPLIT: the only one)
@@ -285,21 +270,29 @@ k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, cons
     const int buf = t & 1;
     if (t + 1 < tiles) fetch(kbeg + (t + 1) * F32_BK);
     __syncthreads();
-    const float *as = As + buf * F32_BK * AROW + 2 * TM * ty, *ws = Ws + buf * F32_BK * F32_WROW + 4 * tx;
+    const float *as = As + buf * F32_BK * AROW + TM * ty, *ws = Ws + buf * F32_BK * F32_WROW + 4 * tx;
 #pragma unroll
     for (int k = 0; k < F32_BK; k++) {
-      unsigned long long a[TM], w[4];
+      float a[TM], w[8];
+      if constexpr (TM >= 4) {
 #pragma unroll
-      for (int i = 0; i < TM; i += 2) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(as + k * AROW + 2 * i);
-        a[i] = v.x; a[i + 1] = v.y;
+        for (int i = 0; i < TM; i += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(as + k * AROW + i);
+          a[i] = v.x; a[i + 1] = v.y; a[i + 2] = v.z; a[i + 3] = v.w;
+        }
+      } else {
+        const float2 v = *reinterpret_cast<const float2*>(as + k * AROW);
+        a[0] = v.x; a[1] = v.y;
       }
-      const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(ws + k * F32_WROW), v = *reinterpret_cast<const ulonglong2*>(ws + k * F32_WROW + 64);
-      w[0] = u.x; w[1] = u.y; w[2] = v.x; w[3] = v.y;
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(ws + k * F32_WROW + 16 * j);
+        w[j] = v.x; w[j + 1] = v.y; w[j + 2] = v.z; w[j + 3] = v.w;
+      }
 #pragma unroll
       for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) f32_fma2(acc[i][j], a[i], w[j]);
+        for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
     }
     if constexpr (!SPLIT) {
       if (--until == 0 || t + 1 == tiles) {             // a range is complete
@@ -307,11 +300,9 @@ k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, cons
 #pragma unroll
         for (int i = 0; i < TM; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const float2 v = f32_unpair(acc[i][j]);
-            total[i][2 * j] += v.x;
-            total[i][2 * j + 1] += v.y;
-            acc[i][j] = 0ull;
+          for (int j = 0; j < 8; j++) {
+            total[i][j] += acc[i][j];
+            acc[i][j] = 0.f;
           }
       }
     }
@@ -343,8 +334,7 @@ k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, cons
     for (int i = 0; i < TM; i++)
 #pragma unroll
       for (int j = 0; j < 2; j++) {
-        const float2 x = f32_unpair(acc[i][2 * j]), y = f32_unpair(acc[i][2 * j + 1]);
-        *reinterpret_cast<float4*>(f32_smem + (ty * TM + i) * ROW + 64 * j + 4 * tx) = make_float4(x.x, x.y, y.x, y.y);
+        *reinterpret_cast<float4*>(f32_smem + (ty * TM + i) * ROW + 64 * j + 4 * tx) = make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
       }
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     const unsigned base = (unsigned)__cvta_generic_to_shared(f32_smem);
@@ -375,7 +365,7 @@ k_linear_f32_tile(const float* __restrict__ A, const float* __restrict__ W, cons
 
 template <typename Kern>
 static int f32_allow(Kern kern, size_t smem) {
-  if (smem <= 48 * 1024) return 0;
+  if (smem <= 44 * 1024) return 0;                      // (48 KB are a kernel's without asking, its own static arrays among them)
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   return e == cudaSuccess ? 0 : cima_fail((int)e, "linear_plain: %zu bytes of shared memory are not available: %s", smem, cudaGetErrorString(e));
 }
@@ -396,19 +386,29 @@ static int launch_f32(const float* A, const float* W, const float* bias, float* 
   if (M <= FEW_ROWS) {
     const int chunks = (f32_group_len(K) + FEW_K - 1) / FEW_K, unit = (FEW_F + M) * FEW_PITCH * (int)sizeof(float) * FEW_WARPS;
     const int blocks = (N + FEW_F - 1) / FEW_F;
-    // the most pieces in flight that leave room for two blocks on an SM (one, where there are not two for each)
-    const int room = blocks > 148 ? 110 * 1024 : 220 * 1024;
+    // the most pieces in flight that leave room for two blocks on an SM: its own, or the next launch's, whose weights are then
+    // requested while this one ends
+    const int room = 110 * 1024;
     const int stages = chunks >= FEW_STAGES && FEW_STAGES * unit <= room ? FEW_STAGES : chunks >= 2 ? 2 : 1;
     const size_t smem = (size_t)stages * unit;
     auto kern = M <= 4 ? k_linear_f32_few<1, VEC> : k_linear_f32_few<2, VEC>;
     if (int rc = f32_allow(kern, smem)) return rc;
     return cima_launch(kern, dim3((unsigned)blocks), dim3(32 * FEW_WARPS), smem, stream, 1, A, W, bias, out, M, N, K, lda, ldo, mode, stages);
   }
-  // Tiles of 128 rows, or of 64 or 32 where those leave less of them empty; fewer tiles than three quarters of the SMs are shared by
-  // clusters of 8 blocks.
-  const int nt = (N + F32_BN - 1) / F32_BN;
-  const int bm = M <= 32 ? 32 : (M + 63) / 64 % 2 && M < 512 ? 64 : 128;
-  const bool split = K >= 2 * F32_GROUPS * F32_BK && (long long)nt * ((M + bm - 1) / bm) <= 111;
+  // The tile's rows, and whether clusters share a tile, by the time of the SM that gets the most blocks: a block's rows (a lower tile
+  // reads more of shared memory for a product: measured at 0.9 and 0.7 of the rate), an eighth of them where a cluster shares the tile (and
+  // a sixth more for the sums' way through the cluster).
+  const long long nt = (N + F32_BN - 1) / F32_BN;
+  int bm = 128;
+  bool split = false;
+  double best = 1e30;
+  for (int rows = 128; rows >= 32; rows /= 2)
+    for (int shared = 0; shared < 2; shared++) {
+      if (shared && K <= F32_ONE_RANGE) continue;
+      const long long blocks = nt * ((M + rows - 1) / rows) * (shared ? F32_GROUPS : 1);
+      const double cost = (double)((blocks + 147) / 148) * rows * (rows == 128 ? 1.0 : rows == 64 ? 1.1 : 1.4) * (shared ? 1.17 / F32_GROUPS : 1.0);
+      if (cost < best) { best = cost; bm = rows; split = shared; }
+    }
 #define F32_RUN(BM) return split ? launch_f32_tile<BM, true, VEC>(A, W, bias, out, mode, M, N, K, lda, ldo, stream) \
                                  : launch_f32_tile<BM, false, VEC>(A, W, bias, out, mode, M, N, K, lda, ldo, stream)
   if (bm == 32) F32_RUN(32);
