@@ -99,7 +99,7 @@ __device__ __forceinline__ void f32_finish(float* o, float v, const float* bias,
 // to FEW_STAGES pieces in flight, the first ones before the kernel ahead has finished (weights do not depend on it).  Lane =
 // (feature, row mod 4): a lane walks its feature's range in order for one or two rows of A.  8 features a block and not more:
 // a narrow product (896 features) still covers 112 SMs, and a wide one keeps several blocks on each.  Measured inside a decode
-// step of the 0.5B shape, 2 rows: 9.5 us a product on average, 2.2 TB/s (74.8 us and 0.27 TB/s with a thread an output feature).
+// step of the 0.5B shape, 2 rows: 9.3 us a product on average, 2.2 TB/s (74.8 us and 0.27 TB/s with a thread an output feature).
 constexpr int FEW_ROWS = 8, FEW_F = 8, FEW_K = 64, FEW_PITCH = FEW_K + 4, FEW_STAGES = 4, FEW_WARPS = F32_GROUPS;
 
 template <int MR, bool VEC>        // MR: rows of A a lane takes (rows r, r + 4)
@@ -191,8 +191,8 @@ k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const
 // More rows: bound by the FP32 pipe.  Tiles of BM x 128 outputs, 256 threads with BM / 16 x 8 outputs each.  The next 16 k travel
 // through registers while the current ones are multiplied.  (Products two at a time, fma.rn.f32x2, want every value of A twice in
 // shared memory and were no faster.)  SPLIT: a cluster of 8 blocks shares a tile, a range of k each, and adds the ranges' sums in
-// order through distributed shared memory (see launch_f32 for when).  Measured, the 0.5B shape's products of 324 rows: 93 us on
-// average, 26 TFLOP/s (322 us with tiles of 64 x 64 and 4 x 4 a thread); alone and shared: 1,152 x 896 95 and 30 us, 9,728 x 896 187 and
+// order through distributed shared memory (see launch_f32 for when).  Measured inside a prompt step of the 0.5B shape, 201 + 123
+// rows: 112 us a product on average, 26 TFLOP/s (322 us with tiles of 64 x 64 and 4 x 4 a thread); by themselves, alone and shared: 1,152 x 896 95 and 30 us, 9,728 x 896 187 and
 // 186, 896 x 4,864 491 and 124; tiles of 64 rows for 37 rows of 1,152 x 896: 11.5, of 128: 17.
 constexpr int F32_BN = 128, F32_BK = 16, F32_WROW = F32_BN + 4;
 
