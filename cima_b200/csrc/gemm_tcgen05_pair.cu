@@ -193,35 +193,25 @@ k_gemm_tcgen05_pair(const __grid_constant__ CUtensorMap map_p, const __grid_cons
 #pragma unroll 1
       for (int c0 = 0; c0 < OUT_COLS; c0 += 32) {
         float v[32];
+        tmem_ld32(acc + (unsigned)c0, v);
         if (GATED) {
-          // Gate and up come together.  The quotient is the fast one (2 ulp of float32, in front of a rounding to bfloat16; 0 for gates
-          // below -87.3, whose share is less than 88 * 2^-126): the IEEE
-          // division's steps and its branch made this loop, not the tensor cores, set the time of a tile of fewer than some 2,000 k
-          // (4 warps x 128 values a lane; main loop of 1,536 k: 6.6 us at 1.9 GHz).
-          unsigned rv[32], ru[32];
-          tmem_ld32_issue(acc + (unsigned)c0, rv);
-          tmem_ld32_issue(acc + (unsigned)(BN / 2 + c0), ru);
-          tmem_ld_wait();
           float u[32];
-#pragma unroll
-          for (int e = 0; e < 32; e++) { v[e] = __uint_as_float(rv[e]); u[e] = __uint_as_float(ru[e]); }
+          tmem_ld32(acc + (unsigned)(BN / 2 + c0), u);
           // one loop per form: the four epilogue warps have nothing to hide a branch or a call behind
           if (a.act == CIMA_ACT_SILU) {
 #pragma unroll
-            for (int e = 0; e < 32; e++) v[e] = __fdividef(v[e], 1.0f + expf(-v[e])) * u[e];
+            for (int e = 0; e < 32; e++) v[e] = v[e] / (1.0f + expf(-v[e])) * u[e];
           } else if (a.act == CIMA_GATED_SWISH_CLAMPED) {
             const float lim = a.act_limit;
 #pragma unroll
             for (int e = 0; e < 32; e++) {
               const float g = fminf(v[e], lim);
-              v[e] = __fdividef(g, 1.0f + expf(-1.702f * g)) * (fminf(fmaxf(u[e], -lim), lim) + 1.0f);
+              v[e] = g / (1.0f + expf(-1.702f * g)) * (fminf(fmaxf(u[e], -lim), lim) + 1.0f);
             }
           } else {
 #pragma unroll
             for (int e = 0; e < 32; e++) v[e] = cima_gated(v[e], u[e], a.act, a.act_limit);
           }
-        } else {
-          tmem_ld32(acc + (unsigned)c0, v);
         }
         if (EPI == EPI_ACT) {
           if (a.act == CIMA_UNGATED_RELU2) {

@@ -151,15 +151,18 @@ class GatedLinearPair:
 
     def _gated_on_tcgen05(self, rows: int) -> bool:
         """Whether the tcgen05 product with the fused activation beats the library product plus the activation
-        kernel.  Measured with full tiles of 256 rows, K 896 / 1,536 / 2,048 / 3,584, in us against the library's two
-        launches inside a step: 2,048 rows 35 / 88 / 138 / 373 against 41 / 96 / 147 / 385; 512 rows 17 / 26 / 46 / 103 against
-        17 / 32 / 52 / 105.  A last tile that is mostly padding costs a whole one, where the library's time follows the rows
-        (K 3,584 inside a 7B prompt step: 300 rows 115 us against 65 + 11, 1,000: 209 against 167 + 25): of its tiles' rows at most
-        2 % may be padding where the two are that close, 8 % below K 3,072."""
+        kernel.  With a short sum the tile's epilogue (256 x 256 accumulators through the activation) outlasts
+        its main loop: measured at 2,048 rows, K 896 / 1,536 / 2,048 / 3,584: 55 / 93 / 136 / 366 us against
+        41 / 96 / 147 / 385; at 512 rows 31 / 36 / 54 / 101 against 17 / 32 / 52 / 105.  And the kernel works in
+        tiles of 256 rows, a last tile that is mostly padding costing a whole one, where the library's time follows
+        the rows: inside a prompt step of the 7B shape (K 3,584) 300 rows took 115 us against 65 + 11 for the
+        library and the activation, 600: 163 against 103 + 16, 1,000: 209 against 167 + 25; with full tiles the two
+        are within 5 % (256: 72 / 80, 1,024: 194 / 192, 2,048: 375 / 379, 4,096: 749 / 772, 8,192: 1,576 / 1,586).
+        So the kernel takes the product when at most 2 % of its tiles' rows are padding."""
         K = self.lin.K
-        if K % 8 or K < 768 or rows < (TCGEN05_ROWS if K >= 1536 else 1024):
+        if K % 8 or K < 1536 or rows < (TCGEN05_ROWS if K >= 3072 else 1024):
             return False
-        return rows >= (0.98 if K >= 3072 else 0.92) * TCGEN05_ROWS * -(-rows // TCGEN05_ROWS)
+        return rows >= 0.98 * TCGEN05_ROWS * -(-rows // TCGEN05_ROWS)
 
     def activated(self, a) -> torch.Tensor:
         """act(a Wg^T) * (a Wu^T) in the activation dtype, [M, I]."""

@@ -793,9 +793,10 @@ def test_gemm_tcgen05_pair_modes(K, M, N, K_):
 
 
 def test_gemm_tcgen05_pair_gate_over_its_whole_range(K):
-    """SiLU in the gated epilogue, gates of either sign from 1e-30 to 1e30 and every hundredth up to 130: float32's quotient (2 ulp) and
-    exponential (2 ulp) in front of the rounding to bfloat16 (8 bits: at most 2^-8 of the value); a quotient by more than 2^126 is 0, so that of a gate
-    below -87.3 less than 88 * 2^-126 goes, times the up value's 3 at most."""
+    """SiLU in the gated epilogue, gates of either sign from 1e-30 to 1e30 and every hundredth up to 130: float32's quotient and
+    exponential (2 ulp) in front of the rounding to bfloat16 (8 bits: at most 2^-8 of the value).  The exponential of a gate below -88.72 is
+    infinite, so less than 89 * 2^-128 goes there, times the up value's 3 at most; down to it nothing does, so an infinite up value
+    stays infinite."""
     from cima_b200.kernels import SK_SWIGLU
     v = torch.cat([torch.arange(-13000, 13000).double() / 100, 10.0 ** torch.arange(-30, 31).double(), -10.0 ** torch.arange(-30, 31).double(), torch.zeros(1).double()])
     v = v.to(torch.bfloat16)
@@ -805,20 +806,35 @@ def test_gemm_tcgen05_pair_gate_over_its_whole_range(K):
     out = torch.empty(len(v), 16, dtype=torch.bfloat16, device="cuda")
     K.gemm_tc_pair(a.cuda(), w.cuda(), None, out, SK_SWIGLU)
     want = (v.double() * torch.sigmoid(v.double()))[:, None] * w[16:, 1].double()
-    assert bool(((out.cpu().double() - want).abs() <= 2.0 ** -8 * (1 + 2.0 ** -12) * want.abs() + 88 * 2.0 ** -126 * 3).all())
+    assert bool(((out.cpu().double() - want).abs() <= 2.0 ** -8 * (1 + 2.0 ** -12) * want.abs() + 89 * 2.0 ** -128 * 3).all())
+    w[16:, 1] = float("inf")
+    K.gemm_tc_pair(a.cuda(), w.cuda(), None, out, SK_SWIGLU)
+    some = (v > -88.7) & (v != 0)
+    assert torch.equal(out.cpu()[some].float(), (torch.sign(v[some].float()) * float("inf"))[:, None].expand(-1, 16))
     assert K.device_errors() == 0
 
 
-@pytest.mark.parametrize("inter,width,rows", [(40, 768, 943), (40, 768, 1500), (72, 1536, 236), (72, 1536, 300), (40, 3072, 251), (24, 760, 1024)])
-def test_gated_pair_on_the_kernel_its_rule_picks(K, inter, width, rows):
-    """Rows and sums on both sides of the rule that picks the fused tcgen05 product or the library's and the activation kernel.
-    Tolerance: gate, up and their product rounded to bfloat16 each, 2^-8 of the largest value they can pass on."""
+@pytest.mark.parametrize("inter,width,rows,fused", [(40, 768, 943, False), (40, 768, 1500, False), (72, 1536, 236, False), (72, 1536, 300, False),
+                                                    (40, 3072, 251, False), (24, 760, 1024, False), (40, 3072, 256, True), (40, 3072, 501, False),
+                                                    (40, 3072, 502, True), (24, 3064, 512, False),
+                                                    (24, 1536, 1024, True), (24, 1528, 1024, False), (24, 1536, 1023, False), (24, 1536, 1254, False),
+                                                    (24, 1536, 1255, True)])
+def test_gated_pair_on_the_kernel_its_rule_picks(K, inter, width, rows, fused):
+    """Rows and sums on both sides of the rule that picks the fused tcgen05 product or the library's and the activation kernel, and
+    which of them ran.  Tolerance: gate, up and their product rounded to bfloat16 each, 2^-8 of the largest value they can pass on."""
+    from cima_b200.engine.profile import StepProfile
     from cima_b200.parts.linear import GatedLinearPair
     from cima_b200.parts.runtime import Runtime
-    gate, up = (g(inter, width, seed=s, scale=1.0 / math.sqrt(width)) for s in (1, 2))
+    gate, up = (g(inter, width, dtype=torch.bfloat16, seed=s, scale=1.0 / math.sqrt(width)) for s in (1, 2))
     pair = GatedLinearPair(gate, up, Runtime(kernels=K, dtype=torch.bfloat16, device="cuda:0"))
     a = g(rows, width, dtype=torch.bfloat16, seed=rows)
-    got = pair.activated(a.cuda())
+    K.profile = seen = StepProfile()
+    try:
+        got = pair.activated(a.cuda())
+    finally:
+        K.profile = None
+    names = [launch.name for launch in seen.launches]
+    assert any("tcgen05" in n for n in names) == fused and any("swiglu" in n for n in names) != fused, names
     z = a.double() @ pair.lin.weight.cpu().double().t()
     want = REF.gate_act(z[:, :inter], 0) * z[:, inter:]
     assert err(got, want) <= 3 * 2.0 ** -8 * (z[:, :inter].abs().max() * z[:, inter:].abs().max()).item()
