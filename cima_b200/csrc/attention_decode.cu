@@ -292,8 +292,10 @@ k_attention_decode(const __nv_bfloat16* __restrict__ qkv, int ld, const __nv_bfl
     }
     const int h = h0 + r;
     if (n_splits == 1) {
-      // `sink` entries of score 0 without a value (0: an ordinary softmax), or one entry of the head's own score
-      l += (head_sink ? expf(head_sink[h]) : sink) * ex2(-Ms);
+      // `sink` entries of score 0 without a value (0: an ordinary softmax), or one entry of the head's own score; none is not
+      // added as 0 times the power of a low maximum, which may be infinite
+      const float extra = head_sink ? expf(head_sink[h]) : sink;
+      if (extra != 0.f) l += extra * ex2(-Ms);
       float res = l > 0.f ? acc / l : 0.f;
       if (gate_col > 0) res *= cima_sigmoid(__bfloat162float(qkv[(size_t)b * ld + gate_col + (size_t)h * HD + d]));      // the row's own gate
       out[(size_t)b * ldo + (size_t)h * HD + d] = __float2bfloat16_rn(res);
@@ -343,7 +345,8 @@ k_attention_combine(const float* __restrict__ part_o, const float* __restrict__ 
       L += ws * l[i];
     }
     for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-    L += (head_sink ? expf(head_sink[h]) : sink) * ex2(-Ms);
+    const float extra = head_sink ? expf(head_sink[h]) : sink;
+    if (extra != 0.f) L += extra * ex2(-Ms);
     if (threadIdx.x == 0) s_inv = L > 0.f ? 1.0f / L : 0.f;
   }
   __syncthreads();

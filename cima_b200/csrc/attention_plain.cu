@@ -80,7 +80,9 @@ k_attention_plain(const TA* __restrict__ qkv, int ld, const TA* __restrict__ cac
   TA* op = out + (size_t)row * ldo + (size_t)h * hd;
   // `sink` entries of score 0 that carry no value (0: an ordinary softmax); or, with `head_sink`, one entry whose score is
   // the head's own number (neither scaled nor attached to a value)
-  l += head_sink ? expf(head_sink[h] - m) : sink * expf(-m);
+  // (without either nothing is added: the exponential of a low maximum is infinite, and 0 times that no number)
+  if (head_sink) l += expf(head_sink[h] - m);
+  else if (sink != 0.f) l += sink * expf(-m);
   const float inv = l > 0.f ? 1.0f / l : 0.f;
 #pragma unroll
   for (int i = 0; i < NI; i++) {
@@ -309,7 +311,10 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
       const int v = i / HDP, d = i - v * HDP;
       if (d >= hd) continue;
       const int row = r0 + v / heads, h = h0 + v % heads;
-      const float m = run_m[v], l = run_l[v] + (a.head_sink ? expf(a.head_sink[h] - m) : a.sink * expf(-m));
+      const float m = run_m[v];
+      float l = run_l[v];
+      if (a.head_sink) l += expf(a.head_sink[h] - m);
+      else if (a.sink != 0.f) l += a.sink * expf(-m);    // (see k_attention_plain)
       const float gate = a.gate_col > 0 ? cima_sigmoid(a.qkv[(size_t)row * a.ld + a.gate_col + (size_t)h * hd + d]) : 1.0f;
       a.out[(size_t)row * a.ldo + (size_t)h * hd + d] = O[i] * (l > 0.f ? 1.0f / l : 0.f) * gate;
     }

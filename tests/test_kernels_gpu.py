@@ -389,6 +389,31 @@ def test_attention_float32_the_same_bits_however_cut(K, nh, nkv, hd, window, kee
     assert err(step[:n - 1], want[:n - 1]) <= TOL["float32"]
 
 
+@pytest.mark.parametrize("dtype,hd,n_splits", [("float32", 64, 0), ("float32", 300, 0), ("bfloat16", 64, 1), ("bfloat16", 64, 3)])
+def test_attention_without_a_sink_at_low_scores(K, dtype, hd, n_splits):
+    """An ordinary softmax whose scores all lie near -150, from one key (a sequence's first row) to 140: the exponential of minus the
+    maximum is infinite, and no entry is there for it to multiply.  ``n_splits``: the decode attention with so many splits (0: the plain
+    kernels, the two head sizes on the two of them)."""
+    nh, nkv, page, lens = 4, 2, 64, [1, 2, 65, 140]
+    tables, n_pages, width = scattered_tables(lens, list(range(4)), page, seed=hd)
+    cpu, gpu = make_kv(n_pages, nkv, page, hd, 4, width, 0, 0, DT[dtype], tables)
+    scale, size = 1.0 / math.sqrt(hd), math.sqrt(150 / math.sqrt(hd))
+    qkv = torch.full((4, (nh + 2 * nkv) * hd), -size).to(DT[dtype])
+    for slot, n in enumerate(lens):
+        fill_cache(cpu, gpu, slot, (size + 0.01 * g(n, nkv, hd, seed=slot)).to(DT[dtype]), g(n, nkv, hd, dtype=DT[dtype], seed=9 + slot))
+    seqs = [(slot, n - 1, 1) for slot, n in enumerate(lens)]
+    bc, bg = batch_of(seqs, "cpu"), batch_of(seqs, "cuda")
+    want = torch.zeros(4, nh * hd, dtype=torch.float64)
+    REF.attention_plain(qkv, cpu, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_first_row, want, nh, nkv, hd, scale, 0, True)
+    out = torch.full((4, nh * hd), 7.0, dtype=DT[dtype], device="cuda")
+    if n_splits:
+        K.attention_decode(qkv.cuda(), gpu, bg.seq_slot, bg.seq_len, out, nh, nkv, hd, scale, 0, n_splits=n_splits)
+    else:
+        K.attention_plain(qkv.cuda(), gpu, bg.row_pos, bg.row_seq, bg.seq_slot, bg.seq_first_row, out, nh, nkv, hd, scale, 0, True)
+    # float32: a score of 150 is off by the sum's steps, hd half ulps of it at most, and its exponential by that factor
+    assert err(out, want) <= (TOL["bfloat16"] if dtype == "bfloat16" else 2 * hd * 150 * 2.0 ** -24 * want.abs().max().item())
+
+
 @pytest.mark.parametrize("dtype,page", [("float32", 16), ("bfloat16", 16), ("bfloat16", 64)])
 @pytest.mark.parametrize("nh,nkv,hd", [(6, 2, 48), (7, 1, 128), (4, 4, 16), (28, 4, 128), (3, 3, 80), (40, 2, 64), (2, 1, 112)])
 def test_attention_decode_over_cache(K, dtype, page, nh, nkv, hd):
