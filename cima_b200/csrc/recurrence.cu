@@ -19,7 +19,8 @@
 //
 // A token is a chain of some 600 cycles (measured: 315 ns a token of the gate rule at key and value size 128), of which its
 // instructions fill a sixth, so few sequences leave the SMs waiting.  Long steps of the decay and the gate rule, whose states
-// nothing reads back before they are written, are therefore cut into segments of `seg` tokens that run side by side:
+// nothing reads back before they are written, are therefore cut into segments of `seg` tokens (counted from a sequence's first
+// row in the step) that run side by side:
 //   PHASE 1   every segment but a sequence's last, from S = 0, without read-out: what it adds, E (and the product of its
 //             gates, D; the decay rule's is a power of its constant)
 //   combine   the state in front of every segment: S_0 = the stored state, S_(i+1) = D_i S_i + E_i
@@ -46,11 +47,24 @@ __device__ __forceinline__ float rec_sum_over_lanes(float v) {        // over th
 // both, but a block covers 64 columns and a sequence gets half as many blocks: measured slower for one prompt (1.2 ms
 // against 0.97 ms a layer of 2,048 tokens at key and value size 128), so the launch takes one where a step is not cut.
 // MODE: 0 the decay rule, 1 the delta rule, 2 the gate rule.
+// The scratch follows the rows of the sequences that are cut, not the longest one's times their number: a sequence of r > seg rows from
+// row F of the step on has the places from 2 F / seg on (the next one's begin at 2 (F + r) / seg, at least r / seg rounded up later),
+// one of at most seg rows has none and works on its state as it is.  Blocks are numbered likewise, from F / seg + s on for sequence s.
 struct RecSegments {
-  float* buf;                  // [sequence x max_segs, heads, dim, vdim]: what a segment adds, then the state in front of it
-  float* prod;                 // the gate rule: [sequence x max_segs, heads, dim], a segment's product of gates
-  int seg, max_segs;
+  float* buf;                  // [2 rows / seg, heads, dim, vdim]: what a segment adds, then the state in front of it
+  float* prod;                 // the gate rule: [2 rows / seg, heads, dim], a segment's product of gates
+  int seg, n_seqs;             // seg 0: not cut
 };
+__device__ __forceinline__ int rec_sequence_of(const int* __restrict__ first, const RecSegments& s, int block) {
+  int lo = 0, hi = s.n_seqs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (first[mid] / s.seg + mid <= block) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+__device__ __forceinline__ size_t rec_place(int first, const RecSegments& s) { return (size_t)(2ll * first / s.seg); }
 
 template <typename TQ, typename TV, int DIMP, int MODE, int CPT, int PHASE>
 __global__ void __launch_bounds__(REC_THREADS)
@@ -70,18 +84,21 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
   __shared__ float sv[CH][COLS];
   __shared__ float so[CH][COLS];
   __shared__ float sb[CH];
-  const int seq = PHASE == 0 ? blockIdx.z : blockIdx.z / sg_.max_segs, h = blockIdx.y, col0 = blockIdx.x * COLS;
-  const int skip = PHASE == 0 ? 0 : (blockIdx.z - seq * sg_.max_segs) * sg_.seg;      // the sequence's tokens in front of the segment
+  const int seq = PHASE == 0 ? blockIdx.z : rec_sequence_of(seq_first_row, sg_, blockIdx.z), h = blockIdx.y, col0 = blockIdx.x * COLS;
+  const int row0 = seq_first_row[seq], rows = seq_first_row[seq + 1] - row0;
+  const int sidx = PHASE == 0 ? 0 : blockIdx.z - (row0 / sg_.seg + seq), skip = sidx * sg_.seg;      // the sequence's tokens in front of the segment
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rg = lane >> 2, lc = warp * 4 + (lane & 3);  // row group; the thread's columns are col0 + lc + 32 x
   const int kvh = h / (heads / kv_heads);
-  const int first = seq_first_row[seq] + skip, left = seq_first_row[seq + 1] - first;
+  const int first = row0 + skip, left = rows - skip;
   if (PHASE != 0 && left <= 0) return;
   const bool last = PHASE == 0 || left <= sg_.seg;
   if (PHASE == 1 && last) return;
   const int n = last ? left : sg_.seg;
   const size_t in_unit = ((size_t)h * dim) * (size_t)vdim + col0 + lc, unit = (size_t)heads * dim * vdim;
-  float* st = PHASE == 0 ? state + seq_slot[seq] * unit + in_unit : sg_.buf + blockIdx.z * unit + in_unit;
+  const bool whole = PHASE == 0 || rows <= sg_.seg;
+  const size_t place = whole ? 0 : rec_place(row0, sg_) + sidx;
+  float* st = whole ? state + seq_slot[seq] * unit + in_unit : sg_.buf + place * unit + in_unit;
   float S[CPT][RP];
 #pragma unroll
   for (int x = 0; x < CPT; x++)
@@ -289,7 +306,7 @@ k_recurrence(const TQ* __restrict__ q, int ldq, const TQ* __restrict__ k, int ld
     if (!last) return;
     st = state + seq_slot[seq] * unit + in_unit;
   }
-  if (GATE && PHASE == 1 && blockIdx.x == 0 && (int)threadIdx.x < dim) sg_.prod[((size_t)blockIdx.z * heads + h) * dim + threadIdx.x] = prod;
+  if (GATE && PHASE == 1 && blockIdx.x == 0 && (int)threadIdx.x < dim) sg_.prod[(place * heads + h) * dim + threadIdx.x] = prod;
 #pragma unroll
   for (int x = 0; x < CPT; x++)
 #pragma unroll
@@ -307,7 +324,9 @@ k_recurrence_combine(const float* __restrict__ state, const int* __restrict__ se
   cima_pdl_wait();
   const int size = dim * vdim, e = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, seq = blockIdx.z;
   if (e >= size) return;
-  const int segs = (seq_first_row[seq + 1] - seq_first_row[seq] + sg_.seg - 1) / sg_.seg;
+  const int row0 = seq_first_row[seq], segs = (seq_first_row[seq + 1] - row0 + sg_.seg - 1) / sg_.seg;
+  if (segs <= 1) return;
+  const size_t place = rec_place(row0, sg_);
   const float power = GATE ? 0.f : powf(decay[h], (float)sg_.seg);
   float S = state[((size_t)seq_slot[seq] * heads + h) * size + e];
   for (int s0 = 0; s0 < segs; s0 += 8) {                 // eight segments' values requested before the first is used
@@ -315,13 +334,13 @@ k_recurrence_combine(const float* __restrict__ state, const int* __restrict__ se
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const bool ok = s0 + i < segs - 1;                  // what the last segment adds was not made
-      const size_t at = ((size_t)seq * sg_.max_segs + (ok ? s0 + i : 0)) * heads + h;
+      const size_t at = (place + (ok ? s0 + i : 0)) * heads + h;
       E[i] = ok ? sg_.buf[at * size + e] : 0.f;
       D[i] = !ok ? 0.f : GATE ? sg_.prod[at * dim + e / vdim] : power;
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      if (s0 + i < segs) sg_.buf[(((size_t)seq * sg_.max_segs + s0 + i) * heads + h) * size + e] = S;
+      if (s0 + i < segs) sg_.buf[((place + s0 + i) * heads + h) * size + e] = S;
       S = fmaf(D[i], S, E[i]);
     }
   }
@@ -349,14 +368,15 @@ int launch_phase(const void* q, int ldq, const void* k, int ldk, const void* v, 
 template <typename TQ, typename TV, int MODE>
 int launch_recurrence(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const float* g, const float* beta,
                       const float* decay, float* state, const int* seq_slot, const int* seq_first_row, float* out,
-                      int n_seqs, int heads, int kv_heads, int dim, int vdim, const RecSegments& sg, cudaStream_t stream) {
+                      int T, int n_seqs, int heads, int kv_heads, int dim, int vdim, const RecSegments& sg, cudaStream_t stream) {
 #define PHASE_ARGS q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out
   if constexpr (MODE != 1) {
-    if (sg.max_segs > 1) {
-      if (int rc = launch_phase<TQ, TV, MODE, 1>(PHASE_ARGS, n_seqs * sg.max_segs, heads, kv_heads, dim, vdim, sg, stream)) return rc;
+    if (sg.seg > 0) {
+      const int blocks = T / sg.seg + n_seqs;
+      if (int rc = launch_phase<TQ, TV, MODE, 1>(PHASE_ARGS, blocks, heads, kv_heads, dim, vdim, sg, stream)) return rc;
       if (int rc = cima_launch(k_recurrence_combine<MODE == 2>, dim3((unsigned)((dim * vdim + 255) / 256), (unsigned)heads, (unsigned)n_seqs), dim3(256), (size_t)0,
                                stream, 1, (const float*)state, seq_slot, seq_first_row, decay, heads, dim, vdim, sg)) return rc;
-      return launch_phase<TQ, TV, MODE, 2>(PHASE_ARGS, n_seqs * sg.max_segs, heads, kv_heads, dim, vdim, sg, stream);
+      return launch_phase<TQ, TV, MODE, 2>(PHASE_ARGS, blocks, heads, kv_heads, dim, vdim, sg, stream);
     }
   }
   return launch_phase<TQ, TV, MODE, 0>(PHASE_ARGS, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
@@ -423,17 +443,16 @@ k_delta_prepare(const TA* __restrict__ qk, int ldqk, const TA* __restrict__ a, i
 // delta != 0: q, k float32 [T, kv_heads * dim] (prepared), v (vdtype) [T, ldv], g [T, heads * dim], beta [T, heads].
 // delta == 0: q, k, v of one dtype (vdtype), SiLU applied here; decay [heads].  out [T, heads * vdim] float32.
 // delta == 2 (the gate rule): q and k of v's dtype, k holding the gate's projection; g its bias and decay its lower bound,
-// both [heads * dim] and shared by all tokens.  max_segs > 1 (not the delta rule): the sequences are cut into at most so many
-// segments of `seg` tokens; buf [n_seqs * max_segs, heads, dim, vdim] and, for the gate rule, prod [n_seqs * max_segs, heads, dim]
-// float32 are their scratch.
+// both [heads * dim] and shared by all tokens.  seg > 0 (not the delta rule): sequences of more tokens are cut into segments of so
+// many; buf [2 T / seg, heads, dim, vdim] and, for the gate rule, prod [2 T / seg, heads, dim] float32 are their scratch.
 extern "C" int cima_recurrence(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, int vdtype,
                                const float* g, const float* beta, const float* decay, float* state, const int* seq_slot,
                                const int* seq_first_row, float* out, int T, int n_seqs, int heads, int kv_heads, int dim,
-                               int vdim, int delta, int seg, int max_segs, float* buf, float* prod, cudaStream_t stream) {
+                               int vdim, int delta, int seg, float* buf, float* prod, cudaStream_t stream) {
   if (T <= 0 || n_seqs <= 0) return 0;
-  if (max_segs > 1 && (delta == 1 || seg < 1 || !buf || (delta == 2 && !prod) || (long long)n_seqs * max_segs > 65535))
-    return cima_fail(CIMA_E_ARG, "recurrence: %d segments of %d tokens in %d sequences need their scratch, a rule without a delta and at most 65535 units", max_segs, seg, n_seqs);
-  const RecSegments sg{buf, prod, seg, max_segs};
+  if (seg < 0 || (seg > 0 && (delta == 1 || !buf || (delta == 2 && !prod) || (long long)T / seg + n_seqs > 65535)))
+    return cima_fail(CIMA_E_ARG, "recurrence: segments of %d of %d tokens in %d sequences need their scratch, a rule without a delta and at most 65535 blocks", seg, T, n_seqs);
+  const RecSegments sg{buf, prod, seg, n_seqs};
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || heads > 65535 || n_seqs > 65535)
     return cima_fail(CIMA_E_SIZE, "recurrence: %d heads on %d key heads in %d sequences are not accepted", heads, kv_heads, n_seqs);
   if (dim <= 0 || dim > 256 || vdim <= 0) return cima_fail(CIMA_E_SIZE, "recurrence: key size %d must lie in 1..256 and value size %d be positive", dim, vdim);
@@ -441,8 +460,8 @@ extern "C" int cima_recurrence(const void* q, int ldq, const void* k, int ldk, c
   if (delta == 2) {
     if (!g || !decay) return cima_fail(CIMA_E_ARG, "recurrence: the gate rule needs the gate's bias and lower bound");
     int rc2;
-    if (vdtype == CIMA_F32) rc2 = launch_recurrence<float, float, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
-    else if (vdtype == CIMA_BF16) rc2 = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    if (vdtype == CIMA_F32) rc2 = launch_recurrence<float, float, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, T, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    else if (vdtype == CIMA_BF16) rc2 = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 2>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, T, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
     else return cima_fail(CIMA_E_DTYPE, "recurrence: dtype code %d is neither float32 nor bfloat16", vdtype);
     return rc2 ? rc2 : cima_launch_result();
   }
@@ -450,12 +469,12 @@ extern "C" int cima_recurrence(const void* q, int ldq, const void* k, int ldk, c
   if (!delta && !decay) return cima_fail(CIMA_E_ARG, "recurrence: the decay rule needs the heads' decays");
   int rc;
   if (delta) {
-    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
-    else if (vdtype == CIMA_BF16) rc = launch_recurrence<float, __nv_bfloat16, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, T, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    else if (vdtype == CIMA_BF16) rc = launch_recurrence<float, __nv_bfloat16, 1>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, T, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
     else return cima_fail(CIMA_E_DTYPE, "recurrence: dtype code %d is neither float32 nor bfloat16", vdtype);
   } else {
-    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
-    else if (vdtype == CIMA_BF16) rc = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    if (vdtype == CIMA_F32) rc = launch_recurrence<float, float, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, T, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
+    else if (vdtype == CIMA_BF16) rc = launch_recurrence<__nv_bfloat16, __nv_bfloat16, 0>(q, ldq, k, ldk, v, ldv, g, beta, decay, state, seq_slot, seq_first_row, out, T, n_seqs, heads, kv_heads, dim, vdim, sg, stream);
     else return cima_fail(CIMA_E_DTYPE, "recurrence: dtype code %d is neither float32 nor bfloat16", vdtype);
   }
   return rc ? rc : cima_launch_result();

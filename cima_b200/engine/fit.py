@@ -40,11 +40,12 @@ class Forecast:
 
 def forecast(plan: Dict[str, object], requests: Sequence[Sequence[object]], dtype: torch.dtype, max_tokens: int,
              hidden: int, vocab: int, widest: int, page_size: int = 64, shares: Sequence[int] = (),
-             extra_state: Sequence[StateRequest] = (), max_seqs: int = 0, streams: int = 1) -> Forecast:
+             extra_state: Sequence[StateRequest] = (), max_seqs: int = 0, streams: int = 1, segment_row: float = 0.0) -> Forecast:
     """``plan``: name -> TensorSpec (matrices are kept in ``dtype``, vectors in float32).  ``requests[i]``: what
     the mixer at site i asks of the cache.  ``widest``: the widest activation row of a layer (its gated
     intermediate, twice, or its q/k/v row).  ``streams``: float32 copies of the residual stream that a step holds
-    (1, or with a depth average one per site and two more)."""
+    (1, or with a depth average one per site and two more).  ``segment_row``: bytes a row of the states that a recurrence keeps
+    while a long step runs in segments."""
     elt = 4 if dtype is torch.float32 else 2
     weights = 0
     for spec in plan.values():
@@ -73,7 +74,7 @@ def forecast(plan: Dict[str, object], requests: Sequence[Sequence[object]], dtyp
     from .graph import MAX_PROMPT_GRAPHS, recorded_prompt_rows
     row = hidden * 4 * max(1, streams) + (widest + 2 * hidden) * elt
     rows = min(max_tokens, STEP_ROWS)
-    scratch = rows * row + min(n_slots, 256) * vocab * 4 * 2
+    scratch = int(rows * (row + segment_row)) + min(n_slots, 256) * vocab * 4 * 2
     scratch += MAX_PROMPT_GRAPHS * min(max_tokens, recorded_prompt_rows(weights, len(requests), elt)) * row
     return Forecast(weights, cache, scratch)
 

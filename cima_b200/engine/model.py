@@ -215,10 +215,13 @@ class Model:
         sched = self.spec.schedule
         shares = [site for site, layer in enumerate(sched) if self.spec.layers[layer].mixer.cache_from is not None]
         widest = max([int(getattr(b, "scratch_row", lambda: 0)()) for b in self.blocks] + [self.spec.hidden])
+        mixers = [m for b in self.blocks if hasattr(b, "mixer") for m in getattr(b.mixer, "branches", [b.mixer])]
+        segment_row = max([float(getattr(m, "segment_row", 0.0)) for m in mixers], default=0.0) if self.rt.dtype is torch.bfloat16 else 0.0
         return forecast(self.plan(), self._cache_requests(),
                         self.rt.dtype, max_tokens, self.spec.hidden, self.spec.vocab, widest, page_size, shares,
                         extra_state, max_seqs or 0,
-                        streams=len(sched) + 2 if self.depth is not None else (self.spec.streams + 1 if self.spec.stream == "hyper" else 1))
+                        streams=len(sched) + 2 if self.depth is not None else (self.spec.streams + 1 if self.spec.stream == "hyper" else 1),
+                        segment_row=segment_row)
 
     # ------------------------------------------------------------------ the step
     def step(self, entries: Sequence[StepEntry]) -> torch.Tensor:

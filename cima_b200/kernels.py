@@ -15,7 +15,7 @@ import torch
 from .csrc.build import BuildError, library_path
 
 F32, BF16 = 0, 1
-ABI_VERSION = 34
+ABI_VERSION = 35
 SPLIT_BLOCKS = 296          # blocks of the decode attention that one wave holds (two per SM, 148 SMs)
 TC_ATTENTION_MIN_LEN = 256  # prompts from this length on take the tcgen05 attention (head_dim 64 or 128)
 SPLIT_FEW_BLOCKS = 148      # below this many blocks at 8 splits, more splits are taken
@@ -101,7 +101,7 @@ _SIGNATURES = {
     "cima_dyt_add": [_vp, _vp, _vp, _vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _i, _i, _vp],
     "cima_embed_bigram": [_vp, _vp, _vp, _i, _vp, _i, _i, _i, _f, _i, ctypes.c_longlong, ctypes.c_longlong, _vp, _vp, _vp, _vp, _vp,
                           _i, _vp],
-    "cima_recurrence": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
+    "cima_recurrence": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp],
     "cima_delta_prepare": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "cima_delta_rule": [_vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "cima_group_rmsnorm_gate": [_vp, _vp, _vp, _i, _i, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _f, _vp],
@@ -1037,12 +1037,16 @@ class Kernels:
         blocks of 32 value channels, all heads.  Uncut, a sequence takes 600 cycles a token; cut, a block's token costs the SM some
         110 cycles of instructions, half as many again for the first phase, and three launches and the states' way through memory
         come to some 30,000 cycles: cut where that is less than the longest sequence's chain.  bfloat16 rows only (a 32-bit row has
-        the same bits however its sequence is cut)."""
+        the same bits however its sequence is cut).  Where a sequence is cut depends on the step, so a bfloat16 sequence's bits do."""
         rows = int(getattr(batch, "max_rows", 0) or 0)
         segs = -(-rows // self.RECURRENCE_SEGMENT)
-        if dtype is not torch.bfloat16 or rows < 2 * self.RECURRENCE_SEGMENT or 1.2 * batch.n_rows * columns + 30000 > 600 * rows or batch.n_seqs * segs > 65535:
+        if dtype is not torch.bfloat16 or rows < 2 * self.RECURRENCE_SEGMENT or 1.2 * batch.n_rows * columns + 30000 > 600 * rows or batch.n_rows // self.RECURRENCE_SEGMENT + batch.n_seqs > 65535:
             return 1
         return segs
+
+    def _segment_scratch(self, batch, values: int, device) -> torch.Tensor:
+        """Scratch of a cut step: ``values`` float32 a segment, two places for every full segment's worth of rows (recurrence.cu)."""
+        return torch.empty(2 * batch.n_rows // self.RECURRENCE_SEGMENT * values, dtype=torch.float32, device=device)
 
     def recurrence(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, batch, out: torch.Tensor,
                    heads: int, kv_heads: int, dim: int, vdim: int, g: Optional[torch.Tensor] = None,
@@ -1078,14 +1082,14 @@ class Kernels:
                            batch.n_seqs * heads * dim * vdim * 8 + T * (2 * kv_heads * dim * q.element_size() + heads * vdim * (4 + v.element_size())
                                                                         + (heads * dim * 4 if delta else 0)),
                            (8.0 if delta else 5.0) * T * heads * dim * vdim): return
-        segs = 1 if delta else self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype)
-        buf = torch.empty(batch.n_seqs * segs * heads * dim * vdim, dtype=torch.float32, device=q.device) if segs > 1 else None
+        cut = not delta and self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype) > 1
+        buf = self._segment_scratch(batch, heads * dim * vdim, q.device) if cut else None
         self._check(self.lib.cima_recurrence(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
                                              dtype_code(v.dtype), _ptr(g), _ptr(beta), _ptr(decay), state.data_ptr(),
                                              batch.seq_slot.data_ptr(), batch.seq_first_row.data_ptr(), out.data_ptr(), T,
-                                             batch.n_seqs, heads, kv_heads, dim, vdim, int(delta), self.RECURRENCE_SEGMENT, segs, _ptr(buf), None,
+                                             batch.n_seqs, heads, kv_heads, dim, vdim, int(delta), self.RECURRENCE_SEGMENT if cut else 0, _ptr(buf), None,
                                              self._stream()), "recurrence")
-        if segs > 1:
+        if cut:
             self.launches += 2
 
     def _recurrence_gate(self, q, k, v, state, batch, out, heads, kv_heads, dim, vdim, bias, lower) -> None:
@@ -1102,17 +1106,17 @@ class Kernels:
                               f"out {tuple(out.shape)} and the gate's vectors do not agree with {heads} heads of {dim} x {vdim}")
         if not self._admit("recurrence[gate]", batch.n_seqs * heads * dim * vdim * 8 + T * heads * ((2 * dim + vdim) * v.element_size() + vdim * 4),
                            5.0 * T * heads * dim * vdim): return
-        segs = self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype)
+        cut = self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype) > 1
         buf = prod = None
-        if segs > 1:
-            buf = torch.empty(batch.n_seqs * segs * heads * dim * vdim, dtype=torch.float32, device=q.device)
-            prod = torch.empty(batch.n_seqs * segs * heads * dim, dtype=torch.float32, device=q.device)
+        if cut:
+            buf = self._segment_scratch(batch, heads * dim * vdim, q.device)
+            prod = self._segment_scratch(batch, heads * dim, q.device)
         self._check(self.lib.cima_recurrence(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
                                              dtype_code(v.dtype), bias.data_ptr(), None, lower.data_ptr(), state.data_ptr(),
                                              batch.seq_slot.data_ptr(), batch.seq_first_row.data_ptr(), out.data_ptr(), T,
-                                             batch.n_seqs, heads, kv_heads, dim, vdim, 2, self.RECURRENCE_SEGMENT, segs, _ptr(buf), _ptr(prod),
+                                             batch.n_seqs, heads, kv_heads, dim, vdim, 2, self.RECURRENCE_SEGMENT if cut else 0, _ptr(buf), _ptr(prod),
                                              self._stream()), "recurrence")
-        if segs > 1:
+        if cut:
             self.launches += 2
 
     def delta_prepare(self, qk: torch.Tensor, a: torch.Tensor, b: torch.Tensor, A_log: torch.Tensor, dt_bias: torch.Tensor,

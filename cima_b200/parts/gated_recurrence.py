@@ -69,6 +69,13 @@ class GatedRecurrence:
     def scratch_row(self) -> int:
         return 2 * self.qd + 4 * self.vd
 
+    @property
+    def segment_row(self) -> float:
+        """Bytes a row of the segments' states in a long bfloat16 step: two places of a state (and of a column of it) for every
+        full segment's worth of rows."""
+        from ..kernels import Kernels
+        return 2.0 * self.heads * self.dim * (self.vdim + 1) * 4 / Kernels.RECURRENCE_SEGMENT
+
     graph_safe = True
 
     @staticmethod

@@ -31,6 +31,33 @@ def test_forecast_counts_what_is_allocated():
     assert half.cache * 2 == fc.cache          # bfloat16 keys and values
 
 
+def test_forecast_counts_the_segments_of_a_long_steps_recurrence():
+    """Two states (and a column of one) for every 128 rows of the largest step, of the mixer with the largest state; bfloat16 only,
+    as 32-bit sequences are not cut."""
+    import gisirax_cases
+    from cima_b200.engine import fit
+    m = gisirax_cases.cpu_model("C", "bfloat16", max_tokens=640)
+    seen = {}
+    plain, fit.forecast = fit.forecast, lambda *a, **kw: (seen.update(kw), plain(*a, **kw))[1]
+    try:
+        with_segments = m.forecast(20000)
+    finally:
+        fit.forecast = plain
+    rights = [l["mixer"]["right"] for l in gisirax_cases.CONFIGS["C"]["layers"] if l["type"] == "parallel"]
+    row = max(2.0 * r["heads"] * r["dim"] * (r["vdim"] + 1) * 4 / 128 for r in rights)
+    assert seen["segment_row"] == row
+    args = (m.plan(), m._cache_requests(), torch.bfloat16, 20000, 256, 640, 512)
+    assert plain(*args, segment_row=row).scratch - plain(*args).scratch == int(fit.STEP_ROWS * row)
+    assert with_segments.scratch > plain(*args).scratch
+    seen.clear()
+    fit.forecast = lambda *a, **kw: (seen.update(kw), plain(*a, **kw))[1]
+    try:
+        gisirax_cases.cpu_model("C", "float32", max_tokens=640).forecast(640)
+    finally:
+        fit.forecast = plain
+    assert seen["segment_row"] == 0.0
+
+
 @pytest.mark.gpu
 def test_a_cache_that_cannot_fit_is_refused_before_allocating():
     from cima_b200.engine import load_model

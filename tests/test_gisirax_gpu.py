@@ -203,6 +203,39 @@ def test_decay_rule_of_long_sequences_in_segments(heads, dim, vdim):
     _recurrence_case(False, heads, heads, dim, vdim, "bfloat16", steps, seed=dim)
 
 
+@pytest.mark.parametrize("gate", [False, True])
+def test_segments_scratch_follows_the_rows_that_are_cut(gate):
+    """One sequence of 2,048 tokens, one of 300 and 62 of one to eleven: the scratch is two states for every segment's worth of rows,
+    not the longest one's segments times the sequences; each sequence gives what it gives alone, and its state with it."""
+    heads, dim, vdim = 2, 64, 64
+    counts = [1 + i % 11 for i in range(30)] + [2048] + [1 + i % 7 for i in range(20)] + [300] + [1 + i % 5 for i in range(12)]
+    assert len(counts) == 64 and K().recurrence_segments(SimpleNamespace(max_rows=2048, n_rows=sum(counts), n_seqs=64), 2 * heads, torch.bfloat16) == 16
+    g = torch.Generator().manual_seed(3)
+    rows = torch.randn(sum(counts), heads * (2 * dim + vdim), generator=g).bfloat16().to(DEV)
+    start = torch.randn(64, heads, dim, vdim, generator=g).to(DEV)
+    kw = dict(gate=(torch.randn(heads * dim, generator=g).to(DEV), (torch.rand(heads * dim, generator=g) * 0.9).to(DEV))) if gate else dict(decay=torch.tensor([0.9, 0.99]).to(DEV))
+
+    def run(x, state, b):
+        o = torch.empty(b.n_rows, heads * vdim, dtype=torch.float32, device=DEV)
+        K().recurrence(x[:, :heads * dim], x[:, heads * dim:2 * heads * dim], x[:, 2 * heads * dim:], state, b, o, heads, heads, dim, vdim, **kw)
+        return o
+
+    state = start.clone()
+    b = entries_batch(counts, [0] * 64, list(range(64)))
+    run(rows[:1], state.clone(), entries_batch([1], [0], [0]))
+    torch.cuda.synchronize(); torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    out = run(rows, state, b)
+    torch.cuda.synchronize()
+    own = out.numel() * 4 + 2 * sum(counts) // K().RECURRENCE_SEGMENT * heads * dim * (vdim + 1) * 4
+    assert torch.cuda.max_memory_allocated() - before <= own + 4096          # (allocations are rounded up to 512 bytes)
+    alone, r = start.clone(), 0
+    for i, n in enumerate(counts):
+        assert torch.equal(run(rows[r:r + n], alone, entries_batch([n], [0], [i])), out[r:r + n]), (i, n)
+        r += n
+    assert torch.equal(alone, state)
+
+
 def test_recurrence_long_decoding_holds_its_state():
     _recurrence_case(True, 2, 1, 32, 32, "float32", [[3, 1]] + [[1, 1]] * 150, seed=5)
     _recurrence_case(False, 2, 2, 32, 32, "bfloat16", [[3, 1]] + [[1, 1]] * 150, seed=6)
