@@ -173,8 +173,6 @@ class Kernels:
             fn.restype = ctypes.c_int
         self.launches = 0
         self.library_launches = 0   # matrix products handed to the library (not counted in ``launches``)
-        self._scratch_bufs = {}
-        self._retired = []          # replaced scratch buffers, kept alive for the graphs recorded with them
         self._error_flag = None
         self.profile = None         # a StepProfile while a step's launches are being counted and timed
 
@@ -706,8 +704,10 @@ class Kernels:
         if not self._admit(f"attention_decode[{n_splits} splits]", *self._attention_work(qkv, n_heads, n_kv_heads, head_dim, kv.planes)): return
         part_o = part_ml = None
         if n_splits > 1:
-            part_o = self._scratch("attn_o", B * n_heads * n_splits * head_dim, qkv.device)
-            part_ml = self._scratch("attn_ml", B * n_heads * n_splits * 2, qkv.device)
+            # this call's own, from the recording's memory where the step is recorded: another stream's step, or another recording's
+            # replay, may be between its splits and their merge at the same time
+            part = torch.empty(B * n_heads * n_splits * (head_dim + 2), dtype=torch.float32, device=qkv.device)
+            part_o, part_ml = part, part[B * n_heads * n_splits * head_dim:]
         self._check(self.lib.cima_attention_decode(
             qkv.data_ptr(), qkv.shape[1], kv.storage.data_ptr(), kv.block_table.data_ptr(), kv.block_table.shape[1],
             kv.ring_pages, kv.page_size, seq_slot.data_ptr(), seq_len.data_ptr(), _ptr(part_o), _ptr(part_ml),
@@ -715,17 +715,6 @@ class Kernels:
             kv.planes, sink, keep_first, v_group, _ptr(head_sink), gate_col, _ptr(slopes), self._stream()), "attention_decode")
         if n_splits > 1:
             self.launches += 1
-
-    def _scratch(self, name: str, numel: int, device) -> torch.Tensor:
-        """Float32 scratch that lives as long as this object (grown on demand, outside graph capture:
-        a captured step always follows an eager one of the same sizes).  A buffer that a larger one replaces is
-        kept, not freed: a captured step holds the address it was recorded with and goes on writing there."""
-        t = self._scratch_bufs.get(name)
-        if t is None or t.numel() < numel or t.device != torch.device(device):
-            if t is not None:
-                self._retired.append(t)
-            t = self._scratch_bufs[name] = torch.empty(numel, dtype=torch.float32, device=device)
-        return t
 
     # ------------------------------------------------------------------ short convolution, depth average, latents
     def short_conv(self, h: torch.Tensor, w: torch.Tensor, state: Optional[torch.Tensor], batch, out: torch.Tensor,

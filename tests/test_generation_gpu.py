@@ -620,3 +620,34 @@ def test_one_token_steps_recorded_give_what_issued_ones_give(name, dtype):
     assert rec.step([StepEntry(slots[0][0], [1], [])]).shape[0] == 0
     ref.step([StepEntry(slots[1][0], [1], [])])
     both([0, 1, 2])
+
+
+def test_one_token_steps_on_two_streams_at_split_contexts():
+    """Two streams, each with two sequences of some 1,500 positions (a decode attention of several splits and their merge), step side by
+    side without waiting for one another: the logits are those of a model whose steps run one after the other on one stream."""
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    kw = dict(config=dict(SHAPES["qwen2.5-0.5b"], num_hidden_layers=4, max_position_embeddings=4096), seed=3, draw="device", max_tokens=8192, max_seqs=4, verbose=False)
+    rec, ref = cima_b200.load(**kw), cima_b200.load(**kw)
+    assert rec.model.short_context < 1400
+    g = torch.Generator().manual_seed(5)
+    prompts = [torch.randint(0, rec.spec.vocab, (n,), generator=g).tolist() for n in (1500, 1411, 1533, 1600)]
+    tokens = torch.randint(0, rec.spec.vocab, (12, 4), generator=g).tolist()
+    pairs = []
+    for lm in (rec, ref):
+        slots = lm.model.cache.open(4)
+        lm.step([StepEntry(s, p, [len(p) - 1]) for s, p in zip(slots, prompts)])
+        pairs.append((slots[:2], slots[2:]))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got, want = [], []
+    for row in tokens:
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got.append(rec.step([StepEntry(s, [t], [0]) for s, t in zip(pairs[0][i], row[2 * i:2 * i + 2])]))
+    torch.cuda.synchronize()
+    for row in tokens:
+        for i in range(2):
+            want.append(ref.step([StepEntry(s, [t], [0]) for s, t in zip(pairs[1][i], row[2 * i:2 * i + 2])]))
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
