@@ -177,7 +177,7 @@ class PromptGraph:
         return self.logits
 
 
-MAX_STEP_GRAPHS = 16      # recorded one-token steps kept (by sequences, context class and stream); the one used longest ago gives way
+MAX_STEP_GRAPHS = 16      # recorded one-token steps kept (by sequences and context class); the one used longest ago gives way
 STEP_GRAPH_ROWS = 64      # most sequences of a recorded one-token step
 
 

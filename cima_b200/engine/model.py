@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import dataclasses
 import sys
+import threading
 from collections import OrderedDict
 from typing import Dict, List, Optional, Sequence
 
@@ -74,7 +75,9 @@ class Model:
         self.config = None                                  # set by load_model
         self.step_rows = STEP_ROWS                          # a step of more rows runs in parts
         self.record_steps = False                           # record one-token steps (``StepGraph``); an ``LM`` with graphs says so
-        self._step_graphs = OrderedDict()                   # (sequences, context bound, stream) -> StepGraph, the newest last
+        self._step_graphs = OrderedDict()                   # (sequences, context bound) -> StepGraph, the newest last
+        self._step_lock = threading.Lock()                  # a recorded step's inputs and launch belong together
+        self._step_done = None                              # event behind the last recorded step, whatever stream it ran on
         self.embedding: Optional[torch.Tensor] = None
         self.bigram: Optional[torch.Tensor] = None          # the hashed bigram table, where the spec has one
         self.positions: Optional[torch.Tensor] = None       # the vectors added at each position, where the spec has a table
@@ -247,7 +250,8 @@ class Model:
         if limit is not None and any(starts) and max(len(e.tokens) for e in entries) > limit:
             return self._step_in_rounds(entries, limit)
         if self._recordable(entries):
-            return self._step_recorded(entries, starts)
+            with self._step_lock:
+                return self._step_recorded(entries, starts)
         batch = build_batch(entries, starts, self.spec.vocab, self.rt.device)
         for e, s in zip(entries, starts):
             cache.reserve(e.slot, s + len(e.tokens))
@@ -269,11 +273,16 @@ class Model:
         from .graph import MAX_STEP_GRAPHS, StepGraph
         check_entries(entries, self.spec.vocab)
         cache, short = self.cache, self.short_context
+        # The recordings' inputs and memory serve every stream and thread: a step waits for the one before it, wherever that ran.
+        stream = torch.cuda.current_stream()
+        if self._step_done is None:
+            self._step_done = torch.cuda.Event()
+        else:
+            stream.wait_event(self._step_done)
         for e, s in zip(entries, starts):
             cache.reserve(e.slot, s + 1)
         cache.flush()
-        # a stream's steps follow one another; another stream's have buffers of their own
-        key = (len(entries), short if max(starts) + 1 <= short else 0, torch.cuda.current_stream().cuda_stream)
+        key = (len(entries), short if max(starts) + 1 <= short else 0)
         g = self._step_graphs.get(key)
         if g is None:
             g = self._step_graphs[key] = StepGraph(self, key[0], key[1])
@@ -281,7 +290,10 @@ class Model:
                 torch.cuda.synchronize()                    # the one that goes may still be running
                 self._step_graphs.popitem(last=False)
         self._step_graphs.move_to_end(key)
-        logits = g.run([e.slot for e in entries], [int(e.tokens[0]) for e in entries], starts)
+        try:
+            logits = g.run([e.slot for e in entries], [int(e.tokens[0]) for e in entries], starts)
+        finally:
+            self._step_done.record(stream)
         for e, s in zip(entries, starts):
             cache.commit(e.slot, s + 1)
         return logits

@@ -651,3 +651,42 @@ def test_one_token_steps_on_two_streams_at_split_contexts():
             want.append(ref.step([StepEntry(s, [t], [0]) for s, t in zip(pairs[1][i], row[2 * i:2 * i + 2])]))
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_one_token_steps_from_several_threads():
+    """Four threads, each with a sequence of its own, feed tokens at the same time, two on the default stream and two on streams of
+    their own: each gets the logits that it gets alone."""
+    import threading
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    kw = dict(config=SHAPES["tiny-b"], seed=3, max_tokens=1024, max_seqs=4, verbose=False)
+    rec, ref = cima_b200.load(**kw), cima_b200.load(**kw)
+    g = torch.Generator().manual_seed(5)
+    feeds = torch.randint(0, rec.spec.vocab, (4, 25), generator=g).tolist()
+    slots = [lm.model.cache.open(4) for lm in (rec, ref)]
+    for lm, held in zip((rec, ref), slots):
+        lm.step([StepEntry(s, [7 + i, 3], [1]) for i, s in enumerate(held)])
+    torch.cuda.synchronize()
+    got, wrong = [[] for _ in range(4)], []
+
+    def feed(i):
+        try:
+            stream = torch.cuda.Stream() if i % 2 else torch.cuda.default_stream()
+            with torch.cuda.stream(stream):
+                for t in feeds[i]:
+                    got[i].append(rec.step([StepEntry(slots[0][i], [t], [0])]))
+                stream.synchronize()
+        except Exception as e:                               # (a thread's exception is not pytest's)
+            wrong.append(e)
+
+    threads = [threading.Thread(target=feed, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not wrong, wrong
+    for i in range(4):
+        for t, logits in zip(feeds[i], got[i]):
+            assert torch.equal(logits, ref.step([StepEntry(slots[1][i], [t], [0])])), i
+    assert len(rec.model._step_graphs) == 1                  # whatever the stream, one recording
