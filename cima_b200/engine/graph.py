@@ -185,7 +185,8 @@ class StepGraph:
     """``Model.step`` for sequences that bring one token each, all logits wanted, recorded: what a caller that feeds tokens
     itself runs again and again.  Issued launch by launch, such a step waits for the host (about 100 us a layer: 2.75 ms at the
     24 layers of the 0.5B shape, where the device works 0.5; 3.4 against 1.2 at 1.5B).  A shape's first step is issued as it is,
-    its second is recorded as well, from the third on the recording is replayed; every call gets logits of its own."""
+    its second is recorded as well, from the third on the recording is replayed; every call gets logits of its own.  A shape that
+    cannot be recorded (no memory left for it) goes on being issued."""
 
     def __init__(self, model, n_seqs: int, max_len: int):
         self.model, self.n_seqs = model, n_seqs
@@ -194,9 +195,11 @@ class StepGraph:
         self.graph = None
         self.logits = None
         self.uses = 0
+        self.recordable = True
 
     def run(self, slots: Sequence[int], tokens: Sequence[int], lengths: Sequence[int]) -> torch.Tensor:
-        """Float32 logits [sequences, vocab].  The caller has reserved the new position of every slot and commits it."""
+        """Float32 logits [sequences, vocab].  The caller has reserved the new position of every slot and commits it, then asks for
+        the recording (``record``)."""
         host = torch.empty(6 * self.n_seqs + 1, dtype=torch.int32, pin_memory=True)      # its own each time: the copy may still be under way
         fill_meta(host.numpy(), slots, tokens, lengths)
         self.meta.copy_(host, non_blocking=True)
@@ -204,15 +207,22 @@ class StepGraph:
             self.graph.replay()
             return self.logits.clone()
         self.uses += 1
-        out = self.model.forward(self.batch)
-        if self.uses >= 2:
-            g, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
-            side.wait_stream(torch.cuda.current_stream())
+        return self.model.forward(self.batch)
+
+    def record(self) -> None:
+        """Behind the shape's second step, when its positions are committed: a step is whole whether or not its recording succeeds."""
+        if self.graph is not None or self.uses < 2 or not self.recordable:
+            return
+        g, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        try:
             with torch.cuda.stream(side):
                 g.capture_begin(capture_error_mode="thread_local")
                 try:
-                    self.logits = self.model.forward(self.batch)      # recorded, not run
+                    logits = self.model.forward(self.batch)      # recorded, not run
                 finally:
                     g.capture_end()
-            self.graph = g
-        return out
+        except RuntimeError:
+            self.recordable = False
+            return
+        self.graph, self.logits = g, logits

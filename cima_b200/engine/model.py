@@ -296,6 +296,7 @@ class Model:
             self._step_done.record(stream)
         for e, s in zip(entries, starts):
             cache.commit(e.slot, s + 1)
+        g.record()
         return logits
 
     def _step_in_parts(self, entries: Sequence[StepEntry]) -> torch.Tensor:

@@ -690,3 +690,31 @@ def test_one_token_steps_from_several_threads():
         for t, logits in zip(feeds[i], got[i]):
             assert torch.equal(logits, ref.step([StepEntry(slots[1][i], [t], [0])])), i
     assert len(rec.model._step_graphs) == 1                  # whatever the stream, one recording
+
+
+@pytest.mark.parametrize("name", ["tiny-b", "gisirax-tiny"])
+def test_a_one_token_step_whose_recording_fails_is_a_step(name, monkeypatch):
+    """The recording behind a shape's second step has no memory: the step's logits come back, its token is counted once (recurrent
+    states have moved on with it) and later steps of the shape are issued, without another attempt."""
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    kw = dict(config=SHAPES[name], seed=3, max_tokens=1024, max_seqs=4, verbose=False)
+    rec, ref = cima_b200.load(**kw), cima_b200.load(use_graphs=False, **kw)
+    slots = [lm.model.cache.open(2) for lm in (rec, ref)]
+    for lm, held in zip((rec, ref), slots):
+        lm.step([StepEntry(s, [7 + i, 3, 5], [2]) for i, s in enumerate(held)])
+    issue, attempts = rec.model.forward, []
+
+    def forward(batch):
+        if torch.cuda.is_current_stream_capturing():
+            attempts.append(1)
+            issue(batch)
+            raise torch.OutOfMemoryError("planted")
+        return issue(batch)
+
+    monkeypatch.setattr(rec.model, "forward", forward)
+    for n, t in enumerate([11, 12, 13, 14]):
+        out = [lm.step([StepEntry(s, [t + i], [0]) for i, s in enumerate(held)]) for lm, held in zip((rec, ref), slots)]
+        assert (out[0] - out[1]).abs().max() <= 2e-2 * out[1].std()
+        assert [rec.model.cache.length(s) for s in slots[0]] == [4 + n] * 2
+    assert len(attempts) == 1 and not any(x.graph for x in rec.model._step_graphs.values())
