@@ -177,7 +177,8 @@ class PromptGraph:
         return self.logits
 
 
-MAX_STEP_GRAPHS = 16      # recorded one-token steps kept (by sequences and context class); the one used longest ago gives way
+MAX_STEP_GRAPHS = 16      # recorded one-token steps kept (by sequences and context class)
+STEP_GRAPH_IDLE = 256     # with so many kept, a new shape takes the place of one that the last so many steps did not use, or is issued
 STEP_GRAPH_ROWS = 64      # most sequences of a recorded one-token step
 
 
@@ -195,6 +196,7 @@ class StepGraph:
         self.graph = None
         self.logits = None
         self.uses = 0
+        self.last = 0                              # number of the model's one-token step that used it last
         self.recordable = True
 
     def run(self, slots: Sequence[int], tokens: Sequence[int], lengths: Sequence[int]) -> torch.Tensor:

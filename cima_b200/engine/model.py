@@ -76,6 +76,7 @@ class Model:
         self.step_rows = STEP_ROWS                          # a step of more rows runs in parts
         self.record_steps = False                           # record one-token steps (``StepGraph``); an ``LM`` with graphs says so
         self._step_graphs = OrderedDict()                   # (sequences, context bound) -> StepGraph, the newest last
+        self._steps = 0                                     # one-token steps so far
         self._step_lock = threading.Lock()                  # a recorded step's inputs and launch belong together
         self._step_done = None                              # event behind the last recorded step, whatever stream it ran on
         self.embedding: Optional[torch.Tensor] = None
@@ -115,7 +116,7 @@ class Model:
         """``tensors``: name -> tensor, a dict or a ``TensorSource`` that fetches each tensor when it is asked for
         (every name of the plan is asked for once)."""
         s = self.spec
-        self._step_graphs.clear()
+        self._forget_step_graphs()
         table = tensors[s.embed_name]
         self.embedding = self.rt.matrix(table)
         if s.tie_head:
@@ -192,7 +193,7 @@ class Model:
         sched = self.spec.schedule
         shares = {site: self.spec.layers[layer].mixer.cache_from for site, layer in enumerate(sched)
                   if self.spec.layers[layer].mixer.cache_from is not None}
-        self._step_graphs.clear()                           # recorded with the cache before
+        self._forget_step_graphs()                          # recorded with the cache before
         self.cache = KVCache(self._cache_requests(),
                              max_tokens, self.spec.max_position,
                              self.rt.dtype, self.rt.device, page_size=page_size, max_seqs=max_seqs,
@@ -251,7 +252,9 @@ class Model:
             return self._step_in_rounds(entries, limit)
         if self._recordable(entries):
             with self._step_lock:
-                return self._step_recorded(entries, starts)
+                g = self._step_graph(len(entries), max(starts) + 1)
+                if g is not None:
+                    return self._step_recorded(g, entries, starts)
         batch = build_batch(entries, starts, self.spec.vocab, self.rt.device)
         for e, s in zip(entries, starts):
             cache.reserve(e.slot, s + len(e.tokens))
@@ -269,10 +272,34 @@ class Model:
                 and self.graph_safe and torch.device(self.rt.device).type == "cuda" and getattr(self.rt.kernels, "profile", None) is None
                 and not torch.cuda.is_current_stream_capturing())
 
-    def _step_recorded(self, entries: Sequence[StepEntry], starts: Sequence[int]) -> torch.Tensor:
-        from .graph import MAX_STEP_GRAPHS, StepGraph
+    def _step_graph(self, n_seqs: int, max_len: int):
+        """The ``StepGraph`` of this shape, or None where as many others as are kept have been in use of late: a caller that goes
+        round among more shapes replays some and issues the rest, rather than recording each anew."""
+        from . import graph
+        short, graphs = self.short_context, self._step_graphs
+        key = (n_seqs, short if max_len <= short else 0)
+        self._steps += 1
+        g = graphs.get(key)
+        if g is None:
+            if len(graphs) >= graph.MAX_STEP_GRAPHS:
+                if self._steps - next(iter(graphs.values())).last <= graph.STEP_GRAPH_IDLE:
+                    return None
+                torch.cuda.synchronize()                    # the one that goes may still be running
+                graphs.popitem(last=False)
+            g = graphs[key] = graph.StepGraph(self, *key)
+        graphs.move_to_end(key)
+        g.last = self._steps
+        return g
+
+    def _forget_step_graphs(self) -> None:
+        with self._step_lock:
+            if self._step_graphs:
+                torch.cuda.synchronize()                    # one may still be running
+                self._step_graphs.clear()
+
+    def _step_recorded(self, g, entries: Sequence[StepEntry], starts: Sequence[int]) -> torch.Tensor:
         check_entries(entries, self.spec.vocab)
-        cache, short = self.cache, self.short_context
+        cache = self.cache
         # The recordings' inputs and memory serve every stream and thread: a step waits for the one before it, wherever that ran.
         stream = torch.cuda.current_stream()
         if self._step_done is None:
@@ -282,14 +309,6 @@ class Model:
         for e, s in zip(entries, starts):
             cache.reserve(e.slot, s + 1)
         cache.flush()
-        key = (len(entries), short if max(starts) + 1 <= short else 0)
-        g = self._step_graphs.get(key)
-        if g is None:
-            g = self._step_graphs[key] = StepGraph(self, key[0], key[1])
-            while len(self._step_graphs) > MAX_STEP_GRAPHS:
-                torch.cuda.synchronize()                    # the one that goes may still be running
-                self._step_graphs.popitem(last=False)
-        self._step_graphs.move_to_end(key)
         try:
             logits = g.run([e.slot for e in entries], [int(e.tokens[0]) for e in entries], starts)
         finally:

@@ -718,3 +718,32 @@ def test_a_one_token_step_whose_recording_fails_is_a_step(name, monkeypatch):
         assert (out[0] - out[1]).abs().max() <= 2e-2 * out[1].std()
         assert [rec.model.cache.length(s) for s in slots[0]] == [4 + n] * 2
     assert len(attempts) == 1 and not any(x.graph for x in rec.model._step_graphs.values())
+
+
+def test_more_shapes_of_one_token_steps_than_are_recorded(monkeypatch):
+    """A caller that goes round among six batch sizes where two recordings are kept: two sizes are replayed, the others issued, none
+    recorded anew; a recording that went unused for long enough gives its place away."""
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry, graph
+    monkeypatch.setattr(graph, "MAX_STEP_GRAPHS", 2)
+    monkeypatch.setattr(graph, "STEP_GRAPH_IDLE", 12)
+    kw = dict(config=SHAPES["tiny-b"], seed=3, max_tokens=2048, max_seqs=6, verbose=False)
+    rec, ref = cima_b200.load(**kw), cima_b200.load(use_graphs=False, **kw)
+    slots = [lm.model.cache.open(6) for lm in (rec, ref)]
+    for lm, held in zip((rec, ref), slots):
+        lm.step([StepEntry(s, [7 + i, 3, 5], [2]) for i, s in enumerate(held)])
+    made, start = [], graph.StepGraph.__init__
+    monkeypatch.setattr(graph.StepGraph, "__init__", lambda self, *a: (made.append(a[1]), start(self, *a))[1])
+
+    def both(n, t):
+        out = [lm.step([StepEntry(s, [t + i], [0]) for i, s in enumerate(held[:n])]) for lm, held in zip((rec, ref), slots)]
+        assert (out[0] - out[1]).abs().max() <= 2e-2 * out[1].std()
+
+    for turn in range(4):
+        for n in range(1, 7):
+            both(n, 20 * turn + n)
+    assert made == [1, 2] and all(x.graph is not None for x in rec.model._step_graphs.values())
+    for turn in range(13):
+        both(2, 100 + turn)
+    both(5, 120); both(5, 121); both(5, 122)
+    assert made == [1, 2, 5] and sorted(k[0] for k in rec.model._step_graphs) == [2, 5] and rec.model._step_graphs[(5, rec.model.short_context)].graph is not None
