@@ -187,10 +187,11 @@ class StepGraph:
     itself runs again and again.  Issued launch by launch, such a step waits for the host (about 100 us a layer: 2.75 ms at the
     24 layers of the 0.5B shape, where the device works 0.5; 3.4 against 1.2 at 1.5B).  A shape's first step is issued as it is,
     its second is recorded as well, from the third on the recording is replayed; every call gets logits of its own.  A shape that
-    cannot be recorded (no memory left for it) goes on being issued."""
+    cannot be recorded (no memory left for it) goes on being issued.  (The model holds its recordings; they do not hold it, so that
+    its memory is given back with the last reference to it.)"""
 
     def __init__(self, model, n_seqs: int, max_len: int):
-        self.model, self.n_seqs = model, n_seqs
+        self.n_seqs = n_seqs
         self.meta = torch.zeros(6 * n_seqs + 1, dtype=torch.int32, device=model.rt.device)
         self.batch = one_token_batch(self.meta, n_seqs, max_len)
         self.graph = None
@@ -199,7 +200,7 @@ class StepGraph:
         self.last = 0                              # number of the model's one-token step that used it last
         self.recordable = True
 
-    def run(self, slots: Sequence[int], tokens: Sequence[int], lengths: Sequence[int]) -> torch.Tensor:
+    def run(self, model, slots: Sequence[int], tokens: Sequence[int], lengths: Sequence[int]) -> torch.Tensor:
         """Float32 logits [sequences, vocab].  The caller has reserved the new position of every slot and commits it, then asks for
         the recording (``record``)."""
         host = torch.empty(6 * self.n_seqs + 1, dtype=torch.int32, pin_memory=True)      # its own each time: the copy may still be under way
@@ -209,9 +210,9 @@ class StepGraph:
             self.graph.replay()
             return self.logits.clone()
         self.uses += 1
-        return self.model.forward(self.batch)
+        return model.forward(self.batch)
 
-    def record(self) -> None:
+    def record(self, model) -> None:
         """Behind the shape's second step, when its positions are committed: a step is whole whether or not its recording succeeds."""
         if self.graph is not None or self.uses < 2 or not self.recordable:
             return
@@ -221,7 +222,7 @@ class StepGraph:
             with torch.cuda.stream(side):
                 g.capture_begin(capture_error_mode="thread_local")
                 try:
-                    logits = self.model.forward(self.batch)      # recorded, not run
+                    logits = model.forward(self.batch)      # recorded, not run
                 finally:
                     g.capture_end()
         except RuntimeError:

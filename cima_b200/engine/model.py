@@ -310,12 +310,12 @@ class Model:
             cache.reserve(e.slot, s + 1)
         cache.flush()
         try:
-            logits = g.run([e.slot for e in entries], [int(e.tokens[0]) for e in entries], starts)
+            logits = g.run(self, [e.slot for e in entries], [int(e.tokens[0]) for e in entries], starts)
         finally:
             self._step_done.record(stream)
         for e, s in zip(entries, starts):
             cache.commit(e.slot, s + 1)
-        g.record()
+        g.record(self)
         return logits
 
     def _step_in_parts(self, entries: Sequence[StepEntry]) -> torch.Tensor:

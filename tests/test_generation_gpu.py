@@ -747,3 +747,25 @@ def test_more_shapes_of_one_token_steps_than_are_recorded(monkeypatch):
         both(2, 100 + turn)
     both(5, 120); both(5, 121); both(5, 122)
     assert made == [1, 2, 5] and sorted(k[0] for k in rec.model._step_graphs) == [2, 5] and rec.model._step_graphs[(5, rec.model.short_context)].graph is not None
+
+
+def test_a_model_with_recorded_steps_goes_with_its_last_reference():
+    """One-token steps recorded and replayed: the model and its memory are given back when the handle goes, without waiting for the
+    collector of reference cycles."""
+    import gc
+    import weakref
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    lm = cima_b200.load(config=SHAPES["tiny-b"], seed=3, max_tokens=1024, max_seqs=4, verbose=False)
+    (slot,) = lm.model.cache.open(1)
+    for t in (5, 6, 7):
+        lm.step([StepEntry(slot, [t], [0])])
+    torch.cuda.synchronize()
+    assert any(x.graph is not None for x in lm.model._step_graphs.values())
+    model = weakref.ref(lm.model)
+    gc.collect(); gc.disable()
+    try:
+        del lm
+        assert model() is None
+    finally:
+        gc.enable()
