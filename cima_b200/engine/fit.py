@@ -70,12 +70,14 @@ def forecast(plan: Dict[str, object], requests: Sequence[Sequence[object]], dtyp
     for r, sites in groups.items():
         cache += sites * n_pages * r.planes * r.n_kv_heads * page_size * r.head_dim * elt
     # a step of the longest prompt: the float32 residual, the widest activation and its input, logits of a batch;
-    # and the recorded prompt steps that are kept, each with the activations of its rows
-    from .graph import MAX_PROMPT_GRAPHS, recorded_prompt_rows
+    # and the recorded prompt steps that are kept, each with the activations of its rows; the recorded one-token steps, each with its
+    # logits, and the activations of the largest
+    from .graph import MAX_PROMPT_GRAPHS, MAX_STEP_GRAPHS, STEP_GRAPH_ROWS, recorded_prompt_rows
     row = hidden * 4 * max(1, streams) + (widest + 2 * hidden) * elt
     rows = min(max_tokens, STEP_ROWS)
     scratch = int(rows * (row + segment_row)) + min(n_slots, 256) * vocab * 4 * 2
     scratch += MAX_PROMPT_GRAPHS * min(max_tokens, recorded_prompt_rows(weights, len(requests), elt)) * row
+    scratch += min(n_slots, STEP_GRAPH_ROWS) * (MAX_STEP_GRAPHS * vocab * 4 + row)
     return Forecast(weights, cache, scratch)
 
 

@@ -188,7 +188,8 @@ class StepGraph:
     24 layers of the 0.5B shape, where the device works 0.5; 3.4 against 1.2 at 1.5B).  A shape's first step is issued as it is,
     its second is recorded as well, from the third on the recording is replayed; every call gets logits of its own.  A shape that
     cannot be recorded (no memory left for it) goes on being issued.  (The model holds its recordings; they do not hold it, so that
-    its memory is given back with the last reference to it.)"""
+    its memory is given back with the last reference to it.)  A model's recordings share one pool of memory, and one stream to be
+    recorded on: they run one after another, and nothing but their logits outlives a replay (``engine.fit`` counts both)."""
 
     def __init__(self, model, n_seqs: int, max_len: int):
         self.n_seqs = n_seqs
@@ -216,11 +217,11 @@ class StepGraph:
         """Behind the shape's second step, when its positions are committed: a step is whole whether or not its recording succeeds."""
         if self.graph is not None or self.uses < 2 or not self.recordable:
             return
-        g, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        g, (pool, side) = torch.cuda.CUDAGraph(), model.step_pool()
         side.wait_stream(torch.cuda.current_stream())
         try:
             with torch.cuda.stream(side):
-                g.capture_begin(capture_error_mode="thread_local")
+                g.capture_begin(pool=pool, capture_error_mode="thread_local")
                 try:
                     logits = model.forward(self.batch)      # recorded, not run
                 finally:

@@ -76,6 +76,7 @@ class Model:
         self.step_rows = STEP_ROWS                          # a step of more rows runs in parts
         self.record_steps = False                           # record one-token steps (``StepGraph``); an ``LM`` with graphs says so
         self._step_graphs = OrderedDict()                   # (sequences, context bound) -> StepGraph, the newest last
+        self._step_pool = None                              # (memory pool, stream) that the recordings share
         self._steps = 0                                     # one-token steps so far
         self._step_lock = threading.Lock()                  # a recorded step's inputs and launch belong together
         self._step_done = None                              # event behind the last recorded step, whatever stream it ran on
@@ -296,6 +297,12 @@ class Model:
             if self._step_graphs:
                 torch.cuda.synchronize()                    # one may still be running
                 self._step_graphs.clear()
+                self._step_pool = None
+
+    def step_pool(self):
+        if self._step_pool is None:
+            self._step_pool = (torch.cuda.graph_pool_handle(), torch.cuda.Stream())
+        return self._step_pool
 
     def _step_recorded(self, g, entries: Sequence[StepEntry], starts: Sequence[int]) -> torch.Tensor:
         check_entries(entries, self.spec.vocab)

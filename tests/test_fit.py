@@ -59,6 +59,34 @@ def test_forecast_counts_the_segments_of_a_long_steps_recurrence():
 
 
 @pytest.mark.gpu
+def test_recorded_one_token_steps_stay_within_their_part_of_the_forecast():
+    """Steps of 33 to 48 sequences recorded, sixteen of them: the memory that stays taken is their logits and one step's activations
+    (and what the allocator rounds up to, blocks of 20 MiB), as the forecast has it."""
+    import cima_b200
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    from cima_b200.engine.graph import MAX_STEP_GRAPHS
+    lm = cima_b200.load(config=dict(SHAPES["qwen2.5-0.5b"], num_hidden_layers=2), draw="device", max_tokens=64 * 64, max_seqs=64, verbose=False)
+    slots = lm.model.cache.open(48)
+    lm.step([StepEntry(s, [1, 2], [1]) for s in slots])
+    for n in range(33, 49):                              # (a size's first step needs what a step needs)
+        lm.step([StepEntry(s, [3], [0]) for s in slots[:n]])
+    torch.cuda.synchronize(); torch.cuda.empty_cache()
+    before = torch.cuda.memory_reserved()
+    for n in range(33, 49):
+        lm.step([StepEntry(s, [4], [0]) for s in slots[:n]])
+        lm.step([StepEntry(s, [5], [0]) for s in slots[:n]])
+    torch.cuda.synchronize(); torch.cuda.empty_cache()
+    assert len(lm.model._step_graphs) == MAX_STEP_GRAPHS and all(g.graph is not None for g in lm.model._step_graphs.values())
+    vocab, row = lm.spec.vocab, 896 * 4 + (2 * 4864 + 2 * 896) * 2
+    assert torch.cuda.memory_reserved() - before <= 64 * (MAX_STEP_GRAPHS * vocab * 4 + row)
+    from cima_b200.engine import fit
+    m, held = lm.model, fit.forecast
+    plan = (m.plan(), m._cache_requests(), torch.bfloat16, 4096, 896, vocab, 2 * 4864)
+    assert held(*plan, max_seqs=64).scratch - held(*plan, max_seqs=63).scratch == MAX_STEP_GRAPHS * vocab * 4 + row + 2 * vocab * 4
+
+
+@pytest.mark.gpu
 def test_a_cache_that_cannot_fit_is_refused_before_allocating():
     from cima_b200.engine import load_model
     from cima_b200.engine.fit import DoesNotFit
