@@ -47,7 +47,7 @@ class LM:
                  use_graphs: bool = True):
         from .engine import GenerationLoop, ModelStepper
         self.model = model
-        model.record_steps = use_graphs
+        model.record_steps = self._record = use_graphs
         self.stepper = ModelStepper(model, max_batch=max_batch, use_graphs=use_graphs, pipeline=pipeline, retain=retain)
         self.loop = GenerationLoop(self.stepper, eos_ids)
 
@@ -67,7 +67,7 @@ class LM:
     def step(self, entries):
         """The model's step function (``cima_b200.engine.StepEntry`` per sequence): float32 logits at the wanted
         places.  The caller opens and closes the slots (``lm.model.cache``)."""
-        return self.model.step(entries)
+        return self.model.step(entries, record=self._record)
 
     def generate(self, prompts: Sequence[Sequence[int]], options: Union[GenOptions, Sequence[GenOptions], None] = None,
                  on_token=None, **named):

@@ -229,9 +229,10 @@ class Model:
                         segment_row=segment_row)
 
     # ------------------------------------------------------------------ the step
-    def step(self, entries: Sequence[StepEntry]) -> torch.Tensor:
+    def step(self, entries: Sequence[StepEntry], record: Optional[bool] = None) -> torch.Tensor:
         """Run the tokens the entries bring, from the cache earlier steps left; float32 logits
-        ``[wanted, vocab]`` in the order of the entries and of their ``want``."""
+        ``[wanted, vocab]`` in the order of the entries and of their ``want``.  ``record``: whether one-token steps may run through
+        a recording (None: as ``record_steps`` says)."""
         cache = self.cache
         if cache is None:
             raise RuntimeError("the model has no cache yet: call make_cache first")
@@ -244,14 +245,14 @@ class Model:
         cache.must_fit([(e.slot, s + len(e.tokens)) for e, s in zip(entries, starts)])
         if sum(len(e.tokens) for e in entries) > self.step_rows:
             return self._step_in_parts(entries)
-        return self._step_within_bound(entries, starts)
+        return self._step_within_bound(entries, starts, self.record_steps if record is None else record)
 
-    def _step_within_bound(self, entries: Sequence[StepEntry], starts: Sequence[int]) -> torch.Tensor:
+    def _step_within_bound(self, entries: Sequence[StepEntry], starts: Sequence[int], record: bool = False) -> torch.Tensor:
         cache = self.cache
         limit = cache.most_tokens_going_on()
         if limit is not None and any(starts) and max(len(e.tokens) for e in entries) > limit:
             return self._step_in_rounds(entries, limit)
-        if self._recordable(entries):
+        if record and self._recordable(entries):
             with self._step_lock:
                 g = self._step_graph(len(entries), max(starts) + 1)
                 if g is not None:
@@ -269,7 +270,7 @@ class Model:
         """Whether the step runs through a ``StepGraph``: one token a sequence, every sequence's logits wanted, parts that may
         be recorded, and nobody else recording or profiling."""
         from .graph import STEP_GRAPH_ROWS
-        return (self.record_steps and len(entries) <= STEP_GRAPH_ROWS and all(len(e.tokens) == 1 and list(e.want) == [0] for e in entries)
+        return (len(entries) <= STEP_GRAPH_ROWS and all(len(e.tokens) == 1 and list(e.want) == [0] for e in entries)
                 and self.graph_safe and torch.device(self.rt.device).type == "cuda" and getattr(self.rt.kernels, "profile", None) is None
                 and not torch.cuda.is_current_stream_capturing())
 

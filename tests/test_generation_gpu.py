@@ -769,3 +769,17 @@ def test_a_model_with_recorded_steps_goes_with_its_last_reference():
         assert model() is None
     finally:
         gc.enable()
+
+
+def test_two_handles_on_one_model_record_as_each_was_asked():
+    """An ``LM`` made with ``use_graphs`` and one made without share a model: each one's one-token steps are recorded, or not, as it was
+    asked, whichever was made last."""
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    first = cima_b200.load(config=SHAPES["tiny-b"], seed=3, max_tokens=1024, max_seqs=4, verbose=False)
+    second = cima_b200.LM(first.model, use_graphs=False)
+    (slot,) = first.model.cache.open(1)
+    for lm, kept in ((second, 0), (first, 1)):
+        for t in (5, 6, 7):
+            lm.step([StepEntry(slot, [t], [0])])
+        assert len(first.model._step_graphs) == kept
