@@ -96,7 +96,7 @@ __device__ __forceinline__ void f32_finish(float* o, float v, const float* bias,
 
 // At most 8 rows (a decode step): bound by the weights' bytes.  A block takes 8 output features, a warp one range of k of
 // them: its pieces of the 8 weight rows travel through shared memory by cp.async, 256-byte runs of a row at a time, up
-// to FEW_STAGES pieces in flight, the first ones before the kernel ahead has finished (weights do not depend on it).  Lane =
+// to FEW_STAGES pieces in flight, the first ones before the kernel ahead has finished where the caller says that it does not write them (`early`).  Lane =
 // (feature, row mod 4): a lane walks its feature's range in order for one or two rows of A.  8 features a block and not more:
 // a narrow product (896 features) still covers 112 SMs, and a wide one keeps several blocks on each.  Measured inside a decode
 // step of the 0.5B shape, 2 rows: 9.3 us a product on average, 2.2 TB/s (74.8 us and 0.27 TB/s with a thread an output feature).
@@ -105,7 +105,7 @@ constexpr int FEW_ROWS = 8, FEW_F = 8, FEW_K = 64, FEW_PITCH = FEW_K + 4, FEW_ST
 template <int MR, bool VEC>        // MR: rows of A a lane takes (rows r, r + 4)
 __global__ void __launch_bounds__(32 * FEW_WARPS)
 k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out,
-                 int M, int N, int K, int lda, int ldo, int mode, int stages) {
+                 int M, int N, int K, int lda, int ldo, int mode, int stages, int early) {
   extern __shared__ __align__(16) float few_smem[];
   __shared__ float red[FEW_WARPS][FEW_ROWS][FEW_F];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * FEW_F;
@@ -134,8 +134,9 @@ k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const
     float* s = mine + (c % stages) * unit + FEW_F * FEW_PITCH;
     for (int m = half; m < M; m += 2) piece(s + m * FEW_PITCH, A + (size_t)m * lda, c);
   };
+  if (!early) cima_pdl_wait();
   for (int c = 0; c < min(stages, chunks); c++) weights(c);
-  cima_pdl_wait();
+  if (early) cima_pdl_wait();
   for (int c = 0; c < stages; c++) {
     if (c < chunks) rows(c);
     f32_commit();                                       // (the first of these groups holds all the weights requested above)
@@ -382,7 +383,7 @@ static int launch_f32_tile(const float* A, const float* W, const float* bias, fl
 
 template <bool VEC>
 static int launch_f32(const float* A, const float* W, const float* bias, float* out, int mode, int M, int N, int K, int lda, int ldo,
-                      cudaStream_t stream) {
+                      int early, cudaStream_t stream) {
   if (M <= FEW_ROWS) {
     const int chunks = (f32_group_len(K) + FEW_K - 1) / FEW_K, unit = (FEW_F + M) * FEW_PITCH * (int)sizeof(float) * FEW_WARPS;
     const int blocks = (N + FEW_F - 1) / FEW_F;
@@ -393,7 +394,7 @@ static int launch_f32(const float* A, const float* W, const float* bias, float* 
     const size_t smem = (size_t)stages * unit;
     auto kern = M <= 4 ? k_linear_f32_few<1, VEC> : k_linear_f32_few<2, VEC>;
     if (int rc = f32_allow(kern, smem)) return rc;
-    return cima_launch(kern, dim3((unsigned)blocks), dim3(32 * FEW_WARPS), smem, stream, 1, A, W, bias, out, M, N, K, lda, ldo, mode, stages);
+    return cima_launch(kern, dim3((unsigned)blocks), dim3(32 * FEW_WARPS), smem, stream, 1, A, W, bias, out, M, N, K, lda, ldo, mode, stages, early);
   }
   // The tile's rows, and whether clusters share a tile, by the time of the SM that gets the most blocks: a block's rows (a lower tile
   // reads more of shared memory for a product: measured at 0.9 and 0.7 of the rate), an eighth of them where a cluster shares the tile (and
@@ -419,11 +420,11 @@ static int launch_f32(const float* A, const float* W, const float* bias, float* 
 
 template <typename TA, typename TW, typename TO>
 static int launch_plain(const void* A, const void* W, const float* bias, void* out, int mode, int M, int N, int K,
-                        int lda, int ldo, cudaStream_t stream) {
+                        int lda, int ldo, int early, cudaStream_t stream) {
   if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4 && sizeof(TO) == 4) {
     const bool vec = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-    const int rc = vec ? launch_f32<true>((const float*)A, (const float*)W, bias, (float*)out, mode, M, N, K, lda, ldo, stream)
-                       : launch_f32<false>((const float*)A, (const float*)W, bias, (float*)out, mode, M, N, K, lda, ldo, stream);
+    const int rc = vec ? launch_f32<true>((const float*)A, (const float*)W, bias, (float*)out, mode, M, N, K, lda, ldo, early, stream)
+                       : launch_f32<false>((const float*)A, (const float*)W, bias, (float*)out, mode, M, N, K, lda, ldo, early, stream);
     return rc ? rc : cima_launch_result();
   } else {
   dim3 grid((N + 63) / 64, (M + 63) / 64);
@@ -436,9 +437,10 @@ static int launch_plain(const void* A, const void* W, const float* bias, void* o
 }
 
 // mode 0: out = A W^T (+ bias), stored as out_dtype.  mode 1: out += A W^T (+ bias); out must be float32.
+// early != 0: the kernel launched just before this one on the stream does not write W, so W may be read while it finishes.
 extern "C" int cima_linear_plain(const void* A, int a_dtype, const void* W, int w_dtype, const float* bias,
                                  void* out, int out_dtype, int mode, int M, int N, int K, int lda, int ldo,
-                                 cudaStream_t stream) {
+                                 int early, cudaStream_t stream) {
   if (M <= 0) return 0;
   if (N <= 0 || K <= 0) return cima_fail(CIMA_E_SIZE, "linear_plain: N %d and K %d must be positive", N, K);
   if (lda < K || ldo < N) return cima_fail(CIMA_E_SIZE, "linear_plain: leading dimensions (%d, %d) are smaller than the rows (%d, %d)", lda, ldo, K, N);
@@ -447,11 +449,11 @@ extern "C" int cima_linear_plain(const void* A, int a_dtype, const void* W, int 
   if ((long long)((M + 63) / 64) > 65535) return cima_fail(CIMA_E_SIZE, "linear_plain: %d rows exceed one launch; the caller cuts them", M);
   const int key = a_dtype * 4 + w_dtype * 2 + out_dtype;
   switch (key) {
-    case 0: return launch_plain<float, float, float>(A, W, bias, out, mode, M, N, K, lda, ldo, stream);
-    case 4 + 0 + 0: return launch_plain<__nv_bfloat16, float, float>(A, W, bias, out, mode, M, N, K, lda, ldo, stream);
-    case 4 + 0 + 1: return launch_plain<__nv_bfloat16, float, __nv_bfloat16>(A, W, bias, out, mode, M, N, K, lda, ldo, stream);
-    case 4 + 2 + 0: return launch_plain<__nv_bfloat16, __nv_bfloat16, float>(A, W, bias, out, mode, M, N, K, lda, ldo, stream);
-    case 4 + 2 + 1: return launch_plain<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(A, W, bias, out, mode, M, N, K, lda, ldo, stream);
+    case 0: return launch_plain<float, float, float>(A, W, bias, out, mode, M, N, K, lda, ldo, early, stream);
+    case 4 + 0 + 0: return launch_plain<__nv_bfloat16, float, float>(A, W, bias, out, mode, M, N, K, lda, ldo, early, stream);
+    case 4 + 0 + 1: return launch_plain<__nv_bfloat16, float, __nv_bfloat16>(A, W, bias, out, mode, M, N, K, lda, ldo, early, stream);
+    case 4 + 2 + 0: return launch_plain<__nv_bfloat16, __nv_bfloat16, float>(A, W, bias, out, mode, M, N, K, lda, ldo, early, stream);
+    case 4 + 2 + 1: return launch_plain<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(A, W, bias, out, mode, M, N, K, lda, ldo, early, stream);
     default:
       return cima_fail(CIMA_E_DTYPE, "linear_plain: dtypes (A %d, W %d, out %d) are not a supported combination", a_dtype, w_dtype, out_dtype);
   }

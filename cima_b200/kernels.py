@@ -15,7 +15,7 @@ import torch
 from .csrc.build import BuildError, library_path
 
 F32, BF16 = 0, 1
-ABI_VERSION = 35
+ABI_VERSION = 36
 SPLIT_BLOCKS = 296          # blocks of the decode attention that one wave holds (two per SM, 148 SMs)
 TC_ATTENTION_MIN_LEN = 256  # prompts from this length on take the tcgen05 attention (head_dim 64 or 128)
 SPLIT_FEW_BLOCKS = 148      # below this many blocks at 8 splits, more splits are taken
@@ -78,7 +78,7 @@ _SIGNATURES = {
     "cima_gather_rows": [_vp, _vp, _vp, _i, _i, _vp],
     "cima_add_rmsnorm": [_vp, _vp, _vp, _vp, _i, _i, _i, _f, _vp],
     "cima_decode_advance": [_vp, _vp, _vp, _vp, _i, _vp],
-    "cima_linear_plain": [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
+    "cima_linear_plain": [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "cima_linear_skinny": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _f, _vp],
     "cima_linear_skinny_norm": [_vp, _vp, _i, _f, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "cima_qkv_rope_skinny": [_vp, _vp, _i, _f, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i,
@@ -297,8 +297,9 @@ class Kernels:
 
     # ------------------------------------------------------------------ matrix products
     def linear_plain(self, a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
-                     accumulate: bool = False) -> None:
-        """out = a @ w.T (+ bias), or out += ... when ``accumulate`` (out float32)."""
+                     accumulate: bool = False, early: bool = False) -> None:
+        """out = a @ w.T (+ bias), or out += ... when ``accumulate`` (out float32).  ``early``: the kernel launched just before this one
+        does not write ``w``, so ``w`` may be read while it finishes (a model's weights; ``linear_plain_of_weights``)."""
         self._need(a, "a", None, 2); self._need(w, "w", None, 2); self._need(out, "out", None, 2)
         M, K = a.shape
         N = w.shape[0]
@@ -316,12 +317,18 @@ class Kernels:
             self._check(self.lib.cima_linear_plain(a[m0:m1].data_ptr(), dtype_code(a.dtype), w.data_ptr(),
                                                    dtype_code(w.dtype), _ptr(bias), out[m0:m1].data_ptr(),
                                                    dtype_code(out.dtype), 1 if accumulate else 0, m1 - m0, N, K,
-                                                   K, N, self._stream()), "linear_plain")
+                                                   K, N, int(early), self._stream()), "linear_plain")
+
+    def linear_plain_of_weights(self, a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
+                                accumulate: bool = False) -> None:
+        """``linear_plain`` by weights, which no kernel of a step writes."""
+        self.linear_plain(a, w, bias, out, accumulate, early=True)
 
     def linear_skinny(self, a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
                       mode: int, ssq_out: Optional[torch.Tensor] = None, w_next: Optional[torch.Tensor] = None,
                       xw_out: Optional[torch.Tensor] = None, act: int = 0, limit: float = 0.0) -> None:
-        """Few rows (<= 8), bf16 operands; ``mode`` is one of SK_*.  For SK_SWIGLU ``w`` is [2N, K].
+        """Few rows (<= 8), bf16 operands; ``mode`` is one of SK_*.  For SK_SWIGLU ``w`` is [2N, K].  ``w`` must be older than the kernel
+        launched just before this one: it is read while that one finishes.
         With SK_ACCUM, ``ssq_out`` [M, ceil(N / 16)] receives partial sums of squares of the updated rows and
         ``xw_out`` [M, N] bf16 the updated rows times ``w_next`` (the weight of the norm that follows)."""
         self._need(a, "a", torch.bfloat16, 2); self._need(w, "w", torch.bfloat16, 2); self._need(out, "out", None, 2)

@@ -23,6 +23,11 @@ TCGEN05_ROWS = 256       # rows of a tile of the tcgen05 kernel, and the fewest 
 SKINNY_ROWS = 8
 
 
+def _plain_product(kernels):
+    """The plain product by a model's weights, which the kernels before it in a step do not write."""
+    return getattr(kernels, "linear_plain_of_weights", kernels.linear_plain)
+
+
 class Linear:
     def __init__(self, weight, bias: Optional[torch.Tensor], rt):
         """``weight``: a matrix [N, K], or a list of matrices of one width that are stacked by rows."""
@@ -63,7 +68,7 @@ class Linear:
         if hasattr(a, "tensor"):
             a = a.tensor()
         if self._plain():
-            K_.linear_plain(a, self.weight, self.bias, out)
+            _plain_product(K_)(a, self.weight, self.bias, out)
         elif self._skinny(M):
             K_.linear_skinny(a, self.weight, self.bias, out, SK_STORE)
         else:
@@ -83,7 +88,7 @@ class Linear:
         if M == 0:
             return None
         if self._plain():
-            K_.linear_plain(a, self.weight, self.bias, x, accumulate=True)
+            _plain_product(K_)(a, self.weight, self.bias, x, accumulate=True)
         elif self._skinny(M):
             if M > FOLDED_NORM_ROWS:
                 K_.linear_skinny(a, self.weight, self.bias, x, SK_ACCUM)
@@ -120,7 +125,7 @@ class Linear:
         if hasattr(a, "tensor"):
             a = a.tensor()
         if self._plain() or self.K % 8:
-            K_.linear_plain(a, self.weight, self.bias, out)
+            _plain_product(K_)(a, self.weight, self.bias, out)
         elif self._skinny(M):
             K_.linear_skinny(a, self.weight, self.bias, out, SK_STORE_F32)
         else:

@@ -135,6 +135,26 @@ def test_linear_float32_the_same_bits_from_every_kernel(K, N, K_):
         assert torch.equal(acc, acc_full[50:50 + rows]), rows
 
 
+@pytest.mark.parametrize("rows", [1, 5, 8])
+def test_linear_float32_by_a_matrix_that_the_kernel_before_it_wrote(K, rows):
+    """A product whose matrix is the result of the product launched just before it, without waiting in between: the new matrix is
+    read, not what stood there before; as weights (``linear_plain_of_weights``) once it is old."""
+    N, K_ = 4096, 1024
+    a, left, right = g(rows, K_, seed=1).cuda(), g(N, 64, seed=2).cuda(), g(K_, 64, seed=3, scale=0.1).cuda()
+    w, out, again = torch.empty(N, K_, device="cuda"), torch.empty(rows, N, device="cuda"), torch.empty(rows, N, device="cuda")
+    want = a.double() @ (left.double() @ right.double().t()).t()
+    for _ in range(10):
+        w.fill_(float("nan"))
+        torch.cuda.synchronize()
+        K.linear_plain(left, right, None, w)
+        K.linear_plain(a, w, None, out)
+        # float32 sums of 64 and of 1,024 products
+        assert err(out, want) <= (64 + 1024 / 8 + 23) * 2.0 ** -24 * (a.double().abs() @ (left.double().abs() @ right.double().abs().t()).t()).max().item()
+    torch.cuda.synchronize()
+    K.linear_plain_of_weights(a, w, None, again)
+    assert torch.equal(out, again)
+
+
 @pytest.mark.parametrize("M", [1, 3, 7, 8])
 @pytest.mark.parametrize("N,K_", [(200, 328), (1000, 192), (4608, 3584), (17, 8)])
 def test_linear_skinny_modes(K, M, N, K_):
