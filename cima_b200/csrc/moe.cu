@@ -20,8 +20,8 @@
 //   many pairs, bfloat16   moe_sort_tiles lays every expert's pairs out from a multiple of 256 rows on and names each row
 //                          tile's expert; moe_gather_rows copies the rows of h to their places; the two products run on
 //                          the tcgen05 kernel (gemm_tcgen05_pair_grouped); moe_combine reads y through the pairs' places
-//   fewer, bfloat16        moe_few: a block computes 16 output features for up to 8 (32 where there are more) pairs of an expert
-//                          at a time, its warps streaming a range of k each with 16-byte loads (every touched expert is read once)
+//   fewer, bfloat16        moe_few: a block computes 16 output features for some pairs of an expert at a time, its warps streaming a
+//                          range of k each with 16-byte loads: multiply-adds up to 128 pairs, mma.sync beyond (32 pairs at a time)
 #include "common.cuh"
 
 namespace {
@@ -507,19 +507,14 @@ k_moe_gather_rows(const uint4* __restrict__ src, const int* __restrict__ pos, ui
   for (int v = threadIdx.x; v < vecs; v += blockDim.x) d[v] = s[v];
 }
 
-// Few pairs (a decode step): bound by the touched experts' weights.  Block (x = tile of 32 pairs of one expert as moe_sort laid
-// them out, y = 16 output features): the weights are the 16-row operand of mma.m16n8k16, up to 8 pairs its columns.  The sum
-// over k is shared by the block's 8 warps, a range each, whose sums are added in their order, so that a down product (few
-// features, a long sum) has work for every SM in more than one wave.  The order of k inside a product is free as long as both
-// operands follow it: lane (g, t) loads 16 neighbouring bytes of weight rows g and g + 8 and of pair g, 8 t values into each 32,
-// and uses them as its parts of two k-steps.  FEW_AHEAD such pieces are requested before the first is used.  MODE as in k_moe_gemm.
-// (A warp a feature with multiply-adds stood at 4.2 TB/s in the down product of 16 experts of 1,536 x 4,480 and 8 rows, 52.8 us: its
-// 1,536 blocks are 1.3 waves, and each began with a chain of dependent look-ups of its expert.)
+// Up to 1,023 pairs: bound by the touched experts' weights.  Block (x = tile of 32 pairs of one expert as moe_sort laid them out, y = 16
+// output features); the sum over k is shared by its 8 warps, a range each, so that a down product (few features, a long sum) has work
+// for every SM in more than one wave.  Lane (g, t) loads 16 neighbouring bytes of weight rows g and g + 8 and of its pairs' rows, 8 t
+// values into each 32 ("a piece"); several pieces are requested before the first is used.  MODE as in k_moe_gemm.
+// (A warp a feature stood at 4.2 TB/s in the down product of 16 experts of 1,536 x 4,480 and 8 rows, 52.8 us: its 1,536 blocks are 1.3
+// waves, and each began with a chain of dependent look-ups of its expert.)
+constexpr int FEW_MOST = 128;           // pairs up to which the sums are multiply-adds (k_moe_few); beyond, k_moe_some
 constexpr int FEW_PAIRS = 8, FEW_FEATURES = 16, FEW_WARPS = 8;
-__device__ __forceinline__ void few_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 // 16 bytes, or zeros; volatile, so that a piece's requests stay in front of the products they are requested for
 __device__ __forceinline__ uint4 few_load(const void* p, bool ok) {
   uint4 v;
@@ -527,54 +522,194 @@ __device__ __forceinline__ uint4 few_load(const void* p, bool ok) {
                : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)ok));
   return v;
 }
-// NB: pairs of eight that a piece of weights serves at once (1 in a decode step of few sequences; 4, a whole tile of 32 pairs, where
-// an expert has more than eight on average: 192 pairs of 16 gated experts of 1,536 x 2,240 in 109 us, 1,024 in 248).  A row's sums
-// are the same either way.
-template <int MODE, int NB>
-__global__ void __launch_bounds__(32 * FEW_WARPS)
-k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
-          const int* __restrict__ offsets, const int* __restrict__ tiles, const int* __restrict__ perm, int E, int top, int N,
-          int K, int act, float limit, const float* __restrict__ weigh) {
-  constexpr int MT = MODE == 0 ? 2 : 1;                 // operand tiles of a block: gate and up
-  constexpr int AHEAD = MODE == 0 || NB > 1 ? 2 : 4, COLS = NB * FEW_PAIRS;
-  cima_pdl_wait();
-  __shared__ int s_row[BM], s_pair[BM], s_e, s_i0, s_n;
-  __shared__ float s_w[BM];
-  __shared__ float red[FEW_WARPS][MT * FEW_FEATURES][COLS + 1];
-  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
-  if (tid == 0) s_e = -1;
+__device__ __forceinline__ void few_unpack(float (&f)[8], const uint4& v) {
+  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) { f[2 * i] = __uint_as_float(u[i] << 16); f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
+}
+// The pairs of a block's tile: expert e, the pairs i0 .. i0 + n - 1 of the sorted order.
+struct FewTile {
+  int row[BM], pair[BM], e, i0, n;
+  float w[BM];
+};
+template <int MODE>
+__device__ __forceinline__ bool few_tile(FewTile& s, const int* __restrict__ offsets, const int* __restrict__ tiles, const int* __restrict__ perm,
+                                         int E, int top, const float* __restrict__ weigh) {
+  const int tid = (int)threadIdx.x, tile = blockIdx.x;
+  if (tid == 0) s.e = -1;
   __syncthreads();
   for (int e = tid; e < E; e += 32 * FEW_WARPS) {       // the expert whose row tiles hold this one
     const int t0 = tiles[e], t1 = tiles[e + 1], o0 = offsets[e], o1 = offsets[e + 1];
     if (t0 <= tile && tile < t1) {
-      s_e = e;
-      s_i0 = o0 + (tile - t0) * BM;
-      s_n = min(BM, o1 - s_i0);
+      s.e = e;
+      s.i0 = o0 + (tile - t0) * BM;
+      s.n = min(BM, o1 - s.i0);
     }
   }
   __syncthreads();
-  const int e = s_e;
-  if (e < 0) return;
-  const int i0 = s_i0, nrows = s_n, n0 = blockIdx.y * FEW_FEATURES;
-  if (tid < nrows) {
-    const int pair = perm[i0 + tid];
-    s_pair[tid] = pair;
-    s_row[tid] = MODE != 1 ? pair / top : i0 + tid;
-    s_w[tid] = MODE != 1 && weigh ? weigh[pair] : 1.0f;
+  if (s.e < 0) return false;
+  if (tid < s.n) {
+    const int pair = perm[s.i0 + tid];
+    s.pair[tid] = pair;
+    s.row[tid] = MODE != 1 ? pair / top : s.i0 + tid;
+    s.w[tid] = MODE != 1 && weigh ? weigh[pair] : 1.0f;
   }
-  const int g = lane >> 2, t = lane & 3;
+  __syncthreads();
+  return true;
+}
+// What leaves for pair r of the tile and feature n; v: its sum (gate: v0, up: v1).
+template <int MODE>
+__device__ __forceinline__ void few_store(const FewTile& s, void* __restrict__ out, int r, int n, int N, float v0, float v1, int act, float limit) {
+  if (MODE == 2) {
+    const float z = __bfloat162float(__float2bfloat16_rn(v0 * s.w[r]));
+    reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(s.i0 + r) * N + n] = __float2bfloat16_rn(cima_ungated_act(z, act));
+  } else if (MODE == 0) {
+    // gate and up are rounded to bfloat16 before the activation, as stored projections would be
+    const float gt = __bfloat162float(__float2bfloat16_rn(v0 * s.w[r])), uv = __bfloat162float(__float2bfloat16_rn(v1 * s.w[r]));
+    reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(s.i0 + r) * N + n] = __float2bfloat16_rn(cima_gated(gt, uv, act, limit));
+  } else {
+    reinterpret_cast<float*>(out)[(size_t)s.pair[r] * N + n] = v0;
+  }
+}
+
+// Up to FEW_MOST pairs (a decode step): multiply-adds, each rounded to float32.  (mma.sync cuts its sums off instead; over 4,480 values of k
+// they stand five times as far from 64 bits, 5.3e-7 against 1.0e-7, and 27 times where all products have one sign.)  A lane's products of a
+// feature and pair are added in ascending k, then lanes and warps by halves, whatever NP, the pairs that a piece of weights serves at
+// once.  The next piece is requested before the one at hand is used.  Sort, both products and sum aside, us, a warp a feature / this / mma.sync:
+// 16 gated experts of 1,536 x 2,240, 16 pairs: 47 / 37 / 31 and down 23 / 20 / 19, 64 pairs: 93 / 81 / 40 and 52 / 49 / 28; 16 ungated ones of
+// 1,536 x 4,480, 24 pairs: 56 / 44 / 37 and 55 / 47 / 35.  NP 1 is the better one for gate and up where most experts have one pair
+// (8 pairs of 16 experts: 22 us, NP 2 25), NP 2 elsewhere (32: 51, NP 1 55); NP 4 costs a decode step its blocks (106 registers).
+template <int MODE, int NP>
+__global__ void __launch_bounds__(32 * FEW_WARPS)
+k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
+          const int* __restrict__ offsets, const int* __restrict__ tiles, const int* __restrict__ perm, int E, int top, int N,
+          int K, int act, float limit, const float* __restrict__ weigh) {
+  constexpr int MT = MODE == 0 ? 2 : 1;                 // rows of weights of a feature: gate and up
+  cima_pdl_wait();
+  __shared__ FewTile s;
+  __shared__ float red[FEW_WARPS][MT * FEW_FEATURES][NP];
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  if (!few_tile<MODE>(s, offsets, tiles, perm, E, top, weigh)) return;
+  const int nrows = s.n, n0 = blockIdx.y * FEW_FEATURES;
   const __nv_bfloat16* w[MT][2];
 #pragma unroll
   for (int m = 0; m < MT; m++)
 #pragma unroll
-    for (int x = 0; x < 2; x++) w[m][x] = W + ((size_t)e * (MT * N) + (size_t)m * N + min(n0 + g + 8 * x, N - 1)) * K + 8 * t;
+    for (int x = 0; x < 2; x++) w[m][x] = W + ((size_t)s.e * (MT * N) + (size_t)m * N + min(n0 + g + 8 * x, N - 1)) * K + 8 * t;
   const int pieces = (K + 31) / 32, share = (pieces + FEW_WARPS - 1) / FEW_WARPS;
   const int beg = min(pieces, warp * share), end = min(pieces, beg + share);
-  __syncthreads();
+  struct Piece { uint4 w[MT][2], a[NP]; };
+  for (int r0 = 0; r0 < nrows; r0 += NP) {
+    const __nv_bfloat16* a[NP];
+#pragma unroll
+    for (int y = 0; y < NP; y++) a[y] = A + (size_t)s.row[min(r0 + y, nrows - 1)] * lda + 8 * t;
+    float acc[MT][2][NP];
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int y = 0; y < NP; y++) acc[m][x][y] = 0.f;
+    auto fetch = [&](Piece& f, int p) {
+      const int k = 32 * p;
+      const bool ok = p < end && k + 8 * t < K;
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int x = 0; x < 2; x++) f.w[m][x] = few_load(w[m][x] + k, ok);
+#pragma unroll
+      for (int y = 0; y < NP; y++) f.a[y] = few_load(a[y] + k, ok && r0 + y < nrows);
+    };
+    auto use = [&](const Piece& f) {
+      float wf[MT][2][8];
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int x = 0; x < 2; x++) few_unpack(wf[m][x], f.w[m][x]);
+#pragma unroll
+      for (int y = 0; y < NP; y++) {
+        if (r0 + y >= nrows) break;                       // (the same for the whole block)
+        float af[8];
+        few_unpack(af, f.a[y]);
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+#pragma unroll
+          for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int x = 0; x < 2; x++) acc[m][x][y] = fmaf(af[q], wf[m][x][q], acc[m][x][y]);
+      }
+    };
+    Piece one, two;
+    fetch(one, beg);
+#pragma unroll 1
+    for (int p = beg; p < end; p += 2) {
+      fetch(two, p + 1);
+      use(one);
+      fetch(one, p + 2);
+      use(two);
+    }
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int y = 0; y < NP; y++) {
+          float v = acc[m][x][y];
+          v += __shfl_xor_sync(0xffffffffu, v, 1);
+          v += __shfl_xor_sync(0xffffffffu, v, 2);
+          if (t == 0) red[warp][m * FEW_FEATURES + g + 8 * x][y] = v;
+        }
+    __syncthreads();
+    for (int o = tid; o < FEW_FEATURES * NP; o += 32 * FEW_WARPS) {
+      const int f = o / NP, r = o % NP, n = n0 + f;
+      if (n >= N || r0 + r >= nrows) continue;
+      float v[MT];
+#pragma unroll
+      for (int m = 0; m < MT; m++) {
+        float p[FEW_WARPS];
+#pragma unroll
+        for (int x = 0; x < FEW_WARPS; x++) p[x] = red[x][m * FEW_FEATURES + f][r];
+        v[m] = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+      }
+      few_store<MODE>(s, out, r0 + r, n, N, v[0], v[MT - 1], act, limit);
+    }
+    __syncthreads();
+  }
+}
+
+// More pairs: bound by the weights still.  The weights are the 16-row operand of mma.m16n8k16, NB times 8 pairs its columns (4, a whole tile of 32 pairs, where an
+// expert has more than eight on average: 192 pairs of 16 gated experts of 1,536 x 2,240 in 109 us, 1,024 in 248).  The order of k inside
+// a product is free as long as both operands follow it: a lane uses its 16 bytes as its parts of two k-steps.  The warps' sums are
+// added in their order; a row's sums are the same for either NB.  (The plain tiles, which add all of k one by one, stand further from
+// 64 bits: 6.6e-7 against 5.3e-7 over 4,480 values of k, 1.6e-7 against 0.9e-7 over 512.)
+__device__ __forceinline__ void some_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <int MODE, int NB>
+__global__ void __launch_bounds__(32 * FEW_WARPS)
+k_moe_some(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
+           const int* __restrict__ offsets, const int* __restrict__ tiles, const int* __restrict__ perm, int E, int top, int N,
+           int K, int act, float limit, const float* __restrict__ weigh) {
+  constexpr int MT = MODE == 0 ? 2 : 1;                 // operand tiles of a block: gate and up
+  constexpr int AHEAD = MODE == 0 || NB > 1 ? 2 : 4, COLS = NB * FEW_PAIRS;
+  cima_pdl_wait();
+  __shared__ FewTile s;
+  __shared__ float red[FEW_WARPS][MT * FEW_FEATURES][COLS + 1];
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  if (!few_tile<MODE>(s, offsets, tiles, perm, E, top, weigh)) return;
+  const int nrows = s.n, n0 = blockIdx.y * FEW_FEATURES;
+  const __nv_bfloat16* w[MT][2];
+#pragma unroll
+  for (int m = 0; m < MT; m++)
+#pragma unroll
+    for (int x = 0; x < 2; x++) w[m][x] = W + ((size_t)s.e * (MT * N) + (size_t)m * N + min(n0 + g + 8 * x, N - 1)) * K + 8 * t;
+  const int pieces = (K + 31) / 32, share = (pieces + FEW_WARPS - 1) / FEW_WARPS;
+  const int beg = min(pieces, warp * share), end = min(pieces, beg + share);
   for (int r0 = 0; r0 < nrows; r0 += COLS) {
     const __nv_bfloat16* a[NB];                           // (a column without a pair is not read below)
 #pragma unroll
-    for (int y = 0; y < NB; y++) a[y] = A + (size_t)s_row[min(r0 + FEW_PAIRS * y + g, nrows - 1)] * lda + 8 * t;
+    for (int y = 0; y < NB; y++) a[y] = A + (size_t)s.row[min(r0 + FEW_PAIRS * y + g, nrows - 1)] * lda + 8 * t;
     float acc[MT][NB][4];
 #pragma unroll
     for (int m = 0; m < MT; m++)
@@ -601,9 +736,9 @@ k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __r
 #pragma unroll
         for (int m = 0; m < MT; m++) {
 #pragma unroll
-          for (int y = 0; y < NB; y++) few_mma(acc[m][y], wv[u][m][0].x, wv[u][m][1].x, wv[u][m][0].y, wv[u][m][1].y, av[u][y].x, av[u][y].y);
+          for (int y = 0; y < NB; y++) some_mma(acc[m][y], wv[u][m][0].x, wv[u][m][1].x, wv[u][m][0].y, wv[u][m][1].y, av[u][y].x, av[u][y].y);
 #pragma unroll
-          for (int y = 0; y < NB; y++) few_mma(acc[m][y], wv[u][m][0].z, wv[u][m][1].z, wv[u][m][0].w, wv[u][m][1].w, av[u][y].z, av[u][y].w);
+          for (int y = 0; y < NB; y++) some_mma(acc[m][y], wv[u][m][0].z, wv[u][m][1].z, wv[u][m][0].w, wv[u][m][1].w, av[u][y].z, av[u][y].w);
         }
     }
 #pragma unroll
@@ -623,16 +758,7 @@ k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __r
 #pragma unroll
         for (int x = 1; x < FEW_WARPS; x++) v[m] += red[x][m * FEW_FEATURES + f][r];
       }
-      if (MODE == 2) {
-        const float z = __bfloat162float(__float2bfloat16_rn(v[0] * s_w[r0 + r]));
-        reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(i0 + r0 + r) * N + n] = __float2bfloat16_rn(cima_ungated_act(z, act));
-      } else if (MODE == 0) {
-        // gate and up are rounded to bfloat16 before the activation, as stored projections would be
-        const float gt = __bfloat162float(__float2bfloat16_rn(v[0] * s_w[r0 + r])), uv = __bfloat162float(__float2bfloat16_rn(v[MT - 1] * s_w[r0 + r]));
-        reinterpret_cast<__nv_bfloat16*>(out)[(size_t)(i0 + r0 + r) * N + n] = __float2bfloat16_rn(cima_gated(gt, uv, act, limit));
-      } else {
-        reinterpret_cast<float*>(out)[(size_t)s_pair[r0 + r] * N + n] = v[0];
-      }
+      few_store<MODE>(s, out, r0 + r, n, N, v[0], v[MT - 1], act, limit);
     }
     __syncthreads();
   }
@@ -743,9 +869,14 @@ extern "C" int cima_moe_few(const void* a, int lda, const void* w, void* out, co
   const dim3 grid((unsigned)((P + BM - 1) / BM + E), (unsigned)((N + FEW_FEATURES - 1) / FEW_FEATURES));
   if (grid.y > 65535) return cima_fail(CIMA_E_SIZE, "moe_few: %d outputs exceed one launch", N);
   int rc;
-#define RUN(M, NB) rc = cima_launch(k_moe_few<M, NB>, grid, dim3(256), (size_t)0, stream, 1, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, out, offsets, tiles, perm, E, top, N, K, act, limit, weigh)
-#define WIDTH(M) { if (P > FEW_PAIRS * E) RUN(M, 4); else RUN(M, 1); }
-  if (mode == 0) WIDTH(0)
+#define RUN(...) rc = cima_launch(__VA_ARGS__, grid, dim3(32 * FEW_WARPS), (size_t)0, stream, 1, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, out, offsets, tiles, perm, E, top, N, K, act, limit, weigh)
+#define WIDTH(M) { if (P > FEW_PAIRS * E) RUN(k_moe_some<M, 4>); else RUN(k_moe_some<M, 1>); }
+  if (P <= FEW_MOST) {
+    if (mode == 1) RUN(k_moe_few<1, 2>);
+    else if (mode == 2) RUN(k_moe_few<2, 2>);
+    else if (2 * P <= E) RUN(k_moe_few<0, 1>);
+    else RUN(k_moe_few<0, 2>);
+  } else if (mode == 0) WIDTH(0)
   else if (mode == 2) WIDTH(2)
   else WIDTH(1)
 #undef WIDTH

@@ -1468,7 +1468,7 @@ class Kernels:
         gate_up [E, 2 ff, H] (an expert's gate rows, then its up rows), down [E, H, ff]; x float32 [T, H].  Four launches:
         the pairs sorted by expert, the two grouped products over tiles of one expert's pairs, the weighted sum.  The
         products take one of three roads by the step's size, layout and dtype alone (``MOE_TC_PAIRS``): tcgen05 tiles of 256 pairs,
-        ``mma.sync`` tiles of 16 features and up to 32 pairs (bfloat16), or the plain tiles (any dtype, size and address).
+        ``moe_few``'s blocks of 16 features (bfloat16), or the plain tiles (any dtype and size; any address beyond ``MOE_FEW_PAIRS``).
         ``limit`` goes with the clamped form of the middle.  ``shared = (rows, gate, col)``: float32 rows [T, H] (a shared
         expert's output) that join the weighted sum in its launch, each row times sigmoid(gate[t, col]) (gate float32
         [T, n]; None: unweighted).  ``identity``: indices from E on are identity experts: their pairs are in no product and
@@ -1539,12 +1539,14 @@ class Kernels:
             self._check(self.lib.cima_moe_combine(y.data_ptr(), given, None, x.data_ptr(), T, top, H, int(assign), *tail, *own,
                                                   self._stream()), "moe_combine")
 
-    # From MOE_TC_PAIRS (row, choice) pairs on bfloat16 experts run on the tcgen05 tiles of 256 pairs, below on the mma.sync kernel: such
-    # steps are the experts' weights read once, which both do, the mma.sync one with less beside it, until its pairs take several
-    # passes over a tile of weights.  Sort, products and sum of 16 gated experts of 1,536 x 2,240, mma.sync, tcgen05 and plain tiles, us:
-    # 64 pairs 73 / 113 / 1,223, 192: 109 / 114 / 1,413, 512: 160 / 114 / 1,671, 1,024: 248 / 114 / 2,373; ungated ones of 1,536 x 4,480: 96: 104 / 208 /
-    # 1,740, 288: 157 / 265 / 1,800, 768: 289 / 292 / 2,943; 64 gated ones of 2,048 x 512, 256: 92 / 186, 1,024: 160 / 193, 2,048: 235 / 195.
-    # MOE_FEW_PAIRS: up to there the mma.sync kernel refuses operands off 16 bytes; beyond, those go to the plain tiles.
+    # From MOE_TC_PAIRS (row, choice) pairs on bfloat16 experts run on the tcgen05 tiles of 256 pairs, below on moe_few's kernels:
+    # multiply-adds up to 128 pairs, mma.sync beyond.  Such steps are the experts' weights read once, which all do, moe_few with less
+    # beside it, until its pairs take several passes over a tile of weights.  Where the two cross follows the pairs an expert has (some 20),
+    # so the line lies right for 64 experts and late for 16, whose 192 to 1,023 pairs the tcgen05 tiles would take in up to half the time.
+    # Sort, products and sum of 16 gated experts of 1,536 x 2,240, mma.sync, tcgen05 and plain tiles, us:
+    # 192 pairs: 109 / 114 / 1,413, 512: 160 / 114 / 1,671, 1,024: 248 / 114 / 2,373; ungated ones of 1,536 x 4,480: 288: 157 / 265 / 1,800,
+    # 768: 289 / 292 / 2,943; 64 gated ones of 2,048 x 512, 256: 92 / 186, 1,024: 160 / 193, 2,048: 235 / 195.
+    # MOE_FEW_PAIRS: up to there operands off 16 bytes are refused (by moe_few); beyond, they go to the plain tiles.
     MOE_TC_PAIRS, MOE_FEW_PAIRS = 1024, 128
 
     def _moe_experts_tc(self, h, gate_up, down, idx, wgt, x, act, assign=False, limit: float = 0.0, tail=(None, None, 0, None, 0, None, F32),

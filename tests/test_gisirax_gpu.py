@@ -317,6 +317,28 @@ def test_experts_of_few_pairs(T, H, ff, E, top, gated):
     assert close(xd - x.to(DEV), xr - x, 1.2e-2)          # the middle's rounding to bfloat16 (2^-8) at its largest, and the weighted rows'
 
 
+@pytest.mark.parametrize("ff", [1536, 4480])
+@pytest.mark.parametrize("T", [1, 3, 8, 40, 128])
+def test_experts_of_a_decode_step_add_in_rounded_float32(T, ff):
+    """A down product of positive values (its input is h itself: an identity in front and ReLU): rounded sums stand on both sides of the
+    64-bit ones, half a unit in the last place off in each of the last few steps and less in the earlier ones, so their mean error is a
+    small part of 2^-24; sums that are cut off all fall short, by more the longer they are (4,480: 9e-7)."""
+    N = 1024
+    g = torch.Generator().manual_seed(T + ff)
+    h, dn = torch.rand(T, ff, generator=g).bfloat16(), torch.rand(2, N, ff, generator=g).bfloat16()
+    up = torch.eye(ff).bfloat16().repeat(2, 1, 1)
+    idx = (torch.arange(T) % 2).view(T, 1).to(torch.int32)
+    # the sums are N wide, x as wide as h: rows of dn beyond N are zero
+    wide = torch.zeros(2, ff, ff, dtype=torch.bfloat16)
+    wide[:, :N] = dn
+    x = torch.zeros(T, ff, device=DEV)
+    K().moe_experts(h.to(DEV), up.to(DEV), wide.to(DEV), idx.to(DEV), torch.ones(T, 1, device=DEV), x, 3, gated=False)
+    wants = [h.double() @ d.double().t() for d in dn]
+    want = torch.stack([wants[t % 2][t] for t in range(T)])
+    off = (x[:, :N].double().cpu() - want) / want
+    assert off.abs().max() <= 6 * 2.0 ** -24 and abs(off.mean().item()) <= 2.0 ** -26 and off.square().mean().sqrt() <= 2.0 ** -24
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("T,H,ff,E,top", [(1, 40, 24, 3, 3), (5, 96, 40, 8, 2), (200, 64, 56, 6, 1), (70, 100, 33, 10, 4),
                                           (1100, 64, 56, 6, 1), (600, 128, 200, 5, 2), (30, 256, 64, 4, 4)])
