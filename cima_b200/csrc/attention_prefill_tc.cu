@@ -30,6 +30,12 @@
 // first, under the mask.  `v_group` neighbouring key heads share one value head.  (A layer of differential attention of the
 // 3B Lipizen shape, 2,048 tokens: 46 us; 109 on the mma.sync kernel, which took these two before.)
 //
+// NEAR: the reference point of the probabilities is the row's maximum, as on the mma.sync kernel, so that the largest is exactly 1 when it
+// is rounded to bfloat16, and the denominator sums them as they are rounded.  Otherwise the point lies up to 2^8 below, which spares O most
+// of its rescaling, and a row of few large probabilities stands 1.2 times as far from 64 bits (2.09e-3 against 1.72e-3; 1.73e-3 on
+// mma.sync).  Taken for the two forms above, which came from there: 2,048 rows, 32 heads of 64, window 1,024 and 64 kept, 42 us
+// (37 without, 67 on mma.sync); the other forms keep what they had.
+//
 // The reference's prefill attention is k_attn_prefill_tiled (src/kernels.cu:659-753): one warp per query row,
 // online softmax on CUDA cores; it has no tensor-core attention.
 #include "tcgen05.cuh"
@@ -81,7 +87,7 @@ __device__ __forceinline__ void key_tiles(int p0, int len, int window, int& firs
   last = q_hi / BN;
 }
 
-template <int HD, bool FROM_CACHE>
+template <int HD, bool FROM_CACHE, bool NEAR>
 __global__ void __launch_bounds__(THREADS, 2)
 k_attention_prefill_tc(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_k,
                        AttnArgs a) {
@@ -275,17 +281,17 @@ k_attention_prefill_tc(const __grid_constant__ CUtensorMap map_qkv, const __grid
           for (int e = 0; e < 32; e++) mx4[e & 3] = fmaxf(mx4[e & 3], __uint_as_float(raw[c][e]));
       }
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sc2;
-      // The reference point of the exponentials moves only when the row's maximum has grown by more than 2^8
+      // The reference point of the exponentials moves only when the row's maximum has grown by more than 2^8 (NEAR: at all)
       // since it was set: O and the sum stay consistent with whatever reference they were made with, the
       // probabilities stay below 2^8 (no harm in float32 or bfloat16), and O is rarely rescaled.
       float alpha = 1.0f;
-      if (mx > m_run + 8.0f) {                          // also the first tile with a visible key (m_run = -inf)
+      if (mx > m_run + (NEAR ? 0.0f : 8.0f)) {          // also the first tile with a visible key (m_run = -inf)
         alpha = ex2(m_run - mx);                        // 2^(-inf) = 0 while nothing was seen
         m_run = mx;
       }
       const float neg_m = m_run == -INFINITY ? 0.f : -m_run;
       l_run *= alpha;
-      // probabilities 2^(s * scale - m), summed in float32, packed as bfloat16 pairs in place
+      // probabilities 2^(s * scale - m), packed as bfloat16 pairs in place, summed in float32 (NEAR: as packed)
       float ps4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < NC; c++)
@@ -293,9 +299,11 @@ k_attention_prefill_tc(const __grid_constant__ CUtensorMap map_qkv, const __grid
         for (int e = 0; e < 32; e += 2) {
           const float p0 = ex2(fmaf(__uint_as_float(raw[c][e]), sc2, neg_m));
           const float p1 = ex2(fmaf(__uint_as_float(raw[c][e + 1]), sc2, neg_m));
-          ps4[(e >> 1) & 3] += p0 + p1;
           const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
-          raw[c][e >> 1] = *reinterpret_cast<const unsigned*>(&h2);
+          const unsigned both = *reinterpret_cast<const unsigned*>(&h2);
+          raw[c][e >> 1] = both;
+          if constexpr (NEAR) ps4[(e >> 1) & 3] += __uint_as_float(both << 16) + __uint_as_float(both & 0xffff0000u);
+          else ps4[(e >> 1) & 3] += p0 + p1;
         }
       l_run += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
       // O may be touched once the previous tile's P V has completed
@@ -387,7 +395,7 @@ struct CacheSource {              // keys and values from a layer's pages; cache
   int planes = 2;
 };
 
-template <int HD, bool FROM_CACHE>
+template <int HD, bool FROM_CACHE, bool NEAR>
 int launch_attention_tc(const void* qkv, int ld, const int* tile_seq, const int* tile_row0, const int* seq_first_row,
                         const CacheSource& c, void* out, int ldo, int T, int n_tiles, int nh, int nkv, float scale,
                         int window, int* error_flag, float sink, const float* head_sink, int gate_col, const float* slopes, int keep_first, int v_group,
@@ -406,17 +414,20 @@ int launch_attention_tc(const void* qkv, int ld, const int* tile_seq, const int*
   static_assert(14 * 8 + 8 <= 14 * 8 + 16, "barriers and flags fit their place");
   static bool raised = false;
   if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(k_attention_prefill_tc<HD, FROM_CACHE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_attention_prefill_tc<HD, FROM_CACHE, NEAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cima_fail((int)e, "attention_prefill_tc: cannot raise shared memory to %zu bytes: %s", smem, cudaGetErrorString(e));
     raised = true;
   }
   AttnArgs a{tile_seq, tile_row0, seq_first_row, c.seq_len, c.seq_slot, c.table, c.table_width, c.ring,
              (__nv_bfloat16*)out, ldo, nh, nkv, window, scale, error_flag, c.planes, sink, head_sink, gate_col > 0 ? (const __nv_bfloat16*)qkv + gate_col : nullptr, ld, slopes, keep_first, v_group};
-  { int rc_ = cima_launch(k_attention_prefill_tc<HD, FROM_CACHE>, dim3((unsigned)n_tiles * (unsigned)nh), dim3(THREADS), smem, stream, 1, mq, mk, a); if (rc_) return rc_; }
+  { int rc_ = cima_launch(k_attention_prefill_tc<HD, FROM_CACHE, NEAR>, dim3((unsigned)n_tiles * (unsigned)nh), dim3(THREADS), smem, stream, 1, mq, mk, a); if (rc_) return rc_; }
   return cima_launch_result();
 }
 
 }  // namespace
+
+#define RUN(H, C) ((keep_first > 0 || v_group > 1) ? LAUNCH(H, C, true) : LAUNCH(H, C, false))
+#define LAUNCH(H, C, R) launch_attention_tc<H, C, R>(qkv, ld, tile_seq, tile_row0, seq_first_row, source, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream)
 
 static int tc_checks(const char* who, const void* qkv, int ld, const void* out, int ldo, int nh, int nkv, int hd, const int* error_flag,
                      int gate_col, int keep_first, int v_group, bool queries_only = false) {
@@ -441,10 +452,8 @@ extern "C" int cima_attention_prefill_tc(const void* qkv, int ld, const int* til
                                          int gate_col, const float* slopes, int keep_first, int v_group, cudaStream_t stream) {
   if (T <= 0 || n_tiles <= 0) return 0;
   if (int rc = tc_checks("attention_prefill_tc", qkv, ld, out, ldo, nh, nkv, hd, error_flag, gate_col, keep_first, v_group)) return rc;
-  const CacheSource none{nullptr, 0, nullptr, nullptr, nullptr, 0, 0};
-  if (hd == 64)
-    return launch_attention_tc<64, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, none, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
-  return launch_attention_tc<128, false>(qkv, ld, tile_seq, tile_row0, seq_first_row, none, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
+  const CacheSource source{nullptr, 0, nullptr, nullptr, nullptr, 0, 0};
+  return hd == 64 ? RUN(64, false) : RUN(128, false);
 }
 
 // The same for sequences that go on: the rows of sequence s are the positions seq_len[s] - rows .. seq_len[s] - 1, and
@@ -462,8 +471,8 @@ extern "C" int cima_attention_extend_tc(const void* qkv, int ld, const int* tile
   if (!cache || !table || !seq_slot || !seq_len || ((uintptr_t)cache & 15) || n_pages <= 0)
     return cima_fail(CIMA_E_ARG, "attention_extend_tc: the cache (16-byte aligned), its block table, slots and lengths are needed");
   if (n_pages * planes * nkv * BN >= (1ll << 31)) return cima_fail(CIMA_E_SIZE, "attention_extend_tc: %lld pages exceed a tensor map's 32-bit row coordinate", n_pages);
-  const CacheSource c{cache, n_pages, table, seq_slot, seq_len, table_width, ring, planes};
-  if (hd == 64)
-    return launch_attention_tc<64, true>(qkv, ld, tile_seq, tile_row0, seq_first_row, c, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
-  return launch_attention_tc<128, true>(qkv, ld, tile_seq, tile_row0, seq_first_row, c, out, ldo, T, n_tiles, nh, nkv, scale, window, error_flag, sink, head_sink, gate_col, slopes, keep_first, v_group, stream);
+  const CacheSource source{cache, n_pages, table, seq_slot, seq_len, table_width, ring, planes};
+  return hd == 64 ? RUN(64, true) : RUN(128, true);
 }
+#undef RUN
+#undef LAUNCH

@@ -691,6 +691,35 @@ def test_attention_tcgen05_with_kept_positions_and_shared_values(K, nh, nkv, hd,
         assert torch.equal(out, out2), cached
 
 
+@pytest.mark.parametrize("spread", [1.0, 2.0])
+@pytest.mark.parametrize("T,nh,nkv,hd,v_group,window,keep", [(700, 24, 4, 64, 2, 0, 0), (1100, 16, 4, 64, 2, 512, 64), (900, 12, 2, 128, 1, 300, 64)])
+def test_attention_tcgen05_as_near_to_64_bits_as_mma_sync(K, T, nh, nkv, hd, v_group, window, keep, spread):
+    """The forms that came to the tcgen05 kernel from the mma.sync one, from flat scores to rows of a few large probabilities: prompts
+    and the same rows from the cache.  Both round each probability to bfloat16 once, the largest being exactly 1, and here the denominator
+    has the same roundings: no further off than there."""
+    nv, scale = nkv // v_group, 1.0 / math.sqrt(hd)
+    qkv = g(T, (nh + nkv + nv) * hd, dtype=torch.bfloat16, seed=T, scale=spread).cuda()
+    b = batch_of([(0, 0, T)], "cuda")
+    q, k, v = (t.double().view(T, -1, hd).transpose(0, 1) for t in qkv.split([nh * hd, nkv * hd, nv * hd], dim=1))
+    i = torch.arange(T, device="cuda")
+    seen = i[None] <= i[:, None]
+    if window:
+        seen &= (i[:, None] - i[None] < window) | (i[None] < keep)
+    want = torch.stack([(q[h] @ k[h // (nh // nkv)].t() * scale).masked_fill(~seen, -math.inf).softmax(-1) @ v[h // (nh // nkv) // v_group] for h in range(nh)], 1).reshape(T, -1)
+    pages = -(-T // 64)
+    cpu, gpu = make_kv(pages, nkv, 64, hd, 1, pages, 0, window, torch.bfloat16, {0: list(range(pages))})
+    fill_cache(cpu, gpu, 0, qkv[:, nh * hd:(nh + nkv) * hd].view(T, nkv, hd).cpu(), torch.nn.functional.pad(qkv[:, (nh + nkv) * hd:].view(T, nv, hd), (0, 0, 0, nkv - nv)).cpu())
+    off = {}
+    for name, call in (("mma", lambda o: K.attention_prefill(qkv, b.q_tile_seq, b.q_tile_row0, b.seq_first_row, o, nh, nkv, hd, scale, window, keep_first=keep, v_group=v_group)),
+                       ("tc", lambda o: K.attention_prefill_tc(qkv, b, o, nh, nkv, hd, scale, window, keep_first=keep, v_group=v_group)),
+                       ("tc cached", lambda o: K.attention_prefill_tc(qkv, b, o, nh, nkv, hd, scale, window, kv=gpu, keep_first=keep, v_group=v_group))):
+        o = torch.empty(T, nh * hd, dtype=torch.bfloat16, device="cuda")
+        call(o)
+        off[name] = ((o.double() - want).norm() / want.norm()).item()
+    assert K.device_errors() == 0
+    assert max(off["tc"], off["tc cached"]) <= off["mma"], off
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 128), (6, 1, 64)])
 @pytest.mark.parametrize("window", [0, 90, 300])
 def test_attention_of_sequences_that_go_on_by_many_rows_tcgen05(K, nh, nkv, hd, window):
