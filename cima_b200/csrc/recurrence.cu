@@ -13,9 +13,9 @@
 // lanes' 16-byte reads of k, q and g from shared memory cover 32 consecutive words).  The step's tokens are walked in
 // order, 16 (8 for key sizes above 128) at a time: their k, q, g, v and beta are staged in shared memory, and the outputs
 // leave through it in whole rows.  A sum over the key channels is a lane's own rows in ascending order in two interleaved
-// partial sums, then a fixed shuffle tree over the 8 lanes, whatever the step: a token's result has the same bits whether
-// its sequence came whole, in pieces or one token at a time, alone or in a batch.  Everything is float32 but the loads of
-// q, k, v.
+// partial sums, then a fixed shuffle tree over the 8 lanes, whatever the step: a walked token's result has the same bits
+// whether its sequence came whole, in pieces or one token at a time, alone or in a batch.  Everything is float32 but the loads
+// of q, k, v.
 //
 // A token is a chain of some 600 cycles (measured: 315 ns a token of the gate rule at key and value size 128), of which its
 // instructions fill a sixth, so few sequences leave the SMs waiting.  Long steps of the decay and the gate rule, whose states
@@ -26,7 +26,8 @@
 //   combine   the state in front of every segment: S_0 = the stored state, S_(i+1) = D_i S_i + E_i
 //   PHASE 2   every segment from the state in front of it, with read-out; a sequence's last one stores the state
 // One and a half times the work, in place of the chain; PHASE 0 is the one launch for everything else.  Only bfloat16 rows are
-// cut: the 32-bit path keeps a token's bits whatever the cutting.
+// cut, and whether they are follows from the whole step (kernels.py, recurrence_segments), so a bfloat16 token's last bits depend
+// on what its sequence came with; the 32-bit path keeps a token's bits whatever the cutting.
 #include "common.cuh"
 
 namespace {

@@ -1028,17 +1028,23 @@ class Kernels:
     # ------------------------------------------------------------------ recurrent mixers
     RECURRENCE_SEGMENT = 128    # tokens of a segment of a long step's decay or gate rule
 
-    def recurrence_segments(self, batch, columns: int, dtype: torch.dtype) -> int:
+    def recurrence_segments(self, batch, columns: int, dtype: torch.dtype, dim: int = 128) -> int:
         """Into how many segments at most the step's sequences are cut by the decay and the gate rule (1: not at all); ``columns``:
-        blocks of 32 value channels, all heads.  Uncut, a sequence takes 600 cycles a token; cut, a block's token costs the SM some
-        110 cycles of instructions, half as many again for the first phase, and three launches and the states' way through memory
-        come to some 30,000 cycles: cut where that is less than the longest sequence's chain.  bfloat16 rows only (a 32-bit row has
-        the same bits however its sequence is cut).  Where a sequence is cut depends on the step, so a bfloat16 sequence's bits do."""
+        blocks of 32 value channels, all heads; ``dim``: the key size.  Cut where that is expected to be faster, in us at key size 128 (a
+        smaller one takes 0.7 of all but the launches): uncut, a token is 0.25 of the longest sequence's chain, 0.345 for each two blocks that
+        an SM has at once; cut, two segments' chains are 66 at least, and the SMs' instructions, two phases and the combination of the
+        states 30 + 0.2 for each of an SM's block-tokens.  Measured, uncut and cut, us: 16 heads of 128 x 128, one sequence of 256 tokens 66 / 76, of
+        512: 129 / 76, of 2,048: 503 / 212, two of 512: 129 / 117, four of 300: 108 / 158, four of 1,024: 350 / 378; 12 heads, eight of 1,024:
+        591 / 566; 28 heads, two of 300: 108 / 138, one of 2,048: 504 / 351.  bfloat16 rows only (a 32-bit row has the same bits
+        however its sequence is cut).  Where a sequence is cut depends on the step, so a bfloat16 sequence's bits do."""
         rows = int(getattr(batch, "max_rows", 0) or 0)
-        segs = -(-rows // self.RECURRENCE_SEGMENT)
-        if dtype is not torch.bfloat16 or rows < 2 * self.RECURRENCE_SEGMENT or 1.2 * batch.n_rows * columns + 30000 > 600 * rows or batch.n_rows // self.RECURRENCE_SEGMENT + batch.n_seqs > 65535:
+        if dtype is not torch.bfloat16 or rows < 2 * self.RECURRENCE_SEGMENT or batch.n_rows // self.RECURRENCE_SEGMENT + batch.n_seqs > 65535:
             return 1
-        return segs
+        per_sm = batch.n_rows * columns / 148                       # block-tokens
+        blocks = -(-batch.n_rows * columns // (148 * rows))         # on an SM at once, were all sequences as long as the longest
+        whole = rows * (0.345 * (blocks // 2) + 0.25 * (blocks % 2))
+        cut = max(66.0, (30.0 if dim > 64 else 43.0) + 0.2 * per_sm)
+        return -(-rows // self.RECURRENCE_SEGMENT) if cut < 0.95 * whole else 1
 
     def _segment_scratch(self, batch, values: int, device) -> torch.Tensor:
         """Scratch of a cut step: ``values`` float32 a segment, two places for every full segment's worth of rows (recurrence.cu)."""
@@ -1078,7 +1084,7 @@ class Kernels:
                            batch.n_seqs * heads * dim * vdim * 8 + T * (2 * kv_heads * dim * q.element_size() + heads * vdim * (4 + v.element_size())
                                                                         + (heads * dim * 4 if delta else 0)),
                            (8.0 if delta else 5.0) * T * heads * dim * vdim): return
-        cut = not delta and self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype) > 1
+        cut = not delta and self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype, dim) > 1
         buf = self._segment_scratch(batch, heads * dim * vdim, q.device) if cut else None
         self._check(self.lib.cima_recurrence(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
                                              dtype_code(v.dtype), _ptr(g), _ptr(beta), _ptr(decay), state.data_ptr(),
@@ -1102,7 +1108,7 @@ class Kernels:
                               f"out {tuple(out.shape)} and the gate's vectors do not agree with {heads} heads of {dim} x {vdim}")
         if not self._admit("recurrence[gate]", batch.n_seqs * heads * dim * vdim * 8 + T * heads * ((2 * dim + vdim) * v.element_size() + vdim * 4),
                            5.0 * T * heads * dim * vdim): return
-        cut = self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype) > 1
+        cut = self.recurrence_segments(batch, heads * -(-vdim // 32), v.dtype, dim) > 1
         buf = prod = None
         if cut:
             buf = self._segment_scratch(batch, heads * dim * vdim, q.device)

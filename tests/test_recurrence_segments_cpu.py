@@ -1,6 +1,10 @@
 """Where a cut step's segments stand: the numbers that the recurrence's kernels give their blocks and the places of the
 scratch (csrc/recurrence.cu, ``RecSegments``), over drawn steps."""
 import random
+from types import SimpleNamespace
+
+import pytest
+import torch
 
 
 def test_segments_have_blocks_and_places_of_their_own():
@@ -26,3 +30,17 @@ def test_segments_have_blocks_and_places_of_their_own():
                 lo, hi = (mid, hi) if first[mid] // seg + mid <= b else (lo, mid - 1)
             i = b - (first[lo] // seg + lo)
             assert i >= 0 and ((lo, i) == blocks[b] if b in blocks else i * seg >= rows[lo])
+
+
+@pytest.mark.parametrize("heads,dim,vdim,counts,cut", [
+    (16, 128, 128, [255], False), (16, 128, 128, [256], False), (16, 128, 128, [512], True), (16, 128, 128, [2048], True), (16, 128, 128, [300] * 4, False),
+    (16, 128, 128, [512] * 4, False), (16, 128, 128, [1024] * 4, False), (28, 128, 128, [300] * 2, False), (28, 128, 128, [2048], True),
+    (28, 128, 128, [512] * 2, False), (12, 128, 128, [900, 883, 531, 1080], True), (16, 128, 128, [4000] + [60] * 60, True), (8, 64, 64, [256] * 16, False),
+    (2, 64, 64, [256], False), (2, 64, 64, [2048], True), (4, 200, 64, [256] * 16, False), (14, 64, 64, [300] * 4, False), (1, 16, 8, [700, 5, 256], True)])
+def test_long_steps_are_cut_where_that_is_faster(heads, dim, vdim, counts, cut):
+    """Steps measured both ways: the ones that were 4 % and more faster whole are left whole, the others cut."""
+    from cima_b200.kernels import Kernels
+    batch = SimpleNamespace(max_rows=max(counts), n_rows=sum(counts), n_seqs=len(counts))
+    columns = heads * -(-vdim // 32)
+    assert Kernels.recurrence_segments(Kernels, batch, columns, torch.bfloat16, dim) == (-(-max(counts) // 128) if cut else 1)
+    assert Kernels.recurrence_segments(Kernels, batch, columns, torch.float32, dim) == 1
