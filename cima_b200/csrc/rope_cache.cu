@@ -263,10 +263,10 @@ k_norm_rope_append(TA* __restrict__ qkv, int ld, const float* __restrict__ inv_f
 // The norm, the rotation (ROT), the queries' factor and the append for heads of at most 128 values in multiples of 4: a block a
 // row, a lane four neighbouring values of a head in registers, a warp NORM_HEADS heads at a time with all their loads requested
 // before the first use.  The row's angles are made once (a block of four heads a row, as in the kernel above, made them sixteen
-// times at 32 + 32 heads); the value that one turns with stands rotary_dim / 8 lanes away.  Few rows (a decode step) share a row's
-// heads among blocks.  Bound by the rows' way through memory.  (2,048 rows of the 3B Lipizen shape: 22 us, 30 before.)
-constexpr int NORM_HEADS = 4;
-template <typename TA, bool ROT>
+// times at 32 + 32 heads); the value that one turns with stands rotary_dim / 8 lanes away.  Where few rows leave SMs idle, blocks
+// share a row's heads, a warp taking two or one of them (the angles made again; see the launch).  Bound by the rows' way through
+// memory, with few rows by a block's chain of loads.  (2,048 rows of the 3B Lipizen shape: 22 us, 30 before.)
+template <typename TA, bool ROT, int NORM_HEADS>
 __global__ void __launch_bounds__(128)
 k_norm_append(TA* __restrict__ qkv, int ld, const float* __restrict__ inv_freq, int rotary_dim, const int* __restrict__ row_pos,
               const int* __restrict__ row_seq, const int* __restrict__ seq_slot, const int* __restrict__ seq_len, TA* __restrict__ cache_in,
@@ -484,12 +484,18 @@ extern "C" int cima_rope_append(void* qkv, int dtype, int ld, const float* inv_f
     const size_t bytes = dtype == CIMA_F32 ? 4 : 2;
     const bool vec = hd % 4 == 0 && ld % 4 == 0 && ((uintptr_t)qkv % (4 * bytes)) == 0 && ((uintptr_t)cache % (4 * bytes)) == 0;
     if (vec && hd <= 128 && rotary_dim % 8 == 0) {
-      const dim3 rows((unsigned)T, T < 296 ? (unsigned)((nh + nkv + nv + 4 * NORM_HEADS - 1) / (4 * NORM_HEADS)) : 1u);
-#define RUN(TA, R) cima_launch(k_norm_append<TA, R>, rows, dim3(128), (size_t)0, stream, 1, (TA*)qkv, ld, inv_freq, rotary_dim, row_pos, row_seq, seq_slot, seq_len, (TA*)cache, pg, nh, nkv, nv, hd, q_norm, k_norm, norm_dim, eps, amp, temp_coef, temp_every)
+      // Heads a warp: one while that is a dozen blocks an SM or fewer, four (a block a row) from 2,048 rows on, else two.  40 heads of 64,
+      // one / two / four, us: 1 row 2.6 / 2.9 / 8.0, 64: 3.1 / 3.3 / 8.3, 400: 6.6 / 6.2 / 9.0, 1,400: 18.8 / 15.4 / 15.8, 4,096: 51 / 41 / 39
+      // (the kernel above: 3.1, 3.7 and 8.1 for 1, 64 and 400 rows).
+      const int heads = nh + nkv + nv, each = (long long)T * ((heads + 3) / 4) <= 1800 ? 1 : T < 2048 ? 2 : 4;
+      const dim3 rows((unsigned)T, each == 4 ? 1u : (unsigned)((heads + 4 * each - 1) / (4 * each)));
+#define RUN(TA, R) (each == 1 ? RUN_EACH(TA, R, 1) : each == 2 ? RUN_EACH(TA, R, 2) : RUN_EACH(TA, R, 4))
+#define RUN_EACH(TA, R, H) cima_launch(k_norm_append<TA, R, H>, rows, dim3(128), (size_t)0, stream, 1, (TA*)qkv, ld, inv_freq, rotary_dim, row_pos, row_seq, seq_slot, seq_len, (TA*)cache, pg, nh, nkv, nv, hd, q_norm, k_norm, norm_dim, eps, amp, temp_coef, temp_every)
       if (dtype == CIMA_F32) rc_ = rotary_dim ? RUN(float, true) : RUN(float, false);
       else if (dtype == CIMA_BF16) rc_ = rotary_dim ? RUN(__nv_bfloat16, true) : RUN(__nv_bfloat16, false);
       else return cima_fail(CIMA_E_DTYPE, "rope_append: dtype code %d is neither float32 nor bfloat16", dtype);
 #undef RUN
+#undef RUN_EACH
       return rc_ ? rc_ : cima_launch_result();
     }
     if (vec) {

@@ -914,6 +914,45 @@ def test_gated_pair_on_the_kernel_its_rule_picks(K, inter, width, rows, fused):
     assert err(got, want) <= 3 * 2.0 ** -8 * (z[:, :inter].abs().max() * z[:, inter:].abs().max()).item()
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("nh,nkv,hd,rotary,nd", [(5, 2, 64, 64, 64), (28, 4, 128, 64, 128), (3, 1, 16, 0, 8)])
+def test_norm_rotation_and_append_the_same_bits_for_any_number_of_rows(K, nh, nkv, hd, rotary, nd, dtype):
+    """Rows that a launch gives a warp one, two and four heads of (few, hundreds, 2,048 and more), at the lines between: each row and
+    its keys and values in the pages as when it comes alone; against the float64 statement."""
+    heads, T = nh + 2 * nkv, 2100
+    edge = 1800 // -(-heads // 4)
+    qkv = g(T, heads * hd, dtype=DT[dtype], seed=hd)
+    inv, norm = torch.rand(rotary // 2, generator=torch.Generator().manual_seed(2)), [1 + g(nd, seed=s, scale=0.1) for s in (3, 4)]
+    pages = -(-T // 64)
+
+    def run(first, n):
+        cpu, gpu = make_kv(pages, nkv, 64, hd, 1, pages, 0, 0, DT[dtype], {0: list(range(pages))})
+        b = batch_of([(0, first, n)], "cuda")
+        q = qkv[first:first + n].contiguous().cuda()
+        K.rope_append(q, inv.cuda(), rotary, b.row_pos, b.row_seq, b.seq_slot, torch.tensor([first + n], dtype=torch.int32, device="cuda"), gpu, nh, nkv, hd,
+                      qk_norm=(norm[0].cuda(), norm[1].cuda(), nd, 1e-6))
+        return q, gpu.storage.transpose(2, 3).reshape(pages, 2, 64, nkv, hd).transpose(1, 2).reshape(pages * 64, 2, nkv, hd)[first:first + n]
+
+    whole, kept = run(0, T)
+    for n in (edge, edge + 1, 2047, 2048):
+        part, kept_part = run(0, n)
+        assert torch.equal(part, whole[:n]) and torch.equal(kept_part, kept[:n]), n
+    for first in (0, 1, 777, T - 1):
+        part, kept_part = run(first, 1)
+        assert torch.equal(part[0], whole[first]) and torch.equal(kept_part[0], kept[first]), first
+    x = qkv.double().view(T, heads, hd)[:, :nh + nkv].clone()
+    r = 1.0 / torch.sqrt((x[..., :nd] ** 2).mean(-1, keepdim=True) + 1e-6)
+    w = torch.cat([norm[0].double().expand(nh, nd), norm[1].double().expand(nkv, nd)])
+    x[..., :nd] = x[..., :nd] * r * w
+    if rotary:
+        # the angle as the kernel has it, a float32 product: its sine and cosine move by that rounding, not by the kernel's own
+        angle = (torch.arange(T).float()[:, None] * inv).double()[:, None]
+        a, c = x[..., :rotary // 2].clone(), x[..., rotary // 2:rotary].clone()
+        x[..., :rotary // 2], x[..., rotary // 2:rotary] = a * angle.cos() - c * angle.sin(), a * angle.sin() + c * angle.cos()
+    assert err(whole[:, :(nh + nkv) * hd], x.reshape(T, -1)) <= TOL[dtype] * x.abs().max().item()
+    assert torch.equal(whole[:, nh * hd:].view(T, 2, nkv, hd)[:, 0], kept[:, 0]) and torch.equal(whole[:, nh * hd:].view(T, 2, nkv, hd)[:, 1], kept[:, 1])
+
+
 @pytest.mark.parametrize("M", [1, 5, 7, 8])
 @pytest.mark.parametrize("nh,nkv,hd,H", [(6, 2, 48, 200), (28, 4, 128, 3584), (3, 1, 64, 192), (4, 4, 16, 64)])
 def test_qkv_rope_skinny_equals_projection_then_rope_append(K, M, nh, nkv, hd, H):
