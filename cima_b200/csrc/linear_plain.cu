@@ -98,18 +98,20 @@ __device__ __forceinline__ void f32_finish(float* o, float v, const float* bias,
 // them: its pieces of the 8 weight rows travel through shared memory by cp.async, 256-byte runs of a row at a time, up
 // to FEW_STAGES pieces in flight, the first ones before the kernel ahead has finished where the caller says that it does not write them (`early`).  Lane =
 // (feature, row mod 4): a lane walks its feature's range in order for one or two rows of A.  8 features a block and not more:
-// a narrow product (896 features) still covers 112 SMs, and a wide one keeps several blocks on each.  Measured inside a decode
+// a narrow product (896 features) still covers 112 SMs, and a wide one keeps several blocks on each.  A sum of one range has no
+// work for a second warp, so there (ONE) each warp takes 8 features of its own, as many warps a block as leave a block for every SM
+// (16,384 features of 512 k, one row: 17 us; with one working warp of 8 a block 51).  Measured inside a decode
 // step of the 0.5B shape, 2 rows: 9.3 us a product on average, 2.2 TB/s (74.8 us and 0.27 TB/s with a thread an output feature).
 constexpr int FEW_ROWS = 8, FEW_F = 8, FEW_K = 64, FEW_PITCH = FEW_K + 4, FEW_STAGES = 4, FEW_WARPS = F32_GROUPS;
 
-template <int MR, bool VEC>        // MR: rows of A a lane takes (rows r, r + 4)
+template <int MR, bool VEC, bool ONE>        // MR: rows of A a lane takes (rows r, r + 4)
 __global__ void __launch_bounds__(32 * FEW_WARPS)
 k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out,
                  int M, int N, int K, int lda, int ldo, int mode, int stages, int early) {
   extern __shared__ __align__(16) float few_smem[];
   __shared__ float red[FEW_WARPS][FEW_ROWS][FEW_F];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * FEW_F;
-  const int len = f32_group_len(K), k0 = min(K, warp * len), kn = min(K, k0 + len) - k0, chunks = (kn + FEW_K - 1) / FEW_K;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = (ONE ? blockIdx.x * (blockDim.x >> 5) + warp : blockIdx.x) * FEW_F;
+  const int len = f32_group_len(K), k0 = ONE ? 0 : min(K, warp * len), kn = min(K, k0 + len) - k0, chunks = (kn + FEW_K - 1) / FEW_K;
   const int unit = (FEW_F + M) * FEW_PITCH;             // a stage: 8 rows of W, then M rows of A
   float* mine = few_smem + (size_t)warp * stages * unit;
   // half a warp brings a piece of one row (from k0 + c FEW_K on) to dst; what lies beyond the range is zero
@@ -175,6 +177,13 @@ k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const
   }
   f32_wait<0>();
   cima_pdl_trigger();
+  if constexpr (ONE) {
+    if (live && n0 + f < N) {
+      f32_finish(out + (size_t)r * ldo + n0 + f, acc[0], bias, n0 + f, mode);
+      if (MR > 1 && r + 4 < M) f32_finish(out + (size_t)(r + 4) * ldo + n0 + f, acc[MR - 1], bias, n0 + f, mode);
+    }
+    return;
+  }
   if (live) {
     red[warp][r][f] = acc[0];
     if (MR > 1 && r + 4 < M) red[warp][r + 4][f] = acc[MR - 1];
@@ -192,7 +201,7 @@ k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const
 // More rows: bound by the FP32 pipe.  Tiles of BM x 128 outputs, 256 threads with BM / 16 x 8 outputs each.  The next 16 k travel
 // through registers while the current ones are multiplied.  (Products two at a time, fma.rn.f32x2, want every value of A twice in
 // shared memory and were no faster.)  SPLIT: a cluster of 8 blocks shares a tile, a range of k each, and adds the ranges' sums in
-// order through distributed shared memory (see launch_f32 for when).  Measured inside a prompt step of the 0.5B shape, 201 + 123
+// order through distributed shared memory (see launch_f32 for when).  Measured inside a prompt step of the 0.5B shape, 201 + 197
 // rows: 112 us a product on average, 26 TFLOP/s (322 us with tiles of 64 x 64 and 4 x 4 a thread); by themselves, alone and shared: 1,152 x 896 95 and 30 us, 9,728 x 896 187 and
 // 186, 896 x 4,864 491 and 124; tiles of 64 rows for 37 rows of 1,152 x 896: 11.5, of 128: 17.
 constexpr int F32_BN = 128, F32_BK = 16, F32_WROW = F32_BN + 4;
@@ -385,16 +394,18 @@ template <bool VEC>
 static int launch_f32(const float* A, const float* W, const float* bias, float* out, int mode, int M, int N, int K, int lda, int ldo,
                       int early, cudaStream_t stream) {
   if (M <= FEW_ROWS) {
-    const int chunks = (f32_group_len(K) + FEW_K - 1) / FEW_K, unit = (FEW_F + M) * FEW_PITCH * (int)sizeof(float) * FEW_WARPS;
-    const int blocks = (N + FEW_F - 1) / FEW_F;
+    const bool one = K <= F32_ONE_RANGE;
+    const int parts = (N + FEW_F - 1) / FEW_F, warps = one ? max(1, min(FEW_WARPS, parts / 148)) : FEW_WARPS;
+    const int chunks = (f32_group_len(K) + FEW_K - 1) / FEW_K, unit = (FEW_F + M) * FEW_PITCH * (int)sizeof(float) * warps;
+    const int blocks = one ? (parts + warps - 1) / warps : parts;
     // the most pieces in flight that leave room for two blocks on an SM: its own, or the next launch's, whose weights are then
     // requested while this one ends
     const int room = 110 * 1024;
     const int stages = chunks >= FEW_STAGES && FEW_STAGES * unit <= room ? FEW_STAGES : chunks >= 2 ? 2 : 1;
     const size_t smem = (size_t)stages * unit;
-    auto kern = M <= 4 ? k_linear_f32_few<1, VEC> : k_linear_f32_few<2, VEC>;
+    auto kern = one ? (M <= 4 ? k_linear_f32_few<1, VEC, true> : k_linear_f32_few<2, VEC, true>) : M <= 4 ? k_linear_f32_few<1, VEC, false> : k_linear_f32_few<2, VEC, false>;
     if (int rc = f32_allow(kern, smem)) return rc;
-    return cima_launch(kern, dim3((unsigned)blocks), dim3(32 * FEW_WARPS), smem, stream, 1, A, W, bias, out, M, N, K, lda, ldo, mode, stages, early);
+    return cima_launch(kern, dim3((unsigned)blocks), dim3(32 * warps), smem, stream, 1, A, W, bias, out, M, N, K, lda, ldo, mode, stages, early);
   }
   // The tile's rows, and whether clusters share a tile, by the time of the SM that gets the most blocks: a block's rows (a lower tile
   // reads more of shared memory for a product: measured at 0.9 and 0.7 of the rate), an eighth of them where a cluster shares the tile (and

@@ -112,11 +112,12 @@ def test_linear_plain_rows_are_independent(K, rows, N, K_):
     assert torch.equal(acc_full[33:33 + rows], acc_few)
 
 
-@pytest.mark.parametrize("N,K_", [(129, 256), (127, 512), (128, 513), (127, 516), (896, 4864), (20000, 896), (260, 1000), (130, 1021), (40, 4864)])
+@pytest.mark.parametrize("N,K_", [(129, 256), (127, 512), (128, 513), (127, 516), (896, 4864), (20000, 896), (260, 1000), (130, 1021), (40, 4864), (2367, 200), (2377, 510),
+                                  (9473, 72), (9479, 37)])
 def test_linear_float32_the_same_bits_from_every_kernel(K, N, K_):
     """Rows 1 to 8 (a warp a range of k), 9 to 32, 33 to 64, 65 and more (tiles of 32, 64 and 128 rows; shared by a cluster where a
     product has few tiles, alone where it has many): one order of the sums, so one result; sizes around the tiles' edges, sums of one
-    range of k (up to 512) and of eight, ranges that end early, rows whose bytes are no multiple of 16.  Tolerance: a range's steps (K, or
+    range of k (up to 512; one, two and eight warps a block with 8 features each) and of eight, ranges that end early, rows whose bytes are no multiple of 16.  Tolerance: a range's steps (K, or
     at most K / 8 + 15) and the eight ranges', each half an ulp of a sum that stays below the sum of the magnitudes."""
     M = 200
     a, w, b = g(M, K_, seed=4), g(N, K_, seed=5, scale=0.1), g(N, seed=6)
