@@ -102,10 +102,12 @@ k_attention_plain(const TA* __restrict__ qkv, int ld, const TA* __restrict__ cac
 // 200 positions, a chain of some 1.4 us a key; bound by latency.)
 //
 // A block owns up to QV query vectors of one sequence and key head: neighbouring rows times the heads that share the key head,
-// so that a piece's keys and values serve them all.  Its warps take the pieces in turn, each through its own shared memory
-// (cp.async), a lane a key for the scores and a lane NI dims for the weighted sums; what a round of pieces gives is merged by
-// the block in their order.  A decode step has a row a block and 8 warps, a prompt as many rows as QV allows and 4.
-// Measured at the 0.5B shape: 14.0 us for 2 rows at some 200 positions (294), 109 us for prompts of 201 and 123 rows (153).
+// so that a piece's keys and values serve them all.  Its teams of warps take the pieces in turn, each team through its own shared
+// memory (cp.async), a lane a key for the scores and a lane NI dims for the weighted sums, the vectors in eights over the team's
+// warps; what a round of pieces gives is merged by the block in their order.  Rows, teams and warps a team: launch_attention_f32.
+// Measured, us (a warp that walks one key after another): 14 heads of 64 on 2, one row at 100 positions 11.8 (75), at 1,000: 43 (721), two
+// prompts of 200 rows 57 (135), one of 1,000: 304 (1,171).  A sequence of a dozen positions or fewer does not repay a piece's own chain: one
+// row at 8 positions 10 (8.7), a prompt of 5 rows 8.9 (5.4); it stays here, as its later rows' bits follow from this order.
 constexpr int AF_KEYS = 32;
 
 struct AfArgs {
@@ -113,17 +115,18 @@ struct AfArgs {
   const int *row_pos, *row_seq, *seq_slot, *seq_first_row;
   float* out;
   CimaPaged pg;
-  int ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, rows, heads;      // a block's rows, and heads of a key head
+  int ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, rows, heads, team;      // a block's rows, and heads of a key head; warps of a team
   float scale, sink;
 };
 
 template <int HDP> constexpr int AF_QV = HDP <= 64 ? 32 : HDP <= 128 ? 24 : 16;
-static size_t af_smem(int hdp, int warps, int qv) {
-  return sizeof(float) * ((size_t)warps * 2 * AF_KEYS * (hdp + 4) + (size_t)2 * qv * hdp + (size_t)warps * qv * (hdp + 4) + (size_t)warps * 8 * AF_KEYS);
+template <int HDP> constexpr int AF_THREADS = HDP <= 128 ? 256 : 128;
+static size_t af_smem(int hdp, int teams, int team, int qv) {
+  return sizeof(float) * ((size_t)teams * 2 * AF_KEYS * (hdp + 4) + (size_t)2 * qv * hdp + (size_t)teams * qv * (hdp + 4) + (size_t)teams * team * 8 * AF_KEYS);
 }
 
 template <int HDP, bool FROM_CACHE, bool VEC>
-__global__ void __launch_bounds__(HDP <= 64 ? 256 : 128)
+__global__ void __launch_bounds__(AF_THREADS<HDP>)
 k_attention_f32(const __grid_constant__ AfArgs a) {
   constexpr int NI = HDP / 32, PITCH = HDP + 4, QVM = AF_QV<HDP>;
   extern __shared__ __align__(16) float af[];
@@ -131,16 +134,17 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
   __shared__ int s_any[8][QVM];
   cima_pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  const int teams = warps / a.team, slot_of = warp / a.team, member = warp - slot_of * a.team;
   const int group = a.nh / a.nkv, per_kv = (group + a.heads - 1) / a.heads;      // blocks of heads of one key head
   const int kvh = blockIdx.y / per_kv, h0 = kvh * group + (blockIdx.y % per_kv) * a.heads;
   const int heads = min(a.heads, (kvh + 1) * group - h0), vh = kvh / a.v_group;
   const int qvs_max = a.rows * a.heads, hd = a.hd, hdr = (hd + 3) & ~3;
-  float* Kt = af + (size_t)warp * 2 * AF_KEYS * PITCH;
+  float* Kt = af + (size_t)slot_of * 2 * AF_KEYS * PITCH;
   float* Vt = Kt + AF_KEYS * PITCH;
-  float* Q = af + (size_t)warps * 2 * AF_KEYS * PITCH;          // [qv][HDP]
+  float* Q = af + (size_t)teams * 2 * AF_KEYS * PITCH;          // [qv][HDP]
   float* O = Q + (size_t)qvs_max * HDP;                          // [qv][HDP], the running weighted sums
-  float* part = O + (size_t)qvs_max * HDP;                       // [warp][qv][PITCH], a round's pieces
-  float* P = part + (size_t)warps * qvs_max * PITCH + (size_t)warp * 8 * AF_KEYS;      // [8][32], the warp's weights
+  float* part = O + (size_t)qvs_max * HDP;                       // [team][qv][PITCH], a round's pieces
+  float* P = part + (size_t)teams * qvs_max * PITCH + (size_t)warp * 8 * AF_KEYS;      // [8][32], the warp's weights
   const int t0 = blockIdx.x * a.rows, t1 = min(a.T, t0 + a.rows);
 
   for (int r0 = t0; r0 < t1;) {                          // rows of one sequence at a time
@@ -161,13 +165,15 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
     }
     for (int i = tid; i < qvs; i += blockDim.x) { run_m[i] = -1e30f; run_l[i] = 0.f; }
     __syncthreads();
-    for (int base = 0; base < pieces; base += warps) {
-      const int mine = base + warp;
+    for (int base = 0; base < pieces; base += teams) {
+      const int mine = base + slot_of;
+      const int b = mine < kept_pieces ? mine : b0 + mine - kept_pieces;
+      const int j = b * AF_KEYS + lane;
+      // what no row sees is not read (pages may hold anything there), and its place in shared memory not used
+      const bool seen = mine < pieces && j <= pmax && (j >= lo || j < kept);
+      const unsigned have = __ballot_sync(0xffffffffu, seen);
+      const int keys = 32 - __clz(have);                 // behind the last one that is seen
       if (mine < pieces) {
-        const int b = mine < kept_pieces ? mine : b0 + mine - kept_pieces;
-        const int j = b * AF_KEYS + lane;
-        // what no row sees is not read (pages may hold anything there)
-        const bool seen = j <= pmax && (j >= lo || j < kept);
         const float *kp = nullptr, *vp = nullptr;
         if (seen) {
           if (FROM_CACHE) {
@@ -179,8 +185,7 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
             vp = a.qkv + (size_t)(first + j) * a.ld + (size_t)(a.nh + a.nkv + vh) * hd;
           }
         }
-        const unsigned have = __ballot_sync(0xffffffffu, seen);
-        for (int key = 0; key < AF_KEYS; key++) {
+        auto bring = [&](int key) {
           const float* ks = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(kp), key));
           const float* vs = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(vp), key));
           const bool ok = have >> key & 1;
@@ -202,11 +207,19 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
               Vt[key * PITCH + d] = ok && d < hd ? vs[d] : 0.f;
             }
           }
+        };
+        if (a.team == 1 && keys == AF_KEYS) {
+          for (int key = 0; key < AF_KEYS; key++) bring(key);
+        } else {
+          for (int key = member; key < keys; key += a.team) bring(key);
         }
         if constexpr (VEC) asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-        __syncwarp();
-        float* mypart = part + (size_t)warp * qvs_max * PITCH;
-        for (int v0 = 0; v0 < qvs; v0 += 8) {            // eight query vectors at a time
+      }
+      if (a.team > 1) __syncthreads();
+      else __syncwarp();
+      if (mine < pieces) {
+        float* mypart = part + (size_t)slot_of * qvs_max * PITCH;
+        for (int v0 = 8 * member; v0 < qvs; v0 += 8 * a.team) {      // eight query vectors at a time
           float s[8];
           const float* q[8];
 #pragma unroll
@@ -238,7 +251,7 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
             P[x * AF_KEYS + lane] = p;
-            if (lane == 0 && v0 + x < qvs) { s_m[warp][v] = m; s_l[warp][v] = l; s_any[warp][v] = vis[x] != 0u; }
+            if (lane == 0 && v0 + x < qvs) { s_m[slot_of][v] = m; s_l[slot_of][v] = l; s_any[slot_of][v] = vis[x] != 0u; }
           }
           __syncwarp();
           float o[8][NI];
@@ -246,8 +259,7 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
           for (int x = 0; x < 8; x++)
 #pragma unroll
             for (int i = 0; i < NI; i++) o[x][i] = 0.f;
-#pragma unroll 2
-          for (int k = 0; k < AF_KEYS; k += 4) {
+          auto weigh = [&](int k, bool whole) {
             float vv[4][NI];
 #pragma unroll
             for (int e = 0; e < 4; e++)
@@ -257,20 +269,20 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
             for (int x = 0; x < 8; x++) {
               const float4 p4 = *reinterpret_cast<const float4*>(P + x * AF_KEYS + k);
               const float p[4] = {p4.x, p4.y, p4.z, p4.w};
-              if (all == 0xffffffffu) {
 #pragma unroll
-                for (int e = 0; e < 4; e++)
+              for (int e = 0; e < 4; e++)
+                if (whole || (vis[x] >> (k + e) & 1)) {
 #pragma unroll
                   for (int i = 0; i < NI; i++) o[x][i] = fmaf(p[e], vv[e][i], o[x][i]);
-              } else {                                   // a value that the row does not see stays out, whatever it is
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                  if (vis[x] >> (k + e) & 1) {
-#pragma unroll
-                    for (int i = 0; i < NI; i++) o[x][i] = fmaf(p[e], vv[e][i], o[x][i]);
-                  }
-              }
+                }
             }
+          };
+          if (all == 0xffffffffu) {
+#pragma unroll 2
+            for (int k = 0; k < AF_KEYS; k += 4) weigh(k, true);
+          } else {                                       // a value that the row does not see stays out, whatever it is
+#pragma unroll 1
+            for (int k = 0; k < keys; k += 4) weigh(k, false);
           }
 #pragma unroll
           for (int x = 0; x < 8; x++)
@@ -282,7 +294,7 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
         }
       }
       __syncthreads();
-      const int there = min(warps, pieces - base);
+      const int there = min(teams, pieces - base);
       for (int v = tid; v < qvs; v += blockDim.x) {      // the factors of the round's pieces, in their order
         float m = run_m[v], l = run_l[v];
         for (int w = 0; w < there; w++) {
@@ -322,17 +334,28 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
   }
 }
 
+// max_keys: positions of the longest sequence after the step.  The bits do not depend on rows, teams or warps.
 template <int HDP, bool FROM_CACHE>
-static int launch_attention_f32(AfArgs a, bool vec, cudaStream_t stream) {
+static int launch_attention_f32(AfArgs a, bool vec, int n_seqs, int max_keys, cudaStream_t stream) {
   const int group = a.nh / a.nkv;
   a.heads = group < AF_QV<HDP> ? group : AF_QV<HDP>;
   const int per_kv = (group + a.heads - 1) / a.heads;
-  // few rows: a row a block, so that rows do not wait for one another; many: as many rows as share a block's keys
+  // Few rows: a row a block, so that rows do not wait for one another; many: as many rows as share a block's keys, and no more than a
+  // sequence has (64 sequences' decode rows in blocks of 32 took 917 us, one after another in each block; 201 so).
   const bool few = (long long)a.T * a.nkv * per_kv <= 592;
-  a.rows = few ? 1 : AF_QV<HDP> / a.heads;
-  int warps = HDP <= 64 ? (few ? 8 : 4) : HDP <= 128 ? 4 : 2;
-  if (af_smem(HDP, warps, a.rows * a.heads) > 220 * 1024) warps /= 2;
-  const size_t smem = af_smem(HDP, warps, a.rows * a.heads);
+  const int vectors = AF_QV<HDP>;
+  const int average = (a.T + n_seqs - 1) / n_seqs, most = max(1, vectors / a.heads), parts = (average + most - 1) / most;
+  a.rows = few ? 1 : (average + parts - 1) / parts;
+  // A team a piece, no more than there are pieces (a team's shared memory is another block's: 16 prompts of 20 rows, 32 heads of 64, took 148 us; 29 so),
+  // and the spare warps are the teams': they share its loads and vectors.
+  int teams = HDP <= 64 ? (few ? 8 : 4) : HDP <= 128 ? 4 : 2;
+  while (teams > 1 && (teams - 1) * AF_KEYS >= max_keys) teams--;
+  for (;; teams--) {
+    a.team = AF_THREADS<HDP> / 32 / teams;
+    if (teams == 1 || af_smem(HDP, teams, a.team, a.rows * a.heads) <= 220 * 1024) break;
+  }
+  const int warps = teams * a.team;
+  const size_t smem = af_smem(HDP, teams, a.team, a.rows * a.heads);
   auto kern = vec ? k_attention_f32<HDP, FROM_CACHE, true> : k_attention_f32<HDP, FROM_CACHE, false>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cima_fail((int)e, "attention_plain: %zu bytes of shared memory are not available: %s", smem, cudaGetErrorString(e));
@@ -341,12 +364,13 @@ static int launch_attention_f32(AfArgs a, bool vec, cudaStream_t stream) {
 }
 
 // from_cache 0: keys/values of the step (seq_first_row needed); 1: of the cache (table, seq_slot needed).
+// n_seqs: sequences of the step; max_keys: positions of the longest after it (0: not known).  Neither changes a result.
 extern "C" int cima_attention_plain(const void* qkv, int dtype, int ld, const void* cache, const int* table,
                                     int table_width, int ring, int page_size, const int* row_pos,
                                     const int* row_seq, const int* seq_slot, const int* seq_first_row, void* out,
                                     int ldo, int T, int nh, int nkv, int hd, float scale, int window,
                                     int from_cache, int planes, float sink, int keep_first, int v_group, const float* head_sink,
-                                    int gate_col, const float* slopes, cudaStream_t stream) {
+                                    int gate_col, const float* slopes, int n_seqs, int max_keys, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (hd <= 0 || hd > 1024) return cima_fail(CIMA_E_SIZE, "attention_plain: head_dim %d is outside 1..1024", hd);
   if (planes != 1 && planes != 2) return cima_fail(CIMA_E_ARG, "attention_plain: %d planes; pages hold keys | values (2) or one shared vector (1)", planes);
@@ -356,14 +380,16 @@ extern "C" int cima_attention_plain(const void* qkv, int dtype, int ld, const vo
   if (from_cache && (!cache || !table)) return cima_fail(CIMA_E_ARG, "attention_plain: decoding needs the cache and its block table");
   if (gate_col < 0 || (gate_col > 0 && gate_col + nh * hd > ld)) return cima_fail(CIMA_E_ARG, "attention_plain: %d gate values from column %d on exceed the rows of %d", nh * hd, gate_col, ld);
   CimaPaged pg{table, table_width, ring, page_size, nkv, hd, planes};
+  if (n_seqs <= 0) n_seqs = T;
+  if (max_keys <= 0) max_keys = from_cache ? 0x7fffffff : T;
   if (dtype == CIMA_F32 && hd <= 256) {
     AfArgs a{(const float*)qkv, (const float*)cache, head_sink, slopes, row_pos, row_seq, seq_slot, seq_first_row, (float*)out, pg,
-             ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, 1, 1, scale, sink};
+             ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, 1, 1, 1, scale, sink};
     const bool vec = hd % 4 == 0 && (from_cache || ld % 4 == 0) && ((from_cache ? (uintptr_t)cache : (uintptr_t)qkv) & 15) == 0;
     int rc;
-    if (hd <= 64) rc = from_cache ? launch_attention_f32<64, true>(a, vec, stream) : launch_attention_f32<64, false>(a, vec, stream);
-    else if (hd <= 128) rc = from_cache ? launch_attention_f32<128, true>(a, vec, stream) : launch_attention_f32<128, false>(a, vec, stream);
-    else rc = from_cache ? launch_attention_f32<256, true>(a, vec, stream) : launch_attention_f32<256, false>(a, vec, stream);
+    if (hd <= 64) rc = from_cache ? launch_attention_f32<64, true>(a, vec, n_seqs, max_keys, stream) : launch_attention_f32<64, false>(a, vec, n_seqs, max_keys, stream);
+    else if (hd <= 128) rc = from_cache ? launch_attention_f32<128, true>(a, vec, n_seqs, max_keys, stream) : launch_attention_f32<128, false>(a, vec, n_seqs, max_keys, stream);
+    else rc = from_cache ? launch_attention_f32<256, true>(a, vec, n_seqs, max_keys, stream) : launch_attention_f32<256, false>(a, vec, n_seqs, max_keys, stream);
     return rc ? rc : cima_launch_result();
   }
   dim3 grid((T + 3) / 4, nh);

@@ -15,7 +15,7 @@ import torch
 from .csrc.build import BuildError, library_path
 
 F32, BF16 = 0, 1
-ABI_VERSION = 36
+ABI_VERSION = 37
 SPLIT_BLOCKS = 296          # blocks of the decode attention that one wave holds (two per SM, 148 SMs)
 TC_ATTENTION_MIN_LEN = 256  # prompts from this length on take the tcgen05 attention (head_dim 64 or 128)
 SPLIT_FEW_BLOCKS = 148      # below this many blocks at 8 splits, more splits are taken
@@ -37,7 +37,8 @@ EXTEND_BLOCKS = 444         # blocks of the attention of going-on rows that one 
 
 def extend_splits(blocks: int, max_len: int, window: int, keep_first: int) -> int:
     """How many blocks share the key tiles of a block of rows that goes on from the cache: as many as fill one wave, each with
-    at least four tiles of 64 keys (a split costs its sums' way through memory and the merge's launch), 64 at most.
+    at least four tiles of 64 keys (a split costs its sums' way through memory and the merge's launch), 64 at most.  The number
+    follows from the step, so a row's last bits depend on what it came with.
     ``max_len``: positions of the longest sequence after the step (0: not known, one block then)."""
     seen = max_len if window <= 0 else min(max_len, window + 128 + -(-keep_first // 64) * 64)
     tiles = -(-seen // 64)
@@ -85,7 +86,7 @@ _SIGNATURES = {
                              _i, _i, _i, _i, _vp],
     "cima_rope_append": [_vp, _i, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _f, _f, _f, _i, _vp],
     "cima_attention_plain": [_vp, _i, _i, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i,
-                             _f, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _vp],
+                             _f, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _i, _i, _vp],
     "cima_attention_decode": [_vp, _i, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _vp],
     "cima_attention_prefill": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _vp, _i, _vp, _vp],
     "cima_attention_extend": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _f, _i, _i, _vp, _i, _vp,
@@ -496,7 +497,9 @@ class Kernels:
     def attention_plain(self, qkv: torch.Tensor, kv, row_pos, row_seq, seq_slot, seq_first_row, out: torch.Tensor,
                         n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int,
                         from_cache: bool, sink: float = 0.0, keep_first: int = 0, v_group: int = 1, head_sink=None, gate_col: int = 0,
-                        slopes=None) -> None:
+                        slopes=None, max_len: int = 0) -> None:
+        """``attention`` by the plain kernels, for any dtype and head size.  ``max_len``: positions of the longest sequence after the step
+        (0: not known); it changes how the work is shared, not the result."""
         self._need(qkv, "qkv", None, 2); self._need(out, "out", qkv.dtype, 2)
         self._need_head_sink(head_sink, n_heads, slopes)
         T = qkv.shape[0]
@@ -516,7 +519,7 @@ class Kernels:
                                                   seq_first_row.data_ptr(), out.data_ptr(), out.shape[1], T,
                                                   n_heads, n_kv_heads, head_dim, scale, window,
                                                   1 if from_cache else 0, planes, sink, keep_first, v_group, _ptr(head_sink),
-                                                  gate_col, _ptr(slopes), self._stream()), "attention_plain")
+                                                  gate_col, _ptr(slopes), seq_first_row.numel() - 1, max_len, self._stream()), "attention_plain")
 
     def _need_head_sink(self, head_sink, n_heads: int, slopes=None) -> None:
         if slopes is not None:
@@ -593,7 +596,7 @@ class Kernels:
                                           keep_first=keep_first, v_group=v_group, head_sink=head_sink, gate_col=gate_col, slopes=slopes)
         self.attention_plain(qkv, kv, batch.row_pos, batch.row_seq, batch.seq_slot, batch.seq_first_row, out,
                              n_heads, n_kv_heads, head_dim, scale, window, from_cache, sink=sink, keep_first=keep_first,
-                             v_group=v_group, head_sink=head_sink, gate_col=gate_col, slopes=slopes)
+                             v_group=v_group, head_sink=head_sink, gate_col=gate_col, slopes=slopes, max_len=int(getattr(batch, "max_len", 0) or 0))
 
     def attention_prefill(self, qkv: torch.Tensor, tile_seq, tile_row0, seq_first_row, out: torch.Tensor,
                           n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int, sink: float = 0.0,

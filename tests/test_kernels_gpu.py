@@ -410,6 +410,41 @@ def test_attention_float32_the_same_bits_however_cut(K, nh, nkv, hd, window, kee
     assert err(step[:n - 1], want[:n - 1]) <= TOL["float32"]
 
 
+@pytest.mark.parametrize("nh,nkv,hd,window,keep", [(14, 2, 64, 0, 0), (6, 6, 64, 0, 0), (40, 2, 32, 50, 9), (12, 1, 96, 0, 0), (3, 3, 200, 64, 40), (2, 1, 30, 0, 0)])
+def test_attention_float32_the_same_bits_in_any_company(K, nh, nkv, hd, window, keep):
+    """Prompts of 1 to 131 rows and of 20 rows sixteen times in one step, and one more row of each from the cache in one step: each
+    sequence as when it comes alone, whatever rows, teams and warps a block has there and whether the longest length is known."""
+    page, rows = 16, [1, 5, 31, 32, 33, 64, 131] + [20] * 16
+    n = len(rows)
+    tables, n_pages, width = scattered_tables([r + 1 for r in rows], list(range(n)), page, seed=hd)
+    cpu, gpu = make_kv(n_pages, nkv, page, hd, n, width, 0, 0, torch.float32, tables)
+    qkv, last = g(sum(rows), (nh + 2 * nkv) * hd, seed=7), g(n, (nh + 2 * nkv) * hd, seed=8)
+    first = [sum(rows[:i]) for i in range(n + 1)]
+    for i, r in enumerate(rows):
+        all_rows = torch.cat([qkv[first[i]:first[i] + r], last[i:i + 1]])
+        fill_cache(cpu, gpu, i, all_rows[:, nh * hd:(nh + nkv) * hd].reshape(r + 1, nkv, hd), all_rows[:, (nh + nkv) * hd:].reshape(r + 1, nkv, hd))
+
+    def run(seqs, x, cached, max_len):
+        b, out = batch_of(seqs, "cuda"), torch.full((len(x), nh * hd), 7.0, device="cuda")
+        K.attention_plain(x.cuda(), gpu if cached else None, b.row_pos, b.row_seq, b.seq_slot, b.seq_first_row, out, nh, nkv, hd, 1.0 / math.sqrt(hd), window,
+                          cached, keep_first=keep, max_len=max_len)
+        return out
+
+    prompts = [(i, 0, r) for i, r in enumerate(rows)]
+    whole, known = run(prompts, qkv, False, 0), run(prompts, qkv, False, max(rows))
+    more = [(i, r, 1) for i, r in enumerate(rows)]
+    steps, steps_known = run(more, last, True, 0), run(more, last, True, max(rows) + 1)
+    assert torch.equal(whole, known) and torch.equal(steps, steps_known)
+    for i, r in enumerate(rows[:9]):
+        x = qkv[first[i]:first[i] + r]
+        assert torch.equal(run([(i, 0, r)], x, False, r), whole[first[i]:first[i] + r]), r
+        assert torch.equal(run([(i, 0, r)], x, True, 0), whole[first[i]:first[i] + r]), r
+        assert torch.equal(run([(i, r, 1)], last[i:i + 1], True, r + 1)[0], steps[i]) and torch.equal(run([(i, r, 1)], last[i:i + 1], True, 0)[0], steps[i]), r
+    bc, want = batch_of(prompts, "cpu"), torch.zeros(sum(rows), nh * hd, dtype=torch.float64)
+    REF.attention_plain(qkv, None, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_first_row, want, nh, nkv, hd, 1.0 / math.sqrt(hd), window, False, keep_first=keep)
+    assert err(whole, want) <= TOL["float32"]
+
+
 @pytest.mark.parametrize("dtype,hd,n_splits", [("float32", 64, 0), ("float32", 300, 0), ("bfloat16", 64, 1), ("bfloat16", 64, 3)])
 def test_attention_without_a_sink_at_low_scores(K, dtype, hd, n_splits):
     """An ordinary softmax whose scores all lie near -150, from one key (a sequence's first row) to 140: the exponential of minus the
