@@ -633,15 +633,15 @@ class Kernels:
         if n_splits is None:
             n_splits = extend_splits(batch.q_tile_seq.numel() * n_heads, int(getattr(batch, "max_len", 0) or 0), window, keep_first)
         part_o = part_ml = None
-        if n_splits > 1:
-            part_o = torch.empty(T * n_heads * n_splits * head_dim, dtype=torch.float32, device=qkv.device)
-            part_ml = torch.empty(T * n_heads * n_splits * 2, dtype=torch.float32, device=qkv.device)
+        if n_splits > 1:                                  # (one allocation: such a step waits for its launches' host)
+            part = torch.empty(T * n_heads * n_splits * (head_dim + 2), dtype=torch.float32, device=qkv.device)
+            part_o, part_ml = part.data_ptr(), part.data_ptr() + 4 * T * n_heads * n_splits * head_dim
         self._check(self.lib.cima_attention_extend(
             qkv.data_ptr(), qkv.shape[1], batch.q_tile_seq.data_ptr(), batch.q_tile_row0.data_ptr(),
             batch.seq_first_row.data_ptr(), kv.storage.data_ptr(), kv.block_table.data_ptr(), kv.block_table.shape[1],
             kv.ring_pages, kv.page_size, batch.seq_slot.data_ptr(), batch.seq_len.data_ptr(), out.data_ptr(), out.shape[1],
             T, batch.q_tile_seq.numel(), n_heads, n_kv_heads, head_dim, scale, window, kv.planes, sink, keep_first, v_group,
-            _ptr(head_sink), gate_col, _ptr(slopes), n_splits, _ptr(part_o), _ptr(part_ml), self._stream()), "attention_extend")
+            _ptr(head_sink), gate_col, _ptr(slopes), n_splits, part_o, part_ml, self._stream()), "attention_extend")
         if n_splits > 1:
             self.launches += 1
 
@@ -717,10 +717,10 @@ class Kernels:
             # this call's own, from the recording's memory where the step is recorded: another stream's step, or another recording's
             # replay, may be between its splits and their merge at the same time
             part = torch.empty(B * n_heads * n_splits * (head_dim + 2), dtype=torch.float32, device=qkv.device)
-            part_o, part_ml = part, part[B * n_heads * n_splits * head_dim:]
+            part_o, part_ml = part.data_ptr(), part.data_ptr() + 4 * B * n_heads * n_splits * head_dim
         self._check(self.lib.cima_attention_decode(
             qkv.data_ptr(), qkv.shape[1], kv.storage.data_ptr(), kv.block_table.data_ptr(), kv.block_table.shape[1],
-            kv.ring_pages, kv.page_size, seq_slot.data_ptr(), seq_len.data_ptr(), _ptr(part_o), _ptr(part_ml),
+            kv.ring_pages, kv.page_size, seq_slot.data_ptr(), seq_len.data_ptr(), part_o, part_ml,
             out.data_ptr(), out.shape[1], B, n_heads, n_kv_heads, head_dim, scale, window, n_splits, int(early),
             kv.planes, sink, keep_first, v_group, _ptr(head_sink), gate_col, _ptr(slopes), self._stream()), "attention_decode")
         if n_splits > 1:
