@@ -94,7 +94,8 @@ __device__ __forceinline__ void f32_finish(float* o, float v, const float* bias,
   *o = mode == LIN_ACCUM ? *o + v : v;
 }
 
-// At most 8 rows (a decode step): bound by the weights' bytes.  A block takes 8 output features, a warp one range of k of
+// At most 8 rows (a decode step): the weights' bytes are the floor; at a third to a half of the bandwidth it stands between its loads'
+// latency and shared memory.  A block takes 8 output features, a warp one range of k of
 // them: its pieces of the 8 weight rows travel through shared memory by cp.async, 256-byte runs of a row at a time, up
 // to FEW_STAGES pieces in flight, the first ones before the kernel ahead has finished where the caller says that it does not write them (`early`).  Lane =
 // (feature, row mod 4): a lane walks its feature's range in order for one or two rows of A.  8 features a block and not more:
@@ -198,7 +199,7 @@ k_linear_f32_few(const float* __restrict__ A, const float* __restrict__ W, const
   }
 }
 
-// More rows: bound by the FP32 pipe.  Tiles of BM x 128 outputs, 256 threads with BM / 16 x 8 outputs each.  The next 16 k travel
+// More rows: bound by shared memory (64-row tiles, 398 rows of 9,728 x 896: 89 % of its rate, issue slots 69 %).  Tiles of BM x 128 outputs, 256 threads with BM / 16 x 8 outputs each.  The next 16 k travel
 // through registers while the current ones are multiplied.  (Products two at a time, fma.rn.f32x2, want every value of A twice in
 // shared memory and were no faster.)  SPLIT: a cluster of 8 blocks shares a tile, a range of k each, and adds the ranges' sums in
 // order through distributed shared memory (see launch_f32 for when).  Measured inside a prompt step of the 0.5B shape, 201 + 197

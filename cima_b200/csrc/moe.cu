@@ -507,10 +507,11 @@ k_moe_gather_rows(const uint4* __restrict__ src, const int* __restrict__ pos, ui
   for (int v = threadIdx.x; v < vecs; v += blockDim.x) d[v] = s[v];
 }
 
-// Up to 1,023 pairs: bound by the touched experts' weights.  Block (x = tile of 32 pairs of one expert as moe_sort laid them out, y = 16
-// output features); the sum over k is shared by its 8 warps, a range each, so that a down product (few features, a long sum) has work
-// for every SM in more than one wave.  Lane (g, t) loads 16 neighbouring bytes of weight rows g and g + 8 and of its pairs' rows, 8 t
-// values into each 32 ("a piece"); several pieces are requested before the first is used.  MODE as in k_moe_gemm.
+// Up to 1,023 pairs: the touched experts' weights are the floor; at half the bandwidth the warps wait for them, two to four blocks on an
+// SM.  Block (x = tile of 32 pairs of one expert as moe_sort laid them out, y = 16 output features); the sum over k is shared by its
+// 8 warps, a range each, so that a down product (few features, a long sum) has work for every SM in more than one wave.  Lane (g, t)
+// loads 16 neighbouring bytes of weight rows g and g + 8 and of its pairs' rows, 8 t values into each 32 ("a piece"), ahead of their use.
+// MODE as in k_moe_gemm.
 // (A warp a feature stood at 4.2 TB/s in the down product of 16 experts of 1,536 x 4,480 and 8 rows, 52.8 us: its 1,536 blocks are 1.3
 // waves, and each began with a chain of dependent look-ups of its expert.)
 constexpr int FEW_MOST = 128;           // pairs up to which the sums are multiply-adds (k_moe_few); beyond, k_moe_some
@@ -578,7 +579,7 @@ __device__ __forceinline__ void few_store(const FewTile& s, void* __restrict__ o
 // once.  The next piece is requested before the one at hand is used.  Sort, both products and sum aside, us, a warp a feature / this / mma.sync:
 // 16 gated experts of 1,536 x 2,240, 16 pairs: 47 / 37 / 31 and down 23 / 20 / 19, 64 pairs: 93 / 81 / 40 and 52 / 49 / 28; 16 ungated ones of
 // 1,536 x 4,480, 24 pairs: 56 / 44 / 37 and 55 / 47 / 35.  NP 1 is the better one for gate and up where most experts have one pair
-// (8 pairs of 16 experts: 22 us, NP 2 25), NP 2 elsewhere (32: 51, NP 1 55); NP 4 costs a decode step its blocks (106 registers).
+// (8 pairs of 16 experts: 22 us, NP 2 25), NP 2 elsewhere (32: 51, NP 1 55); NP 4 is slower everywhere (98 registers).
 template <int MODE, int NP>
 __global__ void __launch_bounds__(32 * FEW_WARPS)
 k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
@@ -677,7 +678,7 @@ k_moe_few(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __r
   }
 }
 
-// More pairs: bound by the weights still.  The weights are the 16-row operand of mma.m16n8k16, NB times 8 pairs its columns (4, a whole tile of 32 pairs, where an
+// More pairs: the weights are the 16-row operand of mma.m16n8k16, NB times 8 pairs its columns (4, a whole tile of 32 pairs, where an
 // expert has more than eight on average: 192 pairs of 16 gated experts of 1,536 x 2,240 in 109 us, 1,024 in 248).  The order of k inside
 // a product is free as long as both operands follow it: a lane uses its 16 bytes as its parts of two k-steps.  The warps' sums are
 // added in their order; a row's sums are the same for either NB.  (The plain tiles, which add all of k one by one, stand further from

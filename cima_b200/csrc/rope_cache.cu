@@ -264,8 +264,8 @@ k_norm_rope_append(TA* __restrict__ qkv, int ld, const float* __restrict__ inv_f
 // row, a lane four neighbouring values of a head in registers, a warp NORM_HEADS heads at a time with all their loads requested
 // before the first use.  The row's angles are made once (a block of four heads a row, as in the kernel above, made them sixteen
 // times at 32 + 32 heads); the value that one turns with stands rotary_dim / 8 lanes away.  Where few rows leave SMs idle, blocks
-// share a row's heads, a warp taking two or one of them (the angles made again; see the launch).  Bound by the rows' way through
-// memory, with few rows by a block's chain of loads.  (2,048 rows of the 3B Lipizen shape: 22 us, 30 before.)
+// share a row's heads, a warp taking two or one of them (the angles made again; see the launch).  Bound by its instructions (2,048 rows:
+// issue slots 68 %, DRAM 5 %), with few rows by a block's chain of loads.  (2,048 rows of the 3B Lipizen shape: 22 us, 30 before.)
 template <typename TA, bool ROT, int NORM_HEADS>
 __global__ void __launch_bounds__(128)
 k_norm_append(TA* __restrict__ qkv, int ld, const float* __restrict__ inv_freq, int rotary_dim, const int* __restrict__ row_pos,
