@@ -44,10 +44,9 @@ class DecodeGraph:
     does one step (the first run after construction executes eagerly and captures)."""
 
     def __init__(self, model, sampler, n_seqs: int, all_greedy: bool, max_len: int = 0):
-        """``max_len``: the most positions that a sequence may hold after a step of this graph (0: any number).  A
-        recorded step fixes its launches; one recorded for short contexts takes the kernels' choices for them
-        (the decode attention without splits), and the stepper moves to the unbounded graph when a sequence
-        outgrows the bound."""
+        """``max_len``: the most positions that a sequence may hold after a step of this graph (0: as many as the model
+        takes).  A recorded step fixes its launches; one recorded for short or middling contexts takes the kernels' choices
+        for them, and the stepper moves on to the next graph when a sequence outgrows the bound."""
         self.model, self.sampler = model, sampler
         self.B = B = n_seqs
         self.all_greedy = all_greedy
@@ -55,7 +54,7 @@ class DecodeGraph:
         dev = model.rt.device
         self.meta = torch.zeros(6 * B + 1, dtype=torch.int32, device=dev)
         self.meta_host = torch.zeros(6 * B + 1, dtype=torch.int32).pin_memory()
-        self.batch = b = one_token_batch(self.meta, B, max_len)
+        self.batch = b = one_token_batch(self.meta, B, max_len or model.spec.max_position)
         self.tokens, self.row_pos, self.row_seq = b.tokens, b.row_pos, b.row_seq
         self.seq_slot, self.seq_first_row, self.seq_len = b.seq_slot, b.seq_first_row, b.seq_len
         self.params = torch.zeros(B, 4, dtype=torch.float32, device=dev)
@@ -194,7 +193,7 @@ class StepGraph:
     def __init__(self, model, n_seqs: int, max_len: int):
         self.n_seqs = n_seqs
         self.meta = torch.zeros(6 * n_seqs + 1, dtype=torch.int32, device=model.rt.device)
-        self.batch = one_token_batch(self.meta, n_seqs, max_len)
+        self.batch = one_token_batch(self.meta, n_seqs, max_len or model.spec.max_position)
         self.graph = None
         self.logits = None
         self.uses = 0

@@ -75,6 +75,7 @@ class Model:
         self.config = None                                  # set by load_model
         self.step_rows = STEP_ROWS                          # a step of more rows runs in parts
         self.record_steps = False                           # record one-token steps (``StepGraph``); an ``LM`` with graphs says so
+        self._context_bounds: Dict[int, List[int]] = {}     # sequences -> bounds of their context classes
         self._step_graphs = OrderedDict()                   # (sequences, context bound) -> StepGraph, the newest last
         self._step_pool = None                              # (memory pool, stream) that the recordings share
         self._steps = 0                                     # one-token steps so far
@@ -166,6 +167,17 @@ class Model:
         named = [int(getattr(b.mixer, "short_context", 0) or 0) for b in self.blocks if hasattr(b, "mixer")]
         named = [n for n in named if n > 0]
         return min(named) if named else 0
+
+    def context_bound(self, n_seqs: int, longest: int) -> int:
+        """The context class of a one-token step of ``n_seqs`` sequences, the longest of ``longest`` positions after it: the smallest
+        bound that holds it among ``short_context`` and the reach of the kernels for middling contexts (``mixer.near_context``),
+        0 for any number of positions."""
+        bounds = self._context_bounds.get(n_seqs)
+        if bounds is None:                                  # (asked for at every step)
+            named = [b.mixer.near_context(n_seqs) for b in self.blocks if hasattr(getattr(b, "mixer", None), "near_context")]
+            near = min([n for n in named if n > 0], default=0)
+            bounds = self._context_bounds[n_seqs] = [self.short_context] + ([near] if near < self.spec.max_position else [])
+        return next((n for n in bounds if longest <= n), 0)
 
     @property
     def graph_safe(self) -> bool:
@@ -278,8 +290,8 @@ class Model:
         """The ``StepGraph`` of this shape, or None where as many others as are kept have been in use of late: a caller that goes
         round among more shapes replays some and issues the rest, rather than recording each anew."""
         from . import graph
-        short, graphs = self.short_context, self._step_graphs
-        key = (n_seqs, short if max_len <= short else 0)
+        graphs = self._step_graphs
+        key = (n_seqs, self.context_bound(n_seqs, max_len))
         self._steps += 1
         g = graphs.get(key)
         if g is None:

@@ -40,7 +40,6 @@ class ModelStepper:
         self.use_graphs = (use_graphs and torch.device(model.rt.device).type == "cuda"
                            and getattr(model, "graph_safe", False))
         self._graphs = {}
-        self.short_context = int(getattr(model, "short_context", 0) or 0)
         self._prompt_graphs = OrderedDict()      # (sequences, rows of the bucket) -> PromptGraph, the newest last
         from .graph import recorded_prompt_rows
         self.prompt_rows = (recorded_prompt_rows(model.weight_bytes(), len(model.spec.schedule), (4 if model.rt.dtype is torch.float32 else 2))
@@ -257,12 +256,10 @@ class ModelStepper:
         self._inflight.clear()
 
     def _context_bound(self, slots, ahead: int) -> int:
-        """The bound of the graph that may run the next ``ahead`` steps of these sequences: the short-context bound
-        while every sequence stays within it, else 0 (no bound)."""
+        """The bound of the graph that may run the next ``ahead`` steps of these sequences: the smallest that every sequence
+        stays within (``Model.context_bound``), 0 for none."""
         cache = self.model.cache
-        short = self.short_context
-        longest = max(cache.length(s) + self._inflight.get(s, 0) for s in slots) + ahead
-        return short if longest <= short else 0
+        return self.model.context_bound(len(slots), max(cache.length(s) + self._inflight.get(s, 0) for s in slots) + ahead)
 
     def _decode_pipelined(self, slots, last_tokens, options) -> List[int]:
         fl = self._flight

@@ -15,7 +15,7 @@ import torch
 from .csrc.build import BuildError, library_path
 
 F32, BF16 = 0, 1
-ABI_VERSION = 37
+ABI_VERSION = 38
 SPLIT_BLOCKS = 296          # blocks of the decode attention that one wave holds (two per SM, 148 SMs)
 TC_ATTENTION_MIN_LEN = 256  # prompts from this length on take the tcgen05 attention (head_dim 64 or 128)
 SPLIT_FEW_BLOCKS = 148      # below this many blocks at 8 splits, more splits are taken
@@ -30,6 +30,31 @@ SHORT_CONTEXT_BYTES = 96 * 1024   # up to this many bytes of keys and values (on
 def short_context(head_dim: int) -> int:
     """Positions (whole pages of 64) up to which the decode attention of this head size runs without splits."""
     return SHORT_CONTEXT_BYTES // (4 * head_dim) // 64 * 64
+
+
+NEAR_KEYS = 832             # positions a block of a cluster, up to which the cluster kernel beats the splits where it leaves SMs idle
+NEAR_FULL = 96              # blocks from which on it does so at every length
+
+
+def near_cluster(pairs: int, head_dim: int) -> int:
+    """Blocks of the cluster that shares one of ``pairs`` (sequence, kv head) pairs: as many as one wave holds (an SM holds one block at
+    head_dim 128, two at 64), in the clusters that the GPU's groups of SMs can place: at head_dim 128 one of 16 a group (measured: 4
+    pairs in clusters of 16 against 8: 7B, 2,000 positions 2,658 against 2,676 us a step; 8 pairs 2,939 against 2,759), 14 of 8
+    (16 pairs, 1.5B, 1,000 positions: clusters of 8 1,218 us, of 4 1,100), 37 of 4, 74 of 2."""
+    for cluster, most in ((16, 4), (8, 14), (4, 37), (2, 74)):
+        if pairs <= most * (2 if head_dim == 64 else 1):
+            return cluster
+    return 1
+
+
+def near_context(pairs: int, head_dim: int) -> int:
+    """Positions up to which the cluster kernel takes ``pairs`` (sequence, kv head) pairs; 0: any number.  Where its blocks fill
+    the GPU it is the faster one throughout (us a layer against the splits and their merge: 7B, 8 sequences, 2,048 to 24,000
+    positions -6.5 to -7.1; 32 sequences, 270 to 4,000 -5 to -6; 64, 2,000 -1.2; 1.5B, 64 sequences, 3,000 -4.6).  Where it leaves
+    SMs idle the splits read more at a time: at 4,000 / 7,000 / 16,000 positions of one sequence in a cluster of 8 -2.5 / +0.3 / +8.3
+    (1.5B, 2 pairs), in one of 16 -3.5 / -2.1 (8,000) / +0.4, at 3,000 / 6,000 in 16 clusters of 4 -2.3 / +1.0."""
+    cluster = near_cluster(pairs, head_dim)
+    return 0 if pairs * cluster >= NEAR_FULL * (2 if head_dim == 64 else 1) else NEAR_KEYS * cluster
 
 
 EXTEND_BLOCKS = 444         # blocks of the attention of going-on rows that one wave holds (three per SM, 148 SMs)
@@ -88,6 +113,7 @@ _SIGNATURES = {
     "cima_attention_plain": [_vp, _i, _i, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i,
                              _f, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _i, _i, _vp],
     "cima_attention_decode": [_vp, _i, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _vp],
+    "cima_attention_decode_near": [_vp, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _vp],
     "cima_attention_prefill": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _vp, _i, _vp, _vp],
     "cima_attention_extend": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _f, _i, _i, _vp, _i, _vp,
                               _i, _vp, _vp, _vp],
@@ -574,6 +600,11 @@ class Kernels:
         off the scaled score of the query at position i with the key at j."""
         if (from_cache and qkv.dtype is torch.bfloat16 and kv.page_size == 64 and head_dim % 16 == 0
                 and head_dim <= 128 and batch.n_rows == batch.n_seqs):
+            plain = not (sink or keep_first or v_group > 1 or head_sink is not None or gate_col or slopes is not None)
+            near = self._near(qkv, kv, batch, n_heads, n_kv_heads, head_dim, window) if plain else 0
+            if near:
+                return self.attention_decode_near(qkv, kv, batch.seq_slot, batch.seq_len, out, n_heads, n_kv_heads, head_dim, scale, window, near,
+                                                  early=after_append)
             return self.attention_decode(qkv, kv, batch.seq_slot, batch.seq_len, out, n_heads, n_kv_heads, head_dim,
                                          scale, window, batch.max_len, early=after_append, sink=sink,
                                          keep_first=keep_first, v_group=v_group, head_sink=head_sink, gate_col=gate_col, slopes=slopes)
@@ -725,6 +756,35 @@ class Kernels:
             kv.planes, sink, keep_first, v_group, _ptr(head_sink), gate_col, _ptr(slopes), self._stream()), "attention_decode")
         if n_splits > 1:
             self.launches += 1
+
+    def _near(self, qkv: torch.Tensor, kv, batch, n_heads: int, n_kv_heads: int, head_dim: int, window: int) -> int:
+        """Blocks of a cluster where a one-token step's plain attention is the cluster kernel's, else 0."""
+        if (kv.planes != 2 or head_dim not in (64, 128) or n_heads // n_kv_heads > 8 or qkv.shape[1] % 8 or qkv.data_ptr() % 16):
+            return 0
+        pairs, seen = batch.n_rows * n_kv_heads, int(getattr(batch, "max_len", 0) or 0)        # positions that a row reads at most (0: not known)
+        if window > 0:
+            seen = min(seen or window + 64, window + 64)
+        if 0 < seen <= short_context(head_dim):           # one block a pair reads them in less time than a cluster needs to meet
+            return 1
+        bound = near_context(pairs, head_dim)
+        return near_cluster(pairs, head_dim) if bound == 0 or 0 < seen <= bound else 0
+
+    def attention_decode_near(self, qkv: torch.Tensor, kv, seq_slot, seq_len, out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int,
+                              scale: float, window: int, cluster: int, early: bool = False) -> None:
+        """``attention_decode`` by a cluster of ``cluster`` blocks a (sequence, kv head) (head sizes 64 and 128, at most 8 query heads a
+        kv head, keys | values, no sinks, kept first positions, gates or slopes): one launch, no scratch."""
+        self._need(qkv, "qkv", torch.bfloat16, 2); self._need(out, "out", torch.bfloat16, 2)
+        self._need(kv.storage, "cache", torch.bfloat16, 5); self._need(kv.block_table, "block_table", torch.int32, 2)
+        B = qkv.shape[0]
+        if tuple(out.shape) != (B, n_heads * head_dim) or seq_slot.numel() < B or seq_len.numel() < B:
+            raise KernelError(f"attention_decode_near: out {tuple(out.shape)} / sequences do not fit {B} rows")
+        if tuple(kv.storage.shape[1:]) != (2, n_kv_heads, 64, head_dim):
+            raise KernelError(f"attention_decode_near: cache pages are {tuple(kv.storage.shape)}")
+        if not self._admit(f"attention_decode[cluster of {cluster}]", *self._attention_work(qkv, n_heads, n_kv_heads, head_dim, kv.planes)): return
+        self._check(self.lib.cima_attention_decode_near(
+            qkv.data_ptr(), qkv.shape[1], kv.storage.data_ptr(), kv.block_table.data_ptr(), kv.block_table.shape[1], kv.ring_pages,
+            seq_slot.data_ptr(), seq_len.data_ptr(), out.data_ptr(), out.shape[1], B, n_heads, n_kv_heads, head_dim, scale, window, cluster,
+            int(early), self._stream()), "attention_decode_near")
 
     # ------------------------------------------------------------------ short convolution, depth average, latents
     def short_conv(self, h: torch.Tensor, w: torch.Tensor, state: Optional[torch.Tensor], batch, out: torch.Tensor,

@@ -214,6 +214,15 @@ class Attention:
         from ..kernels import short_context
         return short_context(self.hd)
 
+    def near_context(self, n_seqs: int) -> int:
+        """The same for the decode kernel of middling contexts, whose reach follows from the number of sequences (0: no bound)."""
+        from ..kernels import near_context
+        if (self.rt.full_precision or self.hd not in (64, 128) or self.spec.n_heads // self.spec.n_kv_heads > 8 or self.sink or self.keep_first
+                or self.has_sink or self.gated or self.slopes_host is not None):
+            return 0
+        bound = near_context(n_seqs * self.spec.n_kv_heads, self.hd)
+        return 0 if self.spec.window and self.spec.window + 64 <= bound else bound
+
     # ------------------------------------------------------------------ cache
     def cache_requests(self, site: int) -> List[object]:
         if self.spec.cache_from is not None:

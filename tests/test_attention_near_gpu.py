@@ -1,0 +1,84 @@
+"""The decode attention whose blocks are clusters that merge their own results: every cluster size at the edges of its pieces (16 keys a
+warp, 128 a block, pages of 64), windows and rings against float64; and which step takes it."""
+import math
+
+import pytest
+import torch
+
+from cima_b200.cache.kv import LayerKV
+from cima_b200.kernels import Kernels, near_cluster, near_context
+
+TOL = 2e-2          # bfloat16 values of magnitude 1 to 4 and their weighted means, as in test_kernels_gpu.py
+LENS = [1, 2, 16, 17, 64, 65, 128, 129, 300, 1100]
+
+
+def test_the_rule_covers_every_number_of_pairs():
+    """At most one block an SM (two at head size 64) where a cluster has more than one, and no bound where they fill the GPU."""
+    for hd, room in ((64, 296), (128, 148)):
+        last = 16
+        for pairs in range(1, 600):
+            c = near_cluster(pairs, hd)
+            assert c in (1, 2, 4, 8, 16) and c <= last and (c == 1 or pairs * c <= room)
+            assert (near_context(pairs, hd) == 0) == (pairs * c >= (192 if hd == 64 else 96))
+            last = c
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nh,nkv,hd,window,more", [
+    (14, 2, 64, 0, ""), (28, 4, 128, 0, "early"), (6, 6, 128, 0, ""), (8, 1, 64, 0, "early"), (6, 2, 128, 40, "early"), (4, 4, 64, 129, "ring"),
+    (15, 3, 64, 64, "ring early")])
+def test_attention_near(nh, nkv, hd, window, more):
+    K, B, page, G = Kernels(verbose=False), len(LENS), 64, nh // nkv
+    gen = torch.Generator().manual_seed(nh + hd + window)
+    randn = lambda *s: torch.randn(*s, generator=gen)                                           # noqa: E731
+    ring = -(-window // page) + 1 if "ring" in more else 0
+    width = ring or -(-max(LENS) // page)
+    storage = torch.full((B * width + 3, 2, nkv, page, hd), float("nan"), dtype=torch.bfloat16)      # what no sequence holds must not be seen
+    table = torch.randperm(B * width + 3, generator=gen)[:B * width].view(B, width).int()
+    slots = torch.randperm(B, generator=gen).int()
+    qkv = randn(B, (nh + 2 * nkv) * hd).bfloat16()
+    want = torch.empty(B, nh * hd, dtype=torch.float64)
+    for b, n in enumerate(LENS):
+        k, v = randn(n, nkv, hd).bfloat16(), randn(n, nkv, hd).bfloat16()
+        lo = max(0, n - window) if window else 0
+        k[lo, 0] = qkv[b, :hd] * 3.0                               # the oldest visible key stands out for head 0, the one below it more
+        if lo:
+            k[lo - 1, 0] = qkv[b, :hd] * 9.0
+        for p in range(max(0, n - ring * page + page) if ring else 0, n):
+            e = (p // page) % ring if ring else p // page
+            at = table[slots[b], e]
+            storage[at, 0, :, p % page], storage[at, 1, :, p % page] = k[p], v[p]
+        for h in range(nh):
+            s = (k[lo:, h // G].double() @ qkv[b, h * hd:(h + 1) * hd].double()) * 0.3 / math.sqrt(hd)
+            want[b, h * hd:(h + 1) * hd] = torch.softmax(s, 0) @ v[lo:, h // G].double()
+    kv = LayerKV(storage.cuda(), table.cuda(), page, ring, window, 0)
+    args = (qkv.cuda(), kv, slots.cuda(), torch.tensor(LENS, dtype=torch.int32, device="cuda"))
+    for cluster in (1, 2, 4, 8, 16):
+        out = torch.full((B, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        K.attention_decode_near(*args, out, nh, nkv, hd, 0.3 / math.sqrt(hd), window, cluster, early="early" in more)
+        got = out.cpu().double()
+        assert ((got - want).abs() <= TOL * want.abs().clamp(min=1.0)).all(), (cluster, (got - want).abs().max().item())
+    one = torch.full((1, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")      # a sequence alone: the same bits
+    K.attention_decode_near(qkv[-1:].cuda(), kv, slots[-1:].cuda(), args[3][-1:], one, nh, nkv, hd, 0.3 / math.sqrt(hd), window, 16, early="early" in more)
+    assert torch.equal(one[0], out[-1])
+
+
+@pytest.mark.gpu
+def test_steps_cross_the_reach_of_the_clusters(monkeypatch):
+    """Decoding across the bound behind which the splits take over (lowered, so that a short walk crosses it): the same logits as
+    steps that are issued one by one, to the rounding of bfloat16."""
+    import cima_b200
+    from cima_b200 import kernels
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    monkeypatch.setattr(kernels, "NEAR_KEYS", 32)                   # 512 positions for a cluster of 16
+    kw = dict(config=dict(SHAPES["qwen2.5-0.5b"], num_hidden_layers=2, max_position_embeddings=4096), seed=3, draw="device", max_tokens=4096, max_seqs=2, verbose=False)
+    rec, ref = cima_b200.load(**kw), cima_b200.load(use_graphs=False, **kw)
+    prompt = torch.randint(0, rec.spec.vocab, (505,), generator=torch.Generator().manual_seed(1)).tolist()
+    outs = []
+    for lm in (rec, ref):
+        (slot,) = lm.model.cache.open(1)
+        lm.step([StepEntry(slot, prompt)])
+        outs.append(torch.cat([lm.step([StepEntry(slot, [t], [0])]) for t in range(100, 116)]))
+    assert {k[1] for k in rec.model._step_graphs} == {512, 0}
+    assert (outs[0] - outs[1]).abs().max() <= 2e-2 * outs[1].std()
