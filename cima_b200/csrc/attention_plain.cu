@@ -334,6 +334,120 @@ k_attention_f32(const __grid_constant__ AfArgs a) {
   }
 }
 
+// The same sums for steps of few rows (a decode step), head sizes 64 and 128, all keys visible below a row's position but for a window's.
+// A block owns ONE head of one row, a warp a piece, its keys and values straight to registers: a lane a key for the scores, a lane
+// HD / 32 neighbouring dims for the weighted sum.  What bounds such a step is the chain and not the bytes: the kernel above takes
+// 13 us for one or two rows at 200 positions, most of it the pieces' way through shared memory and the seven heads of a key
+// head one after the other; here each head has a block, and its keys are read from L2 as often as heads share them.  The order of
+// every sum is the other kernel's.  Measured, us a decode step of the 0.5B shape in 32 bits, the kernel above / this one: one row at
+// 10 / 1,000 / 8,000 positions 1,332 / 1,190, 2,151 / 1,601, 8,998 / 5,067, two at 205 1,428 / 1,260, 8 at 300 1,824 / 1,550, 20 at 1,500
+// 4,498 / 3,948.
+// (Volatile, so that a batch of loads stays in front of the sums it is asked for: left to the compiler, each waits for its own.)
+__device__ __forceinline__ float4 ld_f4(const float* p, bool ok) {
+  float4 v;
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %5, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\nmov.b32 %2, 0;\nmov.b32 %3, 0;\n@p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n}\n"
+               : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(p), "r"((int)ok));
+  return v;
+}
+__device__ __forceinline__ float2 ld_f2(const float* p, bool ok) {
+  float2 v;
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %3, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\n@p ld.global.v2.f32 {%0, %1}, [%2];\n}\n"
+               : "=&f"(v.x), "=&f"(v.y) : "l"(p), "r"((int)ok));
+  return v;
+}
+template <int HD>
+__global__ void __launch_bounds__(256)
+k_attention_f32_row(const __grid_constant__ AfArgs a) {
+  constexpr int NI = HD / 32, PARTS = HD / 64, BATCH = AF_KEYS / PARTS;      // K in pieces of 64 dims, V in batches of so many keys
+  __shared__ __align__(16) float q[HD];
+  __shared__ float part[8][HD], s_m[8], s_l[8];
+  __shared__ int s_any[8];
+  cima_pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = blockIdx.x, h = blockIdx.y, kvh = h / (a.nh / a.nkv);
+  const int pos = a.row_pos[row], slot = a.seq_slot[a.row_seq[row]];
+  const int lo = a.window > 0 && pos + 1 > a.window ? pos + 1 - a.window : 0, b0 = lo / AF_KEYS, pieces = pos / AF_KEYS - b0 + 1;
+  if (tid < HD) q[tid] = a.qkv[(size_t)row * a.ld + (size_t)h * HD + tid];
+  __syncthreads();
+  float m = -1e30f, l = 0.f, acc = 0.f;                  // of dim `tid`, over the pieces so far
+  for (int base = 0; base < pieces; base += 8) {
+    if (base + warp < pieces) {
+      const int j0 = (b0 + base + warp) * AF_KEYS, j = j0 + lane;
+      const bool see = j <= pos && j >= lo;
+      const unsigned vis = __ballot_sync(0xffffffffu, see);
+      const float* kp = a.cache + a.pg.offset(slot, j0, 0, kvh);      // (a piece lies in one page)
+      const float* vp = kp + a.pg.value_offset() + NI * lane;
+      kp += (size_t)lane * HD;
+      float s = 0.f;
+      float v[BATCH][NI];
+      auto values = [&](int from) {
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {
+          const bool ok = vis >> (from + k) & 1;         // (what no row sees is not read)
+          if constexpr (NI == 2) {
+            const float2 x = ld_f2(vp + (size_t)(from + k) * HD, ok);
+            v[k][0] = x.x; v[k][1] = x.y;
+          } else {
+            const float4 x = ld_f4(vp + (size_t)(from + k) * HD, ok);
+            v[k][0] = x.x; v[k][1] = x.y; v[k][2] = x.z; v[k][3] = x.w;
+          }
+        }
+      };
+#pragma unroll 1
+      for (int part0 = 0; part0 < HD; part0 += 64) {
+        float4 k4[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) k4[i] = ld_f4(kp + part0 + 4 * i, see);
+        if (part0 + 64 == HD) values(0);                 // on their way while the scores are made
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          const float4 q4 = *reinterpret_cast<const float4*>(q + part0 + 4 * i);
+          s = fmaf(q4.x, k4[i].x, s); s = fmaf(q4.y, k4[i].y, s);
+          s = fmaf(q4.z, k4[i].z, s); s = fmaf(q4.w, k4[i].w, s);
+        }
+      }
+      s *= a.scale;
+      float mp = see ? fmaxf(s, -1e30f) : -1e30f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mp = fmaxf(mp, __shfl_xor_sync(0xffffffffu, mp, o));
+      const float p = see ? expf(s - mp) : 0.f;
+      float lp = p;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) lp += __shfl_xor_sync(0xffffffffu, lp, o);
+      float o[NI];
+#pragma unroll
+      for (int i = 0; i < NI; i++) o[i] = 0.f;
+#pragma unroll
+      for (int from = 0; from < AF_KEYS; from += BATCH) {
+        if (from > 0) values(from);
+#pragma unroll
+        for (int k = 0; k < BATCH; k++) {
+          const float pk = __shfl_sync(0xffffffffu, p, from + k);
+          if (vis >> (from + k) & 1) {
+#pragma unroll
+            for (int i = 0; i < NI; i++) o[i] = fmaf(pk, v[k][i], o[i]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NI; i++) part[warp][NI * lane + i] = o[i];
+      if (lane == 0) { s_m[warp] = mp; s_l[warp] = lp; s_any[warp] = vis != 0u; }
+    }
+    __syncthreads();
+    if (tid < HD) {
+      const int there = min(8, pieces - base);
+      for (int w = 0; w < there; w++)
+        if (s_any[w]) {
+          const float m2 = fmaxf(m, s_m[w]), c = expf(m - m2), k = expf(s_m[w] - m2);
+          l = l * c + s_l[w] * k;
+          m = m2;
+          acc = fmaf(part[w][tid], k, acc * c);
+        }
+    }
+    __syncthreads();
+  }
+  if (tid < HD) a.out[(size_t)row * a.ldo + (size_t)h * HD + tid] = acc * (l > 0.f ? 1.0f / l : 0.f);
+}
+
 // max_keys: positions of the longest sequence after the step.  The bits do not depend on rows, teams or warps.
 template <int HDP, bool FROM_CACHE>
 static int launch_attention_f32(AfArgs a, bool vec, int n_seqs, int max_keys, cudaStream_t stream) {
@@ -387,6 +501,13 @@ extern "C" int cima_attention_plain(const void* qkv, int dtype, int ld, const vo
              ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, 1, 1, 1, scale, sink};
     const bool vec = hd % 4 == 0 && (from_cache || ld % 4 == 0) && ((from_cache ? (uintptr_t)cache : (uintptr_t)qkv) & 15) == 0;
     int rc;
+    // One head of one row a block as long as they are one wave of the GPU (two blocks an SM: 280 of them, 20 rows of 14 heads at 300
+    // positions, 3,464 -> 3,231 us a step); with more the heads that share keys share a block.
+    if (from_cache && (hd == 64 || hd == 128) && (long long)T * nh <= 296 && T <= n_seqs && page_size % AF_KEYS == 0 && planes == 2 && ((uintptr_t)cache & 15) == 0 &&
+        sink == 0.f && keep_first == 0 && v_group == 1 && !head_sink && gate_col == 0 && !slopes) {
+      rc = hd == 64 ? cima_launch(k_attention_f32_row<64>, dim3(T, nh), dim3(256), (size_t)0, stream, 1, a) : cima_launch(k_attention_f32_row<128>, dim3(T, nh), dim3(256), (size_t)0, stream, 1, a);
+      return rc ? rc : cima_launch_result();
+    }
     if (hd <= 64) rc = from_cache ? launch_attention_f32<64, true>(a, vec, n_seqs, max_keys, stream) : launch_attention_f32<64, false>(a, vec, n_seqs, max_keys, stream);
     else if (hd <= 128) rc = from_cache ? launch_attention_f32<128, true>(a, vec, n_seqs, max_keys, stream) : launch_attention_f32<128, false>(a, vec, n_seqs, max_keys, stream);
     else rc = from_cache ? launch_attention_f32<256, true>(a, vec, n_seqs, max_keys, stream) : launch_attention_f32<256, false>(a, vec, n_seqs, max_keys, stream);

@@ -1031,3 +1031,34 @@ def test_qkv_rope_skinny_equals_projection_then_rope_append(K, M, nh, nkv, hd, H
                norm=(ssq, 1e-6))
     assert err(qkv[:, :nh * hd], want2[:, :nh * hd]) <= TOL["bfloat16"] * 4
     assert err(gpu2.storage, cpu2.storage) <= TOL["bfloat16"] * 4
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window", [(14, 2, 64, 0), (15, 3, 64, 40), (16, 2, 128, 0), (28, 4, 128, 129)])
+def test_float32_attention_of_few_rows_has_the_bits_of_many(K, nh, nkv, hd, window):
+    """Decode rows in 32 bits, one head a block while they are few, and together with others, as many rows share a block's keys: the
+    same bits at the ends of a piece (32 positions), a page (64) and a block's round (256), and near float64."""
+    lens = [1, 2, 31, 32, 33, 63, 64, 65, 128, 255, 256, 257, 300, 513, 700]
+    lens += lens[:max(0, 296 // nh + 1 - len(lens))]
+    B = len(lens)
+    assert B * nh > 296
+    tables, n_pages, width = scattered_tables(lens, list(range(B)), 64, seed=hd + window)
+    cpu, gpu = make_kv(n_pages, nkv, 64, hd, B, width, 0, window, torch.float32, tables)
+    cpu.storage.fill_(float("nan"))                       # what no row sees is not read
+    for i, n in enumerate(lens):
+        fill_cache(cpu, gpu, i, g(n, nkv, hd, seed=50 + i), g(n, nkv, hd, seed=90 + i))
+    qkv, scale = g(B, (nh + 2 * nkv) * hd, seed=6), 1.0 / math.sqrt(hd)
+    seqs = [(i, n - 1, 1) for i, n in enumerate(lens)]
+
+    def run(which):
+        b = batch_of([seqs[i] for i in which], "cuda")
+        out = torch.full((len(which), nh * hd), 7.0, device="cuda")
+        K.attention_plain(qkv[which].cuda(), gpu, b.row_pos, b.row_seq, b.seq_slot, b.seq_first_row, out, nh, nkv, hd, scale, window, True)
+        return out
+
+    many = run(list(range(B)))
+    for i in range(B):
+        assert torch.equal(run([i])[0], many[i]), lens[i]
+    assert torch.equal(run([0, B - 1, 3]), many[[0, B - 1, 3]])
+    bc, want = batch_of(seqs, "cpu"), torch.zeros(B, nh * hd, dtype=torch.float64)
+    REF.attention_plain(qkv, cpu, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_first_row, want, nh, nkv, hd, scale, window, True)
+    assert err(many, want) <= TOL["float32"]
