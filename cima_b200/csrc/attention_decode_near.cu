@@ -73,15 +73,19 @@ k_attention_near(const __nv_bfloat16* __restrict__ qkv, int ld, const __nv_bfloa
     if (pg.ring) e %= pg.ring;
     return kbase + (size_t)pg.table[(size_t)slot * pg.width + e] * 2 * nkv * (PS * HD) + (c & 3) * 16 * HD;
   };
-  // Rows that are not loaded keep what the registers hold (0, or an earlier key): their weight is 0.
+  // Rows that are not loaded keep what the registers hold (0, or an earlier key's): a key's score is then masked.  A value's weight is 0, which
+  // an earlier key's infinity would turn into NaN, so a later round clears its values (`clear`).
   uint4 kf[HD / 32][2] = {}, vf[HD / 32][2] = {};
-  auto load = [&](uint4 (&r)[HD / 32][2], const __nv_bfloat16* src, int c, int from, int to) {
+  auto load = [&](uint4 (&r)[HD / 32][2], const __nv_bfloat16* src, int c, int from, int to, bool clear = false) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const int key = c * 16 + g + 8 * h;
       if (key >= from && key < to) {
 #pragma unroll
         for (int d = 0; d < HD / 32; d++) r[d][h] = ld_once16(src + (g + 8 * h) * HD + 32 * d);
+      } else if (clear) {
+#pragma unroll
+        for (int d = 0; d < HD / 32; d++) r[d][h] = make_uint4(0u, 0u, 0u, 0u);
       }
     }
   };
@@ -147,7 +151,7 @@ k_attention_near(const __nv_bfloat16* __restrict__ qkv, int ld, const __nv_bfloa
         mma(o[2 * d], transposed(vf[d][0].x), transposed(vf[d][0].y), transposed(vf[d][1].x), transposed(vf[d][1].y), b0, b1);
         mma(o[2 * d + 1], transposed(vf[d][0].z), transposed(vf[d][0].w), transposed(vf[d][1].z), transposed(vf[d][1].w), b0, b1);
       }
-      if (more) load(vf, src + v_off, c + WARPS, lo, len);
+      if (more) load(vf, src + v_off, c + WARPS, lo, len, true);
     }
   }
   cima_pdl_trigger();

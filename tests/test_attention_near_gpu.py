@@ -64,6 +64,22 @@ def test_attention_near(nh, nkv, hd, window, more):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("hd", [64, 128])
+def test_an_infinite_value_stays_in_its_column(hd):
+    """130 positions: a warp's second 16 keys end after two, and what it has read before of the other fourteen must not come back."""
+    K, n = Kernels(verbose=False), 130
+    storage = torch.zeros(3, 2, 1, 64, hd, dtype=torch.bfloat16)
+    storage[0, 1, 0, 5, 3] = float("inf")                          # weight 1 / 130
+    kv = LayerKV(storage.cuda(), torch.arange(3, dtype=torch.int32, device="cuda").view(1, 3), 64, 0, 0, 0)
+    out = torch.full((1, 2 * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+    slot, length = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((1,), n, dtype=torch.int32, device="cuda")
+    K.attention_decode_near(torch.ones(1, 4 * hd, dtype=torch.bfloat16, device="cuda"), kv, slot, length, out, 2, 1, hd, 1.0, 0, 1)
+    want = torch.zeros(2, hd, dtype=torch.bfloat16)
+    want[:, 3] = float("inf")
+    assert torch.equal(out.cpu().view(2, hd), want)
+
+
+@pytest.mark.gpu
 def test_steps_cross_the_reach_of_the_clusters(monkeypatch):
     """Decoding across the bound behind which the splits take over (lowered, so that a short walk crosses it): the same logits as
     steps that are issued one by one, to the rounding of bfloat16."""
