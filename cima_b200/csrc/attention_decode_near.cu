@@ -235,12 +235,14 @@ template <int HD>
 int launch_near(const void* qkv, int ld, const void* cache, CimaPaged pg, const int* seq_slot, const int* seq_len, void* out, int ldo, int B, int nh,
                 int nkv, float scale, int window, int cluster, int early, cudaStream_t stream) {
   if (cluster > 8) {                                  // more than every device has to offer: this one does
-    static bool allowed = false;
-    if (!allowed) {
-      const cudaError_t e = cudaFuncSetAttribute(k_attention_near<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return cima_fail((int)e, "attention_decode_near: a cluster of %d blocks: %s", cluster, cudaGetErrorString(e));
-      allowed = true;
+    static bool allowed[64] = {false};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && (dev < 0 || dev >= 64 || !allowed[dev])) {
+      e = cudaFuncSetAttribute(k_attention_near<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e == cudaSuccess && dev >= 0 && dev < 64) allowed[dev] = true;
     }
+    if (e != cudaSuccess) return cima_fail((int)e, "attention_decode_near: a cluster of %d blocks: %s", cluster, cudaGetErrorString(e));
   }
   const int rc = cima_launch(k_attention_near<HD>, dim3(cluster, nkv, B), dim3(WARPS * 32), 0, stream, cluster, (const __nv_bfloat16*)qkv, ld,
                              (const __nv_bfloat16*)cache, pg, seq_slot, seq_len, (__nv_bfloat16*)out, ldo, nh, nkv, scale, window, early);
