@@ -49,10 +49,13 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// early: as in attention_decode.cu (what the kernel launched just before this one may have written).
+// early: the kernel launched just before this one has written nothing that this one reads but qkv and, in the cache, the newest position
+// (seq_len[b] - 1) of each sequence: every other position is read before the wait on that kernel, its own page's included.
+// (attention_decode.cu asks for less: it leaves the newest position's whole page until after the wait.)  qkv is not __restrict__, since that
+// kernel may write it during this one's life: its reads must stay behind the wait.
 template <int HD>
 __global__ void __launch_bounds__(WARPS * 32)
-k_attention_near(const __nv_bfloat16* __restrict__ qkv, int ld, const __nv_bfloat16* cache, CimaPaged pg, const int* __restrict__ seq_slot,
+k_attention_near(const __nv_bfloat16* qkv, int ld, const __nv_bfloat16* cache, CimaPaged pg, const int* __restrict__ seq_slot,
                  const int* __restrict__ seq_len, __nv_bfloat16* __restrict__ out, int ldo, int nh, int nkv, float scale, int window, int early) {
   if (!early) cima_pdl_wait();
   __shared__ float so[WARPS][8][HD + 1];             // the warps' results; then [0]: the block's
@@ -253,7 +256,8 @@ int launch_near(const void* qkv, int ld, const void* cache, CimaPaged pg, const 
 
 // One query row a sequence (row b of qkv belongs to sequence b), pages of 64 with keys | values, head sizes 64 and 128, at most 8
 // query heads a kv head; any window (without kept first positions); `cluster` blocks (1, 2, 4, 8 or 16) share a sequence and kv
-// head.  The other arguments are cima_attention_decode's.
+// head.  early: see k_attention_near (more is asked of the kernel before than by cima_attention_decode).  The other arguments are
+// cima_attention_decode's.
 extern "C" int cima_attention_decode_near(const void* qkv, int ld, const void* cache, const int* table, int table_width, int ring, const int* seq_slot,
                                           const int* seq_len, void* out, int ldo, int B, int nh, int nkv, int hd, float scale, int window,
                                           int cluster, int early, cudaStream_t stream) {

@@ -772,7 +772,9 @@ class Kernels:
     def attention_decode_near(self, qkv: torch.Tensor, kv, seq_slot, seq_len, out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int,
                               scale: float, window: int, cluster: int, early: bool = False) -> None:
         """``attention_decode`` by a cluster of ``cluster`` blocks a (sequence, kv head) (head sizes 64 and 128, at most 8 query heads a
-        kv head, keys | values, no sinks, kept first positions, gates or slopes): one launch, no scratch."""
+        kv head, keys | values, no sinks, kept first positions, gates or slopes): one launch, no scratch.  ``early`` promises more than
+        there: the kernel launched just before this one wrote nothing that this one reads but ``qkv`` and each sequence's newest position
+        in the cache (no other position of its page)."""
         self._need(qkv, "qkv", torch.bfloat16, 2); self._need(out, "out", torch.bfloat16, 2)
         self._need(kv.storage, "cache", torch.bfloat16, 5); self._need(kv.block_table, "block_table", torch.int32, 2)
         B = qkv.shape[0]

@@ -98,3 +98,47 @@ def test_steps_cross_the_reach_of_the_clusters(monkeypatch):
         outs.append(torch.cat([lm.step([StepEntry(slot, [t], [0])]) for t in range(100, 116)]))
     assert {k[1] for k in rec.model._step_graphs} == {512, 0}
     assert (outs[0] - outs[1]).abs().max() <= 2e-2 * outs[1].std()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [3, 11])
+@pytest.mark.parametrize("nh,nkv,hd", [(14, 2, 64), (28, 4, 128)])
+def test_the_newest_position_is_read_behind_its_append(rows, nh, nkv, hd, monkeypatch):
+    """The kernel that rotates and appends (the skinny product's epilogue up to 8 rows, the rotation by itself above), then at once the
+    attention by every cluster: NaN stands in the cache at the newest position until the append, whose key is the row's own query
+    of head 0 and outweighs the others.  Against append and softmax in float64."""
+    from reference_kernels import ReferenceKernels
+    from test_kernels_gpu import batch_of, fill_cache, g, make_kv, scattered_tables
+    K, ref, H = Kernels(verbose=False), ReferenceKernels(compute=torch.float64), 256
+    lens = ([1, 450, 1300, 64, 65, 129, 128, 17, 900, 577, 2048])[:rows]
+    slots = list(range(rows, 0, -1))
+    tables, n_pages, width = scattered_tables(lens, slots, 64, seed=hd)
+    cpu, gpu = make_kv(n_pages, nkv, 64, hd, rows + 1, width, 0, 0, torch.bfloat16, tables)
+    for i, (slot, n) in enumerate(zip(slots, lens)):
+        fill_cache(cpu, gpu, slot, g(n, nkv, hd, dtype=torch.bfloat16, seed=10 + i), g(n, nkv, hd, dtype=torch.bfloat16, seed=40 + i))
+        at = cpu.block_table[slot, (n - 1) // 64]
+        cpu.storage[at, :, :, (n - 1) % 64] = float("nan")
+    a, w, b = g(rows, H, dtype=torch.bfloat16, seed=1), g((nh + 2 * nkv) * hd, H, dtype=torch.bfloat16, seed=2, scale=1.0 / math.sqrt(H)), torch.zeros((nh + 2 * nkv) * hd)
+    w[nh * hd:(nh + 1) * hd] = 2.0 * w[:hd]                        # kv head 0's newest key: twice query head 0
+    inv = torch.pow(torch.tensor(10000.0, dtype=torch.float64), -2.0 * torch.arange(hd // 2, dtype=torch.float64) / hd).float()
+    seqs = [(slot, n - 1, 1) for slot, n in zip(slots, lens)]
+    bc, bg = batch_of(seqs, "cpu"), batch_of(seqs, "cuda")
+    qkv, kept = (a.double() @ w.double().t()).bfloat16(), cpu.storage.clone()
+    q64, want = qkv.double(), torch.empty(rows, nh * hd, dtype=torch.float64)
+    ref.rope_append(q64, inv, hd, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_len, cpu, nh, nkv, hd)
+    ref.attention(q64, cpu, bc, want, nh, nkv, hd, 1.0 / math.sqrt(hd), 0, True)
+    for cluster in (1, 2, 4, 8, 16):
+        monkeypatch.setattr(Kernels, "_near", lambda *x, c=cluster: c)
+        gpu.storage.copy_(kept)
+        if rows <= 8:
+            row = torch.empty(rows, (nh + 2 * nkv) * hd, dtype=torch.bfloat16, device="cuda")
+            args = a.cuda(), w.cuda(), b.cuda(), row, inv.cuda(), bg.row_pos, bg.row_seq, bg.seq_slot, gpu, nh, nkv, hd
+        else:
+            row = qkv.cuda()
+            args = row, inv.cuda(), hd, bg.row_pos, bg.row_seq, bg.seq_slot, bg.seq_len, gpu, nh, nkv, hd
+        out = torch.full((rows, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        (K.qkv_rope if rows <= 8 else K.rope_append)(*args)
+        K.attention(row, gpu, bg, out, nh, nkv, hd, 1.0 / math.sqrt(hd), 0, True, after_append=True)
+        # queries and keys of magnitude 1 to 4 rounded once more than in the statement: scores of magnitude 10 to 4e-2, a weight to 4 %
+        got = out.cpu().double()
+        assert ((got - want).abs() <= 5e-2 * want.abs().clamp(min=1.0)).all(), (cluster, (got - want).abs().max().item())
