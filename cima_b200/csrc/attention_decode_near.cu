@@ -234,19 +234,42 @@ k_attention_near(const __nv_bfloat16* qkv, int ld, const __nv_bfloat16* cache, C
   if (CL > 1) cluster.sync();                         // a block's shared memory outlives the others' reads of it
 }
 
+// Clusters of more than 8 blocks are more than every device has to offer: this one may.
+template <int HD>
+cudaError_t allow_near(int cluster) {
+  if (cluster <= 8) return cudaSuccess;
+  static bool allowed[64] = {false};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && (dev < 0 || dev >= 64 || !allowed[dev])) {
+    e = cudaFuncSetAttribute(k_attention_near<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) allowed[dev] = true;
+  }
+  return e;
+}
+
+// Clusters of `cluster` blocks that the current device holds at once; 0 where it cannot place one, or cannot say.
+template <int HD>
+int near_room(int cluster) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(WARPS * 32);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (allow_near<HD>(cluster) == cudaSuccess && cudaOccupancyMaxActiveClusters(&n, k_attention_near<HD>, &cfg) == cudaSuccess) return n;
+  cudaGetLastError();                                 // (what is no launch's error must not become one)
+  return 0;
+}
+
 template <int HD>
 int launch_near(const void* qkv, int ld, const void* cache, CimaPaged pg, const int* seq_slot, const int* seq_len, void* out, int ldo, int B, int nh,
                 int nkv, float scale, int window, int cluster, int early, cudaStream_t stream) {
-  if (cluster > 8) {                                  // more than every device has to offer: this one does
-    static bool allowed[64] = {false};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess && (dev < 0 || dev >= 64 || !allowed[dev])) {
-      e = cudaFuncSetAttribute(k_attention_near<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e == cudaSuccess && dev >= 0 && dev < 64) allowed[dev] = true;
-    }
-    if (e != cudaSuccess) return cima_fail((int)e, "attention_decode_near: a cluster of %d blocks: %s", cluster, cudaGetErrorString(e));
-  }
+  if (const cudaError_t e = allow_near<HD>(cluster)) return cima_fail((int)e, "attention_decode_near: a cluster of %d blocks: %s", cluster, cudaGetErrorString(e));
   const int rc = cima_launch(k_attention_near<HD>, dim3(cluster, nkv, B), dim3(WARPS * 32), 0, stream, cluster, (const __nv_bfloat16*)qkv, ld,
                              (const __nv_bfloat16*)cache, pg, seq_slot, seq_len, (__nv_bfloat16*)out, ldo, nh, nkv, scale, window, early);
   return rc ? rc : cima_launch_result();
@@ -269,4 +292,12 @@ extern "C" int cima_attention_decode_near(const void* qkv, int ld, const void* c
   if (ld % 8 || ((uintptr_t)qkv & 15) || ((uintptr_t)cache & 15)) return cima_fail(CIMA_E_ARG, "attention_decode_near: qkv rows and the cache must be 16-byte aligned");
   const CimaPaged pg{table, table_width, ring, PS, nkv, hd, 2};
   return (hd == 64 ? launch_near<64> : launch_near<128>)(qkv, ld, cache, pg, seq_slot, seq_len, out, ldo, B, nh, nkv, scale, window, cluster, early, stream);
+}
+
+// room[0 .. 3]: clusters of 16, 8, 4 and 2 blocks that the current device holds at once (they follow from how its SMs are grouped, which
+// differs from one device to the next).
+extern "C" int cima_attention_decode_near_room(int hd, int* room) {
+  if (hd != 64 && hd != 128) return cima_fail(CIMA_E_SIZE, "attention_decode_near: head_dim %d; this kernel takes 64 and 128", hd);
+  for (int i = 0; i < 4; i++) room[i] = hd == 64 ? near_room<64>(16 >> i) : near_room<128>(16 >> i);
+  return 0;
 }

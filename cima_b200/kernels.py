@@ -15,7 +15,7 @@ import torch
 from .csrc.build import BuildError, library_path
 
 F32, BF16 = 0, 1
-ABI_VERSION = 38
+ABI_VERSION = 39
 SPLIT_BLOCKS = 296          # blocks of the decode attention that one wave holds (two per SM, 148 SMs)
 TC_ATTENTION_MIN_LEN = 256  # prompts from this length on take the tcgen05 attention (head_dim 64 or 128)
 SPLIT_FEW_BLOCKS = 148      # below this many blocks at 8 splits, more splits are taken
@@ -36,24 +36,27 @@ NEAR_KEYS = 832             # positions a block of a cluster, up to which the cl
 NEAR_FULL = 96              # blocks from which on it does so at every length
 
 
-def near_cluster(pairs: int, head_dim: int) -> int:
+def near_cluster(pairs: int, head_dim: int, room=None) -> int:
     """Blocks of the cluster that shares one of ``pairs`` (sequence, kv head) pairs: as many as one wave holds (an SM holds one block at
     head_dim 128, two at 64), in the clusters that the GPU's groups of SMs can place: at head_dim 128 one of 16 a group (measured: 4
     pairs in clusters of 16 against 8: 7B, 2,000 positions 2,658 against 2,676 us a step; 8 pairs 2,939 against 2,759), 14 of 8
-    (16 pairs, 1.5B, 1,000 positions: clusters of 8 1,218 us, of 4 1,100), 37 of 4, 74 of 2."""
-    for cluster, most in ((16, 4), (8, 14), (4, 37), (2, 74)):
-        if pairs <= most * (2 if head_dim == 64 else 1):
+    (16 pairs, 1.5B, 1,000 positions: clusters of 8 1,218 us, of 4 1,100), 37 of 4, 74 of 2.  ``room``: clusters of 16, 8, 4 and 2 blocks that
+    the device at hand holds at once (``Kernels.near_room``); one that holds fewer gets smaller clusters, and none of a size that it
+    cannot place."""
+    for i, (cluster, most) in enumerate(((16, 4), (8, 14), (4, 37), (2, 74))):
+        most *= 2 if head_dim == 64 else 1
+        if pairs <= (most if room is None else min(most, room[i])):
             return cluster
     return 1
 
 
-def near_context(pairs: int, head_dim: int) -> int:
+def near_context(pairs: int, head_dim: int, room=None) -> int:
     """Positions up to which the cluster kernel takes ``pairs`` (sequence, kv head) pairs; 0: any number.  Where its blocks fill
     the GPU it is the faster one throughout (us a layer against the splits and their merge: 7B, 8 sequences, 2,048 to 24,000
     positions -6.5 to -7.1; 32 sequences, 270 to 4,000 -5 to -6; 64, 2,000 -1.2; 1.5B, 64 sequences, 3,000 -4.6).  Where it leaves
     SMs idle the splits read more at a time: at 4,000 / 7,000 / 16,000 positions of one sequence in a cluster of 8 -2.5 / +0.3 / +8.3
     (1.5B, 2 pairs), in one of 16 -3.5 / -2.1 (8,000) / +0.4, at 3,000 / 6,000 in 16 clusters of 4 -2.3 / +1.0."""
-    cluster = near_cluster(pairs, head_dim)
+    cluster = near_cluster(pairs, head_dim, room)
     return 0 if pairs * cluster >= NEAR_FULL * (2 if head_dim == 64 else 1) else NEAR_KEYS * cluster
 
 
@@ -114,6 +117,7 @@ _SIGNATURES = {
                              _f, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _i, _i, _vp],
     "cima_attention_decode": [_vp, _i, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _i, _f, _i, _i, _vp, _i, _vp, _vp],
     "cima_attention_decode_near": [_vp, _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _i, _i, _vp],
+    "cima_attention_decode_near_room": [_i, _vp],
     "cima_attention_prefill": [_vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i, _i, _vp, _i, _vp, _vp],
     "cima_attention_extend": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _f, _i, _i, _vp, _i, _vp,
                               _i, _vp, _vp, _vp],
@@ -201,6 +205,7 @@ class Kernels:
         self.launches = 0
         self.library_launches = 0   # matrix products handed to the library (not counted in ``launches``)
         self._error_flag = None
+        self._near_room = {}        # (device, head size) -> clusters that it holds
         self.profile = None         # a StepProfile while a step's launches are being counted and timed
 
     # ------------------------------------------------------------------ plumbing
@@ -766,8 +771,21 @@ class Kernels:
             seen = min(seen or window + 64, window + 64)
         if 0 < seen <= short_context(head_dim):           # one block a pair reads them in less time than a cluster needs to meet
             return 1
-        bound = near_context(pairs, head_dim)
-        return near_cluster(pairs, head_dim) if bound == 0 or 0 < seen <= bound else 0
+        room = self.near_room(head_dim)
+        bound = near_context(pairs, head_dim, room)
+        return near_cluster(pairs, head_dim, room) if bound == 0 or 0 < seen <= bound else 0
+
+    def near_room(self, head_dim: int):
+        """Clusters of 16, 8, 4 and 2 blocks of ``attention_decode_near`` that the current device holds at once."""
+        key = (torch.cuda.current_device(), head_dim)
+        room = self._near_room.get(key)
+        if room is None:
+            found = (ctypes.c_int * 4)()
+            code = self.lib.cima_attention_decode_near_room(head_dim, found)
+            if code != 0:
+                raise KernelError(f"attention_decode_near_room: {self.lib.cima_last_error().decode()} (code {code})")
+            room = self._near_room[key] = tuple(found)
+        return room
 
     def attention_decode_near(self, qkv: torch.Tensor, kv, seq_slot, seq_len, out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int,
                               scale: float, window: int, cluster: int, early: bool = False) -> None:

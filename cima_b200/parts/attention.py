@@ -220,7 +220,8 @@ class Attention:
         if (self.rt.full_precision or self.hd not in (64, 128) or self.spec.n_heads // self.spec.n_kv_heads > 8 or self.sink or self.keep_first
                 or self.has_sink or self.gated or self.slopes_host is not None):
             return 0
-        bound = near_context(n_seqs * self.spec.n_kv_heads, self.hd)
+        room = getattr(self.rt.kernels, "near_room", None)               # (a stand-in on the CPU has none)
+        bound = near_context(n_seqs * self.spec.n_kv_heads, self.hd, room and room(self.hd))
         return 0 if self.spec.window and self.spec.window + 64 <= bound else bound
 
     # ------------------------------------------------------------------ cache

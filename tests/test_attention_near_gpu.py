@@ -23,6 +23,15 @@ def test_the_rule_covers_every_number_of_pairs():
             last = c
 
 
+def test_the_clusters_are_those_that_the_device_holds():
+    """A device whose groups of SMs hold fewer clusters, or none of a size: never more blocks to wait for one another than it can place."""
+    for hd in (64, 128):
+        for room in ((0, 0, 0, 0), (0, 14, 33, 72), (2, 6, 12, 30), (0, 0, 35, 74), (100, 100, 100, 200)):
+            for pairs in range(1, 200):
+                c = near_cluster(pairs, hd, room)
+                assert c == 1 or pairs <= room[{16: 0, 8: 1, 4: 2, 2: 3}[c]]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("nh,nkv,hd,window,more", [
     (14, 2, 64, 0, ""), (28, 4, 128, 0, "early"), (6, 6, 128, 0, ""), (8, 1, 64, 0, "early"), (6, 2, 128, 40, "early"), (4, 4, 64, 129, "ring"),
@@ -77,6 +86,23 @@ def test_an_infinite_value_stays_in_its_column(hd):
     want = torch.zeros(2, hd, dtype=torch.bfloat16)
     want[:, 3] = float("inf")
     assert torch.equal(out.cpu().view(2, hd), want)
+
+
+@pytest.mark.gpu
+def test_clusters_stay_within_what_the_device_holds(monkeypatch):
+    """The device is asked once, and a step takes no cluster that it cannot place: with room for none of 16 (as where no group has 16 free
+    SMs) the step runs in smaller ones."""
+    from types import SimpleNamespace
+    K = Kernels(verbose=False)
+    for hd in (64, 128):
+        room = K.near_room(hd)
+        assert len(room) == 4 and room[3] > 0 and all(a <= b for a, b in zip(room, room[1:])), room
+        assert K.near_room(hd) is room
+        qkv, kv = torch.zeros(1, 4 * hd, dtype=torch.bfloat16, device="cuda"), SimpleNamespace(planes=2)
+        batch = SimpleNamespace(n_rows=1, n_seqs=1, max_len=1000)
+        assert K._near(qkv, kv, batch, 2, 1, hd, 0) == near_cluster(1, hd, room)
+        K._near_room[(torch.cuda.current_device(), hd)] = (0,) + room[1:]
+        assert K._near(qkv, kv, batch, 2, 1, hd, 0) == 8
 
 
 @pytest.mark.gpu
