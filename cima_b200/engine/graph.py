@@ -43,18 +43,20 @@ class DecodeGraph:
     """One batch size's captured step.  ``load`` sets its inputs for a set of sequences; ``run``
     does one step (the first run after construction executes eagerly and captures)."""
 
-    def __init__(self, model, sampler, n_seqs: int, all_greedy: bool, max_len: int = 0):
+    def __init__(self, model, sampler, n_seqs: int, all_greedy: bool, max_len: int = 0, pool=None):
         """``max_len``: the most positions that a sequence may hold after a step of this graph (0: as many as the model
         takes).  A recorded step fixes its launches; one recorded for short or middling contexts takes the kernels' choices
-        for them, and the stepper moves on to the next graph when a sequence outgrows the bound."""
+        for them, and the stepper moves on to the next graph when a sequence outgrows the bound.  ``pool``: the memory that its
+        recording shares with others (of the same caller: they run one after another, and nothing in it outlives a step)."""
         self.model, self.sampler = model, sampler
         self.B = B = n_seqs
         self.all_greedy = all_greedy
         self.max_len = max_len
+        self.pool = pool
         dev = model.rt.device
         self.meta = torch.zeros(6 * B + 1, dtype=torch.int32, device=dev)
         self.meta_host = torch.zeros(6 * B + 1, dtype=torch.int32).pin_memory()
-        self.batch = b = one_token_batch(self.meta, B, max_len or model.spec.max_position)
+        self.batch = b = one_token_batch(self.meta, B, max_len or model.most_positions)
         self.tokens, self.row_pos, self.row_seq = b.tokens, b.row_pos, b.row_seq
         self.seq_slot, self.seq_first_row, self.seq_len = b.seq_slot, b.seq_first_row, b.seq_len
         self.params = torch.zeros(B, 4, dtype=torch.float32, device=dev)
@@ -90,7 +92,7 @@ class DecodeGraph:
             g = torch.cuda.CUDAGraph()
             k = self.model.rt.kernels
             before = k.launches
-            with torch.cuda.graph(g):               # records the same step for the following ones; runs nothing
+            with torch.cuda.graph(g, pool=self.pool):      # records the same step for the following ones; runs nothing
                 self._step()
             self.launches_per_step = k.launches - before
             self.graph = g
@@ -193,7 +195,7 @@ class StepGraph:
     def __init__(self, model, n_seqs: int, max_len: int):
         self.n_seqs = n_seqs
         self.meta = torch.zeros(6 * n_seqs + 1, dtype=torch.int32, device=model.rt.device)
-        self.batch = one_token_batch(self.meta, n_seqs, max_len or model.spec.max_position)
+        self.batch = one_token_batch(self.meta, n_seqs, max_len or model.most_positions)
         self.graph = None
         self.logits = None
         self.uses = 0

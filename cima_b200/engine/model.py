@@ -168,6 +168,11 @@ class Model:
         named = [n for n in named if n > 0]
         return min(named) if named else 0
 
+    @property
+    def most_positions(self) -> int:
+        """The most positions that a sequence can come to hold: what the model takes and the cache has room for."""
+        return self.spec.max_position if self.cache is None else min(self.spec.max_position, self.cache.max_tokens)
+
     def context_bound(self, n_seqs: int, longest: int) -> int:
         """The context class of a one-token step of ``n_seqs`` sequences, the longest of ``longest`` positions after it: the smallest
         bound that holds it among ``short_context`` and the reach of the kernels for middling contexts (``mixer.near_context``),
@@ -176,7 +181,8 @@ class Model:
         if bounds is None:                                  # (asked for at every step)
             named = [b.mixer.near_context(n_seqs) for b in self.blocks if hasattr(getattr(b, "mixer", None), "near_context")]
             near = min([n for n in named if n > 0], default=0)
-            bounds = self._context_bounds[n_seqs] = [self.short_context] + ([near] if near < self.spec.max_position else [])
+            # (each class has recordings of its own: one that no sequence can leave is not told apart from that of any length)
+            bounds = self._context_bounds[n_seqs] = [self.short_context] + ([near] if near < self.most_positions else [])
         return next((n for n in bounds if longest <= n), 0)
 
     @property
@@ -207,6 +213,7 @@ class Model:
         shares = {site: self.spec.layers[layer].mixer.cache_from for site, layer in enumerate(sched)
                   if self.spec.layers[layer].mixer.cache_from is not None}
         self._forget_step_graphs()                          # recorded with the cache before
+        self._context_bounds.clear()
         self.cache = KVCache(self._cache_requests(),
                              max_tokens, self.spec.max_position,
                              self.rt.dtype, self.rt.device, page_size=page_size, max_seqs=max_seqs,
@@ -288,18 +295,29 @@ class Model:
 
     def _step_graph(self, n_seqs: int, max_len: int):
         """The ``StepGraph`` of this shape, or None where as many others as are kept have been in use of late: a caller that goes
-        round among more shapes replays some and issues the rest, rather than recording each anew."""
+        round among more shapes replays some and issues the rest, rather than recording each anew.  A batch size takes no more than its
+        share then: one recorded for longer contexts serves the shorter ones too, and takes their recording's place."""
         from . import graph
         graphs = self._step_graphs
         key = (n_seqs, self.context_bound(n_seqs, max_len))
         self._steps += 1
         g = graphs.get(key)
         if g is None:
-            if len(graphs) >= graph.MAX_STEP_GRAPHS:
-                if self._steps - next(iter(graphs.values())).last <= graph.STEP_GRAPH_IDLE:
+            if len(graphs) >= graph.MAX_STEP_GRAPHS and self._steps - next(iter(graphs.values())).last <= graph.STEP_GRAPH_IDLE:
+                reach = lambda k: k[1] or self.most_positions                                       # noqa: E731
+                held = sorted((k for k in graphs if k[0] == n_seqs), key=reach)
+                if not held:
                     return None
-                torch.cuda.synchronize()                    # the one that goes may still be running
+                if reach(held[-1]) > reach(key):
+                    key = next(k for k in held if reach(k) > reach(key))
+                    g = graphs[key]
+                else:
+                    torch.cuda.synchronize()                # the one that goes may still be running
+                    del graphs[held[0]]
+            elif len(graphs) >= graph.MAX_STEP_GRAPHS:
+                torch.cuda.synchronize()
                 graphs.popitem(last=False)
+        if g is None:
             g = graphs[key] = graph.StepGraph(self, *key)
         graphs.move_to_end(key)
         g.last = self._steps

@@ -40,6 +40,9 @@ class ModelStepper:
         self.use_graphs = (use_graphs and torch.device(model.rt.device).type == "cuda"
                            and getattr(model, "graph_safe", False))
         self._graphs = {}
+        # One pool of memory for all of them (a batch size has one by context class and kind of sampling): they run one after another on
+        # the caller's stream, and what outlives a step (tokens, positions, lengths) lies outside the pool.
+        self._graph_pool = torch.cuda.graph_pool_handle() if self.use_graphs else None
         self._prompt_graphs = OrderedDict()      # (sequences, rows of the bucket) -> PromptGraph, the newest last
         from .graph import recorded_prompt_rows
         self.prompt_rows = (recorded_prompt_rows(model.weight_bytes(), len(model.spec.schedule), (4 if model.rt.dtype is torch.float32 else 2))
@@ -307,7 +310,7 @@ class ModelStepper:
         graph = self._graphs.get(key)
         if graph is None:
             from .graph import DecodeGraph
-            graph = self._graphs[key] = DecodeGraph(self.model, self.sampler, len(slots), all_greedy, bound)
+            graph = self._graphs[key] = DecodeGraph(self.model, self.sampler, len(slots), all_greedy, bound, self._graph_pool)
         if self._armed != (key, tuple(slots)):
             params = np.array([[o.temperature, float(o.top_k), o.top_p, o.repeat_penalty] for o in options], dtype=np.float32)
             carried = None

@@ -1,5 +1,7 @@
 """The package's host logic (cache, block tables, step function) driven on the CPU through plain
 statements of the kernels, compared with the plain implementation."""
+import dataclasses
+
 import torch
 import pytest
 
@@ -216,3 +218,40 @@ def test_kept_sequences_give_way_and_rings_do_not_go_back():
     assert [g.tokens for g in got] == [w.tokens for w in plain.generate(big, max_tokens=20, **opts)]
     lm.model.cache.check()
     assert lm.model.cache.slots.held == 2
+
+
+def test_a_context_class_that_no_sequence_can_leave_is_not_told_apart():
+    """A reach of 64 positions more than the short context's: a class of its own while the cache lets a sequence pass it, else that of
+    any length."""
+    model = cpu_model("B", max_tokens=1024)
+    short = model.short_context
+    model.blocks[0].mixer.near_context = lambda n: short + 64
+    model.spec = dataclasses.replace(model.spec, max_position=4096)
+    for tokens, want in ((short + 64, [0, 0]), (short + 128, [short + 64, 0])):
+        model.make_cache(tokens)
+        assert [model.context_bound(2, n) for n in (short, short + 1, short + 65)] == [short] + want, tokens
+
+
+def test_without_room_for_more_recordings_a_batch_size_keeps_the_one_for_its_longest_contexts(monkeypatch):
+    """Two recordings are kept, both in use, each of another batch size; a sequence grows past a class's bound: its recording
+    gives its place to that of the next class, which then serves shorter contexts as well."""
+    from cima_b200.engine import graph
+    model, made = cpu_model("B", max_tokens=1024), []
+
+    class Recording:
+        last = 0
+
+        def __init__(self, model, *key):
+            made.append(key)
+
+    monkeypatch.setattr(graph, "StepGraph", Recording)
+    monkeypatch.setattr(graph, "MAX_STEP_GRAPHS", 2)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    model._context_bounds.update({n: [64, 128] for n in (1, 2, 3)})
+    first, other = model._step_graph(1, 10), model._step_graph(2, 10)
+    second = model._step_graph(1, 65)
+    assert list(model._step_graphs) == [(2, 64), (1, 128)] and model._step_graph(2, 12) is other
+    assert model._step_graph(1, 20) is second and model._step_graph(1, 128) is second
+    last = model._step_graph(1, 129)
+    assert model._step_graph(1, 20) is last and model._step_graph(1, 100) is last and model._step_graph(3, 5) is None
+    assert made == [(1, 64), (2, 64), (1, 128), (1, 0)] and first is not second

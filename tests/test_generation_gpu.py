@@ -783,3 +783,25 @@ def test_two_handles_on_one_model_record_as_each_was_asked():
         for t in (5, 6, 7):
             lm.step([StepEntry(slot, [t], [0])])
         assert len(first.model._step_graphs) == kept
+
+
+def test_recorded_decode_steps_share_their_memory():
+    """Generation in batches of 1 to 12, greedy and sampled, across the short context's bound: some four dozen recorded steps hold one
+    step's memory (7 MB of logits, in the allocator's segments of 20 MiB), not each its own, and each replays right beside the others."""
+    from cima_b200.config.shapes import SHAPES
+    kw = dict(config=dict(SHAPES["qwen2.5-0.5b"], num_hidden_layers=2, max_position_embeddings=4096), seed=3, draw="device", max_tokens=12 * 512, max_seqs=12, verbose=False)
+    rec = cima_b200.load(**kw)
+    prompts = [random_tokens(rec.spec.vocab, rec.model.short_context - 5 - i % 2, seed=70 + i) for i in range(12)]
+
+    def answer(n, t):
+        return [r.tokens for r in rec.generate(prompts[:n], temperature=t, repeat_penalty=1.0, max_tokens=12, seed=5, ignore_eos=True)]
+
+    for t in (0.0, 0.8):                                              # what a step of the largest size needs beside its recording
+        answer(12, t)
+    torch.cuda.synchronize(); torch.cuda.empty_cache()
+    before = torch.cuda.memory_reserved()
+    first = {(n, t): answer(n, t) for n in range(1, 13) for t in (0.0, 0.8)}
+    torch.cuda.synchronize(); torch.cuda.empty_cache()
+    assert len(rec.stepper._graphs) >= 40
+    assert torch.cuda.memory_reserved() - before <= 64 << 20
+    assert all(answer(*key) == want for key, want in first.items())
