@@ -501,8 +501,11 @@ extern "C" int cima_attention_plain(const void* qkv, int dtype, int ld, const vo
              ld, ldo, T, nh, nkv, hd, window, keep_first, v_group, gate_col, 1, 1, 1, scale, sink};
     const bool vec = hd % 4 == 0 && (from_cache || ld % 4 == 0) && ((from_cache ? (uintptr_t)cache : (uintptr_t)qkv) & 15) == 0;
     int rc;
-    // One head of one row a block as long as they are one wave of the GPU (two blocks an SM: 280 of them, 20 rows of 14 heads at 300
-    // positions, 3,464 -> 3,231 us a step); with more the heads that share keys share a block.
+    // One head of one row a block up to 296 of them, two an SM at head size 64 (98 registers); at 128 (170 registers) an SM holds one and more
+    // than 148 run in two waves, which still beat the other kernel at every length.  us a layer against it at 10 / 100 / 1,000 / 8,000 positions:
+    // 280 blocks of 64 (20 rows of 14 heads) -4.7 / -5.8 / -16 / -116, 288 of 128 (24 rows of 12 heads) -3.4 / -1.5 / -23 / -161, 280 of 128
+    // (10 rows of 28 heads) -7.1 / -2.8 / -27 / -186; with one long row beside short ones more.  336 lose (64: 1,000 positions +8.4,
+    // 8,000 +105; 128: 100 positions +3.1, 8,000 +118): there the heads that share keys share a block.
     if (from_cache && (hd == 64 || hd == 128) && (long long)T * nh <= 296 && T <= n_seqs && page_size % AF_KEYS == 0 && planes == 2 && ((uintptr_t)cache & 15) == 0 &&
         sink == 0.f && keep_first == 0 && v_group == 1 && !head_sink && gate_col == 0 && !slopes) {
       rc = hd == 64 ? cima_launch(k_attention_f32_row<64>, dim3(T, nh), dim3(256), (size_t)0, stream, 1, a) : cima_launch(k_attention_f32_row<128>, dim3(T, nh), dim3(256), (size_t)0, stream, 1, a);

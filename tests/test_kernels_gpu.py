@@ -1062,3 +1062,28 @@ def test_float32_attention_of_few_rows_has_the_bits_of_many(K, nh, nkv, hd, wind
     bc, want = batch_of(seqs, "cpu"), torch.zeros(B, nh * hd, dtype=torch.float64)
     REF.attention_plain(qkv, cpu, bc.row_pos, bc.row_seq, bc.seq_slot, bc.seq_first_row, want, nh, nkv, hd, scale, window, True)
     assert err(many, want) <= TOL["float32"]
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window", [(6, 2, 64, 40), (4, 1, 64, 129), (2, 2, 128, 64), (12, 2, 128, 200)])
+def test_float32_attention_of_few_rows_over_a_ring(K, nh, nkv, hd, window):
+    """A window's keys in a ring of pages that has wrapped several times: pieces of 32 keys whose lower part newer positions have
+    overwritten.  Against float64 over the whole sequences; the key just below the window stands out until it is left out."""
+    lens, ring, scale = [1, window - 1, window, window + 1, 449, 640, 707, 1025], -(-window // 64) + 1, 1.0 / math.sqrt(hd)
+    B, G = len(lens), nh // nkv
+    assert B * nh <= 296
+    slots = list(range(B))
+    tables = {i: [ring * i + j for j in range(ring)] for i in slots}
+    cpu, gpu = make_kv(ring * B, nkv, 64, hd, B, ring, ring, window, torch.float32, tables)
+    qkv = g(B, (nh + 2 * nkv) * hd, seed=6)
+    want = torch.empty(B, nh * hd, dtype=torch.float64)
+    for i, n in enumerate(lens):
+        k, v, lo = g(n, nkv, hd, seed=50 + i), g(n, nkv, hd, seed=90 + i), max(0, n - window)
+        if lo:
+            k[lo - 1, 0] = 9.0 * qkv[i, :hd]
+        fill_cache(cpu, gpu, i, k, v)
+        for h in range(nh):
+            p = torch.softmax((k[lo:, h // G].double() @ qkv[i, h * hd:(h + 1) * hd].double()) * scale, 0)
+            want[i, h * hd:(h + 1) * hd] = p @ v[lo:, h // G].double()
+    b, out = batch_of([(i, n - 1, 1) for i, n in enumerate(lens)], "cuda"), torch.full((B, nh * hd), 7.0, device="cuda")
+    K.attention_plain(qkv.cuda(), gpu, b.row_pos, b.row_seq, b.seq_slot, b.seq_first_row, out, nh, nkv, hd, scale, window, True)
+    assert err(out, want) <= TOL["float32"]
