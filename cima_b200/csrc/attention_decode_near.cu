@@ -131,7 +131,11 @@ k_attention_near(const __nv_bfloat16* qkv, int ld, const __nv_bfloat16* cache, C
       }
       if (more) load(kf, src, c + WARPS, lo, len);
       const int key = c * 16 + g;
-      float p[4];
+      // Probabilities against the 16 keys' own maximum, whose key's is 1 and so has no rounding to bfloat16, and the 16 keys' sum from 0, brought
+      // to the running maximum by float32 multiply-adds: against the running maximum the result was the further from 64 bits the fewer
+      // warps shared the keys (relative error at 2,000 positions in clusters of 16 / 4 / 1: 1.94 / 2.04 / 2.14e-3), further than the splits
+      // where those are more than the blocks.
+      float p[4], corr[2], f[2];
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const float v0 = key >= lo && key < len ? (sa[j] + sb[j]) * sc2 : -INFINITY;
@@ -139,20 +143,26 @@ k_attention_near(const __nv_bfloat16* qkv, int ld, const __nv_bfloat16* cache, C
         float mx = fmaxf(v0, v1);
 #pragma unroll
         for (int x = 4; x < 32; x *= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
-        const float mn = fmaxf(mr[j], mx), ms = mn == -INFINITY ? 0.f : mn, corr = ex2(mr[j] - ms);
+        const float own = mx == -INFINITY ? 0.f : mx, mn = fmaxf(mr[j], mx), ms = mn == -INFINITY ? 0.f : mn;
+        p[j] = ex2(v0 - own);
+        p[j + 2] = ex2(v1 - own);
+        corr[j] = ex2(mr[j] - ms);
+        f[j] = ex2(mx - ms);
         mr[j] = mn;
-        p[j] = ex2(v0 - ms);
-        p[j + 2] = ex2(v1 - ms);
-        lr[j] = lr[j] * corr + (p[j] + p[j + 2]);
-#pragma unroll
-        for (int i = 0; i < HD / 16; i++) { o[i][j] *= corr; o[i][j + 2] *= corr; }
+        lr[j] = fmaf(lr[j], corr[j], (p[j] + p[j + 2]) * f[j]);
       }
       const uint32_t b0 = transposed(pack2(p[0], p[1])), b1 = transposed(pack2(p[2], p[3]));
       // O = V^T P^T: tile (d, e) holds dims 32 d + 8 (g / 2) + g % 2 + 4 e (rows g) and those + 2 (rows g + 8)
 #pragma unroll
       for (int d = 0; d < HD / 32; d++) {
-        mma(o[2 * d], transposed(vf[d][0].x), transposed(vf[d][0].y), transposed(vf[d][1].x), transposed(vf[d][1].y), b0, b1);
-        mma(o[2 * d + 1], transposed(vf[d][0].z), transposed(vf[d][0].w), transposed(vf[d][1].z), transposed(vf[d][1].w), b0, b1);
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          float s16[4] = {0.f, 0.f, 0.f, 0.f};
+          if (e == 0) mma(s16, transposed(vf[d][0].x), transposed(vf[d][0].y), transposed(vf[d][1].x), transposed(vf[d][1].y), b0, b1);
+          else mma(s16, transposed(vf[d][0].z), transposed(vf[d][0].w), transposed(vf[d][1].z), transposed(vf[d][1].w), b0, b1);
+#pragma unroll
+          for (int i = 0; i < 4; i++) o[2 * d + e][i] = fmaf(o[2 * d + e][i], corr[i & 1], s16[i] * f[i & 1]);
+        }
       }
       if (more) load(vf, src + v_off, c + WARPS, lo, len, true);
     }

@@ -89,6 +89,34 @@ def test_an_infinite_value_stays_in_its_column(hd):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("signs", ["mixed", "one"])
+@pytest.mark.parametrize("nh,nkv,hd", [(14, 2, 64), (28, 4, 128)])
+def test_long_sums_are_as_near_to_64_bits_as_the_splits(nh, nkv, hd, signs):
+    """Values of mixed and of one sign, up to 8,000 positions: no cluster is further from float64 than the split kernel at 64 splits, whose
+    sums are the shortest (2 % for what the rounding of the result leaves to chance)."""
+    K, B, G = Kernels(verbose=False), 4, nh // nkv
+    for n in (300, 2000, 8000):
+        gen, width = torch.Generator().manual_seed(n + hd), -(-n // 64)
+        storage = torch.randn(B * width, 2, nkv, 64, hd, generator=gen)
+        if signs == "one":
+            storage[:, 1] = storage[:, 1].abs()
+        storage = storage.bfloat16().cuda()
+        table = torch.randperm(B * width, generator=gen).view(B, width).int().cuda()
+        qkv = torch.randn(B, (nh + 2 * nkv) * hd, generator=gen).bfloat16().cuda()
+        held = storage[table.long()].double().permute(0, 2, 3, 1, 4, 5).reshape(B, 2, nkv, width * 64, hd)[..., :n, :]
+        q, scale = qkv[:, :nh * hd].double().view(B, nkv, G, hd), 1.0 / math.sqrt(hd)
+        want = (torch.softmax(q @ held[:, 0].transpose(2, 3) * scale, -1) @ held[:, 1]).reshape(B, nh * hd)
+        args = (qkv, LayerKV(storage, table, 64, 0, 0, 0), torch.arange(B, dtype=torch.int32, device="cuda"), torch.full((B,), n, dtype=torch.int32, device="cuda"))
+        out = torch.empty(B, nh * hd, dtype=torch.bfloat16, device="cuda")
+        off = lambda: ((out.double() - want).norm() / want.norm()).item()                          # noqa: E731
+        K.attention_decode(*args, out, nh, nkv, hd, scale, 0, n_splits=64)
+        splits = off()
+        for cluster in (1, 2, 4, 8, 16):
+            K.attention_decode_near(*args, out, nh, nkv, hd, scale, 0, cluster)
+            assert off() <= 1.02 * splits, (n, cluster, off(), splits)
+
+
+@pytest.mark.gpu
 def test_clusters_stay_within_what_the_device_holds(monkeypatch):
     """The device is asked once, and a step takes no cluster that it cannot place: with room for none of 16 (as where no group has 16 free
     SMs) the step runs in smaller ones."""
