@@ -32,17 +32,25 @@ def short_context(head_dim: int) -> int:
     return SHORT_CONTEXT_BYTES // (4 * head_dim) // 64 * 64
 
 
-NEAR_KEYS = 832             # positions a block of a cluster, up to which the cluster kernel beats the splits where it leaves SMs idle
-NEAR_FULL = 96              # blocks from which on it does so at every length
+def decode_splits(blocks: int) -> int:
+    """Splits of the decode attention's keys for ``blocks`` (sequence, kv head, 16 query heads) at long contexts: one wave of
+    blocks (two of them fit an SM), never a second, nearly empty wave; beyond 8 splits only while the GPU would otherwise stay mostly
+    idle.  32 splits at most, 64 where even 32 leave SMs without a block (one sequence of 4 kv heads: measured at the 7B shape 19 to 25 us
+    against 28 to 31 at 30,000 positions, 15 against 19 at 16,384, the same up to 6,000; with two sequences 32 are the best again)."""
+    splits = max(1, min(64 if blocks * 32 < SPLIT_FEW_BLOCKS else 32, SPLIT_BLOCKS // blocks))
+    return 8 if splits > 8 and blocks * 8 >= SPLIT_FEW_BLOCKS else splits
+
+
+NEAR_KEYS = 832             # positions a block of a cluster, up to which the cluster kernel beats many more splits than it has blocks
 
 
 def near_cluster(pairs: int, head_dim: int, room=None) -> int:
     """Blocks of the cluster that shares one of ``pairs`` (sequence, kv head) pairs: as many as one wave holds (an SM holds one block at
-    head_dim 128, two at 64), in the clusters that the GPU's groups of SMs can place: at head_dim 128 one of 16 a group (measured: 4
-    pairs in clusters of 16 against 8: 7B, 2,000 positions 2,658 against 2,676 us a step; 8 pairs 2,939 against 2,759), 14 of 8
-    (16 pairs, 1.5B, 1,000 positions: clusters of 8 1,218 us, of 4 1,100), 37 of 4, 74 of 2.  ``room``: clusters of 16, 8, 4 and 2 blocks that
-    the device at hand holds at once (``Kernels.near_room``); one that holds fewer gets smaller clusters, and none of a size that it
-    cannot place."""
+    head_dim 128, two at 64), in the clusters that the GPU's groups of SMs can place.  ``room``: clusters of 16, 8, 4 and 2 blocks that the
+    device at hand holds at once (``Kernels.near_room``; one of B200: 7, 15, 33 and 74 at head_dim 128).  One more waits for a whole
+    cluster to finish (us a layer against the splits, 33 / 34 pairs in clusters of 4: 250 positions -2.5 / +1.4, 6,000 -3.0 / +13; 15 / 17 in
+    clusters of 8: 6,000 -2.9 / +7.2).  Of the largest ones fewer than fit are the better choice at short contexts: 4 clusters of 16 (6 pairs
+    of 250 positions: -1.7, in clusters of 8 -2.4), 14 of 8; twice as many at head_dim 64."""
     for i, (cluster, most) in enumerate(((16, 4), (8, 14), (4, 37), (2, 74))):
         most *= 2 if head_dim == 64 else 1
         if pairs <= (most if room is None else min(most, room[i])):
@@ -51,13 +59,29 @@ def near_cluster(pairs: int, head_dim: int, room=None) -> int:
 
 
 def near_context(pairs: int, head_dim: int, room=None) -> int:
-    """Positions up to which the cluster kernel takes ``pairs`` (sequence, kv head) pairs; 0: any number.  Where its blocks fill
-    the GPU it is the faster one throughout (us a layer against the splits and their merge: 7B, 8 sequences, 2,048 to 24,000
-    positions -6.5 to -7.1; 32 sequences, 270 to 4,000 -5 to -6; 64, 2,000 -1.2; 1.5B, 64 sequences, 3,000 -4.6).  Where it leaves
-    SMs idle the splits read more at a time: at 4,000 / 7,000 / 16,000 positions of one sequence in a cluster of 8 -2.5 / +0.3 / +8.3
-    (1.5B, 2 pairs), in one of 16 -3.5 / -2.1 (8,000) / +0.4, at 3,000 / 6,000 in 16 clusters of 4 -2.3 / +1.0."""
-    cluster = near_cluster(pairs, head_dim, room)
-    return 0 if pairs * cluster >= NEAR_FULL * (2 if head_dim == 64 else 1) else NEAR_KEYS * cluster
+    """Positions up to which the cluster kernel takes ``pairs`` (sequence, kv head) pairs; 0: any number.  It saves a launch and a
+    merge, some 3 us a layer, and a block of it walks about 1.5 times as fast as one of the splits'; what it has against them is
+    the number of its blocks a pair.  Measured as us a layer against the splits, at the Qwen2.5 shapes (7B: 4 kv heads, 1.5B: 2), sequences
+    of one length:
+
+    * as many blocks as splits, or half as many at head_dim 128 (where two blocks of the splits share the SM that one of the cluster kernel
+      has for itself): ahead at every length (7B, 8 sequences, 2,000 / 16,000 positions -6.9 / -7.7; 16, -3.3 / -6.0; 28, 8,000 -9.0; 64,
+      4,000 -1.5; 1.5B, 16 sequences, 30,000 -3.5); so too 13 and 14 pairs in clusters of 8 (22 and 21 splits: 1.5B, 30,000 -1.8);
+    * 12 pairs in clusters of 8 (24 splits): 1.5B, 16,000 / 30,000 -0.6 / +1.9; 5 splits against 2 blocks: 1.5B, 4,000 / 8,000 -1.3 / +2.4,
+      7B -2.0 / +1.3; 3 against 1 and 6 against 2: 1.5B, 2,000 / 4,000 -0.7 to -1.4 / +1.1 to +5.1, 7B -1.0 to -2.0 / 0 to +4.6;
+    * more splits yet: 1.5B, one sequence in a cluster of 16, 8,000 / 16,000 -2.1 / +0.4, 8 in clusters of 4, 4,000 / 8,000 -1.4 / +3.5;
+    * head_dim 64 (0.5B): 5 splits against 4 blocks 16,000 -4.5 to -5.0; 6 against 4 16,000 0; 3 against 2 10,000 -0.2; 18 against 8
+      8,000 / 16,000 -1.9 / +1.5."""
+    cluster, splits = near_cluster(pairs, head_dim, room), decode_splits(pairs)
+    if head_dim == 64:
+        keys = 0 if 5 * cluster >= 4 * splits else 4096 if 3 * cluster >= 2 * splits else NEAR_KEYS
+    elif 2 * cluster >= splits or (cluster == 8 and splits <= 22):
+        keys = 0
+    elif cluster == 8 and splits <= 24:
+        keys = 2048
+    else:
+        keys = 2560 if 5 * cluster >= 2 * splits else 1280 if 3 * cluster >= splits else NEAR_KEYS
+    return keys * cluster
 
 
 EXTEND_BLOCKS = 444         # blocks of the attention of going-on rows that one wave holds (three per SM, 148 SMs)
@@ -728,19 +752,10 @@ class Kernels:
         if tuple(out.shape) != (B, n_heads * head_dim) or seq_slot.numel() < B or seq_len.numel() < B:
             raise KernelError(f"attention_decode: out {tuple(out.shape)} / sequences do not fit {B} rows")
         if n_splits is None:
-            mtiles = -(-(n_heads // n_kv_heads) // 16)
-            # one wave of blocks (two of them fit an SM): never a second, nearly empty wave; beyond 8 splits
-            # only while the GPU would otherwise stay mostly idle.  The splits are merged by a second kernel: merging
-            # inside a thread-block cluster (clusters of 8 blocks with 100 KB of shared memory each are slow to
-            # place) and merging in the last block to finish (a fence and a ticket per block) were both measured
-            # slower inside the decode step
-            base = B * n_kv_heads * mtiles
-            # 32 splits at most, 64 where even 32 leave SMs without a block (one sequence of 4 kv heads: measured at
-            # the 7B shape 19 to 25 us against 28 to 31 at 30,000 positions, 15 against 19 at 16,384, the same up to
-            # 6,000; with two sequences 32 are the best again)
-            n_splits = max(1, min(64 if base * 32 < SPLIT_FEW_BLOCKS else 32, SPLIT_BLOCKS // base))
-            if n_splits > 8 and base * 8 >= SPLIT_FEW_BLOCKS:
-                n_splits = 8
+            # The splits are merged by a second kernel.  Merging inside a thread-block cluster (clusters of 8 blocks with 100 KB of shared
+            # memory each are slow to place; ``attention_decode_near``, which does it, keeps keys and values in registers) and merging
+            # in the last block to finish (a fence and a ticket per block) were both measured slower inside the decode step.
+            n_splits = decode_splits(B * n_kv_heads * -(-(n_heads // n_kv_heads) // 16))
             if max_len > 0:
                 seen = max_len if window <= 0 else min(max_len, window + 64 + -(-keep_first // 64) * 64)      # positions whose pages a row reads
                 n_splits = min(n_splits, -(-seen // 64))

@@ -6,21 +6,39 @@ import pytest
 import torch
 
 from cima_b200.cache.kv import LayerKV
-from cima_b200.kernels import Kernels, near_cluster, near_context
+from cima_b200.kernels import Kernels, decode_splits, near_cluster, near_context
 
 TOL = 2e-2          # bfloat16 values of magnitude 1 to 4 and their weighted means, as in test_kernels_gpu.py
 LENS = [1, 2, 16, 17, 64, 65, 128, 129, 300, 1100]
 
 
 def test_the_rule_covers_every_number_of_pairs():
-    """At most one block an SM (two at head size 64) where a cluster has more than one, and no bound where they fill the GPU."""
+    """At most one block an SM (two at head size 64) where a cluster has more than one."""
     for hd, room in ((64, 296), (128, 148)):
         last = 16
         for pairs in range(1, 600):
             c = near_cluster(pairs, hd)
             assert c in (1, 2, 4, 8, 16) and c <= last and (c == 1 or pairs * c <= room)
-            assert (near_context(pairs, hd) == 0) == (pairs * c >= (192 if hd == 64 else 96))
             last = c
+
+
+ROOM = {64: (14, 33, 71, 148), 128: (7, 15, 33, 74)}              # what a B200 answered
+# (head size, pairs, positions): us a layer of the cluster kernel against the splits, sequences of one length, on a B200
+FASTER = {(128, 4, 8000): -3.0, (128, 8, 4000): -3.2, (128, 12, 8000): -2.3, (128, 14, 16000): -2.3, (128, 16, 2000): -3.6, (128, 20, 16000): -4.5,
+          (128, 32, 16000): -3.5, (128, 33, 6000): -3.0, (128, 36, 700): -2.3, (128, 40, 700): -3.5, (128, 48, 2000): -1.3, (128, 56, 4000): -1.3,
+          (128, 60, 12000): -4.7, (128, 74, 4000): -3.4, (128, 76, 700): -2.5, (128, 96, 700): -2.9, (128, 104, 8000): -9.4, (128, 128, 4000): -4.9,
+          (128, 152, 4000): -3.7, (128, 256, 4000): -1.5, (64, 2, 8000): -0.9, (64, 24, 16000): -8.0, (64, 32, 2000): -1.7, (64, 56, 16000): -4.5,
+          (64, 71, 2000): -3.1, (64, 96, 4000): -1.6, (64, 128, 4000): -7.6, (64, 176, 4000): -13.2}
+SLOWER = {(128, 2, 16000): 0.4, (128, 16, 6000): 1.9, (128, 36, 6000): 7.3, (128, 38, 4000): 3.0, (128, 40, 4000): 1.6, (128, 48, 8000): 5.1, (128, 48, 16000): 14.0,
+          (128, 56, 8000): 1.3, (128, 76, 4000): 4.6, (128, 92, 4000): 3.9, (128, 96, 4000): 3.5, (128, 96, 8000): 12.1, (64, 2, 16000): 0.4,
+          (64, 16, 16000): 1.5, (64, 32, 16000): 2.6}
+
+
+def test_the_reach_lies_where_it_was_measured():
+    """No number of pairs at a length at which the splits were faster, and every one well below."""
+    for (hd, pairs, n), us in {**FASTER, **SLOWER}.items():
+        reach = near_context(pairs, hd, ROOM[hd])
+        assert (reach == 0 or n <= reach) == (us < 0), (hd, pairs, n, reach, near_cluster(pairs, hd, ROOM[hd]), decode_splits(pairs))
 
 
 def test_the_clusters_are_those_that_the_device_holds():
