@@ -12,6 +12,8 @@ from typing import Any, Dict, List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..kernels import EVEN
+
 
 Q_TILE = 64        # query rows per block of the prefill attention kernel
 Q_TILE_TC = 128    # ... and of its tcgen05 variant
@@ -48,11 +50,17 @@ class StepBatch:
     n_q_tiles_tc: int = 0             # the same in blocks of 128 rows
     q_tile_tc_seq: torch.Tensor = None
     q_tile_tc_row0: torch.Tensor = None
+    even: bool = True                 # the sequences are of about one length (``lengths_are_even``)
     host_seq_slot: np.ndarray = None
     host_seq_first_row: np.ndarray = None
     host_seq_len: np.ndarray = None
     # what a layer leaves for later layers of the same step, by a name of its kind's own (emptied when the step ends)
     carried: Dict[str, Any] = field(default_factory=dict)
+
+
+def lengths_are_even(lengths) -> bool:
+    """Whether a step's sequences are so near to one length that the kernels' choices for that hold."""
+    return sum(lengths) >= EVEN * len(lengths) * max(lengths)
 
 
 def check_entries(entries: Sequence[StepEntry], vocab: Optional[int] = None) -> None:
@@ -130,7 +138,7 @@ def build_batch(entries: List[StepEntry], starts: Sequence[int], vocab: int, dev
     else:
         dev = host.clone()
     all_in_order = W == T and bool(np.array_equal(want_rows, np.arange(T)))
-    return StepBatch(prefill=prefill, n_rows=T, n_seqs=B, n_want=W, max_len=int(seq_len.max()),
+    return StepBatch(prefill=prefill, n_rows=T, n_seqs=B, n_want=W, max_len=int(seq_len.max()), even=lengths_are_even(seq_len.tolist()),
                      want_all_in_order=all_in_order, max_rows=max(counts),
                      tokens=dev[0:T], row_pos=dev[T:2 * T], row_seq=dev[2 * T:3 * T],
                      seq_slot=dev[o:o + B], seq_first_row=dev[o + B:o + 2 * B + 1],

@@ -17,13 +17,17 @@ import torch
 from .batch import StepBatch, StepEntry, build_batch
 
 
-def one_token_batch(meta: torch.Tensor, n_seqs: int, max_len: int) -> StepBatch:
+UNEVEN = -1     # context class of a step of any length whose sequences are far from one length (``Model.context_bound``)
+
+
+def one_token_batch(meta: torch.Tensor, n_seqs: int, max_len: int, even: bool = True) -> StepBatch:
     """A step of one token a sequence, all logits wanted, whose arrays are views of ``meta`` (int32 [6 n + 1], see
     ``fill_meta``).  What a recorded step may know on the host is what every replay shares: the number of sequences and
     their rows (one each).  Slots, positions and lengths change from replay to replay and exist on the device only
-    (``host_seq_slot`` / ``host_seq_len`` stay None; ``max_len`` bounds the sequences' positions after the step, 0 = unknown)."""
+    (``host_seq_slot`` / ``host_seq_len`` stay None; ``max_len`` bounds the sequences' positions after the step, 0 = unknown;
+    ``even``: they are of about one length)."""
     B, m = n_seqs, meta
-    return StepBatch(prefill=False, n_rows=B, n_seqs=B, n_want=B, max_len=max_len, want_all_in_order=True,
+    return StepBatch(prefill=False, n_rows=B, n_seqs=B, n_want=B, max_len=max_len, even=even, want_all_in_order=True,
                      tokens=m[0:B], row_pos=m[B:2 * B], row_seq=m[2 * B:3 * B], seq_slot=m[3 * B:4 * B], seq_first_row=m[4 * B:5 * B + 1],
                      seq_len=m[5 * B + 1:6 * B + 1], want_rows=m[2 * B:3 * B], max_rows=1, host_seq_first_row=np.arange(B + 1, dtype=np.int32))
 
@@ -45,8 +49,8 @@ class DecodeGraph:
 
     def __init__(self, model, sampler, n_seqs: int, all_greedy: bool, max_len: int = 0, pool=None):
         """``max_len``: the most positions that a sequence may hold after a step of this graph (0: as many as the model
-        takes).  A recorded step fixes its launches; one recorded for short or middling contexts takes the kernels' choices
-        for them, and the stepper moves on to the next graph when a sequence outgrows the bound.  ``pool``: the memory that its
+        takes; ``UNEVEN``: the same, of sequences far from one length).  A recorded step fixes its launches; one recorded for short
+        or middling contexts takes the kernels' choices for them, and the stepper moves on to the next graph when a sequence outgrows the bound.  ``pool``: the memory that its
         recording shares with others (of the same caller: they run one after another, and nothing in it outlives a step)."""
         self.model, self.sampler = model, sampler
         self.B = B = n_seqs
@@ -56,7 +60,7 @@ class DecodeGraph:
         dev = model.rt.device
         self.meta = torch.zeros(6 * B + 1, dtype=torch.int32, device=dev)
         self.meta_host = torch.zeros(6 * B + 1, dtype=torch.int32).pin_memory()
-        self.batch = b = one_token_batch(self.meta, B, max_len or model.most_positions)
+        self.batch = b = one_token_batch(self.meta, B, max_len if max_len > 0 else model.most_positions, max_len != UNEVEN)
         self.tokens, self.row_pos, self.row_seq = b.tokens, b.row_pos, b.row_seq
         self.seq_slot, self.seq_first_row, self.seq_len = b.seq_slot, b.seq_first_row, b.seq_len
         self.params = torch.zeros(B, 4, dtype=torch.float32, device=dev)
@@ -195,7 +199,7 @@ class StepGraph:
     def __init__(self, model, n_seqs: int, max_len: int):
         self.n_seqs = n_seqs
         self.meta = torch.zeros(6 * n_seqs + 1, dtype=torch.int32, device=model.rt.device)
-        self.batch = one_token_batch(self.meta, n_seqs, max_len or model.most_positions)
+        self.batch = one_token_batch(self.meta, n_seqs, max_len if max_len > 0 else model.most_positions, max_len != UNEVEN)
         self.graph = None
         self.logits = None
         self.uses = 0

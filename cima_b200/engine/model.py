@@ -9,6 +9,7 @@ batch of sequences here.
 from __future__ import annotations
 
 import dataclasses
+import math
 import sys
 import threading
 from collections import OrderedDict
@@ -23,7 +24,8 @@ from ..parts import Linear, Runtime, build_block, build_norm
 from ..parts.linear import FOLDED_NORM_ROWS
 from ..parts.norm import RowsInfo
 from ..weights.loader import TensorSpec, tensor_names
-from .batch import StepBatch, StepEntry, build_batch, check_entries
+from .batch import StepBatch, StepEntry, build_batch, check_entries, lengths_are_even
+from .graph import UNEVEN
 from .fit import STEP_ROWS
 
 _DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.float32, "fp32": torch.float32,
@@ -75,7 +77,7 @@ class Model:
         self.config = None                                  # set by load_model
         self.step_rows = STEP_ROWS                          # a step of more rows runs in parts
         self.record_steps = False                           # record one-token steps (``StepGraph``); an ``LM`` with graphs says so
-        self._context_bounds: Dict[int, List[int]] = {}     # sequences -> bounds of their context classes
+        self._context_classes: Dict[int, tuple] = {}        # sequences -> what ``context_bound`` chooses among
         self._step_graphs = OrderedDict()                   # (sequences, context bound) -> StepGraph, the newest last
         self._step_pool = None                              # (memory pool, stream) that the recordings share
         self._steps = 0                                     # one-token steps so far
@@ -173,17 +175,26 @@ class Model:
         """The most positions that a sequence can come to hold: what the model takes and the cache has room for."""
         return self.spec.max_position if self.cache is None else min(self.spec.max_position, self.cache.max_tokens)
 
-    def context_bound(self, n_seqs: int, longest: int) -> int:
-        """The context class of a one-token step of ``n_seqs`` sequences, the longest of ``longest`` positions after it: the smallest
-        bound that holds it among ``short_context`` and the reach of the kernels for middling contexts (``mixer.near_context``),
-        0 for any number of positions."""
-        bounds = self._context_bounds.get(n_seqs)
-        if bounds is None:                                  # (asked for at every step)
-            named = [b.mixer.near_context(n_seqs) for b in self.blocks if hasattr(getattr(b, "mixer", None), "near_context")]
-            near = min([n for n in named if n > 0], default=0)
+    def context_bound(self, lengths: Sequence[int]) -> int:
+        """The context class of a one-token step of sequences that hold ``lengths`` positions after it, named by the most positions that it
+        stands for: ``short_context``, the reach of the kernels for middling contexts (``mixer.near_context``), 0 for any number,
+        ``graph.UNEVEN`` for any number where those kernels would take it but for how far the sequences are from one length."""
+        classes = self._context_classes.get(len(lengths))
+        if classes is None:                                 # (asked for at every step)
+            mixers = [m for b in self.blocks for m in getattr(getattr(b, "mixer", None), "branches", [getattr(b, "mixer", None)]) if hasattr(m, "near_context")]
+            reach = [(m.near_context(len(lengths)), m.near_context(len(lengths), False)) for m in mixers]
             # (each class has recordings of its own: one that no sequence can leave is not told apart from that of any length)
-            bounds = self._context_bounds[n_seqs] = [self.short_context] + ([near] if near < self.most_positions else [])
-        return next((n for n in bounds if longest <= n), 0)
+            reach = [tuple(n if 0 < n < self.most_positions else math.inf for n in r) for r in reach if None not in r]
+            near, uneven = (min((r[i] for r in reach), default=math.inf) for i in (0, 1))
+            classes = self._context_classes[len(lengths)] = (self.short_context, near, uneven, any(e == math.inf > u for e, u in reach))
+        short, near, uneven, apart = classes
+        longest = max(lengths)
+        if longest <= short:
+            return short
+        even = longest <= uneven or lengths_are_even(lengths)
+        if even and longest <= near < math.inf:
+            return near
+        return UNEVEN if apart and not even else 0
 
     @property
     def graph_safe(self) -> bool:
@@ -213,7 +224,7 @@ class Model:
         shares = {site: self.spec.layers[layer].mixer.cache_from for site, layer in enumerate(sched)
                   if self.spec.layers[layer].mixer.cache_from is not None}
         self._forget_step_graphs()                          # recorded with the cache before
-        self._context_bounds.clear()
+        self._context_classes.clear()
         self.cache = KVCache(self._cache_requests(),
                              max_tokens, self.spec.max_position,
                              self.rt.dtype, self.rt.device, page_size=page_size, max_seqs=max_seqs,
@@ -273,7 +284,7 @@ class Model:
             return self._step_in_rounds(entries, limit)
         if record and self._recordable(entries):
             with self._step_lock:
-                g = self._step_graph(len(entries), max(starts) + 1)
+                g = self._step_graph([n + 1 for n in starts])
                 if g is not None:
                     return self._step_recorded(g, entries, starts)
         batch = build_batch(entries, starts, self.spec.vocab, self.rt.device)
@@ -293,23 +304,23 @@ class Model:
                 and self.graph_safe and torch.device(self.rt.device).type == "cuda" and getattr(self.rt.kernels, "profile", None) is None
                 and not torch.cuda.is_current_stream_capturing())
 
-    def _step_graph(self, n_seqs: int, max_len: int):
-        """The ``StepGraph`` of this shape, or None where as many others as are kept have been in use of late: a caller that goes
-        round among more shapes replays some and issues the rest, rather than recording each anew.  A batch size takes no more than its
+    def _step_graph(self, lengths: Sequence[int]):
+        """The ``StepGraph`` of a step that leaves ``lengths``, or None where as many others as are kept have been in use of late: a caller
+        that goes round among more shapes replays some and issues the rest, rather than recording each anew.  A batch size takes no more than its
         share then: one recorded for longer contexts serves the shorter ones too, and takes their recording's place."""
         from . import graph
         graphs = self._step_graphs
-        key = (n_seqs, self.context_bound(n_seqs, max_len))
+        key = (len(lengths), self.context_bound(lengths))
         self._steps += 1
         g = graphs.get(key)
         if g is None:
             if len(graphs) >= graph.MAX_STEP_GRAPHS and self._steps - next(iter(graphs.values())).last <= graph.STEP_GRAPH_IDLE:
-                reach = lambda k: k[1] or self.most_positions                                       # noqa: E731
-                held = sorted((k for k in graphs if k[0] == n_seqs), key=reach)
+                reach = lambda k: k[1] if k[1] > 0 else self.most_positions                         # noqa: E731
+                held = sorted((k for k in graphs if k[0] == key[0]), key=reach)
                 if not held:
                     return None
-                if reach(held[-1]) > reach(key):
-                    key = next(k for k in held if reach(k) > reach(key))
+                if reach(held[-1]) >= reach(key):
+                    key = next(k for k in held if reach(k) >= reach(key))
                     g = graphs[key]
                 else:
                     torch.cuda.synchronize()                # the one that goes may still be running

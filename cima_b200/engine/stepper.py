@@ -259,10 +259,9 @@ class ModelStepper:
         self._inflight.clear()
 
     def _context_bound(self, slots, ahead: int) -> int:
-        """The bound of the graph that may run the next ``ahead`` steps of these sequences: the smallest that every sequence
-        stays within (``Model.context_bound``), 0 for none."""
+        """The context class of the graph that may run the next ``ahead`` steps of these sequences (``Model.context_bound``)."""
         cache = self.model.cache
-        return self.model.context_bound(len(slots), max(cache.length(s) + self._inflight.get(s, 0) for s in slots) + ahead)
+        return self.model.context_bound([cache.length(s) + self._inflight.get(s, 0) + ahead for s in slots])
 
     def _decode_pipelined(self, slots, last_tokens, options) -> List[int]:
         fl = self._flight

@@ -58,8 +58,11 @@ def near_cluster(pairs: int, head_dim: int, room=None) -> int:
     return 1
 
 
-def near_context(pairs: int, head_dim: int, room=None) -> int:
-    """Positions up to which the cluster kernel takes ``pairs`` (sequence, kv head) pairs; 0: any number.  It saves a launch and a
+EVEN = 0.85                 # a batch's mean length over its longest, from which on it counts as one of one length
+
+
+def near_context(n_seqs: int, n_kv_heads: int, head_dim: int, room=None, even: bool = True) -> int:
+    """Positions of the longest sequence up to which the cluster kernel takes a step; 0: any number.  It saves a launch and a
     merge, some 3 us a layer, and a block of it walks about 1.5 times as fast as one of the splits'; what it has against them is
     the number of its blocks a pair.  Measured as us a layer against the splits, at the Qwen2.5 shapes (7B: 4 kv heads, 1.5B: 2), sequences
     of one length:
@@ -71,9 +74,26 @@ def near_context(pairs: int, head_dim: int, room=None) -> int:
       7B -2.0 / +1.3; 3 against 1 and 6 against 2: 1.5B, 2,000 / 4,000 -0.7 to -1.4 / +1.1 to +5.1, 7B -1.0 to -2.0 / 0 to +4.6;
     * more splits yet: 1.5B, one sequence in a cluster of 16, 8,000 / 16,000 -2.1 / +0.4, 8 in clusters of 4, 4,000 / 8,000 -1.4 / +3.5;
     * head_dim 64 (0.5B): 5 splits against 4 blocks 16,000 -4.5 to -5.0; 6 against 4 16,000 0; 3 against 2 10,000 -0.2; 18 against 8
-      8,000 / 16,000 -1.9 / +1.5."""
+      8,000 / 16,000 -1.9 / +1.5.
+
+    Of ``even`` lengths; where one is far longer than the mean its few blocks walk alone in the end, and only the number of blocks counts.
+    One long sequence and the others of 300, 1.5B: 2 splits against 1 block 2,000 / 4,000 / 16,000 -0.3 / +3.5 / +27, 4 against 2
+    -0.2 / +1.8 / +13, 8 against 4 -1.4 / 0 / +5.8, 24 against 8 -1.8 / -0.3 / +5.1, 3 against 1 2,000 +3.3; head_dim 64: 18
+    against 8 4,000 / 8,000 -0.6 / +1.1, 6 against 4 4,000 / 16,000 -1.1 / +2.3, 3 against 2 2,000 / 4,000 -0.6 / +0.4.  As many blocks as
+    splits stay ahead (64 sequences of 4 kv heads -9 at 1,000, -150 at 30,000).  Up to 8 sequences with 4 kv heads and more it is as with
+    even lengths: the projection just before, one kernel with rotation and append, fills the GPU, and the splits of a long sequence, which come
+    first, are placed two an SM as its blocks end, at 20 ns a key and not 14 (7B, 8 sequences, 4,000 / 30,000 -4.6 / -16; 8 kv heads, 8
+    sequences, 30,000 -12, 7, 8,000 / 30,000 -2.0 / +7.3; head_dim 64, 6 sequences of 8, 16,000 -7.0; with 9 of them 2,000 +1.0)."""
+    pairs = n_seqs * n_kv_heads
     cluster, splits = near_cluster(pairs, head_dim, room), decode_splits(pairs)
-    if head_dim == 64:
+    if cluster >= splits:
+        keys = 0
+    elif not even and not (n_seqs <= 8 and n_kv_heads >= 4):
+        if head_dim == 64:
+            keys = 1536 if 3 * cluster >= 2 * splits else 640
+        else:
+            keys = 960 if 2 * cluster >= splits else 512
+    elif head_dim == 64:
         keys = 0 if 5 * cluster >= 4 * splits else 4096 if 3 * cluster >= 2 * splits else NEAR_KEYS
     elif 2 * cluster >= splits or (cluster == 8 and splits <= 22):
         keys = 0
@@ -787,7 +807,7 @@ class Kernels:
         if 0 < seen <= short_context(head_dim):           # one block a pair reads them in less time than a cluster needs to meet
             return 1
         room = self.near_room(head_dim)
-        bound = near_context(pairs, head_dim, room)
+        bound = near_context(batch.n_rows, n_kv_heads, head_dim, room, getattr(batch, "even", True))
         return near_cluster(pairs, head_dim, room) if bound == 0 or 0 < seen <= bound else 0
 
     def near_room(self, head_dim: int):

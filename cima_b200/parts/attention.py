@@ -214,15 +214,16 @@ class Attention:
         from ..kernels import short_context
         return short_context(self.hd)
 
-    def near_context(self, n_seqs: int) -> int:
-        """The same for the decode kernel of middling contexts, whose reach follows from the number of sequences (0: no bound)."""
+    def near_context(self, n_seqs: int, even: bool = True) -> Optional[int]:
+        """Positions up to which the decode kernel of middling contexts takes a step of ``n_seqs`` sequences, of about one length (``even``)
+        or not; 0: any number, None: it takes none."""
         from ..kernels import near_context
         if (self.rt.full_precision or self.hd not in (64, 128) or self.spec.n_heads // self.spec.n_kv_heads > 8 or self.sink or self.keep_first
                 or self.has_sink or self.gated or self.slopes_host is not None):
-            return 0
+            return None
         room = getattr(self.rt.kernels, "near_room", None)               # (a stand-in on the CPU has none)
-        bound = near_context(n_seqs * self.spec.n_kv_heads, self.hd, room and room(self.hd))
-        return 0 if self.spec.window and self.spec.window + 64 <= bound else bound
+        reach = near_context(n_seqs, self.spec.n_kv_heads, self.hd, room and room(self.hd), even)
+        return 0 if self.spec.window and self.spec.window + 64 <= reach else reach
 
     # ------------------------------------------------------------------ cache
     def cache_requests(self, site: int) -> List[object]:

@@ -70,10 +70,6 @@ class SideBySide:
         named = [n for n in named if n > 0]
         return min(named) if named else 0
 
-    def near_context(self, n_seqs: int) -> int:
-        named = [b.near_context(n_seqs) for b in self.branches if hasattr(b, "near_context")]
-        return min([n for n in named if n > 0], default=0)
-
     def cache_requests(self, site: int) -> List[object]:
         reqs: List[object] = []
         for b in self.branches:

@@ -1,6 +1,7 @@
 """The decode attention whose blocks are clusters that merge their own results: every cluster size at the edges of its pieces (16 keys a
 warp, 128 a block, pages of 64), windows and rings against float64; and which step takes it."""
 import math
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -37,8 +38,23 @@ SLOWER = {(128, 2, 16000): 0.4, (128, 16, 6000): 1.9, (128, 36, 6000): 7.3, (128
 def test_the_reach_lies_where_it_was_measured():
     """No number of pairs at a length at which the splits were faster, and every one well below."""
     for (hd, pairs, n), us in {**FASTER, **SLOWER}.items():
-        reach = near_context(pairs, hd, ROOM[hd])
+        reach = near_context(pairs, 1, hd, ROOM[hd])
         assert (reach == 0 or n <= reach) == (us < 0), (hd, pairs, n, reach, near_cluster(pairs, hd, ROOM[hd]), decode_splits(pairs))
+
+
+# (head size, sequences, kv heads, positions of one, the others having 300): the same
+FASTER_UNEVEN = {(128, 16, 2, 2000): -1.5, (128, 3, 4, 8000): -4.2, (128, 6, 4, 30000): -15.7, (128, 8, 4, 30000): -15.8, (128, 32, 4, 700): -2.9, (128, 40, 4, 30000): -151.0,
+                 (128, 64, 4, 1000): -8.8, (64, 8, 2, 4000): -0.6, (64, 24, 2, 4000): -1.1, (64, 64, 2, 30000): -34.4, (64, 48, 2, 2000): -0.6,
+                 (128, 8, 8, 30000): -12.2, (128, 7, 8, 4000): -3.8, (128, 4, 8, 30000): -16.7, (64, 6, 8, 16000): -7.0, (64, 3, 8, 16000): -12.0}
+SLOWER_UNEVEN = {(128, 6, 2, 8000): 0.9, (128, 7, 2, 16000): 4.1, (128, 10, 2, 4000): 0.1, (128, 16, 2, 8000): 2.1, (128, 22, 2, 2000): 1.4, (128, 28, 2, 4000): 3.8,
+                 (128, 12, 4, 2000): 0.3, (128, 16, 4, 4000): 1.3, (128, 24, 4, 2000): 2.8, (128, 32, 4, 4000): 2.6, (128, 60, 2, 4000): 3.4, (64, 8, 2, 8000): 1.1,
+                 (64, 16, 2, 4000): 0.2, (64, 24, 2, 8000): 0.4, (64, 48, 2, 4000): 0.4, (128, 5, 8, 4000): 2.0, (128, 7, 8, 30000): 7.3, (128, 9, 8, 4000): 1.3, (64, 9, 8, 2000): 1.0}
+
+
+def test_the_reach_with_one_long_sequence_lies_where_it_was_measured():
+    for (hd, n_seqs, nkv, n), us in {**FASTER_UNEVEN, **SLOWER_UNEVEN}.items():
+        reach = near_context(n_seqs, nkv, hd, ROOM[hd], even=False)
+        assert (reach == 0 or n <= reach) == (us < 0), (hd, n_seqs, nkv, n, reach)
 
 
 def test_the_clusters_are_those_that_the_device_holds():
@@ -138,7 +154,6 @@ def test_long_sums_are_as_near_to_64_bits_as_the_splits(nh, nkv, hd, signs):
 def test_clusters_stay_within_what_the_device_holds(monkeypatch):
     """The device is asked once, and a step takes no cluster that it cannot place: with room for none of 16 (as where no group has 16 free
     SMs) the step runs in smaller ones."""
-    from types import SimpleNamespace
     K = Kernels(verbose=False)
     for hd in (64, 128):
         room = K.near_room(hd)
@@ -161,15 +176,40 @@ def test_steps_cross_the_reach_of_the_clusters(monkeypatch):
     from cima_b200.engine import StepEntry
     monkeypatch.setattr(kernels, "NEAR_KEYS", 32)                   # 512 positions for a cluster of 16
     kw = dict(config=dict(SHAPES["qwen2.5-0.5b"], num_hidden_layers=2, max_position_embeddings=4096), seed=3, draw="device", max_tokens=4096, max_seqs=2, verbose=False)
-    rec, ref = cima_b200.load(**kw), cima_b200.load(use_graphs=False, **kw)
+    rec, ref, splits = cima_b200.load(**kw), cima_b200.load(use_graphs=False, **kw), cima_b200.load(use_graphs=False, **kw)
+    splits.model.rt.kernels._near = lambda *a: 0                    # (another kernel altogether)
     prompt = torch.randint(0, rec.spec.vocab, (505,), generator=torch.Generator().manual_seed(1)).tolist()
     outs = []
-    for lm in (rec, ref):
+    for lm in (rec, ref, splits):
         (slot,) = lm.model.cache.open(1)
         lm.step([StepEntry(slot, prompt)])
         outs.append(torch.cat([lm.step([StepEntry(slot, [t], [0])]) for t in range(100, 116)]))
     assert {k[1] for k in rec.model._step_graphs} == {512, 0}
     assert (outs[0] - outs[1]).abs().max() <= 2e-2 * outs[1].std()
+    assert (outs[0] - outs[2]).abs().max() <= 2e-2 * outs[2].std()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,seqs,longest,want", [("qwen2.5-0.5b", 25, 6137, {0, -1}), ("qwen2.5-1.5b", 10, 3836, {0, -1}), ("qwen2.5-7b", 3, 500, {0})])
+def test_steps_of_sequences_far_from_one_length(shape, seqs, longest, want):
+    """One long sequence beside short ones: its steps are recorded apart from where the splits are the faster ones for it, and the logits
+    stay those of the split kernel, step by step (two layers; the clusters are of 4, 4 and 8 blocks)."""
+    import cima_b200
+    from cima_b200.config.shapes import SHAPES
+    from cima_b200.engine import StepEntry
+    from cima_b200.engine.graph import UNEVEN
+    kw = dict(config=dict(SHAPES[shape], num_hidden_layers=2, max_position_embeddings=8192), seed=3, draw="device", max_tokens=16384, max_seqs=seqs, verbose=False)
+    rec, ref = cima_b200.load(**kw), cima_b200.load(use_graphs=False, **kw)
+    ref.model.rt.kernels._near = lambda *a: 0
+    g, outs = torch.Generator().manual_seed(1), []
+    prompts = [torch.randint(0, rec.spec.vocab, (longest if i == 0 else 20 + i,), generator=g).tolist() for i in range(seqs)]
+    for lm in (rec, ref):
+        slots = lm.model.cache.open(seqs)
+        lm.step([StepEntry(s, p) for s, p in zip(slots, prompts)])
+        outs.append([lm.step([StepEntry(s, [t + i], [0]) for i, s in enumerate(slots)]) for t in range(100, 114)])
+    for n, (a, b) in enumerate(zip(*outs)):                       # each is up to 0.7 % off its 64-bit result
+        assert ((a - b).norm(dim=1) <= 1.5e-2 * b.norm(dim=1)).all(), n
+    assert UNEVEN == -1 and {k[1] for k in rec.model._step_graphs} == want
 
 
 @pytest.mark.gpu

@@ -225,11 +225,11 @@ def test_a_context_class_that_no_sequence_can_leave_is_not_told_apart():
     any length."""
     model = cpu_model("B", max_tokens=1024)
     short = model.short_context
-    model.blocks[0].mixer.near_context = lambda n: short + 64
+    model.blocks[0].mixer.near_context = lambda n, even=True: short + 64
     model.spec = dataclasses.replace(model.spec, max_position=4096)
     for tokens, want in ((short + 64, [0, 0]), (short + 128, [short + 64, 0])):
         model.make_cache(tokens)
-        assert [model.context_bound(2, n) for n in (short, short + 1, short + 65)] == [short] + want, tokens
+        assert [model.context_bound([n, n]) for n in (short, short + 1, short + 65)] == [short] + want, tokens
 
 
 def test_without_room_for_more_recordings_a_batch_size_keeps_the_one_for_its_longest_contexts(monkeypatch):
@@ -247,11 +247,40 @@ def test_without_room_for_more_recordings_a_batch_size_keeps_the_one_for_its_lon
     monkeypatch.setattr(graph, "StepGraph", Recording)
     monkeypatch.setattr(graph, "MAX_STEP_GRAPHS", 2)
     monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
-    model._context_bounds.update({n: [64, 128] for n in (1, 2, 3)})
-    first, other = model._step_graph(1, 10), model._step_graph(2, 10)
-    second = model._step_graph(1, 65)
-    assert list(model._step_graphs) == [(2, 64), (1, 128)] and model._step_graph(2, 12) is other
-    assert model._step_graph(1, 20) is second and model._step_graph(1, 128) is second
-    last = model._step_graph(1, 129)
-    assert model._step_graph(1, 20) is last and model._step_graph(1, 100) is last and model._step_graph(3, 5) is None
+    monkeypatch.setattr(model, "context_bound", lambda lengths: next((n for n in (64, 128) if max(lengths) <= n), 0))
+    step = lambda n, longest: model._step_graph([longest] * n)                                     # noqa: E731
+    first, other = step(1, 10), step(2, 10)
+    second = step(1, 65)
+    assert list(model._step_graphs) == [(2, 64), (1, 128)] and step(2, 12) is other
+    assert step(1, 20) is second and step(1, 128) is second
+    last = step(1, 129)
+    assert step(1, 20) is last and step(1, 100) is last and step(3, 5) is None
+    monkeypatch.setattr(model, "context_bound", lambda lengths: graph.UNEVEN)
+    assert step(1, 300) is last                                   # of any length, however chosen
     assert made == [(1, 64), (2, 64), (1, 128), (1, 0)] and first is not second
+
+
+def test_context_classes_of_sequences_far_from_one_length():
+    """A kernel that takes sequences of one length at any number of positions and others up to 500, one that takes them up to 700 and
+    300, and one that makes no difference: which class a step's lengths fall into."""
+    from cima_b200.engine.graph import UNEVEN
+    model = cpu_model("B", max_tokens=1024)
+    model.spec = dataclasses.replace(model.spec, max_position=1 << 16)
+    short = model.short_context
+    at = lambda *lengths: model.context_bound([short + n for n in lengths])                        # noqa: E731
+    for reach, want in (((0, short + 500), [short, 0, 0, 0, UNEVEN]), ((short + 700, short + 300), [short, short + 700, short + 700, 0, 0]),
+                        ((short + 5000, 0), [short, short + 5000, short + 5000, 0, short + 5000]), ((0, 0), [short, 0, 0, 0, 0]), ((None, None), [short, 0, 0, 0, 0])):
+        model.blocks[0].mixer.near_context = lambda n, even=True: reach[0] if even else reach[1]
+        model.make_cache(1 << 15)
+        got = [at(0, 0), at(300, -short + 1), at(690, 650), at(9000, 8900), at(4900, -short + 1)]
+        assert got == want, (reach, got)
+    model.blocks[0].mixer.near_context = lambda n, even=True: 0 if even else 9000
+    model.make_cache(2048)                                        # a reach that no sequence can pass
+    assert at(1000, -short + 1) == 0
+
+
+def test_a_batch_says_whether_its_sequences_are_of_one_length():
+    from cima_b200.engine.batch import build_batch
+    for starts, want in (([99, 84], True), ([99, 60], False), ([0], True), ([499, 499, 99], False), ([499] * 9 + [99], True)):
+        entries = [StepEntry(i, [1], [0]) for i in range(len(starts))]
+        assert build_batch(entries, starts, 8, "cpu").even == want, starts
