@@ -57,6 +57,24 @@ def test_the_reach_with_one_long_sequence_lies_where_it_was_measured():
         assert (reach == 0 or n <= reach) == (us < 0), (hd, n_seqs, nkv, n, reach)
 
 
+def test_which_step_takes_it():
+    """The dispatch itself: head sizes, groups, planes, alignment, unknown lengths, windows, short contexts, unevenness."""
+    def near(nh=14, nkv=2, hd=64, rows=1, max_len=1000, window=0, planes=2, width=None, ptr=0, even=True):
+        self = SimpleNamespace(near_room=ROOM.get)
+        qkv = SimpleNamespace(shape=(rows, (nh + 2 * nkv) * hd if width is None else width), data_ptr=lambda: ptr)
+        return Kernels._near(self, qkv, SimpleNamespace(planes=planes), SimpleNamespace(n_rows=rows, max_len=max_len, even=even), nh, nkv, hd, window)
+
+    assert near() == 16 and near(nh=28, nkv=4, hd=128) == 16
+    assert near(hd=96) == near(hd=256) == near(nh=18, nkv=2) == near(planes=1) == near(width=1004) == near(ptr=8) == 0
+    assert near(max_len=384) == 1 and near(max_len=385) == 16 and near(hd=128, max_len=192) == 1
+    assert near(max_len=832 * 16) == 16 and near(max_len=832 * 16 + 1) == 0 == near(max_len=0)
+    assert near(nh=28, nkv=4, hd=128, rows=64, max_len=0) == 1                                     # as many blocks as splits: at any length
+    assert near(nh=28, nkv=4, hd=128, rows=9, max_len=2000) == 0 and near(nh=28, nkv=4, hd=128, rows=9, max_len=1664) == 2
+    assert near(max_len=10 ** 6, window=300) == 1 and near(max_len=0, window=1000) == 16 and near(max_len=10 ** 6, window=20000) == 0
+    assert near(nh=28, nkv=4, hd=128, rows=32, max_len=4000) == 1 and near(nh=28, nkv=4, hd=128, rows=32, max_len=4000, even=False) == 0
+    assert near(nh=28, nkv=4, hd=128, rows=32, max_len=900, even=False) == 1 and near(nh=28, nkv=4, hd=128, rows=8, max_len=30000, even=False) == 4
+
+
 def test_the_clusters_are_those_that_the_device_holds():
     """A device whose groups of SMs hold fewer clusters, or none of a size: never more blocks to wait for one another than it can place."""
     for hd in (64, 128):
@@ -120,6 +138,26 @@ def test_an_infinite_value_stays_in_its_column(hd):
     want = torch.zeros(2, hd, dtype=torch.bfloat16)
     want[:, 3] = float("inf")
     assert torch.equal(out.cpu().view(2, hd), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nh,nkv,hd,B", [(28, 4, 128, 80), (14, 2, 64, 170)])
+def test_more_blocks_than_one_wave(nh, nkv, hd, B):
+    """Some hundred sequences of 1 to 700 positions, up to 5,440 blocks: every row against float64."""
+    K, G, gen, width = Kernels(verbose=False), nh // nkv, torch.Generator().manual_seed(hd), 11
+    lens = torch.randint(1, 700, (B,), generator=gen).int()
+    storage = torch.randn(B * width, 2, nkv, 64, hd, generator=gen).bfloat16().cuda()
+    table, slots = torch.randperm(B * width, generator=gen).view(B, width).int(), torch.randperm(B, generator=gen)
+    qkv = torch.randn(B, (nh + 2 * nkv) * hd, generator=gen).bfloat16().cuda()
+    held = storage[table[slots].long().cuda()].double().permute(0, 2, 3, 1, 4, 5).reshape(B, 2, nkv, width * 64, hd)
+    seen = (torch.arange(width * 64) < lens[:, None]).cuda()
+    s = (qkv[:, :nh * hd].double().view(B, nkv, G, hd) @ held[:, 0].transpose(2, 3) / math.sqrt(hd)).masked_fill(~seen[:, None, None], -math.inf)
+    want = (torch.softmax(s, -1) @ held[:, 1]).reshape(B, nh * hd)
+    kv = LayerKV(storage, table.cuda(), 64, 0, 0, 0)
+    for cluster in (1, 2, 4, 8, 16):
+        out = torch.full((B, nh * hd), 7.0, dtype=torch.bfloat16, device="cuda")
+        K.attention_decode_near(qkv, kv, slots.int().cuda(), lens.cuda(), out, nh, nkv, hd, 1.0 / math.sqrt(hd), 0, cluster)
+        assert ((out.double() - want).abs() <= TOL * want.abs().clamp(min=1.0)).all(), cluster
 
 
 @pytest.mark.gpu
